@@ -15,6 +15,7 @@
 #include <cstring>
 
 #include "bulk_copy.cuh"
+#include "fixed_site.cuh"
 #include "lbswim_device.cuh"
 #include "lbswim_internal.h"
 #include "spread_slab.cuh"
@@ -129,59 +130,127 @@ __device__ __forceinline__ void load_force(const T* F, long long N, long long s,
   }
 }
 
-// FP64 collide + push-stream, lb.cu:72-218.  blockDim = (32, 8); grid.z = x.
-__global__ void __launch_bounds__(256) k_step_push_f64(const double* __restrict__ f,
-                                                       const double* __restrict__ F,
-                                                       double* __restrict__ fn, int nx, int ny,
-                                                       int nz, long long N, Relax<double> k) {
-  const int z = blockIdx.x * 32 + threadIdx.x;
-  const int y = blockIdx.y * 8 + threadIdx.y;
-  const int x = blockIdx.z;
-  if (z >= nz || y >= ny) return;
-  const long long nynz = (long long)ny * nz;
-  const long long s = x * nynz + (long long)y * nz + z;
+// Unsigned division by a divisor fixed at launch: t / d for t < 2^31.
+struct FastDiv {
+  unsigned mul, shift;
+};
+static FastDiv fast_div(unsigned d) {
+  unsigned l = 0;
+  while ((1ull << l) < d) ++l;
+  return FastDiv{(unsigned)(((1ull << 32) * ((1ull << l) - d)) / d + 1), l};
+}
+__device__ __forceinline__ unsigned div_by(unsigned t, FastDiv k) {
+  return (__umulhi(t, k.mul) + t) >> k.shift;
+}
+
+// FP64 collide + push-stream, lb.cu:72-218.  A thread takes site blockIdx.x *
+// F64_THREADS + threadIdx.x of x plane blockIdx.y, so that a ragged nz idles
+// no lanes.  The collision runs on integers (fixed_site.cuh); the sites that do
+// not fit, and every site of a lattice whose relaxation constants do not, take
+// FP64 arithmetic.
+constexpr int F64_THREADS = 128;
+template <bool FORCED>
+__global__ void __launch_bounds__(F64_THREADS, 4) k_step_push_f64(const double* __restrict__ f,
+                                                               const double* __restrict__ F,
+                                                               double* __restrict__ fn, int nx,
+                                                               int ny, int nz, FastDiv by_nz,
+                                                               long long N, Relax<double> k,
+                                                               FixedRelax kf) {
+  const unsigned nynz = (unsigned)ny * (unsigned)nz;
+  const unsigned t = blockIdx.x * F64_THREADS + threadIdx.x;
+  if (t >= nynz) return;
+  const int x = blockIdx.y, y = (int)div_by(t, by_nz), z = (int)(t - (unsigned)y * nz);
+  const long long s = (long long)x * nynz + t;
   double d[15];
 #pragma unroll
   for (int p = 0; p < 15; ++p) d[p] = f[p * N + s];
-  double fx, fy, fz;
-  load_force(F, N, s, fx, fy, fz);
-  collide(d, fx, fy, fz, 0.0, k, d);
+  double Fa[3] = {0.0, 0.0, 0.0};
+  if (FORCED) {
+#pragma unroll
+    for (int a = 0; a < 3; ++a) Fa[a] = F[a * N + s];
+  }
+  unsigned long long X[15];
+  int e;
+  bool fits = site_to_fixed(d, X, e) && kf.usable;
+  long long Fi[3] = {0, 0, 0};
+  if (FORCED) {
+#pragma unroll
+    for (int a = 0; a < 3; ++a) fits = value_to_fixed(Fa[a], e, Fi[a]) && fits;
+  }
+  if (fits) fits = site_collide_fixed<FORCED>(X, Fi, kf);
+  if (fits) {
+#pragma unroll
+    for (int p = 0; p < 15; ++p) d[p] = fixed_to_double(X[p], e);
+  } else {
+    // read again, so that the distributions need no registers meanwhile
+#pragma unroll
+    for (int p = 0; p < 15; ++p) d[p] = f[p * N + s];
+    collide(d, Fa[0], Fa[1], Fa[2], 0.0, k, d);
+  }
   const int xm = wrap_once(x - 1, nx), xp = wrap_once(x + 1, nx);
-  const int ym = wrap_once(y - 1, ny), yp = wrap_once(y + 1, ny);
+  const int ym = wrap_once(y - 1, ny) * nz, yp = wrap_once(y + 1, ny) * nz, y0 = y * nz;
   const int zm = wrap_once(z - 1, nz), zp = wrap_once(z + 1, nz);
 #pragma unroll
   for (int p = 0; p < 15; ++p) {
     const int dx = cx_of(p), dy = cy_of(p), dz = cz_of(p);
-    const long long X = dx > 0 ? xp : (dx < 0 ? xm : x);
-    const long long Y = dy > 0 ? yp : (dy < 0 ? ym : y);
-    const long long Z = dz > 0 ? zp : (dz < 0 ? zm : z);
-    fn[p * N + X * nynz + Y * nz + Z] = d[p];
+    const int X1 = dx > 0 ? xp : (dx < 0 ? xm : x);
+    const int Y1 = dy > 0 ? yp : (dy < 0 ? ym : y0);
+    const int Z1 = dz > 0 ? zp : (dz < 0 ? zm : z);
+    (fn + p * N + (long long)X1 * nynz)[Y1 + Z1] = d[p];
   }
 }
 
-// rho, u from the stored distributions and the force, lb.cu:250-295.
-template <class S, class H>
-__global__ void k_calc_hydro(const S* __restrict__ f, const H* __restrict__ F, H* __restrict__ rho,
-                             H* __restrict__ u, long long N, H rho0, unsigned* status) {
-  using T = H;
+// rho, u from the stored distributions and the force of an FP64 lattice,
+// lb.cu:250-295.  The sums run on integers (fixed_site.cuh: density and
+// momentum are exact and rounded once), and so does the reciprocal; the six
+// operations left keep FP64's relative precision for any force.  Sites that do
+// not fit take FP64 arithmetic throughout.
+template <bool FORCED>
+__global__ void __launch_bounds__(256) k_calc_hydro(const double* __restrict__ f,
+                                                    const double* __restrict__ F,
+                                                    double* __restrict__ rho,
+                                                    double* __restrict__ u, long long N,
+                                                    unsigned* status) {
   for (long long s = blockIdx.x * (long long)blockDim.x + threadIdx.x; s < N;
        s += (long long)gridDim.x * blockDim.x) {
-    T d[15];
+    double d[15];
 #pragma unroll
-    for (int p = 0; p < 15; ++p) d[p] = dev_from_stored<S>((T)Store<S>::ld(f + fidx<S>(p, s, N)), p);
-    T R, jx, jy, jz;
-    hydro_moments(d, R, jx, jy, jz);
-    T fx, fy, fz;
-    load_force(F, N, s, fx, fy, fz);
-    const T r = rho0 + R;
-    // one division per site (GB300's FP64 pipe is narrow; within an ulp of
-    // the reference's three, lb.cu:286-293)
-    const T inv = T(1) / r;
+    for (int p = 0; p < 15; ++p) d[p] = f[p * N + s];
+    double Fa[3] = {0.0, 0.0, 0.0};
+    if (FORCED) {
+#pragma unroll
+      for (int a = 0; a < 3; ++a) Fa[a] = F[a * N + s];
+    }
+    double r, jx, jy, jz, inv;
+    unsigned long long X[15];
+    int e;
+    unsigned long long R;
+    long long ix, iy, iz;
+    const bool fits = site_to_fixed(d, X, e);
+    hydro_fixed(X, R, ix, iy, iz);
+    if (fits && (long long)R > 0) {
+      r = fixed_to_double(R, e);
+      jx = signed_fixed_to_double(ix, e);
+      jy = signed_fixed_to_double(iy, e);
+      jz = signed_fixed_to_double(iz, e);
+      int lz;
+      const unsigned long long y = (unsigned long long)fixed_reciprocal(R, lz);
+      // one division per site: within an ulp of the reference's three, lb.cu:286-293
+      inv = fixed_to_double(y, 2039 + lz - e);
+    } else {
+      hydro_moments(d, r, jx, jy, jz);
+      inv = 1.0 / r;
+      if (!finite_d(r + jx + jy + jz)) raise_status(status, LBSWIM_STATUS_NONFINITE);
+    }
     rho[s] = r;
-    u[s] = (jx + T(0.5) * fx) * inv;
-    u[N + s] = (jy + T(0.5) * fy) * inv;
-    u[2 * N + s] = (jz + T(0.5) * fz) * inv;
-    if (!finite_d((double)(r + jx + jy + jz))) raise_status(status, LBSWIM_STATUS_NONFINITE);
+    if (FORCED) {
+      jx = fma(0.5, Fa[0], jx);
+      jy = fma(0.5, Fa[1], jy);
+      jz = fma(0.5, Fa[2], jz);
+    }
+    u[s] = jx * inv;
+    u[N + s] = jy * inv;
+    u[2 * N + s] = jz * inv;
   }
 }
 
@@ -1183,10 +1252,14 @@ void lattice_step(Lattice* L) {
   if (L->precision == LBSWIM_F64 && (L->compat & LBSWIM_COMPAT_EXACT_F64)) {
     exact_step_f64(L);
   } else if (L->precision == LBSWIM_F64) {
-    dim3 grid((nz + 31) / 32, (ny + 7) / 8, nx);
-    k_step_push_f64<<<grid, dim3(32, 8), 0, L->stream>>>(
-        (const double*)L->f[L->cur], L->force_zero_pending ? nullptr : (const double*)L->force,
-        (double*)L->f[L->cur ^ 1], nx, ny, nz, L->n, make_relax<double>(L->tau_s, L->tau_b));
+    const dim3 grid((unsigned)(((long long)ny * nz + F64_THREADS - 1) / F64_THREADS), nx);
+    const Relax<double> k = make_relax<double>(L->tau_s, L->tau_b);
+    (L->force_zero_pending ? k_step_push_f64<false> : k_step_push_f64<true>)
+        <<<grid, F64_THREADS, 0, L->stream>>>((const double*)L->f[L->cur],
+                                              (const double*)L->force,
+                                              (double*)L->f[L->cur ^ 1], nx, ny, nz,
+                                              fast_div((unsigned)nz), L->n, k,
+                                              make_fixed_relax(k));
     LB_CHECK_LAUNCH(1);
   } else {
     switch (L->precision) {
@@ -1213,10 +1286,11 @@ void lattice_step(Lattice* L) {
 template <class S>
 static void calc_hydro_t(Lattice* L) {
   const long long N = L->n;
-  if (L->precision == LBSWIM_F64)
-    k_calc_hydro<double, double><<<grid_for(N, 256), 256, 0, L->stream>>>(
-        (const double*)L->f[L->cur], L->force_zero_pending ? nullptr : (const double*)L->force,
-        (double*)L->rho, (double*)L->u, N, 0.0, L->status);
+  if constexpr (sizeof(S) == 8)
+    (L->force_zero_pending ? k_calc_hydro<false> : k_calc_hydro<true>)
+        <<<grid_for(N, 256), 256, 0, L->stream>>>((const double*)L->f[L->cur],
+                                                  (const double*)L->force, (double*)L->rho,
+                                                  (double*)L->u, N, L->status);
   else
     k_calc_hydro_packed<S><<<grid_for(N, 256), 256, 0, L->stream>>>(
         (const S*)L->f[L->cur], L->force_zero_pending ? nullptr : (const float*)L->force,
