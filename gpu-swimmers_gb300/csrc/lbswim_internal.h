@@ -76,10 +76,13 @@ struct SpreadScratch {
   int pending = 0;
   bool stepped = false;  // a Step already consumed the pending ends
   unsigned* max_abs_force = nullptr;  // device: largest |F| component of the pending ends
-  TileLists ftiles;      // force tiles, for materialisation
-  // slab buckets of the pending ends, filled as the ends are recorded
+  TileLists ftiles;      // force tiles of a dense FP64 suspension
+  int max_slot = 0;      // FP64: which of the two max-force words is in use
+  // slab buckets of the pending ends, filled as the ends are recorded; an FP64
+  // lattice's force-tile buckets (its bucket_count ends with two words for the
+  // largest force)
   unsigned* bucket_count = nullptr;  // [bucket_slabs]
-  int* bucket_list = nullptr;        // [bucket_slabs][SLAB_BUCKET_CAP]
+  int* bucket_list = nullptr;        // [bucket_slabs][SLAB_BUCKET_CAP], FP64: [][FT_CAP]
   int bucket_slabs = 0;
   int bucket_tile = -1;  // slab shape the buckets hold (Lattice::fused_tile), -1: stale
   // The next step's end records and slab buckets, written by the swimmer move

@@ -4,12 +4,12 @@
 // the tail r - l n and +P n at the head r through the 4^3 Peskin stencil.  The
 // reference scatters with FP64 atomics in arbitrary order.  Here the result is
 // deterministic and uses no floating-point atomics: AddForces records the 2n
-// dipole ends (origin, Peskin weights, force); the ends are then listed under
-// every tile their stencil touches (integer counting sort), and each tile sums,
-// for every site, the covering ends in end order.  The tiles are either force
-// tiles (k_force_tile, which writes the dense force field) or, for FP32/BF16/
-// FP16 lattices, the slabs of the fused step kernel, which spreads the ends
-// itself so the force field never goes through HBM.
+// dipole ends (origin, Peskin weights, force) and lists them under every tile
+// their stencil touches; each tile then sums its ends, in integers or in end
+// order.  The tiles are either force tiles (k_force_fixed and k_force_tile,
+// which write the dense force field of an FP64 lattice) or, for FP32/BF16/FP16
+// lattices, the slabs of the fused step kernel, which spreads the ends itself so
+// the force field never goes through HBM.
 //
 // The original 4^3-origin-bin kernels below (k_spread_bin ... k_spread_gather)
 // serve lbswim_spread_forces_noalloc.
@@ -17,6 +17,7 @@
 #include <mutex>
 #include <string>
 
+#include "fixed_stencil.cuh"
 #include "lbswim_device.cuh"
 #include "lbswim_internal.h"
 
@@ -286,6 +287,12 @@ __device__ __forceinline__ void touched_range(int o, int n, int T, int h, int nt
   }
 }
 
+__device__ __forceinline__ int node_after(int o, int j, int n) {
+  int t = o + j;
+  while (t >= n) t -= n;
+  return t;
+}
+
 constexpr int REC_THREADS = 256;
 
 // Slab shape of a tile choice, as slab_shape_of (lattice.cu): x planes, rows, columns.
@@ -295,8 +302,9 @@ __device__ __forceinline__ void slab_shape_of_dev(int tile, int T[3]) {
   T[2] = tile == 1 ? 16 : 32;
 }
 
-// List end e under every slab of grid G whose extended region its stencil
-// touches (at most SLAB_BUCKET_CAP ends are kept per slab; the count goes on).
+// List end e under every tile of grid G whose extended region its stencil
+// touches (at most CAP ends are kept per tile; the count goes on).
+template <int CAP>
 __device__ __forceinline__ void bucket_end(int e, const int o[3], const Dims& D, const TileGrid& G,
                                            unsigned* __restrict__ count,
                                            int* __restrict__ list) {
@@ -310,7 +318,7 @@ __device__ __forceinline__ void bucket_end(int e, const int o[3], const Dims& D,
         const int kz = f[2] + k < G.nt[2] ? f[2] + k : f[2] + k - G.nt[2];
         const int t = (kx * G.nt[1] + ky) * G.nt[2] + kz;
         const unsigned slot = atomicAdd(count + t, 1u);
-        if (slot < (unsigned)SLAB_BUCKET_CAP) list[(long long)t * SLAB_BUCKET_CAP + slot] = e;
+        if (slot < (unsigned)CAP) list[(long long)t * CAP + slot] = e;
       }
     }
   }
@@ -319,17 +327,15 @@ __device__ __forceinline__ void bucket_end(int e, const int o[3], const Dims& D,
 // One record per dipole end: e = 2i is the tail, 2i + 1 the head.  Records are
 // assembled in shared memory and written out as one contiguous block; with
 // bucket_count set, each end is also listed under the step-kernel slabs it
-// touches (its index among all pending ends is e_base + e).  FP32 records take
-// the stencil origin from the bits of the position (stencil_axis) and the
-// four weights from one square root (peskin_weights4), like the FP32
-// interpolation.
-template <class T>
+// touches (its index among all pending ends is e_base + e).  The stencil origin
+// comes from the bits of the position (stencil_axis) and the four weights from
+// one square root (peskin_weights4), like the FP32 interpolation.
 __device__ __forceinline__ void end_records_block(
     int blk, int nsw, const double* __restrict__ r, const double* __restrict__ nv, double P,
-    double l, Dims D, EndRecord<T>* __restrict__ ends, int e_base,
+    double l, Dims D, EndRecord<float>* __restrict__ ends, int e_base,
     unsigned* __restrict__ max_abs_f, TileGrid G, unsigned* __restrict__ bucket_count,
     int* __restrict__ bucket_list) {
-  __shared__ EndRecord<T> srec[REC_THREADS];
+  __shared__ EndRecord<float> srec[REC_THREADS];
   __shared__ unsigned smax;
   if (threadIdx.x == 0) smax = 0u;
   __syncthreads();
@@ -347,29 +353,25 @@ __device__ __forceinline__ void end_records_block(
       F[a] = -P * na;
       if (head) F[a] *= -1.0;
     }
-    EndRecord<T>& rec = srec[threadIdx.x];
-    if constexpr (sizeof(T) == 4) {
-      for (int a = 0; a < 3; ++a) {
-        int x0;
-        float dr;
-        stencil_axis(rr[a], x0, dr);
-        rec.o[a] = wrap_any(x0, D.n[a]);
-        float w[4];
-        peskin_weights4(dr, w);
+    EndRecord<float>& rec = srec[threadIdx.x];
+    for (int a = 0; a < 3; ++a) {
+      int x0;
+      float dr;
+      stencil_axis(rr[a], x0, dr);
+      rec.o[a] = wrap_any(x0, D.n[a]);
+      float w[4];
+      peskin_weights4(dr, w);
 #pragma unroll
-        for (int j = 0; j < 4; ++j) rec.phi[a][j] = w[j];
-      }
-    } else {
-      stencil_setup<T>(D, rr, rec.o, rec.phi);
+      for (int j = 0; j < 4; ++j) rec.phi[a][j] = w[j];
     }
     rec.pad = 0;
     float m = 0.f;
     for (int a = 0; a < 3; ++a) {
-      rec.F[a] = (T)F[a];
+      rec.F[a] = (float)F[a];
       m = fmaxf(m, fabsf((float)F[a]));
     }
     mbits = __float_as_uint(m);
-    if (bucket_count) bucket_end(e_base + e, rec.o, D, G, bucket_count, bucket_list);
+    if (bucket_count) bucket_end<SLAB_BUCKET_CAP>(e_base + e, rec.o, D, G, bucket_count, bucket_list);
   }
   // non-negative floats order like their bit patterns: a warp's largest, then
   // one shared-memory atomic per warp
@@ -378,18 +380,17 @@ __device__ __forceinline__ void end_records_block(
   __syncthreads();
   if (threadIdx.x == 0 && max_abs_f) atomicMax(max_abs_f, smax);
   const int nrec = min(REC_THREADS, nends - e0);
-  const int words = nrec * (int)(sizeof(EndRecord<T>) / 4);
+  const int words = nrec * (int)(sizeof(EndRecord<float>) / 4);
   const unsigned* src = reinterpret_cast<const unsigned*>(srec);
   unsigned* dst = reinterpret_cast<unsigned*>(ends + e0);
   for (int w = threadIdx.x; w < words; w += REC_THREADS) dst[w] = src[w];
 }
 
-template <class T>
 __global__ void __launch_bounds__(REC_THREADS) k_end_records(
     int nsw, const double* __restrict__ r, const double* __restrict__ nv, double P, double l,
-    Dims D, EndRecord<T>* __restrict__ ends, int e_base, unsigned* __restrict__ max_abs_f,
+    Dims D, EndRecord<float>* __restrict__ ends, int e_base, unsigned* __restrict__ max_abs_f,
     TileGrid G, unsigned* __restrict__ bucket_count, int* __restrict__ bucket_list) {
-  end_records_block<T>(blockIdx.x, nsw, r, nv, P, l, D, ends, e_base, max_abs_f, G, bucket_count,
+  end_records_block(blockIdx.x, nsw, r, nv, P, l, D, ends, e_base, max_abs_f, G, bucket_count,
                        bucket_list);
 }
 
@@ -399,11 +400,11 @@ __global__ void k_bucket_ends(int nends, const EndRecord<float>* __restrict__ en
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= nends) return;
   const int o[3] = {ends[e].o[0], ends[e].o[1], ends[e].o[2]};
-  bucket_end(e, o, D, G, count, list);
+  bucket_end<SLAB_BUCKET_CAP>(e, o, D, G, count, list);
 }
 
-template <class T, int PASS>
-__global__ void k_touch(int nends, const EndRecord<T>* __restrict__ ends, Dims D, TileGrid G,
+template <int PASS>
+__global__ void k_touch(int nends, const EndRecord<double>* __restrict__ ends, Dims D, TileGrid G,
                         unsigned* __restrict__ count, const unsigned* __restrict__ start,
                         int* __restrict__ list) {
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
@@ -453,58 +454,115 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan_apply_total(
   }
 }
 
-// Force tile (FP64 lattices): 8 (x) x 8 (y) x 32 (z) sites, 16 warps, each
-// warp owns 4 of the 64 z-rows; a warp ballot picks the ends covering a row.
-// The ends are put in end order by rank and every site adds their
-// contributions in that order, ((phi_x phi_y) phi_z) F as the reference does
-// (SwimmerArray.cu:64-73).  FP32 lattices spread in the step kernel and in
-// k_force_slab instead.
-constexpr int FT_X = 8, FT_Y = 8, FT_Z = 32, FT_THREADS = 512, FT_CAP = 256;
+// ---- force spreading of FP64 lattices -------------------------------------------
+// Force tiles of 4 (x) x 8 (y) x 32 (z) sites.  The end records list every end
+// under the tiles its stencil touches, in buckets of FT_CAP (a tile with more
+// takes all pending ends).  Two kernels sum them:
+//  * k_force_fixed (default): the (end, node) contributions are 64-bit integers
+//    in units of 2^-60 of the largest force, added as three words of 22, 22 and
+//    20 bits with shared-memory atomics that return nothing, and converted
+//    once.  All 32 lanes work on the nodes of an end.  Integer sums do not
+//    depend on their order.  256^3, 65,536 swimmers: 0.24 ms, against 0.71 ms
+//    in FP64 by site; 65x47x90: 12 us against 29.
+//  * k_force_tile (LBSWIM_COMPAT_EXACT_F64, and suspensions too dense for
+//    buckets): every site adds the ends that cover it in end order,
+//    ((phi_x phi_y) phi_z) F as the reference does (SwimmerArray.cu:64-73).  A
+//    row's 32 lanes have half an end each on average and run as long as the one
+//    with most, on the narrow FP64 pipe.
+constexpr int FT_X = 4, FT_Y = 8, FT_Z = 32, FT_THREADS = 256, FT_CAP = 256;
 static_assert((FT_X & (FT_X - 1)) == 0 && (FT_Y & (FT_Y - 1)) == 0 && (FT_Z & (FT_Z - 1)) == 0,
               "tile edges are powers of two (touched_range shifts)");
 
-__global__ void __launch_bounds__(FT_THREADS) k_force_tile(Dims D, TileGrid G,
-                                                           const EndRecord<double>* __restrict__ ends,
-                                                           const unsigned* __restrict__ start,
-                                                           const int* __restrict__ list,
-                                                           int* __restrict__ sorted,
-                                                           double* __restrict__ force,
-                                                           int accumulate) {
-  using T = double;
-  __shared__ EndRecord<T> srec[FT_CAP];
-  __shared__ int skey[FT_CAP];
-  const int tile = blockIdx.x;
-  const int kz = tile % G.nt[2], ky = (tile / G.nt[2]) % G.nt[1], kx = tile / (G.nt[1] * G.nt[2]);
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const unsigned s0 = start[tile], s1 = start[tile + 1];
-  const int cnt = (int)(s1 - s0);
-  const bool in_smem = cnt <= FT_CAP;
-  if (in_smem) {
-    for (int q = tid; q < cnt; q += FT_THREADS) skey[q] = list[s0 + q];
-    __syncthreads();
-    for (int q = tid; q < cnt; q += FT_THREADS) srec[rank_of(skey[q], skey, cnt)] = ends[skey[q]];
-  } else {
-    // more ends than fit: order them in global scratch and read records from there
-    for (int q = tid; q < cnt; q += FT_THREADS) {
-      const int k = list[s0 + q];
-      int r = 0;
-      for (int j = 0; j < cnt; ++j) r += list[s0 + j] < k;
-      sorted[s0 + r] = k;
+// One thread per (end, axis), 64 ends per block: the axes' chains of FP64
+// operations run side by side.  e = 2i is the tail, 2i + 1 the head.  FIXED:
+// the weights are integers in units of 2^-63 (fixed_weights4) in place of
+// doubles, and *max_f takes the largest high word of |F|; otherwise they are
+// the reference's delta per node.
+constexpr int REC64_ENDS = 64, REC64_THREADS = 3 * REC64_ENDS;
+template <bool FIXED>
+__global__ void __launch_bounds__(REC64_THREADS) k_end_records_f64(
+    int nsw, const double* __restrict__ r, const double* __restrict__ nv, double P, double l,
+    Dims D, EndRecord<double>* __restrict__ ends, unsigned* __restrict__ max_f, TileGrid G,
+    unsigned* __restrict__ bucket_count, int* __restrict__ bucket_list) {
+  __shared__ EndRecord<double> srec[REC64_ENDS];
+  __shared__ unsigned smax, lost[REC64_ENDS];
+  const int q = threadIdx.x % REC64_ENDS, a = threadIdx.x / REC64_ENDS;
+  const int nends = 2 * nsw, e0 = blockIdx.x * REC64_ENDS, e = e0 + q;
+  if (threadIdx.x == 0) smax = 0u;
+  if (a == 0) lost[q] = 0u;
+  __syncthreads();
+  unsigned big = 0u;
+  if (e < nends) {
+    const int i = e >> 1;
+    const bool head = e & 1;
+    const double na = nv[(long long)nsw * a + i], ra = r[(long long)nsw * a + i];
+    const double x = head ? ra : __dsub_rn(ra, __dmul_rn(na, l));
+    double F = -P * na;
+    if (head) F *= -1.0;
+    const double x0 = ceil(x - 2.);
+    EndRecord<double>& rec = srec[q];
+    rec.o[a] = wrap_any((int)x0, D.n[a]);
+    if (FIXED) {
+      long long w[4];
+      const double dr = x - x0;
+      if (dr >= 1.0 && dr <= 2.0) {
+        fixed_weights4(dr, w);
+      } else {  // a coordinate beyond 2^52, or not a number
+        for (int j = 0; j < 4; ++j) w[j] = (long long)(peskin_delta<double>(x - (x0 + j)) * 0x1p63);
+        if (!(dr >= -4.0 && dr <= 4.0)) lost[q] = 1u;
+      }
+#pragma unroll
+      for (int j = 0; j < 4; ++j) rec.phi[a][j] = bits_double((unsigned long long)w[j]);
+      big = hi_word(double_bits(F)) & 0x7fffffffu;
+    } else {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) rec.phi[a][j] = peskin_delta<double>(x - (x0 + j));
     }
+    rec.F[a] = F;
+    if (a == 0) rec.pad = 0;
+  }
+  if (FIXED) {
+    big = __reduce_max_sync(0xffffffffu, big);
+    if ((threadIdx.x & 31) == 0 && big) atomicMax(&smax, big);
   }
   __syncthreads();
-  auto rec = [&](int q) -> const EndRecord<T>& { return in_smem ? srec[q] : ends[sorted[s0 + q]]; };
+  if (a == 0 && e < nends) {
+    if (FIXED && lost[q]) {  // the force of a lost end is not a number
+      for (int c = 0; c < 3; ++c) srec[q].F[c] = bits_double(0x7ff8000000000000ull);
+      atomicMax(max_f, 0x7ff80000u);
+    }
+    if (bucket_count) bucket_end<FT_CAP>(e, srec[q].o, D, G, bucket_count, bucket_list);
+  }
+  if (FIXED && threadIdx.x == 0) atomicMax(max_f, smax);
+  __syncthreads();
+  const int words = min(REC64_ENDS, nends - e0) * (int)(sizeof(EndRecord<double>) / 8);
+  const unsigned long long* src = reinterpret_cast<const unsigned long long*>(srec);
+  unsigned long long* dst = reinterpret_cast<unsigned long long*>(ends + e0);
+  for (int w = threadIdx.x; w < words; w += REC64_THREADS) dst[w] = src[w];
+}
+static_assert(sizeof(EndRecord<double>) % 8 == 0, "records are copied as 64-bit words");
+
+// The ends rec(0), ..., rec(cnt - 1) added to every site of a tile in that order.
+// A warp walks z rows: a ballot picks the ends covering a row, each lane then
+// collects those that cover its own site and adds them.
+template <bool FIXED, class Rec>
+__device__ __forceinline__ void force_gather(const Dims& D, int kx, int ky, int kz, int cnt,
+                                             Rec rec, double* __restrict__ force, int accumulate) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  auto phi = [](const EndRecord<double>& e, int a, int i) {
+    return FIXED ? (double)(long long)double_bits(e.phi[a][i]) * 0x1p-63 : e.phi[a][i];
+  };
   const int z = kz * FT_Z + lane;
   const bool zval = z < D.n[2];
   // no axis shorter than a stencil: one node of an end lands on a site
   const bool single = D.n[0] >= 4 && D.n[1] >= 4 && D.n[2] >= 4;
   for (int row = warp; row < FT_X * FT_Y; row += FT_THREADS / 32) {
-    const int x = kx * FT_X + (row >> 3), y = ky * FT_Y + (row & 7);
+    const int x = kx * FT_X + row / FT_Y, y = ky * FT_Y + row % FT_Y;
     if (x >= D.n[0] || y >= D.n[1]) continue;
     const long long s = (long long)x * D.n[1] * D.n[2] + (long long)y * D.n[2] + z;
     // the sums start from the base force and add the ends in end order, as
     // the oracle's serial spreading does
-    T acc0 = T(0), acc1 = T(0), acc2 = T(0);
+    double acc0 = 0.0, acc1 = 0.0, acc2 = 0.0;
     if (accumulate && zval) {
       acc0 = force[s];
       acc1 = force[D.N + s];
@@ -515,12 +573,9 @@ __global__ void __launch_bounds__(FT_THREADS) k_force_tile(Dims D, TileGrid G,
       const int q = base + lane;
       bool covers = false;
       if (q < cnt) {
-        const EndRecord<T>& e = rec(q);
+        const EndRecord<double>& e = rec(q);
         covers = covers_axis(x, e.o[0], D.n[0]) && covers_axis(y, e.o[1], D.n[1]);
       }
-      // this lane's ends among those covering the row (they also cover its z),
-      // in end order; each lane then adds its own, so that the FP64 work of
-      // the row's ends runs on all the lanes they cover at once
       const unsigned m = __ballot_sync(0xffffffffu, covers);  // every lane takes part
       unsigned mine = 0u;
       if (zval)
@@ -530,15 +585,16 @@ __global__ void __launch_bounds__(FT_THREADS) k_force_tile(Dims D, TileGrid G,
         }
       hit |= mine != 0u;
       for (; mine; mine &= mine - 1) {
-        const EndRecord<T>& e = rec(base + __ffs(mine) - 1);
+        const EndRecord<double>& e = rec(base + __ffs(mine) - 1);
         if (single) {
           int i = x - e.o[0], j = y - e.o[1], k = z - e.o[2];
           i += i < 0 ? D.n[0] : 0;
           j += j < 0 ? D.n[1] : 0;
           k += k < 0 ? D.n[2] : 0;
-          acc0 = __dadd_rn(acc0, end_contrib(e.phi[0][i], e.phi[1][j], e.phi[2][k], e.F[0]));
-          acc1 = __dadd_rn(acc1, end_contrib(e.phi[0][i], e.phi[1][j], e.phi[2][k], e.F[1]));
-          acc2 = __dadd_rn(acc2, end_contrib(e.phi[0][i], e.phi[1][j], e.phi[2][k], e.F[2]));
+          const double px = phi(e, 0, i), py = phi(e, 1, j), pz = phi(e, 2, k);
+          acc0 = __dadd_rn(acc0, end_contrib(px, py, pz, e.F[0]));
+          acc1 = __dadd_rn(acc1, end_contrib(px, py, pz, e.F[1]));
+          acc2 = __dadd_rn(acc2, end_contrib(px, py, pz, e.F[2]));
           continue;
         }
         // node by node in (i, j, k) order, as AccumulateDeltaForce adds them
@@ -549,9 +605,10 @@ __global__ void __launch_bounds__(FT_THREADS) k_force_tile(Dims D, TileGrid G,
             if (wrap_any(e.o[1] + j, D.n[1]) != y) continue;
             for (int k = 0; k < 4; ++k) {
               if (wrap_any(e.o[2] + k, D.n[2]) != z) continue;
-              acc0 = __dadd_rn(acc0, end_contrib(e.phi[0][i], e.phi[1][j], e.phi[2][k], e.F[0]));
-              acc1 = __dadd_rn(acc1, end_contrib(e.phi[0][i], e.phi[1][j], e.phi[2][k], e.F[1]));
-              acc2 = __dadd_rn(acc2, end_contrib(e.phi[0][i], e.phi[1][j], e.phi[2][k], e.F[2]));
+              const double px = phi(e, 0, i), py = phi(e, 1, j), pz = phi(e, 2, k);
+              acc0 = __dadd_rn(acc0, end_contrib(px, py, pz, e.F[0]));
+              acc1 = __dadd_rn(acc1, end_contrib(px, py, pz, e.F[1]));
+              acc2 = __dadd_rn(acc2, end_contrib(px, py, pz, e.F[2]));
             }
           }
         }
@@ -561,6 +618,169 @@ __global__ void __launch_bounds__(FT_THREADS) k_force_tile(Dims D, TileGrid G,
       force[s] = acc0;
       force[D.N + s] = acc1;
       force[2 * D.N + s] = acc2;
+    }
+  }
+}
+
+// The ends of a tile in end order, by rank, then force_gather.  start: counting-
+// sorted lists [start[tile], start[tile + 1]) (with `sorted` as scratch for the
+// long ones); null: buckets, whose count is zeroed for the next call.
+__global__ void __launch_bounds__(FT_THREADS) k_force_tile(
+    Dims D, TileGrid G, const EndRecord<double>* __restrict__ ends, int nends,
+    const unsigned* __restrict__ start, unsigned* __restrict__ count,
+    const int* __restrict__ list, int* __restrict__ sorted, double* __restrict__ force,
+    int accumulate) {
+  __shared__ EndRecord<double> srec[FT_CAP];
+  __shared__ int skey[FT_CAP];
+  const int tile = blockIdx.x;
+  const int kz = tile % G.nt[2], ky = (tile / G.nt[2]) % G.nt[1], kx = tile / (G.nt[1] * G.nt[2]);
+  const int tid = threadIdx.x;
+  const long long s0 = start ? (long long)start[tile] : (long long)tile * FT_CAP;
+  int cnt = (int)(start ? start[tile + 1] - start[tile] : count[tile]);
+  const bool in_smem = cnt <= FT_CAP;
+  if (in_smem) {
+    for (int q = tid; q < cnt; q += FT_THREADS) skey[q] = list[s0 + q];
+    __syncthreads();
+    for (int q = tid; q < cnt; q += FT_THREADS) srec[rank_of(skey[q], skey, cnt)] = ends[skey[q]];
+  } else if (start) {
+    // more ends than fit: order them in global scratch and read records from there
+    for (int q = tid; q < cnt; q += FT_THREADS) {
+      const int k = list[s0 + q];
+      int r = 0;
+      for (int j = 0; j < cnt; ++j) r += list[s0 + j] < k;
+      sorted[s0 + r] = k;
+    }
+  }
+  __syncthreads();
+  if (!start) {
+    if (tid == 0) count[tile] = 0u;  // every thread has read it
+    if (!in_smem) cnt = nends;
+  }
+  auto rec = [&](int q) -> const EndRecord<double>& {
+    return in_smem ? srec[q] : ends[start ? sorted[s0 + q] : q];
+  };
+  force_gather<false>(D, kx, ky, kz, cnt, rec, force, accumulate);
+}
+
+// Words of the fixed-point sums of a tile, [3 components][3 words][sites]: rows
+// are padded by 4 and planes by 16 words, so that the 32 nodes that a warp adds
+// at once (2 planes x 4 rows x 4 columns) fall into 32 banks.
+constexpr int FF_ROW = FT_Z + 4, FF_PLANE = FT_Y * FF_ROW + 16, FF_SITES = FT_X * FF_PLANE;
+constexpr int FF_CHUNK = 32;  // ends staged at a time
+static_assert(FF_ROW % 32 == 4 && FF_PLANE % 32 == 16 && FF_SITES % 4 == 0, "bank layout");
+
+// Default FP64 spreading (see above).  max_f: the largest high word of |F|;
+// next_max_f is zeroed for the next call.  A contribution is below 2^57 of the
+// units (2^60 where stencil nodes fold); with more than 32 ends, or folds, in
+// a tile the units grow so that a site's sum stays within 62 bits.  Tiles whose
+// words could overflow (more than 1024 contributions a site), and forces that
+// are not finite or below 2^-894, take FP64 arithmetic in end order.
+__global__ void __launch_bounds__(FT_THREADS) k_force_fixed(
+    Dims D, TileGrid G, const EndRecord<double>* __restrict__ ends, int nends,
+    unsigned* __restrict__ count, const int* __restrict__ list,
+    const unsigned* __restrict__ max_f, unsigned* __restrict__ next_max_f,
+    double* __restrict__ force, int accumulate) {
+  __shared__ __align__(16) unsigned sums[9 * FF_SITES];
+  __shared__ Digits dig[15][FF_CHUNK];  // 12 weights, 3 force components per end
+  __shared__ int org[3][FF_CHUNK];
+  const int tile = blockIdx.x, tid = threadIdx.x;
+  const int kz = tile % G.nt[2], ky = (tile / G.nt[2]) % G.nt[1], kx = tile / (G.nt[1] * G.nt[2]);
+  const unsigned listed = count[tile];
+  const unsigned fmax = *max_f;
+  const int kf = (int)(fmax >> 20);  // |F| < 2^(kf - 1022)
+  const int cnt = fmax ? (int)listed : 0;  // no force at all: nothing to add
+  // contributions an end can make to one site: stencil nodes that fold onto it
+  int fold = 1;
+  for (int a = 0; a < 3; ++a) fold *= D.n[a] >= 4 ? 1 : (D.n[a] == 1 ? 4 : 2);
+  __syncthreads();
+  if (tid == 0) {
+    count[tile] = 0u;  // every thread has read it
+    if (tile == 0) *next_max_f = 0u;
+  }
+  const int z0 = kz * FT_Z, y0 = ky * FT_Y, x0 = kx * FT_X;
+  if (cnt == 0) {
+    if (!accumulate)
+      for (int t = tid; t < FT_X * FT_Y * FT_Z; t += FT_THREADS) {
+        const int z = z0 + t % FT_Z, y = y0 + (t / FT_Z) % FT_Y, x = x0 + t / (FT_Z * FT_Y);
+        if (x >= D.n[0] || y >= D.n[1] || z >= D.n[2]) continue;
+        const long long s = ((long long)x * D.n[1] + y) * D.n[2] + z;
+        force[s] = force[D.N + s] = force[2 * D.N + s] = 0.0;
+      }
+    return;
+  }
+  if (listed > (unsigned)FT_CAP || cnt * fold > 1024 || kf < FIXED_MIN_K || kf > FIXED_MAX_K) {
+    auto rec = [&](int q) -> const EndRecord<double>& { return ends[q]; };
+    force_gather<true>(D, kx, ky, kz, nends, rec, force, accumulate);
+    return;
+  }
+  for (int i = tid; i < 9 * FF_SITES / 4; i += FT_THREADS)
+    reinterpret_cast<uint4*>(sums)[i] = make_uint4(0u, 0u, 0u, 0u);
+  // coarser units by the doublings of the largest sum over 32 unfolded ends
+  const int most = cnt * (fold > 1 ? 8 : 1);
+  const int coarse = most > 32 ? 32 - __clz((most - 1) >> 5) : 0;
+  const int lane = tid & 31, warp = tid >> 5;
+  const int jy = (lane >> 2) & 3, jz = lane & 3;
+  const long long s0 = (long long)tile * FT_CAP;
+  for (int base = 0; base < cnt; base += FF_CHUNK) {
+    const int m = min(FF_CHUNK, cnt - base);
+    __syncthreads();
+    for (int t = tid; t < 18 * FF_CHUNK; t += FT_THREADS) {
+      const int q = t % FF_CHUNK, w = t / FF_CHUNK;
+      if (q >= m) continue;
+      const EndRecord<double>& e = ends[list[s0 + base + q]];
+      if (w < 12) {
+        dig[w][q] = digits((long long)double_bits(e.phi[w >> 2][w & 3]));
+      } else if (w < 15) {
+        // F in units of 2^(kf - 1022 - 62), to nearest
+        const unsigned long long b = double_bits(e.F[w - 12]);
+        const int drop = kf - (int)((hi_word(b) >> 20) & 0x7ffu);
+        const unsigned long long mant = ((b << 11) | 0x8000000000000000ull);
+        const unsigned long long v = drop > 61 ? 0ull : ((mant >> (drop + 1)) + 1) >> 1;
+        const long long sg = (long long)b >> 63;
+        dig[w][q] = digits(((long long)v ^ sg) - sg);
+      } else {
+        org[w - 15][q] = e.o[w - 15];
+      }
+    }
+    __syncthreads();
+    for (int q = warp; q < m; q += FT_THREADS / 32) {
+      const int ly = node_after(org[1][q], jy, D.n[1]) - y0;
+      const int lz = node_after(org[2][q], jz, D.n[2]) - z0;
+      const bool in_yz = (unsigned)ly < (unsigned)FT_Y && (unsigned)lz < (unsigned)FT_Z;
+      if (!in_yz) continue;
+      const Digits wyz = digits(2 * mul_hi(dig[4 + jy][q], dig[8 + jz][q]));
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int ix = (lane >> 4) + 2 * h;
+        const int lx = node_after(org[0][q], ix, D.n[0]) - x0;
+        if ((unsigned)lx >= (unsigned)FT_X) continue;
+        const Digits w = digits(mul_hi(dig[ix][q], wyz));
+        unsigned* at = sums + lx * FF_PLANE + ly * FF_ROW + lz;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          const long long v = mul_hi(w, dig[12 + c][q]) >> coarse;
+          atomicAdd(at + (3 * c) * FF_SITES, (unsigned)v & 0x3fffffu);
+          atomicAdd(at + (3 * c + 1) * FF_SITES, (unsigned)(v >> 22) & 0x3fffffu);
+          atomicAdd(reinterpret_cast<int*>(at + (3 * c + 2) * FF_SITES), (int)(v >> 44));
+        }
+      }
+    }
+  }
+  __syncthreads();
+  for (int t = tid; t < FT_X * FT_Y * FT_Z; t += FT_THREADS) {
+    const int lz = t % FT_Z, ly = (t / FT_Z) % FT_Y, lx = t / (FT_Z * FT_Y);
+    const int z = z0 + lz, y = y0 + ly, x = x0 + lx;
+    if (x >= D.n[0] || y >= D.n[1] || z >= D.n[2]) continue;
+    const unsigned* at = sums + lx * FF_PLANE + ly * FF_ROW + lz;
+    const long long s = ((long long)x * D.n[1] + y) * D.n[2] + z;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      const long long v = (long long)at[(3 * c) * FF_SITES] +
+                          ((long long)at[(3 * c + 1) * FF_SITES] << 22) +
+                          (long long)((unsigned long long)at[(3 * c + 2) * FF_SITES] << 44);
+      if (accumulate && v == 0) continue;
+      const double f = signed_fixed_to_double(v, kf + coarse);
+      force[c * D.N + s] = accumulate ? force[c * D.N + s] + f : f;
     }
   }
 }
@@ -954,12 +1174,6 @@ __device__ __forceinline__ void point_stencil(const Dims& D, const double r[3],
   }
 }
 
-__device__ __forceinline__ int node_after(int o, int j, int n) {
-  int t = o + j;
-  while (t >= n) t -= n;
-  return t;
-}
-
 // Sum over the L lanes of a point's group (fixed shuffle tree).
 template <int L>
 __device__ __forceinline__ void reduce_lanes(float& vx, float& vy, float& vz) {
@@ -1228,7 +1442,7 @@ __global__ void __launch_bounds__(REC_THREADS) k_ens_records(EnsTable t) {
     slab_shape_of_dev(M.tile, G.T);
     G.h = 1;
     for (int a = 0; a < 3; ++a) G.nt[a] = M.nt[a];
-    end_records_block<float>(vb - t.rec_prefix[m], M.nsw, M.sw_r, M.sw_n, M.common.P,
+    end_records_block(vb - t.rec_prefix[m], M.nsw, M.sw_r, M.sw_n, M.common.P,
                              M.common.l, ens_dims(M), (EndRecord<float>*)M.ends, 0, M.max_abs_f,
                              G, M.bucket_count, M.bucket_list);
     __syncthreads();
@@ -1389,57 +1603,95 @@ static void ensure_lists(Lattice* L, TileLists& TL, const TileGrid& G, int nends
   }
 }
 
-// Lists of the pending ends per tile of G (entries unordered within a tile).
-template <class T>
-static void bin_ends(Lattice* L, TileLists& TL, const TileGrid& G) {
-  const int nends = L->spread.pending;
+// Lists of nends recorded ends per tile of G (entries unordered within a tile).
+static void bin_ends(Lattice* L, TileLists& TL, const TileGrid& G, int nends) {
   ensure_lists(L, TL, G, nends);
   const Dims D = make_dims(L);
-  const EndRecord<T>* ends = (const EndRecord<T>*)L->spread.ends;
-  if (nends > 0) {
-    k_touch<T, 0><<<(nends + 255) / 256, 256, 0, L->stream>>>(nends, ends, D, G, TL.count,
-                                                              nullptr, nullptr);
-    LB_CHECK_LAUNCH(1);
-  }
+  const EndRecord<double>* ends = (const EndRecord<double>*)L->spread.ends;
+  k_touch<0><<<(nends + 255) / 256, 256, 0, L->stream>>>(nends, ends, D, G, TL.count, nullptr,
+                                                         nullptr);
   const int nscan = (TL.ntiles + SCAN_TILE - 1) / SCAN_TILE;
   k_scan_tiles<<<nscan, SCAN_THREADS, 0, L->stream>>>(TL.count, TL.ntiles, TL.scan_tmp);
   k_scan_top<<<1, 1024, 0, L->stream>>>(TL.scan_tmp, nscan);
   k_scan_apply_total<<<nscan, SCAN_THREADS, 0, L->stream>>>(TL.count, TL.ntiles, TL.scan_tmp,
                                                             TL.start);
-  LB_CHECK_LAUNCH(3);
-  if (nends > 0) {
-    k_touch<T, 1><<<(nends + 255) / 256, 256, 0, L->stream>>>(nends, ends, D, G, TL.count,
-                                                              TL.start, TL.list);
-    LB_CHECK_LAUNCH(1);
-  }
+  k_touch<1><<<(nends + 255) / 256, 256, 0, L->stream>>>(nends, ends, D, G, TL.count, TL.start,
+                                                         TL.list);
+  LB_CHECK_LAUNCH(5);
 }
 
-// Fold the pending ends of an FP64 lattice into the dense force buffer
-// (force = base + spread).
-static void materialise_f64(Lattice* L) {
+// Buckets of FT_CAP ends per force tile, counts zero between calls, and the two
+// alternating words for the largest force.
+static void ensure_tile_buckets(Lattice* L, int ntiles) {
   SpreadScratch& S = L->spread;
-  const TileGrid G = force_tiles(L);
-  bin_ends<double>(L, S.ftiles, G);
+  if (S.bucket_count) return;  // the tiles of an FP64 lattice never change
+  unsigned* count = nullptr;
+  LB_CUDA(cudaMalloc(&count, sizeof(unsigned) * (ntiles + 2)));
+  const cudaError_t e = cudaMalloc(&S.bucket_list, sizeof(int) * (size_t)ntiles * FT_CAP);
+  if (e != cudaSuccess) {
+    cudaFree(count);
+    S.bucket_list = nullptr;
+    LB_CUDA(e);
+  }
+  S.bucket_count = count;
+  S.bucket_slabs = ntiles;
+  LB_CUDA(cudaMemsetAsync(count, 0, sizeof(unsigned) * (ntiles + 2), L->stream));
+}
+
+// force = base + the spread of W's dipole ends on an FP64 lattice.  Buckets
+// while the average tile lists at most half of one (each end touches 2.6 tiles
+// of 1024 sites on average): two launches in place of eight, which at 16^3 took
+// 36 us of device time together and take 13 us.  Denser suspensions list their
+// ends by a counting sort (k_force_tile orders long lists in global scratch).
+static void add_forces_f64(Swimmers* W, Lattice* L) {
+  SpreadScratch& S = L->spread;
+  const int nends = 2 * W->n;
+  if (nends == 0) {
+    if (L->force_zero_pending) lattice_zero_force_now(L);
+    return;
+  }
+  const bool exact = L->compat & LBSWIM_COMPAT_EXACT_F64;
   const Dims D = make_dims(L);
-  k_force_tile<<<S.ftiles.ntiles, FT_THREADS, 0, L->stream>>>(
-      D, G, (const EndRecord<double>*)S.ends, S.ftiles.start, S.ftiles.list, S.ftiles.sorted,
-      (double*)L->force, L->force_zero_pending ? 0 : 1);
-  LB_CHECK_LAUNCH(1);
-  S.pending = 0;
-  S.stepped = false;
+  const TileGrid G = force_tiles(L);
+  const long long ntiles = (long long)G.nt[0] * G.nt[1] * G.nt[2];
+  const bool buckets = nends <= 48 * ntiles;
+  ensure_ends(L, nends);
+  if (buckets) ensure_tile_buckets(L, (int)ntiles);
+  EndRecord<double>* ends = (EndRecord<double>*)S.ends;
+  unsigned* max_f = buckets ? S.bucket_count + ntiles : nullptr;
+  const int grid = (nends + REC64_ENDS - 1) / REC64_ENDS;
+  const int accumulate = L->force_zero_pending ? 0 : 1;
+  double* force = (double*)L->force;
+  if (buckets && !exact) {
+    unsigned* now = max_f + S.max_slot;
+    S.max_slot ^= 1;
+    k_end_records_f64<true><<<grid, REC64_THREADS, 0, L->stream>>>(
+        W->n, W->r, W->nv, W->common.P, W->common.l, D, ends, now, G, S.bucket_count,
+        S.bucket_list);
+    k_force_fixed<<<(int)ntiles, FT_THREADS, 0, L->stream>>>(
+        D, G, ends, nends, S.bucket_count, S.bucket_list, now, max_f + S.max_slot, force,
+        accumulate);
+    LB_CHECK_LAUNCH(2);
+  } else {
+    k_end_records_f64<false><<<grid, REC64_THREADS, 0, L->stream>>>(
+        W->n, W->r, W->nv, W->common.P, W->common.l, D, ends, nullptr, G,
+        buckets ? S.bucket_count : nullptr, S.bucket_list);
+    LB_CHECK_LAUNCH(1);
+    if (!buckets) bin_ends(L, S.ftiles, G, nends);
+    k_force_tile<<<(int)ntiles, FT_THREADS, 0, L->stream>>>(
+        D, G, ends, nends, buckets ? nullptr : S.ftiles.start, S.bucket_count,
+        buckets ? S.bucket_list : S.ftiles.list, S.ftiles.sorted, force, accumulate);
+    LB_CHECK_LAUNCH(1);
+  }
   L->force_zero_pending = false;
 }
 
 void spread_materialise(Lattice* L) {
   if (L->spread.pending > 0) {
-    if (L->precision == LBSWIM_F64) {
-      materialise_f64(L);
-    } else {
-      lattice_force_from_slabs(L);
-      L->spread.pending = 0;
-      L->spread.stepped = false;
-      L->force_zero_pending = false;
-    }
+    lattice_force_from_slabs(L);
+    L->spread.pending = 0;
+    L->spread.stepped = false;
+    L->force_zero_pending = false;
   } else if (L->force_zero_pending) {
     lattice_zero_force_now(L);
   }
@@ -1501,30 +1753,26 @@ SlabSpread spread_prepare_slabs(Lattice* L) {
   return out;
 }
 
-template <class T>
-static void append_ends_t(Swimmers* W, Lattice* L) {
+// Records W's ends after the pending ones of a reduced-precision lattice, listed
+// under the step kernel's slabs.
+static void append_ends(Swimmers* W, Lattice* L) {
   SpreadScratch& S = L->spread;
   const int nends = 2 * W->n;
   ensure_ends(L, S.pending + nends);
   if (!S.max_abs_force) LB_CUDA(cudaMalloc(&S.max_abs_force, sizeof(unsigned)));
-  // reduced-precision lattices list the ends under the step kernel's slabs now
-  constexpr bool BUCKETS = sizeof(T) == 4;
-  bool fill = false;
-  if (BUCKETS) {
-    const bool kept = ensure_buckets(L);
-    if (S.pending == 0) {
-      LB_CUDA(cudaMemsetAsync(S.bucket_count, 0, sizeof(unsigned) * S.bucket_slabs, L->stream));
-      S.bucket_tile = L->fused_tile;
-    } else if (!kept) {
-      S.bucket_tile = -1;
-    }
-    fill = S.bucket_tile == L->fused_tile;
+  const bool kept = ensure_buckets(L);
+  if (S.pending == 0) {
+    LB_CUDA(cudaMemsetAsync(S.bucket_count, 0, sizeof(unsigned) * S.bucket_slabs, L->stream));
+    S.bucket_tile = L->fused_tile;
+  } else if (!kept) {
+    S.bucket_tile = -1;
   }
+  const bool fill = S.bucket_tile == L->fused_tile;
   if (S.pending == 0) LB_CUDA(cudaMemsetAsync(S.max_abs_force, 0, sizeof(unsigned), L->stream));
   if (nends > 0) {
-    k_end_records<T><<<(nends + REC_THREADS - 1) / REC_THREADS, REC_THREADS, 0, L->stream>>>(
+    k_end_records<<<(nends + REC_THREADS - 1) / REC_THREADS, REC_THREADS, 0, L->stream>>>(
         W->n, W->r, W->nv, W->common.P, W->common.l, make_dims(L),
-        (EndRecord<T>*)S.ends + S.pending, S.pending, S.max_abs_force, slab_grid(L),
+        (EndRecord<float>*)S.ends + S.pending, S.pending, S.max_abs_force, slab_grid(L),
         fill ? S.bucket_count : nullptr, fill ? S.bucket_list : nullptr);
     LB_CHECK_LAUNCH(1);
   }
@@ -1550,12 +1798,10 @@ void swimmers_wait(Swimmers* W) {
 void swimmers_add_forces(Swimmers* W, Lattice* L) {
   // ends already spread by a Step belong to the base from now on
   if (L->spread.stepped) spread_materialise(L);
-  if (L->precision == LBSWIM_F64) {
-    append_ends_t<double>(W, L);
-    spread_materialise(L);
-  } else {
-    append_ends_t<float>(W, L);
-  }
+  if (L->precision == LBSWIM_F64)
+    add_forces_f64(W, L);
+  else
+    append_ends(W, L);
   swimmers_mark(W, L->stream);
   L->force_version++;
 }
@@ -1629,7 +1875,7 @@ void swimmers_move_preparing(Swimmers* W, Lattice* L, unsigned long long epoch) 
   }
   LB_CUDA(cudaMemsetAsync(P.bucket_count, 0, sizeof(unsigned) * nslabs, L->stream));
   LB_CUDA(cudaMemsetAsync(P.max_abs_force, 0, sizeof(unsigned), L->stream));
-  k_end_records<float><<<(nends + REC_THREADS - 1) / REC_THREADS, REC_THREADS, 0, L->stream>>>(
+  k_end_records<<<(nends + REC_THREADS - 1) / REC_THREADS, REC_THREADS, 0, L->stream>>>(
       W->n, W->r, W->nv, W->common.P, W->common.l, make_dims(L), (EndRecord<float>*)P.ends, 0,
       P.max_abs_force, G, P.bucket_count, P.bucket_list);
   LB_CHECK_LAUNCH(1);
