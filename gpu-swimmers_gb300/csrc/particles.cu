@@ -786,25 +786,24 @@ __global__ void __launch_bounds__(FT_THREADS) k_force_fixed(
 }
 
 // ---- Move kernels -----------------------------------------------------------
-// Stencil nodes and Peskin weights of position r (interp.cu:23-30).  FP64
-// lattices in exact mode keep the reference's arithmetic (a delta per node);
-// the default FP64 moves (FAST) take the four weights of an axis from one
-// square root; the FP32 path takes one FP64 difference per axis and forms the
-// four arguments in FP32 (GB300's FP64 pipe is narrow).
-template <class T, bool FAST = false>
+// Stencil nodes and Peskin weights of position r (interp.cu:23-30).  FP64: the
+// reference's arithmetic (a delta per node), for exact mode and for points
+// given by the caller; FP32: one FP64 difference per axis and one square root
+// for its four weights (GB300's FP64 pipe is narrow).
+template <class T>
 __device__ __forceinline__ void interp_setup(const Dims& D, const double r[3], int idx[3][4],
                                              T phi[3][4]) {
   for (int d = 0; d < 3; ++d) {
     const double x0 = ceil(r[d] - 2.);
     const int o = wrap_any((int)x0, D.n[d]);
     T w[4];
-    if constexpr (sizeof(T) == 4 || FAST) peskin_weights4((T)(r[d] - x0), w);
+    if constexpr (sizeof(T) == 4) peskin_weights4((T)(r[d] - x0), w);
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       int t = o + i;
       while (t >= D.n[d]) t -= D.n[d];
       idx[d][i] = t;
-      if constexpr (sizeof(T) == 8 && !FAST)
+      if constexpr (sizeof(T) == 8)
         phi[d][i] = peskin_delta<T>(r[d] - (x0 + i));
       else
         phi[d][i] = w[i];
@@ -812,140 +811,327 @@ __device__ __forceinline__ void interp_setup(const Dims& D, const double r[3], i
   }
 }
 
-// New periodic coordinate: the reference's fmod(r + size, size) on the FP64
-// path (SwimmerArray.cu:167, TracerArray.cu:40), a compare-and-shift on the
-// FP32 path (valid while a step moves a particle less than one box length).
-template <class T>
-__device__ __forceinline__ double wrap_position(double r, int n) {
-  if constexpr (sizeof(T) == 8) {
-    return fmod(r + n, (double)n);
-  } else {
-    return r >= n ? r - n : (r < 0.0 ? r + n : r);
-  }
+// New periodic coordinate of the FP32 path: a compare-and-shift (valid while a
+// step moves a particle less than one box length).
+__device__ __forceinline__ double wrap_shift(double r, int n) {
+  return r >= n ? r - n : (r < 0.0 ? r + n : r);
+}
+// New periodic coordinate of the FP64 paths, the reference's fmod(x + size, size)
+// (SwimmerArray.cu:167, TracerArray.cu:40).  x + n in [0, 2n), as after any
+// ordinary move, takes no division: x + n - n is exact in [n, 2n).  A result
+// outside [0, n) raises LBSWIM_STATUS_PARTICLE_OUTSIDE.
+__device__ __forceinline__ double wrap_position(double x, int n, unsigned* status) {
+  const double size = (double)n, t = __dadd_rn(x, size);
+  if (t >= 0.0 && t < 2.0 * size) return t >= size ? __dsub_rn(t, size) : t;
+  const double out = fmod(t, size);
+  if (!in_box(out, n)) raise_status(status, LBSWIM_STATUS_PARTICLE_OUTSIDE);
+  return out;
 }
 
 // InterpVelocity, interp.cu:8-47: u at r through the 4^3 Peskin stencil, from
-// the FP64 SoA field (FAST: fused multiply-adds and one square root per axis,
-// the default FP64 moves) ...
-template <class T, bool FAST = false>
+// the FP64 SoA field, every operation rounded in the reference's order ...
 __device__ __forceinline__ void interp_velocity(const double* __restrict__ u, const Dims& D,
-                                                const double r[3], T v[3]) {
+                                                const double r[3], double v[3]) {
   int idx[3][4];
-  T phi[3][4];
-  interp_setup<T, FAST>(D, r, idx, phi);
-  v[0] = v[1] = v[2] = T(0);
+  double phi[3][4];
+  interp_setup<double>(D, r, idx, phi);
+  v[0] = v[1] = v[2] = 0.0;
   const long long nynz = (long long)D.n[1] * D.n[2];
   for (int i = 0; i < 4; ++i)
     for (int j = 0; j < 4; ++j) {
-      const T pij = phi[0][i] * phi[1][j];
+      const double pij = phi[0][i] * phi[1][j];
       const long long row = idx[0][i] * nynz + (long long)idx[1][j] * D.n[2];
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
-        const T d3 = pij * phi[2][k];
+        const double d3 = pij * phi[2][k];
         const long long s = row + idx[2][k];
-        if constexpr (FAST) {
-          v[0] = fma(d3, (T)u[s], v[0]);
-          v[1] = fma(d3, (T)u[D.N + s], v[1]);
-          v[2] = fma(d3, (T)u[2 * D.N + s], v[2]);
-        } else {
-          v[0] = add_prod(v[0], d3, (T)u[s]);
-          v[1] = add_prod(v[1], d3, (T)u[D.N + s]);
-          v[2] = add_prod(v[2], d3, (T)u[2 * D.N + s]);
-        }
+        v[0] = add_prod(v[0], d3, u[s]);
+        v[1] = add_prod(v[1], d3, u[D.N + s]);
+        v[2] = add_prod(v[2], d3, u[2 * D.N + s]);
       }
     }
 }
 
 // ... or from the packed float4 field of a reduced-precision lattice (one 16-byte
 // load per node).
-template <class T>
 __device__ __forceinline__ void interp_velocity(const float4* __restrict__ h, const Dims& D,
-                                                const double r[3], T v[3]) {
+                                                const double r[3], float v[3]) {
   int idx[3][4];
-  T phi[3][4];
-  interp_setup<T>(D, r, idx, phi);
-  v[0] = v[1] = v[2] = T(0);
+  float phi[3][4];
+  interp_setup<float>(D, r, idx, phi);
+  v[0] = v[1] = v[2] = 0.f;
   const long long nynz = (long long)D.n[1] * D.n[2];
   for (int i = 0; i < 4; ++i)
     for (int j = 0; j < 4; ++j) {
-      const T pij = phi[0][i] * phi[1][j];
+      const float pij = phi[0][i] * phi[1][j];
       const long long row = idx[0][i] * nynz + (long long)idx[1][j] * D.n[2];
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
-        const T d3 = pij * phi[2][k];
+        const float d3 = pij * phi[2][k];
         const float4 q = __ldg(h + row + idx[2][k]);
-        v[0] += d3 * (T)q.x;
-        v[1] += d3 * (T)q.y;
-        v[2] += d3 * (T)q.z;
+        v[0] += d3 * q.x;
+        v[1] += d3 * q.y;
+        v[2] += d3 * q.z;
       }
     }
 }
 
-// DoSwimmerArrayMove, SwimmerArray.cu:123-210 (FAST: the default FP64
-// interpolation of interp_velocity).
-template <class U, class T, bool FAST = false>
-__global__ void k_swimmers_move(int nsw, double* __restrict__ swr, double* __restrict__ swv,
-                                double* __restrict__ swn, lbswim_common_params c,
-                                unsigned long long seed, unsigned long long step, Dims D,
-                                const U* __restrict__ u, unsigned* status) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= nsw) return;
-  double r[3], n0[3];
-  for (int d = 0; d < 3; ++d) {
-    r[d] = swr[nsw * d + i];
-    n0[d] = swn[nsw * d + i];
+// FP64 moves in exact mode (LBSWIM_COMPAT_EXACT_F64): the reference's operations
+// in its order.  DoSwimmerArrayMove, SwimmerArray.cu:123-210: two threads per
+// swimmer, one for its own point and one for its rear point, so that the two
+// ordered chains of 450 FP64 operations run side by side.  Small blocks spread
+// a small array over the SMs (a warp's FP64 instruction takes 64 clocks of its
+// scheduler, whatever its active lanes): 1024 swimmers 130 -> 56 us.
+constexpr int EXACT_MOVE_BLOCK = 64;
+__global__ void __launch_bounds__(EXACT_MOVE_BLOCK) k_swimmers_move_exact(
+    int nsw, double* __restrict__ swr, double* __restrict__ swv, double* __restrict__ swn,
+    lbswim_common_params c, unsigned long long seed, unsigned long long step, Dims D,
+    const double* __restrict__ u, unsigned* status) {
+  const int t = blockIdx.x * EXACT_MOVE_BLOCK + threadIdx.x;
+  const int i = t >> 1;
+  const bool rear = t & 1, valid = i < nsw;
+  double r[3] = {0.0, 0.0, 0.0}, n0[3] = {0.0, 0.0, 0.0}, v[3] = {0.0, 0.0, 0.0};
+  bool tumble = false;
+  if (valid) {
+    double p[3];
+    for (int d = 0; d < 3; ++d) {
+      r[d] = swr[(long long)nsw * d + i];
+      n0[d] = swn[(long long)nsw * d + i];
+      p[d] = rear ? __dsub_rn(r[d], __dmul_rn(n0[d], c.l)) : r[d];
+    }
+    tumble = rng_uniform(seed, (uint32_t)i, step) < c.alpha;
+    if (!rear || (!tumble && !c.rotational_advection_off)) interp_velocity(u, D, p, v);
   }
-  T v[3];
-  interp_velocity<T, FAST>(u, D, r, v);
-  double rMinus[3];
+  double vm[3];
+  for (int d = 0; d < 3; ++d) vm[d] = __shfl_xor_sync(0xffffffffu, v[d], 1);
+  if (rear || !valid) return;
   for (int d = 0; d < 3; ++d) {
     double rDot = __dmul_rn(__dmul_rn(c.mobility, c.P), n0[d]);
-    if (!c.translational_advection_off) rDot = __dadd_rn(rDot, (double)v[d]);
-    rMinus[d] = __dsub_rn(r[d], __dmul_rn(n0[d], c.l));
-    swv[nsw * d + i] = rDot;
-    const double rn = wrap_position<T>(r[d] + rDot, D.n[d]);
-    swr[nsw * d + i] = rn;
-    if (!in_box(rn, D.n[d])) raise_status(status, LBSWIM_STATUS_PARTICLE_OUTSIDE);
+    if (!c.translational_advection_off) rDot = __dadd_rn(rDot, v[d]);
+    swv[(long long)nsw * d + i] = rDot;
+    swr[(long long)nsw * d + i] = wrap_position(__dadd_rn(r[d], rDot), D.n[d], status);
   }
-  const float rnd = rng_uniform(seed, (uint32_t)i, step);
   double nn[3];
-  if (rnd < c.alpha) {  // tumble: a direction uniform on the sphere
+  if (tumble) {  // a direction uniform on the sphere
     rng_normal3(seed, (uint32_t)i, step, nn);
   } else if (!c.rotational_advection_off) {  // rotate with the local shear
-    T vm[3];
-    interp_velocity<T, FAST>(u, D, rMinus, vm);
-    for (int d = 0; d < 3; ++d) nn[d] = n0[d] + ((double)v[d] - (double)vm[d]) / c.l;
+    for (int d = 0; d < 3; ++d) nn[d] = __dadd_rn(n0[d], (v[d] - vm[d]) / c.l);
   } else {
     return;  // orientation unchanged
   }
   const double norm = __dsqrt_rn(
       __dadd_rn(__dadd_rn(__dmul_rn(nn[0], nn[0]), __dmul_rn(nn[1], nn[1])), __dmul_rn(nn[2], nn[2])));
-  for (int d = 0; d < 3; ++d) swn[nsw * d + i] = nn[d] / norm;
+  for (int d = 0; d < 3; ++d) swn[(long long)nsw * d + i] = nn[d] / norm;
 }
 
-// DoTracerArrayMove, TracerArray.cu:12-43 (s accumulated per tracer; FAST: the
-// default FP64 interpolation of interp_velocity).
-template <class U, class T, bool FAST = false>
-__global__ void k_tracers_move(int ntr, double* __restrict__ r, double* __restrict__ s,
-                               double* __restrict__ v, Dims D, const U* __restrict__ u,
-                               unsigned* status) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+// DoTracerArrayMove, TracerArray.cu:12-43 (s accumulated per tracer).
+__global__ void __launch_bounds__(EXACT_MOVE_BLOCK) k_tracers_move_exact(
+    int ntr, double* __restrict__ r, double* __restrict__ s, double* __restrict__ v, Dims D,
+    const double* __restrict__ u, unsigned* status) {
+  const int i = blockIdx.x * EXACT_MOVE_BLOCK + threadIdx.x;
   if (i >= ntr) return;
-  double rr[3], ss[3];
+  double rr[3], ss[3], vv[3];
   for (int d = 0; d < 3; ++d) {
-    rr[d] = r[ntr * d + i];
-    ss[d] = s[ntr * d + i];
+    rr[d] = r[(long long)ntr * d + i];
+    ss[d] = s[(long long)ntr * d + i];
   }
-  T vv[3];
-  interp_velocity<T, FAST>(u, D, rr, vv);
+  interp_velocity(u, D, rr, vv);
   for (int d = 0; d < 3; ++d) {
-    const double vd = (double)vv[d];
-    v[ntr * d + i] = vd;
-    const double rn = wrap_position<T>(rr[d] + vd, D.n[d]);
-    r[ntr * d + i] = rn;
-    s[ntr * d + i] = ss[d] + vd;
-    if (!in_box(rn, D.n[d])) raise_status(status, LBSWIM_STATUS_PARTICLE_OUTSIDE);
+    v[(long long)ntr * d + i] = vv[d];
+    r[(long long)ntr * d + i] = wrap_position(__dadd_rn(rr[d], vv[d]), D.n[d], status);
+    s[(long long)ntr * d + i] = __dadd_rn(ss[d], vv[d]);
   }
+}
+
+// ---- FP64 moves (default) ------------------------------------------------------
+// A block interpolates 64 points, four lanes each (one per z node), from integer
+// weights (fixed_weights4), in three phases: a thread per (point, axis) forms the
+// weights, a lane sums its 16 nodes a component, a thread per (particle, axis)
+// updates it.  A lane's 16 velocities become integers below 2^60 under the
+// largest exponent of the point's 64, and are summed over y, x and z with three
+// 32-bit multiply-adds a product: within 2^-57 of the largest velocity in all,
+// where FP64 sums are within 2^-53 of their terms.  The 400 FP64 operations a
+// point took before ran on two lanes per clock and SM.  1,048,576 tracers at
+// 256^3: 748 -> 430 us (2400 instructions per warp, the integer pipe 64% busy);
+// 65,536 swimmers 204 -> 104 us, one swimmer 50 -> 11 us.
+constexpr int MOVE64_BLOCK = 256, MOVE64_POINTS = 64;
+
+struct Stencil64 {
+  Digits w[3][4][MOVE64_POINTS];
+  int o[3][MOVE64_POINTS];
+  double vel[3][MOVE64_POINTS];
+};
+
+// Weights and wrapped origin of coordinate x of point p on axis a.
+__device__ __forceinline__ void point_axis64(const Dims& D, double x, int a, int p, Stencil64& st) {
+  const double x0 = ceil(x - 2.);
+  st.o[a][p] = wrap_any((int)x0, D.n[a]);
+  const double dr = x - x0;
+  long long w[4];
+  if (dr >= 1.0 && dr <= 2.0) {
+    fixed_weights4(dr, w);
+  } else {  // a coordinate beyond 2^52 (or not a number, whose position stays one)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) w[j] = (long long)(peskin_delta<double>(x - (x0 + j)) * 0x1p63);
+  }
+#pragma unroll
+  for (int j = 0; j < 4; ++j) st.w[a][j][p] = digits(w[j]);
+}
+
+// b as digits of an integer below 2^60 in units of 2^(ke - 1082), toward zero,
+// for a double of biased exponent at most ke.
+__device__ __forceinline__ Digits velocity_digits(unsigned long long b, int ke) {
+  const int drop = ke - (int)((hi_word(b) >> 20) & 0x7ffu);
+  const unsigned long long m =
+      ((b & 0xfffffffffffffull) | 0x10000000000000ull) << 10;  // bit 62
+  const long long v = (long long)(m >> min(drop + 3, 63));
+  const long long sg = (long long)b >> 63;
+  return digits((v ^ sg) - sg);
+}
+// acc, t += a b by digits (t holds the cross products, in units of 2^32)
+__device__ __forceinline__ void mul_add(Digits a, Digits b, long long& acc, long long& t) {
+  t += (long long)a.h * b.l;
+  t += (long long)a.l * b.h;
+  acc += (long long)a.h * b.h;
+}
+__device__ __forceinline__ long long sum_of(long long acc, long long t) {
+  return acc + ((t + 0x80000000ll) >> 32);
+}
+
+// Velocity of the block's 64 points; I: the type of the site offsets.
+template <class I>
+__device__ __forceinline__ void gather64(const double* __restrict__ u, const Dims& D,
+                                         Stencil64& st) {
+  const int p = threadIdx.x >> 2, k = threadIdx.x & 3;
+  const I nynz = (I)D.n[1] * D.n[2];
+  I xo[4];
+  int yo[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    xo[i] = (I)node_after(st.o[0][p], i, D.n[0]) * nynz;
+    yo[i] = node_after(st.o[1][p], i, D.n[1]) * D.n[2];
+  }
+  const int z = node_after(st.o[2][p], k, D.n[2]);
+#pragma unroll 1
+  for (int c = 0; c < 3; ++c) {
+    const double* __restrict__ uc = u + c * D.N + z;
+    unsigned long long b[16];
+    unsigned top = 0u;
+#pragma unroll
+    for (int q = 0; q < 16; ++q) {
+      b[q] = double_bits(__ldg(uc + xo[q >> 2] + yo[q & 3]));
+      top = max(top, hi_word(b[q]) & 0x7fffffffu);
+    }
+    top = max(top, __shfl_xor_sync(0xffffffffu, top, 1));
+    top = max(top, __shfl_xor_sync(0xffffffffu, top, 2));
+    const int ke = (int)(top >> 20);
+    long long xa = 0, xt = 0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      long long ya = 0, yt = 0;
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        mul_add(st.w[1][j][p], velocity_digits(b[4 * i + j], ke), ya, yt);
+      mul_add(st.w[0][i][p], digits(sum_of(ya, yt)), xa, xt);
+    }
+    long long v = mul_hi(digits(sum_of(xa, xt)), st.w[2][k][p]);
+    v += __shfl_xor_sync(0xffffffffu, v, 1);
+    v += __shfl_xor_sync(0xffffffffu, v, 2);
+    const bool fits = ke >= FIXED_MIN_K && ke <= FIXED_MAX_K;
+    if (k == 0 && fits) st.vel[c][p] = signed_fixed_to_double(v, ke + 3);
+    // velocities of 0 (a fluid at rest), beyond the integers' range or not
+    // finite: in FP64
+    if (__any_sync(0xffffffffu, !fits && top != 0u)) {
+      double s = 0.0;
+#pragma unroll 1
+      for (int q = 0; q < 16; ++q) {
+        const Digits wx = st.w[0][q >> 2][p], wy = st.w[1][q & 3][p], wz = st.w[2][k][p];
+        const double w = (((double)wx.h * 0x1p32 + wx.l) * ((double)wy.h * 0x1p32 + wy.l)) *
+                         ((double)wz.h * 0x1p32 + wz.l) * 0x1p-189;
+        const I site = (I)node_after(st.o[0][p], q >> 2, D.n[0]) * nynz +
+                       node_after(st.o[1][p], q & 3, D.n[1]) * D.n[2];
+        s = fma(w, uc[site], s);
+      }
+      s += __shfl_xor_sync(0xffffffffu, s, 1);
+      s += __shfl_xor_sync(0xffffffffu, s, 2);
+      if (k == 0 && !fits) st.vel[c][p] = s;
+    } else if (k == 0 && !fits) {
+      st.vel[c][p] = 0.0;
+    }
+  }
+}
+
+template <class I>
+__global__ void __launch_bounds__(MOVE64_BLOCK, 3) k_tracers_move_f64(
+    int ntr, double* __restrict__ r, double* __restrict__ s, double* __restrict__ v, Dims D,
+    const double* __restrict__ u, unsigned* status) {
+  __shared__ Stencil64 st;
+  const int p = threadIdx.x % MOVE64_POINTS, a = threadIdx.x / MOVE64_POINTS;
+  const int i = blockIdx.x * MOVE64_POINTS + p;
+  const long long at = (long long)ntr * a + i;
+  const bool mine = a < 3, valid = mine && i < ntr;
+  double x = 0.0, sa = 0.0;
+  if (valid) {
+    x = r[at];
+    sa = s[at];
+  }
+  if (mine) point_axis64(D, x, a, p, st);
+  __syncthreads();
+  gather64<I>(u, D, st);
+  __syncthreads();
+  if (!valid) return;
+  const double w = st.vel[a][p];
+  v[at] = w;
+  r[at] = wrap_position(x + w, D.n[a], status);
+  s[at] = sa + w;
+}
+
+// Points [0, 32) of a block are the swimmers, [32, 64) their rear points r - l n;
+// the threads (p < 32, axis) update them.
+constexpr int MOVE64_SWIMMERS = MOVE64_POINTS / 2;
+template <class I>
+__global__ void __launch_bounds__(MOVE64_BLOCK, 3) k_swimmers_move_f64(
+    int nsw, double* __restrict__ swr, double* __restrict__ swv, double* __restrict__ swn,
+    lbswim_common_params c, unsigned long long seed, unsigned long long step, Dims D,
+    const double* __restrict__ u, unsigned* status) {
+  __shared__ Stencil64 st;
+  __shared__ double turned[3][MOVE64_SWIMMERS];
+  const int p = threadIdx.x % MOVE64_POINTS, a = threadIdx.x / MOVE64_POINTS;
+  const int q = p % MOVE64_SWIMMERS, i = blockIdx.x * MOVE64_SWIMMERS + q;
+  const long long at = (long long)nsw * a + i;
+  const bool rear = p >= MOVE64_SWIMMERS, mine = a < 3, valid = mine && i < nsw;
+  double x = 0.0, na = 0.0;
+  if (valid) {
+    x = swr[at];
+    na = swn[at];
+  }
+  if (mine) point_axis64(D, rear ? __dsub_rn(x, __dmul_rn(na, c.l)) : x, a, p, st);
+  __syncthreads();
+  gather64<I>(u, D, st);
+  __syncthreads();
+  const bool update = valid && !rear;
+  bool tumble = false;
+  if (update) {
+    tumble = rng_uniform(seed, (uint32_t)i, step) < c.alpha;
+    const double va = st.vel[a][q];
+    double rDot = __dmul_rn(__dmul_rn(c.mobility, c.P), na);
+    if (!c.translational_advection_off) rDot = __dadd_rn(rDot, va);
+    swv[at] = rDot;
+    swr[at] = wrap_position(__dadd_rn(x, rDot), D.n[a], status);
+    if (tumble) {  // a direction uniform on the sphere
+      double g[3];
+      rng_normal3(seed, (uint32_t)i, step, g);
+      turned[a][q] = a == 0 ? g[0] : (a == 1 ? g[1] : g[2]);
+    } else {  // rotate with the local shear
+      turned[a][q] = na + (va - st.vel[a][MOVE64_SWIMMERS + q]) / c.l;
+    }
+  }
+  __syncthreads();
+  if (!update || (!tumble && c.rotational_advection_off)) return;  // orientation unchanged
+  const double nx = turned[0][q], ny = turned[1][q], nz = turned[2][q];
+  const double norm =
+      __dsqrt_rn(__dadd_rn(__dadd_rn(__dmul_rn(nx, nx), __dmul_rn(ny, ny)), __dmul_rn(nz, nz)));
+  swn[at] = turned[a][q] / norm;
 }
 
 template <class U, class T>
@@ -955,7 +1141,7 @@ __global__ void k_interp_points(int np, const double* __restrict__ r, double* __
   if (i >= np) return;
   const double rr[3] = {r[i], r[np + i], r[2 * np + i]};
   T vv[3];
-  interp_velocity<T>(u, D, rr, vv);
+  interp_velocity(u, D, rr, vv);
   for (int d = 0; d < 3; ++d) v[np * d + i] = (double)vv[d];
 }
 
@@ -1104,7 +1290,7 @@ __device__ __forceinline__ double q44_to_pos(long long q) {
       (long long)(((unsigned long long)(e + 1023) << 52) | (m & 0xfffffffffffffull)));
 }
 
-// r + v moved back into [0, n) by one shift, like wrap_position<float>: in Q44
+// r + v moved back into [0, n) by one shift, like wrap_shift: in Q44
 // when r and r + v allow it (the result then lies in the box by construction),
 // else in FP64, where a result outside [0, n) -- a non-finite r or v, or a
 // move longer than the box -- raises LBSWIM_STATUS_PARTICLE_OUTSIDE.
@@ -1116,7 +1302,7 @@ __device__ __forceinline__ double advance_position(double r, float v, int n, uns
     q = q >= nq ? q - nq : (q < 0 ? q + nq : q);
     return q44_to_pos(q);
   }
-  const double out = wrap_position<float>(r + f2d_exact(v), n);
+  const double out = wrap_shift(r + f2d_exact(v), n);
   if (!in_box(out, n)) raise_status(status, LBSWIM_STATUS_PARTICLE_OUTSIDE);
   return out;
 }
@@ -1779,7 +1965,7 @@ static void append_ends(Swimmers* W, Lattice* L) {
   S.pending += nends;
 }
 
-// 64-bit site offsets in the FP32 move kernels: when 32-bit ones would
+// 64-bit site offsets in the move kernels: when 32-bit ones would
 // overflow, or when the lattice asks for them (LBSWIM_COMPAT_WIDE_INDEX).
 static bool wide_particle_index(const Lattice* L) {
   return L->n >= (1ll << 31) || (L->compat & LBSWIM_COMPAT_WIDE_INDEX);
@@ -1809,15 +1995,20 @@ void swimmers_add_forces(Swimmers* W, Lattice* L) {
 void swimmers_move(Swimmers* W, Lattice* L) {
   const Dims D = make_dims(L);
   if (W->n > 0) {
-    const int grid = (W->n + 255) / 256;
-    if (L->precision == LBSWIM_F64 && (L->compat & LBSWIM_COMPAT_EXACT_F64))
-      k_swimmers_move<double, double><<<grid, 256, 0, L->stream>>>(
-          W->n, W->r, W->v, W->nv, W->common, W->seed, W->step, D, (const double*)L->u,
-          L->status);
-    else if (L->precision == LBSWIM_F64)
-      k_swimmers_move<double, double, true><<<grid, 256, 0, L->stream>>>(
-          W->n, W->r, W->v, W->nv, W->common, W->seed, W->step, D, (const double*)L->u,
-          L->status);
+    if (L->precision == LBSWIM_F64) {
+      const double* u = (const double*)L->u;
+      const int grid = (W->n + MOVE64_SWIMMERS - 1) / MOVE64_SWIMMERS;
+      if (L->compat & LBSWIM_COMPAT_EXACT_F64)
+        k_swimmers_move_exact<<<(int)((2ll * W->n + EXACT_MOVE_BLOCK - 1) / EXACT_MOVE_BLOCK),
+                                EXACT_MOVE_BLOCK, 0, L->stream>>>(
+            W->n, W->r, W->v, W->nv, W->common, W->seed, W->step, D, u, L->status);
+      else if (wide_particle_index(L))
+        k_swimmers_move_f64<long long><<<grid, MOVE64_BLOCK, 0, L->stream>>>(
+            W->n, W->r, W->v, W->nv, W->common, W->seed, W->step, D, u, L->status);
+      else
+        k_swimmers_move_f64<int><<<grid, MOVE64_BLOCK, 0, L->stream>>>(
+            W->n, W->r, W->v, W->nv, W->common, W->seed, W->step, D, u, L->status);
+    }
     else if (wide_particle_index(L))
       k_swimmers_move_f32<long long><<<(W->n + SWIMMERS_PER_BLOCK - 1) / SWIMMERS_PER_BLOCK,
                                        SWIMMER_MOVE_BLOCK, 0, L->stream>>>(
@@ -2110,13 +2301,19 @@ static void tracers_move_on(Tracers* T, Lattice* L, cudaStream_t stream) {
   if (T->needs_sort || T->moves_since_sort >= TRACER_RESORT_MOVES) tracers_sort(T, L, stream);
   T->moves_since_sort++;
   const Dims D = make_dims(L);
-  const int grid = (T->n + 255) / 256;
-  if (L->precision == LBSWIM_F64 && (L->compat & LBSWIM_COMPAT_EXACT_F64))
-    k_tracers_move<double, double><<<grid, 256, 0, stream>>>(T->n, T->r, T->s, T->v, D,
-                                                                 (const double*)L->u, L->status);
-  else if (L->precision == LBSWIM_F64)
-    k_tracers_move<double, double, true><<<grid, 256, 0, stream>>>(
-        T->n, T->r, T->s, T->v, D, (const double*)L->u, L->status);
+  if (L->precision == LBSWIM_F64) {
+    const double* u = (const double*)L->u;
+    const int grid = (T->n + MOVE64_POINTS - 1) / MOVE64_POINTS;
+    if (L->compat & LBSWIM_COMPAT_EXACT_F64)
+      k_tracers_move_exact<<<(T->n + EXACT_MOVE_BLOCK - 1) / EXACT_MOVE_BLOCK, EXACT_MOVE_BLOCK,
+                             0, stream>>>(T->n, T->r, T->s, T->v, D, u, L->status);
+    else if (wide_particle_index(L))
+      k_tracers_move_f64<long long><<<grid, MOVE64_BLOCK, 0, stream>>>(T->n, T->r, T->s, T->v, D,
+                                                                       u, L->status);
+    else
+      k_tracers_move_f64<int><<<grid, MOVE64_BLOCK, 0, stream>>>(T->n, T->r, T->s, T->v, D, u,
+                                                                 L->status);
+  }
   else if (wide_particle_index(L))
     k_tracers_move_f32<long long><<<(T->n + TRACER_MOVE_BLOCK - 1) / TRACER_MOVE_BLOCK,
                                     TRACER_MOVE_BLOCK, 0, stream>>>(T->n, T->r, T->s, T->v, D,
