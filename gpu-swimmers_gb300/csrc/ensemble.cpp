@@ -144,6 +144,35 @@ static void capture(Ensemble* E, int nsteps_in_graph, cudaGraphExec_t* out) {
   LB_CUDA(e);
 }
 
+// x planes per slab of every member.  304 CTAs take the slabs from one queue,
+// so a run lasts about the sum of their lx + 5 planes (ring and start) over 304
+// and half a slab more: long slabs for many members, short ones where few
+// members would leave CTAs without a slab.
+static std::vector<int> slab_lengths(const Ensemble* E) {
+  std::vector<int> best;
+  double least = 0.0;
+  for (int cap = 32; cap >= 2; cap /= 2) {
+    std::vector<int> lx(E->lat.size());
+    double planes = 0.0, longest = 0.0;
+    for (size_t m = 0; m < lx.size(); ++m) {
+      const Lattice* L = E->lat[m];
+      int ty, tz;
+      slab_section_of(L->fused_tile, &ty, &tz);
+      lx[m] = slab_lx_within(L->size, L->fused_tile, E->sw[m] ? 2ll * E->sw[m]->n : 0, cap);
+      const double slabs = (double)((L->size[0] + lx[m] - 1) / lx[m]) *
+                           ((L->size[1] + ty - 1) / ty) * ((L->size[2] + tz - 1) / tz);
+      planes += slabs * (lx[m] + 5);
+      longest = std::max(longest, lx[m] + 5.0);
+    }
+    const double cost = std::max(planes / E->grid_step + 0.5 * longest, longest);
+    if (best.empty() || cost < least) {
+      best = lx;
+      least = cost;
+    }
+  }
+  return best;
+}
+
 // The member table of the current run: buffers named relative to the run's
 // start (f[0] = f(t), hyd[p] = the velocity buffer written by steps of
 // parity p, so the last one written is the lattice's current one).
@@ -151,13 +180,15 @@ static void build_tables(Ensemble* E) {
   const int n = (int)E->lat.size();
   E->hmem.assign(n, EnsMember{});
   for (auto& p : E->pre) p.assign(n + 1, 0);
+  const std::vector<int> lx = slab_lengths(E);
   for (int m = 0; m < n; ++m) {
     Lattice* L = E->lat[m];
     Swimmers* W = E->sw[m];
     Tracers* T = E->tr[m];
     EnsMember& M = E->hmem[m];
     const int nsw = W ? W->n : 0, ntr = T ? T->n : 0;
-    spread_reserve(L, 2 * nsw);
+    M.lx = lx[m];
+    spread_reserve(L, 2 * nsw, M.lx);
     for (int a = 0; a < 3; ++a) M.size[a] = L->size[a];
     M.n = L->n;
     M.rho0 = (float)L->rho0;
@@ -168,8 +199,9 @@ static void build_tables(Ensemble* E) {
     M.force_s = (float)(2. * ws * L->tau_s);
     M.force_b = (float)(2. * wb * L->tau_b);
     M.tile = L->fused_tile;
-    int T3[3];
-    slab_shape_of(M.tile, T3);
+    slab_division(M.lx, M.by_lx);
+    int T3[3] = {M.lx, 0, 0};
+    slab_section_of(M.tile, &T3[1], &T3[2]);
     for (int a = 0; a < 3; ++a) M.nt[a] = (L->size[a] + T3[a] - 1) / T3[a];
     M.f[0] = L->f[L->cur];
     M.f[1] = L->f[L->cur ^ 1];
@@ -247,6 +279,7 @@ void ensemble_step(Ensemble* E, int nsteps, const int* limits) {
     L->spread.pending = 2 * (E->sw[m] ? E->sw[m]->n : 0);
     L->spread.stepped = true;
     L->spread.bucket_tile = L->fused_tile;
+    L->spread.lx = E->hmem[m].lx;
     if (E->sw[m]) E->sw[m]->step += k;
     if (E->tr[m]) E->tr[m]->moves_since_sort += k;
   }

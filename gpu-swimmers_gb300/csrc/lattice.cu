@@ -130,19 +130,6 @@ __device__ __forceinline__ void load_force(const T* F, long long N, long long s,
   }
 }
 
-// Unsigned division by a divisor fixed at launch: t / d for t < 2^31.
-struct FastDiv {
-  unsigned mul, shift;
-};
-static FastDiv fast_div(unsigned d) {
-  unsigned l = 0;
-  while ((1ull << l) < d) ++l;
-  return FastDiv{(unsigned)(((1ull << 32) * ((1ull << l) - d)) / d + 1), l};
-}
-__device__ __forceinline__ unsigned div_by(unsigned t, FastDiv k) {
-  return (__umulhi(t, k.mul) + t) >> k.shift;
-}
-
 // FP64 collide + push-stream, lb.cu:72-218.  A thread takes site blockIdx.x *
 // F64_THREADS + threadIdx.x of x plane blockIdx.y, so that a ragged nz idles
 // no lanes.  The collision runs on integers (fixed_site.cuh); the sites that do
@@ -412,7 +399,7 @@ __global__ void k_f32_to_f64(const float* __restrict__ src, double* __restrict__
 // ---------------------------------------------------------------------------
 // Fused collide + stream + hydro kernel (FP32 arithmetic).
 //
-// A CTA owns a TY x TZ cross-section (y, z) of FUSED_LX consecutive x planes
+// A CTA owns a TY x TZ cross-section (y, z) of lx consecutive x planes (choose_slab_lx)
 // and marches along x.  For each plane it collides the cross-section plus a
 // one-site ring (TY*TZ interior threads + up to 96 ring threads) and parks
 // the post-collision values in a ring buffer of shared memory.  Once the
@@ -423,7 +410,6 @@ __global__ void k_f32_to_f64(const float* __restrict__ src, double* __restrict__
 // collisions of the planes x, x-1, x+1 and stay in registers.  The next
 // plane's loads are issued before the current plane is collided.
 // ---------------------------------------------------------------------------
-constexpr int FUSED_LX = SLAB_LX;
 constexpr int FUSED_RING_THREADS = 96;
 
 struct FusedArgs {
@@ -432,6 +418,7 @@ struct FusedArgs {
   const float* force;  // dense force base; null: zero
   float4* hydro;  // {ux, uy, uz, rho} per site
   int nx, ny, nz;
+  int lx;  // x planes per slab
   long long n;
   float rho0;
   Relax<float> k;
@@ -500,7 +487,7 @@ static_assert(2 * (fused_smem_total<float, 32, 8, true, true>() + 1024) <= 228 *
 static_assert(2 * (fused_smem_bytes<32, 8, true>() + 1024) <= 132 * 1024, "SPREAD slab smem");
 static_assert(2 * (fused_smem_bytes<16, 16, true>() + 1024) <= 132 * 1024, "SPREAD slab smem");
 
-// One slab: tile (tz, ty, tx) of the lattice in units of (TZ, TY, FUSED_LX)
+// One slab: tile (tz, ty, tx) of the lattice in units of (TZ, TY, a.lx)
 // sites; `slab` indexes its bucket of pending ends.  Called by one CTA.
 // I is the site-index type: int when 15 N fits it (one multiply-add per
 // address), long long otherwise.
@@ -521,8 +508,8 @@ __device__ __forceinline__ void fused_slab(const FusedArgs& a, int tz, int ty, i
   float* ringC = ringB + NB * RP * PLANE;          // [NC][RP][PLANE]
   const int tid = threadIdx.x;
   const int nx = a.nx, ny = a.ny, nz = a.nz;
-  const int z0 = tz * TZ, y0 = ty * TY, x0 = tx * FUSED_LX;
-  const int ez = min(TZ, nz - z0), ey = min(TY, ny - y0), ex = min(FUSED_LX, nx - x0);
+  const int z0 = tz * TZ, y0 = ty * TY, x0 = tx * a.lx;
+  const int ez = min(TZ, nz - z0), ey = min(TY, ny - y0), ex = min(a.lx, nx - x0);
 
   int ly = 0, lz = 0;
   bool active = false, interior = false;
@@ -776,6 +763,7 @@ __global__ void __launch_bounds__(8 * 32 + FUSED_RING_THREADS, 2) k_ens_step(Ens
     a.nx = M.size[0];
     a.ny = M.size[1];
     a.nz = M.size[2];
+    a.lx = M.lx;
     a.n = M.n;
     a.rho0 = M.rho0;
     a.k = Relax<float>{M.omega_s, M.omega_b, M.force_s, M.force_b};
@@ -813,12 +801,12 @@ void ens_launch_step(const EnsTable& t, int parity, int grid, cudaStream_t s) {
 // ---------------------------------------------------------------------------
 template <int TZ, int TY, bool SPLIT>
 __device__ __forceinline__ void force_slab(const SlabEnds& se, float* __restrict__ force, int nx,
-                                           int ny, int nz, long long N, int accumulate,
+                                           int ny, int nz, int lx, long long N, int accumulate,
                                            int slab) {
   extern __shared__ __align__(16) unsigned char smraw[];
   const int tid = threadIdx.x;
-  const int z0 = blockIdx.x * TZ, y0 = blockIdx.y * TY, x0 = blockIdx.z * SLAB_LX;
-  const int ez = min(TZ, nz - z0), ey = min(TY, ny - y0), ex = min(SLAB_LX, nx - x0);
+  const int z0 = blockIdx.x * TZ, y0 = blockIdx.y * TY, x0 = blockIdx.z * lx;
+  const int ez = min(TZ, nz - z0), ey = min(TY, ny - y0), ex = min(lx, nx - x0);
   SlabSpreader<TZ, TY, 0, 0, SPLIT> sp;
   sp.bind(smraw, se, slab, nx, ny, nz, x0, y0, z0, ex, ey, ez);
   sp.prologue(tid, blockDim.x);
@@ -843,13 +831,13 @@ __device__ __forceinline__ void force_slab(const SlabEnds& se, float* __restrict
 
 template <int TZ, int TY>
 __global__ void __launch_bounds__(TY * TZ) k_force_slab(SlabEnds se, float* __restrict__ force,
-                                                         int nx, int ny, int nz, long long N,
-                                                         int accumulate) {
+                                                         int nx, int ny, int nz, int lx,
+                                                         long long N, int accumulate) {
   const int slab = (blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
   if (slab_sums_split(se, slab, nx, ny, nz))
-    force_slab<TZ, TY, true>(se, force, nx, ny, nz, N, accumulate, slab);
+    force_slab<TZ, TY, true>(se, force, nx, ny, nz, lx, N, accumulate, slab);
   else
-    force_slab<TZ, TY, false>(se, force, nx, ny, nz, N, accumulate, slab);
+    force_slab<TZ, TY, false>(se, force, nx, ny, nz, lx, N, accumulate, slab);
 }
 
 template <int TZ, int TY>
@@ -862,10 +850,11 @@ static void force_slab_launch(Lattice* L, const SlabSpread& sp) {
     configured = true;
   }
   dim3 grid((L->size[2] + TZ - 1) / TZ, (L->size[1] + TY - 1) / TY,
-            (L->size[0] + SLAB_LX - 1) / SLAB_LX);
+            (L->size[0] + sp.lx - 1) / sp.lx);
   k_force_slab<TZ, TY><<<grid, TY * TZ, smem, L->stream>>>(
       SlabEnds{(const EndRecord<float>*)sp.ends, sp.count, sp.list, sp.npending, sp.max_abs_force},
-      (float*)L->force, L->size[0], L->size[1], L->size[2], L->n, L->force_zero_pending ? 0 : 1);
+      (float*)L->force, L->size[0], L->size[1], L->size[2], sp.lx, L->n,
+      L->force_zero_pending ? 0 : 1);
   LB_CHECK_LAUNCH(1);
 }
 
@@ -1123,7 +1112,7 @@ static void launch_fused_i(Lattice* L, const FusedArgs& a) {
                                    cudaSharedmemCarveoutMaxShared));
     configured = true;
   }
-  dim3 grid((a.nz + TZ - 1) / TZ, (a.ny + TY - 1) / TY, (a.nx + FUSED_LX - 1) / FUSED_LX);
+  dim3 grid((a.nz + TZ - 1) / TZ, (a.ny + TY - 1) / TY, (a.nx + a.lx - 1) / a.lx);
   k_fused_step<S, TZ, TY, SPREAD, I, TMA>
       <<<grid, TY * TZ + FUSED_RING_THREADS, smem, L->stream>>>(a);
   LB_CHECK_LAUNCH(1);
@@ -1168,18 +1157,73 @@ static void fused_step_tile(Lattice* L, FusedArgs& a) {
     const SlabSpread sp = spread_prepare_slabs(L);
     a.spread = SlabEnds{(const EndRecord<float>*)sp.ends, sp.count, sp.list, sp.npending,
                         sp.max_abs_force};
+    a.lx = sp.lx;
     launch_fused<S, TZ, TY, true>(L, a);
   } else {
+    a.lx = choose_slab_lx(L->size, L->fused_tile, 0);
     launch_fused<S, TZ, TY, false>(L, a);
   }
 }
 
-void slab_shape_of(int tile, int T[3]) {
-  T[0] = FUSED_LX;
-  T[1] = tile == 1 ? 16 : 8;
-  T[2] = tile == 1 ? 16 : 32;
+void slab_section_of(int tile, int* ty, int* tz) {
+  *ty = tile == 1 ? 16 : 8;
+  *tz = tile == 1 ? 16 : 32;
 }
-void fused_slab_shape(const Lattice* L, int T[3]) { slab_shape_of(L->fused_tile, T); }
+
+void slab_division(int lx, unsigned by[2]) {
+  const FastDiv d = fast_div((unsigned)lx);
+  by[0] = d.mul;
+  by[1] = d.shift;
+}
+
+// Longest slab whose ends, with those that touch its surroundings, fit the
+// SPREAD_CAP held in shared memory: at most 180 of them on average.
+static int longest_slab(const int size[3], int tile, long long nends) {
+  int ty, tz;
+  slab_section_of(tile, &ty, &tz);
+  const double per_plane = (double)nends / ((double)size[0] * size[1] * size[2]) *
+                           std::min(ty + 5, size[1]) * std::min(tz + 5, size[2]);
+  if (std::min(SLAB_LX_MAX + 5, size[0]) * per_plane <= 180.0) return std::min(size[0], SLAB_LX_MAX);
+  return std::max(1, std::min(size[0], (int)(180.0 / per_plane) - 5));
+}
+
+// As many slabs of equal length as slabs of at most lx planes take.
+static int even_slab(int nx, int lx) {
+  const int ns = (nx + lx - 1) / lx;
+  return (nx + ns - 1) / ns;
+}
+
+int slab_lx_within(const int size[3], int tile, long long nends, int cap) {
+  return even_slab(size[0], std::min(cap, longest_slab(size, tile, nends)));
+}
+
+// x planes per slab of a lattice stepped with nends pending ends, by the time
+// its slabs take: a slab takes lx + 2 planes (the ring) and a start that costs
+// about 3 more planes when it lists ends, 1 when not; 304 run at a time, and
+// with half of them or fewer each has an SM to itself and takes about 0.65 of
+// the time a plane takes with two.  A small lattice then has enough slabs for
+// the SMs, and a large one wastes less of its last wave.
+int choose_slab_lx(const int size[3], int tile, long long nends) {
+  int ty, tz;
+  slab_section_of(tile, &ty, &tz);
+  const long long section = (long long)((size[1] + ty - 1) / ty) * ((size[2] + tz - 1) / tz);
+  const int longest = longest_slab(size, tile, nends);
+  constexpr int SLOTS = 304;
+  int best = 1;
+  double least = 0.0;
+  for (int lx = 1; lx <= longest; ++lx) {
+    if (even_slab(size[0], lx) != lx) continue;  // a shorter slab gives as many
+    const long long slabs = (size[0] + lx - 1) / lx * section, rest = slabs % SLOTS;
+    const double waves =
+        (double)(slabs / SLOTS) + (rest == 0 ? 0.0 : rest <= SLOTS / 2 ? 0.65 : 1.0);
+    const double cost = waves * (lx + 2 + (nends > 0 ? 3 : 1));
+    if (least == 0.0 || cost < least) {
+      best = lx;
+      least = cost;
+    }
+  }
+  return best;
+}
 
 template <class S>
 static void fused_step_t(Lattice* L) {

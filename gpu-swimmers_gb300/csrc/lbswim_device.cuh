@@ -30,6 +30,19 @@ __host__ __device__ constexpr double w_of(int p) {
   return p == 0 ? 2.0 / 9.0 : p <= 6 ? 1.0 / 9.0 : 1.0 / 72.0;
 }
 
+// Unsigned division by a divisor fixed at launch: t / d for t < 2^31.
+struct FastDiv {
+  unsigned mul, shift;
+};
+inline FastDiv fast_div(unsigned d) {
+  unsigned l = 0;
+  while ((1ull << l) < d) ++l;
+  return FastDiv{(unsigned)(((1ull << 32) * ((1ull << l) - d)) / d + 1), l};
+}
+__device__ __forceinline__ unsigned div_by(unsigned t, FastDiv k) {
+  return (__umulhi(t, k.mul) + t) >> k.shift;
+}
+
 // Relaxation constants of one lattice (lb.cu:105-108, 165, 174).
 template <class T>
 struct Relax {

@@ -68,6 +68,7 @@ struct TileLists {
 // Ends listed per step-kernel slab, at most SLAB_BUCKET_CAP per slab (a slab
 // with more is spread from the whole list of pending ends).
 constexpr int SLAB_BUCKET_CAP = 1024;
+constexpr int SLAB_LX_MAX = 60;  // x planes of a slab at most
 
 struct SpreadScratch {
   int capacity_ends = 0;
@@ -83,8 +84,10 @@ struct SpreadScratch {
   // largest force)
   unsigned* bucket_count = nullptr;  // [bucket_slabs]
   int* bucket_list = nullptr;        // [bucket_slabs][SLAB_BUCKET_CAP], FP64: [][FT_CAP]
-  int bucket_slabs = 0;
+  int bucket_slabs = 0;  // slabs (or tiles) the buckets have room for
   int bucket_tile = -1;  // slab shape the buckets hold (Lattice::fused_tile), -1: stale
+  int lx = 0;            // x planes per slab of the pending ends' buckets
+  int last_pending = 0;  // ends of the last step: several arrays' ends arrive one by one
   // The next step's end records and slab buckets, written by the swimmer move
   // of lbswim_system_step; its AddForces takes them in place of recording
   // again while nothing has changed since (same swimmers, moved by nothing
@@ -102,6 +105,7 @@ struct SpreadScratch {
     unsigned long long owner_step = 0;    // its move counter after that move
     unsigned long long epoch = 0;         // API-call count then
     int tile = -1;
+    int lx = 0;
     int nends = 0;
   } prep;
 };
@@ -113,6 +117,7 @@ struct SlabSpread {
   const int* list = nullptr;
   int npending = 0;
   const unsigned* max_abs_force = nullptr;
+  int lx = 0;
 };
 
 struct Lattice {
@@ -215,6 +220,8 @@ struct EnsMember {
   float rho0;
   float omega_s, omega_b, force_s, force_b;  // Relax<float>
   int tile;                                  // slab shape: 0 = 8 x 32, 1 = 16 x 16
+  int lx;                                    // x planes per slab
+  unsigned by_lx[2];                         // FastDiv by it
   int nt[3];                                 // slabs per axis
   void* f[2];           // f(t) at the run's start, and the other buffer
   void* hyd[2];         // float4 {u, rho} written by steps 0, 2, 4, ... / 1, 3, 5, ...
@@ -260,8 +267,14 @@ void ens_launch_records(const EnsTable& t, int grid, cudaStream_t s);
 void ens_launch_step(const EnsTable& t, int parity, int grid, cudaStream_t s);
 void ens_launch_move(const EnsTable& t, int parity, int grid, cudaStream_t s);
 int ens_step_ctas_per_sm();
-// Slab shape of a tile choice (x planes, rows, columns).
-void slab_shape_of(int tile, int T[3]);
+// Cross-section (rows, columns) of the slabs of a tile choice, and the x planes
+// per slab of a lattice stepped with nends pending ends.
+void slab_section_of(int tile, int* ty, int* tz);
+int choose_slab_lx(const int size[3], int tile, long long nends);
+// The same with slabs of at most `cap` planes, as even as they come.
+int slab_lx_within(const int size[3], int tile, long long nends, int cap);
+// Multiplier and shift of a division by lx (FastDiv).
+void slab_division(int lx, unsigned by[2]);
 
 // ensemble.cpp
 struct Ensemble;
@@ -304,11 +317,9 @@ void exact_init_from_hydro_f64(Lattice* L);
 // particles.cu: force spreading state
 void spread_materialise(Lattice* L);
 SlabSpread spread_prepare_slabs(Lattice* L);
-// Slab shape of the fused step kernel for a lattice: x planes per slab, rows,
-// columns (lattice.cu).
-void fused_slab_shape(const Lattice* L, int T[3]);
-// Pending-end storage and slab buckets for `nends` ends (particles.cu).
-void spread_reserve(Lattice* L, int nends);
+// Pending-end storage for `nends` ends and buckets for slabs of lx planes
+// (particles.cu).
+void spread_reserve(Lattice* L, int nends, int lx);
 // Dense force (base + spread of the pending ends) of a reduced-precision
 // lattice, bit for bit the force the step kernel spreads (lattice.cu).
 void lattice_force_from_slabs(Lattice* L);

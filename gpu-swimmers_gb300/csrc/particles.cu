@@ -257,6 +257,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan_apply(const unsigned* __r
 // fixed function of the input, so the result is deterministic.
 struct TileGrid {
   int T[3];   // tile edge per axis
+  FastDiv by[3];  // division by it
   int h;      // sites beyond the tile (every side) that also need the force
   int nt[3];  // tiles per axis
 };
@@ -266,9 +267,8 @@ struct TileGrid {
 // range first, first+1, ... (count of them, at most nt).  An interval that
 // wraps past the end covers the tiles from `first` to the last one and from 0
 // to the tile of its wrapped end; if those meet, it covers every tile.  o is a
-// wrapped node (0 <= o < n, as records hold them) and h < n; the tile edge T
-// is a power of two (slab and force-tile shapes all are), so tiles are shifts.
-__device__ __forceinline__ void touched_range(int o, int n, int T, int h, int nt, int& first,
+// wrapped node (0 <= o < n, as records hold them) and h < n.
+__device__ __forceinline__ void touched_range(int o, int n, FastDiv by, int h, int nt, int& first,
                                               int& count) {
   const int len = 4 + 2 * h;
   if (len >= n) {
@@ -276,13 +276,12 @@ __device__ __forceinline__ void touched_range(int o, int n, int T, int h, int nt
     count = nt;
     return;
   }
-  const int sh = __ffs(T) - 1;
   const int a = o - h < 0 ? o - h + n : o - h, b = a + len - 1;
-  first = a >> sh;
+  first = (int)div_by((unsigned)a, by);
   if (b < n) {
-    count = (b >> sh) - first + 1;
+    count = (int)div_by((unsigned)b, by) - first + 1;
   } else {
-    const int last = (b - n) >> sh;
+    const int last = (int)div_by((unsigned)(b - n), by);
     count = last >= first ? nt : (nt - first) + last + 1;
   }
 }
@@ -295,13 +294,6 @@ __device__ __forceinline__ int node_after(int o, int j, int n) {
 
 constexpr int REC_THREADS = 256;
 
-// Slab shape of a tile choice, as slab_shape_of (lattice.cu): x planes, rows, columns.
-__device__ __forceinline__ void slab_shape_of_dev(int tile, int T[3]) {
-  T[0] = 32;
-  T[1] = tile == 1 ? 16 : 8;
-  T[2] = tile == 1 ? 16 : 32;
-}
-
 // List end e under every tile of grid G whose extended region its stencil
 // touches (at most CAP ends are kept per tile; the count goes on).
 template <int CAP>
@@ -309,7 +301,7 @@ __device__ __forceinline__ void bucket_end(int e, const int o[3], const Dims& D,
                                            unsigned* __restrict__ count,
                                            int* __restrict__ list) {
   int f[3], c[3];
-  for (int a = 0; a < 3; ++a) touched_range(o[a], D.n[a], G.T[a], G.h, G.nt[a], f[a], c[a]);
+  for (int a = 0; a < 3; ++a) touched_range(o[a], D.n[a], G.by[a], G.h, G.nt[a], f[a], c[a]);
   for (int i = 0; i < c[0]; ++i) {
     const int kx = f[0] + i < G.nt[0] ? f[0] + i : f[0] + i - G.nt[0];
     for (int j = 0; j < c[1]; ++j) {
@@ -411,9 +403,9 @@ __global__ void k_touch(int nends, const EndRecord<double>* __restrict__ ends, D
   if (e >= nends) return;
   const int ox = ends[e].o[0], oy = ends[e].o[1], oz = ends[e].o[2];
   int fx, cx, fy, cy, fz, cz;
-  touched_range(ox, D.n[0], G.T[0], G.h, G.nt[0], fx, cx);
-  touched_range(oy, D.n[1], G.T[1], G.h, G.nt[1], fy, cy);
-  touched_range(oz, D.n[2], G.T[2], G.h, G.nt[2], fz, cz);
+  touched_range(ox, D.n[0], G.by[0], G.h, G.nt[0], fx, cx);
+  touched_range(oy, D.n[1], G.by[1], G.h, G.nt[1], fy, cy);
+  touched_range(oz, D.n[2], G.by[2], G.h, G.nt[2], fz, cz);
   for (int i = 0; i < cx; ++i) {
     const int kx = fx + i < G.nt[0] ? fx + i : fx + i - G.nt[0];
     for (int j = 0; j < cy; ++j) {
@@ -470,8 +462,6 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan_apply_total(
 //    row's 32 lanes have half an end each on average and run as long as the one
 //    with most, on the narrow FP64 pipe.
 constexpr int FT_X = 4, FT_Y = 8, FT_Z = 32, FT_THREADS = 256, FT_CAP = 256;
-static_assert((FT_X & (FT_X - 1)) == 0 && (FT_Y & (FT_Y - 1)) == 0 && (FT_Z & (FT_Z - 1)) == 0,
-              "tile edges are powers of two (touched_range shifts)");
 
 // One thread per (end, axis), 64 ends per block: the axes' chains of FP64
 // operations run side by side.  e = 2i is the tail, 2i + 1 the head.  FIXED:
@@ -1625,9 +1615,15 @@ __global__ void __launch_bounds__(REC_THREADS) k_ens_records(EnsTable t) {
     const EnsMember& M = t.mem[m];
     if (*t.g_step >= M.limit) continue;
     TileGrid G;
-    slab_shape_of_dev(M.tile, G.T);
+    G.T[0] = M.lx;
+    G.T[1] = M.tile == 1 ? 16 : 8;  // as slab_section_of
+    G.T[2] = M.tile == 1 ? 16 : 32;
     G.h = 1;
-    for (int a = 0; a < 3; ++a) G.nt[a] = M.nt[a];
+    G.by[0] = FastDiv{M.by_lx[0], M.by_lx[1]};
+    for (int a = 0; a < 3; ++a) {
+      G.nt[a] = M.nt[a];
+      if (a) G.by[a] = FastDiv{1u, (unsigned)__ffs(G.T[a]) - 1u};  // powers of two
+    }
     end_records_block(vb - t.rec_prefix[m], M.nsw, M.sw_r, M.sw_n, M.common.P,
                              M.common.l, ens_dims(M), (EndRecord<float>*)M.ends, 0, M.max_abs_f,
                              G, M.bucket_count, M.bucket_list);
@@ -1693,7 +1689,10 @@ static TileGrid force_tiles(const Lattice* L) {
   G.T[1] = FT_Y;
   G.T[2] = FT_Z;
   G.h = 0;
-  for (int a = 0; a < 3; ++a) G.nt[a] = (L->size[a] + G.T[a] - 1) / G.T[a];
+  for (int a = 0; a < 3; ++a) {
+    G.nt[a] = (L->size[a] + G.T[a] - 1) / G.T[a];
+    G.by[a] = fast_div((unsigned)G.T[a]);
+  }
   return G;
 }
 
@@ -1883,52 +1882,64 @@ void spread_materialise(Lattice* L) {
   }
 }
 
-static TileGrid slab_grid(const Lattice* L) {
+static TileGrid slab_grid(const Lattice* L, int lx) {
   TileGrid G;
-  fused_slab_shape(L, G.T);
+  G.T[0] = lx;
+  slab_section_of(L->fused_tile, &G.T[1], &G.T[2]);
   G.h = 1;  // the step kernel collides a one-site ring around its slab
-  for (int a = 0; a < 3; ++a) G.nt[a] = (L->size[a] + G.T[a] - 1) / G.T[a];
+  for (int a = 0; a < 3; ++a) {
+    G.nt[a] = (L->size[a] + G.T[a] - 1) / G.T[a];
+    G.by[a] = fast_div((unsigned)G.T[a]);
+  }
   return G;
 }
 
-// Bucket storage for the current slab grid; false when it had to be replaced
-// (the buckets are then stale).
-static bool ensure_buckets(Lattice* L) {
-  SpreadScratch& S = L->spread;
-  const TileGrid G = slab_grid(L);
-  const int nslabs = G.nt[0] * G.nt[1] * G.nt[2];
-  if (S.bucket_slabs == nslabs && S.bucket_count) return true;
+static int slabs_of(const TileGrid& G) { return G.nt[0] * G.nt[1] * G.nt[2]; }
+
+// Buckets (count and list) for at least nslabs slabs; replacing them waits for
+// the lattice's work.
+static void grow_buckets(Lattice* L, int nslabs, unsigned*& count, int*& list, int& slabs) {
+  if (slabs >= nslabs && count) return;
   LB_CUDA(cudaStreamSynchronize(L->stream));
-  if (S.bucket_count) cudaFree(S.bucket_count);
-  if (S.bucket_list) cudaFree(S.bucket_list);
-  S.bucket_count = nullptr;
-  S.bucket_list = nullptr;
-  LB_CUDA(cudaMalloc(&S.bucket_count, sizeof(unsigned) * nslabs));
-  LB_CUDA(cudaMalloc(&S.bucket_list, sizeof(int) * (size_t)nslabs * SLAB_BUCKET_CAP));
-  S.bucket_slabs = nslabs;
-  S.bucket_tile = -1;
-  return false;
+  if (count) cudaFree(count);
+  if (list) cudaFree(list);
+  count = nullptr;
+  list = nullptr;
+  slabs = 0;
+  LB_CUDA(cudaMalloc(&count, sizeof(unsigned) * nslabs));
+  LB_CUDA(cudaMalloc(&list, sizeof(int) * (size_t)nslabs * SLAB_BUCKET_CAP));
+  slabs = nslabs;
 }
 
-void spread_reserve(Lattice* L, int nends) {
+void spread_reserve(Lattice* L, int nends, int lx) {
   ensure_ends(L, nends);
   SpreadScratch& S = L->spread;
   if (!S.max_abs_force) LB_CUDA(cudaMalloc(&S.max_abs_force, sizeof(unsigned)));
-  ensure_buckets(L);
+  grow_buckets(L, slabs_of(slab_grid(L, lx)), S.bucket_count, S.bucket_list, S.bucket_slabs);
+  S.bucket_tile = -1;
+}
+
+// Empty buckets for slabs of S.lx planes.
+static void clear_buckets(Lattice* L) {
+  SpreadScratch& S = L->spread;
+  const int nslabs = slabs_of(slab_grid(L, S.lx));
+  grow_buckets(L, nslabs, S.bucket_count, S.bucket_list, S.bucket_slabs);
+  LB_CUDA(cudaMemsetAsync(S.bucket_count, 0, sizeof(unsigned) * nslabs, L->stream));
+  S.bucket_tile = L->fused_tile;
 }
 
 SlabSpread spread_prepare_slabs(Lattice* L) {
   SpreadScratch& S = L->spread;
-  if (!ensure_buckets(L) || S.bucket_tile != L->fused_tile) {
-    const TileGrid G = slab_grid(L);
-    LB_CUDA(cudaMemsetAsync(S.bucket_count, 0, sizeof(unsigned) * S.bucket_slabs, L->stream));
+  S.last_pending = S.pending;
+  if (S.bucket_tile != L->fused_tile) {
+    S.lx = choose_slab_lx(L->size, L->fused_tile, S.pending);
+    clear_buckets(L);
     if (S.pending > 0) {
       k_bucket_ends<<<(S.pending + 255) / 256, 256, 0, L->stream>>>(
-          S.pending, (const EndRecord<float>*)S.ends, make_dims(L), G, S.bucket_count,
-          S.bucket_list);
+          S.pending, (const EndRecord<float>*)S.ends, make_dims(L), slab_grid(L, S.lx),
+          S.bucket_count, S.bucket_list);
       LB_CHECK_LAUNCH(1);
     }
-    S.bucket_tile = L->fused_tile;
   }
   SlabSpread out;
   out.ends = S.ends;
@@ -1936,6 +1947,7 @@ SlabSpread spread_prepare_slabs(Lattice* L) {
   out.list = S.bucket_list;
   out.npending = S.pending;
   out.max_abs_force = S.max_abs_force;
+  out.lx = S.lx;
   return out;
 }
 
@@ -1946,19 +1958,16 @@ static void append_ends(Swimmers* W, Lattice* L) {
   const int nends = 2 * W->n;
   ensure_ends(L, S.pending + nends);
   if (!S.max_abs_force) LB_CUDA(cudaMalloc(&S.max_abs_force, sizeof(unsigned)));
-  const bool kept = ensure_buckets(L);
   if (S.pending == 0) {
-    LB_CUDA(cudaMemsetAsync(S.bucket_count, 0, sizeof(unsigned) * S.bucket_slabs, L->stream));
-    S.bucket_tile = L->fused_tile;
-  } else if (!kept) {
-    S.bucket_tile = -1;
+    S.lx = choose_slab_lx(L->size, L->fused_tile, std::max(nends, S.last_pending));
+    clear_buckets(L);
   }
   const bool fill = S.bucket_tile == L->fused_tile;
   if (S.pending == 0) LB_CUDA(cudaMemsetAsync(S.max_abs_force, 0, sizeof(unsigned), L->stream));
   if (nends > 0) {
     k_end_records<<<(nends + REC_THREADS - 1) / REC_THREADS, REC_THREADS, 0, L->stream>>>(
         W->n, W->r, W->nv, W->common.P, W->common.l, make_dims(L),
-        (EndRecord<float>*)S.ends + S.pending, S.pending, S.max_abs_force, slab_grid(L),
+        (EndRecord<float>*)S.ends + S.pending, S.pending, S.max_abs_force, slab_grid(L, S.lx),
         fill ? S.bucket_count : nullptr, fill ? S.bucket_list : nullptr);
     LB_CHECK_LAUNCH(1);
   }
@@ -2036,34 +2045,24 @@ void swimmers_move_preparing(Swimmers* W, Lattice* L, unsigned long long epoch) 
   P.valid = false;
   swimmers_move(W, L);
   if (W->n <= 0 || L->precision == LBSWIM_F64) return;
-  const TileGrid G = slab_grid(L);
-  const int nslabs = G.nt[0] * G.nt[1] * G.nt[2];
   const int nends = 2 * W->n;
+  const int lx = choose_slab_lx(L->size, L->fused_tile, nends);
+  const TileGrid G = slab_grid(L, lx);
+  const int nslabs = slabs_of(G);
   const size_t rec = sizeof(EndRecord<float>);
-  if (P.capacity_ends < nends || P.bucket_slabs != nslabs || !P.max_abs_force) {
+  if (P.capacity_ends < nends) {
     // the buffers may still be read by earlier work on the stream
     LB_CUDA(cudaStreamSynchronize(L->stream));
-    if (P.capacity_ends < nends) {
-      if (P.ends) cudaFree(P.ends);
-      P.ends = nullptr;
-      P.capacity_ends = 0;
-      const int cap = std::max(nends + nends / 2, 64);
-      LB_CUDA(cudaMalloc(&P.ends, rec * cap));
-      P.capacity_ends = cap;
-      P.ends_bytes = rec * cap;
-    }
-    if (P.bucket_slabs != nslabs) {
-      if (P.bucket_count) cudaFree(P.bucket_count);
-      if (P.bucket_list) cudaFree(P.bucket_list);
-      P.bucket_count = nullptr;
-      P.bucket_list = nullptr;
-      P.bucket_slabs = 0;
-      LB_CUDA(cudaMalloc(&P.bucket_count, sizeof(unsigned) * nslabs));
-      LB_CUDA(cudaMalloc(&P.bucket_list, sizeof(int) * (size_t)nslabs * SLAB_BUCKET_CAP));
-      P.bucket_slabs = nslabs;
-    }
-    if (!P.max_abs_force) LB_CUDA(cudaMalloc(&P.max_abs_force, sizeof(unsigned)));
+    if (P.ends) cudaFree(P.ends);
+    P.ends = nullptr;
+    P.capacity_ends = 0;
+    const int cap = std::max(nends + nends / 2, 64);
+    LB_CUDA(cudaMalloc(&P.ends, rec * cap));
+    P.capacity_ends = cap;
+    P.ends_bytes = rec * cap;
   }
+  grow_buckets(L, nslabs, P.bucket_count, P.bucket_list, P.bucket_slabs);
+  if (!P.max_abs_force) LB_CUDA(cudaMalloc(&P.max_abs_force, sizeof(unsigned)));
   LB_CUDA(cudaMemsetAsync(P.bucket_count, 0, sizeof(unsigned) * nslabs, L->stream));
   LB_CUDA(cudaMemsetAsync(P.max_abs_force, 0, sizeof(unsigned), L->stream));
   k_end_records<<<(nends + REC_THREADS - 1) / REC_THREADS, REC_THREADS, 0, L->stream>>>(
@@ -2077,6 +2076,7 @@ void swimmers_move_preparing(Swimmers* W, Lattice* L, unsigned long long epoch) 
   P.owner_step = W->step;
   P.epoch = epoch;
   P.tile = L->fused_tile;
+  P.lx = lx;
   P.nends = nends;
 }
 
@@ -2089,8 +2089,6 @@ bool swimmers_add_forces_prepared(Swimmers* W, Lattice* L, unsigned long long ep
       P.tile != L->fused_tile || L->precision == LBSWIM_F64 || S.pending != 0 || S.stepped ||
       P.nends != 2 * W->n)
     return false;
-  const TileGrid G = slab_grid(L);
-  if (P.bucket_slabs != G.nt[0] * G.nt[1] * G.nt[2]) return false;
   std::swap(S.ends, P.ends);
   std::swap(S.ends_bytes, P.ends_bytes);
   std::swap(S.capacity_ends, P.capacity_ends);
@@ -2099,6 +2097,7 @@ bool swimmers_add_forces_prepared(Swimmers* W, Lattice* L, unsigned long long ep
   std::swap(S.bucket_slabs, P.bucket_slabs);
   std::swap(S.max_abs_force, P.max_abs_force);
   S.bucket_tile = L->fused_tile;
+  S.lx = P.lx;
   S.pending = P.nends;
   P.valid = false;
   swimmers_mark(W, L->stream);

@@ -1,7 +1,7 @@
 // spread_slab.cuh -- spreading the pending dipole ends of one slab into
 // fixed-point force sums, one x plane at a time, in shared memory.
 //
-// A slab is SLAB_LX x planes by TY rows (y) by TZ columns (z) of the lattice,
+// A slab is up to SLAB_LX_MAX x planes by TY rows (y) by TZ columns (z) of the lattice,
 // plus H sites on every side (H = 1 for the step kernel, which collides a ring
 // around its cross-section; H = 0 for the force kernel).  Its ends come from
 // the slab buckets filled when the ends were recorded.  For every local plane
@@ -19,7 +19,6 @@
 
 namespace lbswim {
 
-constexpr int SLAB_LX = 32;                // x planes per slab
 constexpr int SPREAD_CAP = 256;            // ends of one slab held in shared memory
 constexpr int SPREAD_PLANES_PER_END = 8;   // local planes one end can cover (6 at most)
 constexpr unsigned PL_FOLD = 1u << 10;     // nx < 4: several x nodes fold onto the plane
@@ -49,7 +48,7 @@ __device__ __forceinline__ int wrap_small(int i, int n) {
 
 // Byte offsets of the spreading state from byte BASE of shared memory:
 // fixed-point sums of one plane [3][PLANE][2 words], coverage masks [CAP] (u64),
-// ends [CAP], local node rows [CAP], per-plane list offsets [LX + 2H + 1],
+// ends [CAP], local node rows [CAP], per-plane list offsets [LX_MAX + 2H + 1],
 // plane lists [CAP * SPREAD_PLANES_PER_END] (u16).
 template <int TZ, int TY, int H, int BASE>
 struct SpreadLayout {
@@ -59,7 +58,7 @@ struct SpreadLayout {
   static constexpr int ends = align16(xmask + SPREAD_CAP * 8);
   static constexpr int nodes = align16(ends + SPREAD_CAP * (int)sizeof(SlabEnd));
   static constexpr int poff = align16(nodes + SPREAD_CAP * (int)sizeof(NodeLocal));
-  static constexpr int plist = align16(poff + (SLAB_LX + 2 * H + 1) * 4);
+  static constexpr int plist = align16(poff + (SLAB_LX_MAX + 2 * H + 1) * 4);
   static constexpr int total = align16(plist + SPREAD_CAP * SPREAD_PLANES_PER_END * 2);
 };
 
@@ -143,7 +142,7 @@ struct SlabSpreader {
           for (int j = 0; j < 4; ++j) e.phi[c][j] = g.phi[c][j];
         }
         // local planes kk (x = x0 - H + kk) holding one of the x nodes
-        unsigned long long m = 0ull;
+        unsigned long long m = 0ull;  // one bit per plane: SLAB_LX_MAX + 2 < 63
         if (nx >= 4) {
           for (int i = 0; i < 4; ++i)
             for (int d = wrap_small(e.ox + i - x0 + H, nx); d < planes(); d += nx) m |= 1ull << d;
