@@ -457,14 +457,7 @@ int lbswim_swimmers_d2h_all(lbswim_swimmers* sw, double* r, double* v, double* n
   API_BEGIN_READ
   REQUIRE(sw, "swimmers handle is NULL");
   Swimmers* W = SW(sw);
-  swimmers_wait(W);
-  if (!W->copy) LB_CUDA(cudaStreamCreateWithFlags(&W->copy, cudaStreamNonBlocking));
-  const size_t bytes = sizeof(double) * 3 * W->n;
-  double* dst[3] = {r, v, n};
-  const double* src[3] = {W->r, W->v, W->nv};
-  for (int f = 0; f < 3; ++f)
-    if (dst[f] && bytes) LB_CUDA(cudaMemcpyAsync(dst[f], src[f], bytes, cudaMemcpyDeviceToHost, W->copy));
-  LB_CUDA(cudaStreamSynchronize(W->copy));
+  swimmers_read(W, r, v, n);
   API_END
 }
 
@@ -728,6 +721,7 @@ int lbswim_system_step(lbswim_lattice* lat, lbswim_swimmers* const* swimmers, in
     lattice_zero_force(L);  // ZeroForce
     if (n_swimmers != 1 || !swimmers_add_forces_prepared(SW(swimmers[0]), L, calls))
       for (int i = 0; i < n_swimmers; ++i) swimmers_add_forces(SW(swimmers[i]), L);
+    if (n_swimmers == 1) swimmers_prepare_room(SW(swimmers[0]), L);
     lattice_step(L);
     lattice_calc_hydro(L);
     // Tracers move on their own streams while the swimmers move and the next

@@ -424,6 +424,11 @@ struct FusedArgs {
   Relax<float> k;
   SlabEnds spread;  // pending dipole ends spread by the kernel itself (SPREAD instances)
   unsigned* status;  // sticky error bits of the lattice (LBSWIM_STATUS_*)
+  // slab counts and the largest force of the records to be made for the next step,
+  // zeroed by this one
+  unsigned* clear;
+  int nclear;
+  unsigned* clear_max;
 };
 
 // Post-collision populations 3-14 wait in shared memory until the output plane
@@ -707,6 +712,10 @@ __device__ __forceinline__ void fused_slab(const FusedArgs& a, int tz, int ty, i
 template <class S, int TZ, int TY, bool SPREAD, class I, bool TMA>
 __global__ void __launch_bounds__(TY * TZ + FUSED_RING_THREADS, 2) k_fused_step(FusedArgs a) {
   const int slab = (blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
+  for (int i = slab * blockDim.x + threadIdx.x; i < a.nclear;
+       i += gridDim.x * gridDim.y * gridDim.z * blockDim.x)
+    a.clear[i] = 0u;
+  if (a.clear_max && slab == 0 && threadIdx.x == 0) *a.clear_max = 0u;
   if (!SPREAD || slab_sums_split(a.spread, slab, a.nx, a.ny, a.nz))
     fused_slab<S, TZ, TY, SPREAD, I, true, TMA>(a, blockIdx.x, blockIdx.y, blockIdx.z, slab);
   else
@@ -945,7 +954,7 @@ static double* staging(Lattice* L, size_t elems) {
 // staging copy and no serialisation of copy and conversion.  Returns the
 // buffer's device address, or null for pageable memory (which goes through
 // the staging buffer).
-static const void* mapped_host(const void* host) {
+const void* mapped_host(const void* host) {
   cudaPointerAttributes at;
   int dev = -1;
   if (cudaPointerGetAttributes(&at, host) != cudaSuccess || cudaGetDevice(&dev) != cudaSuccess) {
@@ -1201,8 +1210,9 @@ int slab_lx_within(const int size[3], int tile, long long nends, int cap) {
 // its slabs take: a slab takes lx + 2 planes (the ring) and a start that costs
 // about 3 more planes when it lists ends, 1 when not; 304 run at a time, and
 // with half of them or fewer each has an SM to itself and takes about 0.65 of
-// the time a plane takes with two.  A small lattice then has enough slabs for
-// the SMs, and a large one wastes less of its last wave.
+// the time a plane takes with two.  Ends listed in buckets cost an atomic per
+// slab they touch, about 1 + 5 / lx of them along x.  A small lattice then has
+// enough slabs for the SMs, and a large one wastes less of its last wave.
 int choose_slab_lx(const int size[3], int tile, long long nends) {
   int ty, tz;
   slab_section_of(tile, &ty, &tz);
@@ -1216,7 +1226,8 @@ int choose_slab_lx(const int size[3], int tile, long long nends) {
     const long long slabs = (size[0] + lx - 1) / lx * section, rest = slabs % SLOTS;
     const double waves =
         (double)(slabs / SLOTS) + (rest == 0 ? 0.0 : rest <= SLOTS / 2 ? 0.65 : 1.0);
-    const double cost = waves * (lx + 2 + (nends > 0 ? 3 : 1));
+    const double cost = waves * (lx + 2 + (nends > 0 ? 3 : 1)) +
+                        (nends > DIRECT_ENDS ? 1.75 * (1 + 5.0 / lx) : 0.0);
     if (least == 0.0 || cost < least) {
       best = lx;
       least = cost;
@@ -1240,6 +1251,12 @@ static void fused_step_t(Lattice* L) {
   a.rho0 = (float)L->rho0;
   a.k = make_relax<float>(L->tau_s, L->tau_b);
   a.status = L->status;
+  SpreadScratch::Prepared& P = L->spread.prep;
+  a.clear = P.bucket_count;
+  a.nclear = P.clear;
+  a.clear_max = P.clear_max ? P.max_abs_force : nullptr;
+  P.clear = 0;
+  P.clear_max = false;
   if (L->fused_tile == 1)
     fused_step_tile<S, 16, 16>(L, a);
   else

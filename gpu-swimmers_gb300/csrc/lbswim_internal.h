@@ -69,6 +69,11 @@ struct TileLists {
 // with more is spread from the whole list of pending ends).
 constexpr int SLAB_BUCKET_CAP = 1024;
 constexpr int SLAB_LX_MAX = 60;  // x planes of a slab at most
+// Up to this many pending ends, every slab (and force tile of an FP64 lattice) picks
+// its own from all of them and no buckets are filled: their atomics, one after
+// another per end, took longer than the small steps that use them.  A
+// swimmer array with no more ends records them in its move.
+constexpr int DIRECT_ENDS = 512, DIRECT_ENDS_F64 = 64;
 
 struct SpreadScratch {
   int capacity_ends = 0;
@@ -88,10 +93,11 @@ struct SpreadScratch {
   int bucket_tile = -1;  // slab shape the buckets hold (Lattice::fused_tile), -1: stale
   int lx = 0;            // x planes per slab of the pending ends' buckets
   int last_pending = 0;  // ends of the last step: several arrays' ends arrive one by one
-  // The next step's end records and slab buckets, written by the swimmer move
-  // of lbswim_system_step; its AddForces takes them in place of recording
-  // again while nothing has changed since (same swimmers, moved by nothing
-  // else, no other API call in between, same slab shape).
+  // The next step's end records and buckets, made by the swimmer move of
+  // lbswim_system_step; its AddForces takes them in place of recording again
+  // while nothing has changed since (same swimmers, moved by nothing else, no
+  // other API call in between, same slab shape).  FP64 lattices make them in the
+  // buffers above, which are free between AddForces and the next one.
   struct Prepared {
     void* ends = nullptr;
     size_t ends_bytes = 0;
@@ -100,6 +106,9 @@ struct SpreadScratch {
     int* bucket_list = nullptr;
     int bucket_slabs = 0;
     unsigned* max_abs_force = nullptr;
+    int clear = 0;       // counts that the next step kernel clears ...
+    bool clear_max = false;  // ... and the largest force
+    bool dirty = false;  // FP64: the buckets hold records that no step has taken
     bool valid = false;
     const void* owner = nullptr;          // the Swimmers moved
     unsigned long long owner_step = 0;    // its move counter after that move
@@ -257,8 +266,8 @@ struct EnsTable {
 };
 
 // Work items per block of the batched kernels (particles.cu checks them).
-constexpr int ENS_ENDS_PER_BLOCK = 256;
-constexpr int ENS_SWIMMERS_PER_BLOCK = 64;
+constexpr int ENS_ENDS_PER_BLOCK = 64;
+constexpr int ENS_SWIMMERS_PER_BLOCK = 32;
 constexpr int ENS_TRACERS_PER_BLOCK = 256;
 
 // Launches of the batched step (lattice.cu, particles.cu).
@@ -330,11 +339,17 @@ void swimmers_add_forces(Swimmers* S, Lattice* L);
 void swimmers_move(Swimmers* S, Lattice* L);
 // lbswim_system_step with one swimmer array: AddForces from the records the
 // last move prepared (false: nothing prepared that still holds), and the move
-// that prepares them for the next step.  epoch counts the API calls made.
+// that prepares them for the next step (swimmers_prepare_room before the step
+// between them).  epoch counts the API calls made.
 bool swimmers_add_forces_prepared(Swimmers* S, Lattice* L, unsigned long long epoch);
+void swimmers_prepare_room(Swimmers* S, Lattice* L);
 void swimmers_move_preparing(Swimmers* S, Lattice* L, unsigned long long epoch);
 // Wait on the host for the last kernel that used the swimmer arrays.
 void swimmers_wait(Swimmers* S);
+// Host copies (null: none) of the fields, after that kernel; waits for them.
+void swimmers_read(Swimmers* S, double* r, double* v, double* n);
+// Device address of a page-locked host buffer, null for pageable memory (lattice.cu).
+const void* mapped_host(const void* host);
 void tracers_move(Tracers* T, Lattice* L);
 // Move on the tracers' own stream after the point of the lattice stream where
 // L->hydro_ready was last recorded.

@@ -31,6 +31,11 @@ struct Dims {
   long long N;
 };
 
+// Sites along axis a, for a thread's own axis (no local copy of the array).
+__device__ __forceinline__ int dim_of(const Dims& D, int a) {
+  return a == 0 ? D.n[0] : (a == 1 ? D.n[1] : D.n[2]);
+}
+
 // acc + a b: FP64 rounds the product and the sum on their own (the oracle's
 // order, bit for bit); FP32 lets the compiler fuse them.
 template <class T>
@@ -292,7 +297,7 @@ __device__ __forceinline__ int node_after(int o, int j, int n) {
   return t;
 }
 
-constexpr int REC_THREADS = 256;
+constexpr int REC_ENDS = 64, REC_THREADS = 3 * REC_ENDS;  // records of a block
 
 // List end e under every tile of grid G whose extended region its stencil
 // touches (at most CAP ends are kept per tile; the count goes on).
@@ -302,88 +307,122 @@ __device__ __forceinline__ void bucket_end(int e, const int o[3], const Dims& D,
                                            int* __restrict__ list) {
   int f[3], c[3];
   for (int a = 0; a < 3; ++a) touched_range(o[a], D.n[a], G.by[a], G.h, G.nt[a], f[a], c[a]);
-  for (int i = 0; i < c[0]; ++i) {
+  auto tile = [&](int i, int j, int k) {
     const int kx = f[0] + i < G.nt[0] ? f[0] + i : f[0] + i - G.nt[0];
-    for (int j = 0; j < c[1]; ++j) {
-      const int ky = f[1] + j < G.nt[1] ? f[1] + j : f[1] + j - G.nt[1];
-      for (int k = 0; k < c[2]; ++k) {
-        const int kz = f[2] + k < G.nt[2] ? f[2] + k : f[2] + k - G.nt[2];
-        const int t = (kx * G.nt[1] + ky) * G.nt[2] + kz;
-        const unsigned slot = atomicAdd(count + t, 1u);
-        if (slot < (unsigned)CAP) list[(long long)t * CAP + slot] = e;
-      }
+    const int ky = f[1] + j < G.nt[1] ? f[1] + j : f[1] + j - G.nt[1];
+    const int kz = f[2] + k < G.nt[2] ? f[2] + k : f[2] + k - G.nt[2];
+    return (kx * G.nt[1] + ky) * G.nt[2] + kz;
+  };
+  // all of a pair of x tiles' counts in flight before the first is used
+  const bool pairs = c[1] <= 2 && c[2] <= 2;
+  for (int i0 = 0; i0 < c[0]; i0 += 2) {
+    if (pairs) {
+      unsigned slot[8];
+#pragma unroll
+      for (int q = 0; q < 8; ++q)
+        if (i0 + (q >> 2) < c[0] && ((q >> 1) & 1) < c[1] && (q & 1) < c[2])
+          slot[q] = atomicAdd(count + tile(i0 + (q >> 2), (q >> 1) & 1, q & 1), 1u);
+#pragma unroll
+      for (int q = 0; q < 8; ++q)
+        if (i0 + (q >> 2) < c[0] && ((q >> 1) & 1) < c[1] && (q & 1) < c[2] &&
+            slot[q] < (unsigned)CAP)
+          list[(long long)tile(i0 + (q >> 2), (q >> 1) & 1, q & 1) * CAP + slot[q]] = e;
+    } else {
+      for (int i = i0; i < min(i0 + 2, c[0]); ++i)
+        for (int j = 0; j < c[1]; ++j)
+          for (int k = 0; k < c[2]; ++k) {
+            const int t = tile(i, j, k);
+            const unsigned slot = atomicAdd(count + t, 1u);
+            if (slot < (unsigned)CAP) list[(long long)t * CAP + slot] = e;
+          }
     }
   }
 }
 
-// One record per dipole end: e = 2i is the tail, 2i + 1 the head.  Records are
-// assembled in shared memory and written out as one contiguous block; with
-// bucket_count set, each end is also listed under the step-kernel slabs it
-// touches (its index among all pending ends is e_base + e).  The stencil origin
-// comes from the bits of the position (stencil_axis) and the four weights from
-// one square root (peskin_weights4), like the FP32 interpolation.
-__device__ __forceinline__ void end_records_block(
-    int blk, int nsw, const double* __restrict__ r, const double* __restrict__ nv, double P,
-    double l, Dims D, EndRecord<float>* __restrict__ ends, int e_base,
-    unsigned* __restrict__ max_abs_f, TileGrid G, unsigned* __restrict__ bucket_count,
-    int* __restrict__ bucket_list) {
-  __shared__ EndRecord<float> srec[REC_THREADS];
+// Axis a of the FP32 record of one end (tail or head) of a swimmer at r with
+// orientation n; returns |F_a| as float bits.
+__device__ __forceinline__ unsigned record_axis32(double r, double n, bool head, double P,
+                                                  double l, const Dims& D, int a,
+                                                  EndRecord<float>& rec) {
+  const double x = head ? r : __dsub_rn(r, __dmul_rn(n, l));
+  double F = -P * n;
+  if (head) F *= -1.0;
+  int x0;
+  float dr;
+  stencil_axis(x, x0, dr);
+  rec.o[a] = wrap_any(x0, dim_of(D, a));
+  float w[4];
+  peskin_weights4(dr, w);
+#pragma unroll
+  for (int j = 0; j < 4; ++j) rec.phi[a][j] = w[j];
+  rec.F[a] = (float)F;
+  if (a == 0) rec.pad = 0;
+  return __float_as_uint(fmaxf(0.f, fabsf((float)F)));  // 0 for a NaN
+}
+
+// Where the end records of a swimmer array go: the records, the largest |F|, and
+// the buckets of the tiles of G.
+template <class T>
+struct RecordTarget {
+  EndRecord<T>* ends;
+  unsigned* max_f;
+  TileGrid G;
+  unsigned* count;
+  int* list;
+};
+
+// The rest of a block's records e0, e0 + 1, ... (REC_ENDS of them, thread (q, a) for
+// axis a of record q, a <= 2; ids offset by e_base): the largest force, the buckets
+// and the copy to global memory.  Every thread of the block calls it; smax is 0
+// before.  BUCKETS: the records may be listed in buckets.
+template <bool BUCKETS>
+__device__ __forceinline__ void finish_records32(int q, int a, int e0, int nends, int e_base,
+                                                 unsigned big, EndRecord<float>* srec,
+                                                 unsigned& smax, const Dims& D,
+                                                 const RecordTarget<float>& to) {
+  // non-negative floats order like their bit patterns: a warp's largest, then
+  // one shared-memory atomic per warp
+  big = __reduce_max_sync(0xffffffffu, big);
+  if ((threadIdx.x & 31) == 0 && big) atomicMax(&smax, big);
+  __syncthreads();
+  if (BUCKETS && a == 0 && e0 + q < nends && to.count)
+    bucket_end<SLAB_BUCKET_CAP>(e_base + e0 + q, srec[q].o, D, to.G, to.count, to.list);
+  if (threadIdx.x == 0) atomicMax(to.max_f, smax);
+  const int words = min(REC_ENDS, nends - e0) * (int)(sizeof(EndRecord<float>) / 4);
+  const unsigned* src = reinterpret_cast<const unsigned*>(srec);
+  unsigned* dst = reinterpret_cast<unsigned*>(to.ends + e0);
+  for (int w = threadIdx.x; w < words; w += blockDim.x) dst[w] = src[w];
+}
+
+// One record per dipole end: e = 2i is the tail, 2i + 1 the head; a thread per
+// (end, axis).  Records are assembled in shared memory and written out as one
+// contiguous block.  The stencil origin comes from the bits of the position
+// (stencil_axis) and the four weights from one square root (peskin_weights4),
+// like the FP32 interpolation.
+__device__ __forceinline__ void end_records_block(int blk, int nsw, const double* __restrict__ r,
+                                                  const double* __restrict__ nv, double P,
+                                                  double l, const Dims& D, int e_base,
+                                                  const RecordTarget<float>& to) {
+  __shared__ EndRecord<float> srec[REC_ENDS];
   __shared__ unsigned smax;
   if (threadIdx.x == 0) smax = 0u;
   __syncthreads();
-  const int e0 = blk * REC_THREADS;
-  const int e = e0 + threadIdx.x;
-  const int nends = 2 * nsw;
-  unsigned mbits = 0u;  // largest |F| component of this thread's end, as float bits
+  const int q = threadIdx.x % REC_ENDS, a = threadIdx.x / REC_ENDS;
+  const int e0 = blk * REC_ENDS, e = e0 + q, nends = 2 * nsw;
+  unsigned big = 0u;
   if (e < nends) {
-    const int i = e >> 1;
-    const bool head = e & 1;
-    double rr[3], F[3];
-    for (int a = 0; a < 3; ++a) {
-      const double na = nv[nsw * a + i];
-      rr[a] = head ? r[nsw * a + i] : __dsub_rn(r[nsw * a + i], __dmul_rn(na, l));
-      F[a] = -P * na;
-      if (head) F[a] *= -1.0;
-    }
-    EndRecord<float>& rec = srec[threadIdx.x];
-    for (int a = 0; a < 3; ++a) {
-      int x0;
-      float dr;
-      stencil_axis(rr[a], x0, dr);
-      rec.o[a] = wrap_any(x0, D.n[a]);
-      float w[4];
-      peskin_weights4(dr, w);
-#pragma unroll
-      for (int j = 0; j < 4; ++j) rec.phi[a][j] = w[j];
-    }
-    rec.pad = 0;
-    float m = 0.f;
-    for (int a = 0; a < 3; ++a) {
-      rec.F[a] = (float)F[a];
-      m = fmaxf(m, fabsf((float)F[a]));
-    }
-    mbits = __float_as_uint(m);
-    if (bucket_count) bucket_end<SLAB_BUCKET_CAP>(e_base + e, rec.o, D, G, bucket_count, bucket_list);
+    const long long at = (long long)nsw * a + (e >> 1);
+    big = record_axis32(r[at], nv[at], e & 1, P, l, D, a, srec[q]);
   }
-  // non-negative floats order like their bit patterns: a warp's largest, then
-  // one shared-memory atomic per warp
-  mbits = __reduce_max_sync(0xffffffffu, mbits);
-  if ((threadIdx.x & 31) == 0 && mbits) atomicMax(&smax, mbits);
-  __syncthreads();
-  if (threadIdx.x == 0 && max_abs_f) atomicMax(max_abs_f, smax);
-  const int nrec = min(REC_THREADS, nends - e0);
-  const int words = nrec * (int)(sizeof(EndRecord<float>) / 4);
-  const unsigned* src = reinterpret_cast<const unsigned*>(srec);
-  unsigned* dst = reinterpret_cast<unsigned*>(ends + e0);
-  for (int w = threadIdx.x; w < words; w += REC_THREADS) dst[w] = src[w];
+  finish_records32<true>(q, a, e0, nends, e_base, big, srec, smax, D, to);
 }
 
-__global__ void __launch_bounds__(REC_THREADS) k_end_records(
-    int nsw, const double* __restrict__ r, const double* __restrict__ nv, double P, double l,
-    Dims D, EndRecord<float>* __restrict__ ends, int e_base, unsigned* __restrict__ max_abs_f,
-    TileGrid G, unsigned* __restrict__ bucket_count, int* __restrict__ bucket_list) {
-  end_records_block(blockIdx.x, nsw, r, nv, P, l, D, ends, e_base, max_abs_f, G, bucket_count,
-                       bucket_list);
+__global__ void __launch_bounds__(REC_THREADS) k_end_records(int nsw,
+                                                             const double* __restrict__ r,
+                                                             const double* __restrict__ nv,
+                                                             double P, double l, Dims D,
+                                                             int e_base, RecordTarget<float> to) {
+  end_records_block(blockIdx.x, nsw, r, nv, P, l, D, e_base, to);
 }
 
 // Slab buckets of recorded ends (the slab shape changed since they were recorded).
@@ -463,12 +502,70 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan_apply_total(
 //    with most, on the narrow FP64 pipe.
 constexpr int FT_X = 4, FT_Y = 8, FT_Z = 32, FT_THREADS = 256, FT_CAP = 256;
 
-// One thread per (end, axis), 64 ends per block: the axes' chains of FP64
-// operations run side by side.  e = 2i is the tail, 2i + 1 the head.  FIXED:
-// the weights are integers in units of 2^-63 (fixed_weights4) in place of
-// doubles, and *max_f takes the largest high word of |F|; otherwise they are
-// the reference's delta per node.
+// Axis a of the record of an end (tail or head) of a swimmer at r, n.  FIXED: the
+// weights are integers in units of 2^-63 (fixed_weights4) in place of doubles, the
+// result is the high word of |F|, and `lost` is set when the coordinate is not a
+// number; otherwise they are the reference's delta per node.
+template <bool FIXED>
+__device__ __forceinline__ unsigned record_axis64(double r, double n, bool head, double P,
+                                                  double l, const Dims& D, int a,
+                                                  EndRecord<double>& rec, unsigned& lost) {
+  const double x = head ? r : __dsub_rn(r, __dmul_rn(n, l));
+  double F = -P * n;
+  if (head) F *= -1.0;
+  const double x0 = ceil(x - 2.);
+  rec.o[a] = wrap_any((int)x0, dim_of(D, a));
+  rec.F[a] = F;
+  if (!FIXED) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) rec.phi[a][j] = peskin_delta<double>(x - (x0 + j));
+    return 0u;
+  }
+  long long w[4];
+  const double dr = x - x0;
+  if (dr >= 1.0 && dr <= 2.0) {
+    fixed_weights4(dr, w);
+  } else {  // a coordinate beyond 2^52, or not a number
+    for (int j = 0; j < 4; ++j) w[j] = (long long)(peskin_delta<double>(x - (x0 + j)) * 0x1p63);
+    if (!(dr >= -4.0 && dr <= 4.0)) lost = 1u;
+  }
+#pragma unroll
+  for (int j = 0; j < 4; ++j) rec.phi[a][j] = bits_double((unsigned long long)w[j]);
+  return hi_word(double_bits(F)) & 0x7fffffffu;
+}
+
+// The rest of a block's records e0, e0 + 1, ... (REC64_ENDS of them, thread (q, a)
+// for axis a of record q, a <= 2): the force of lost ends, the largest force, the
+// buckets and the copy to global memory.  Every thread of the block calls it.
 constexpr int REC64_ENDS = 64, REC64_THREADS = 3 * REC64_ENDS;
+template <bool FIXED, bool BUCKETS>
+__device__ __forceinline__ void finish_records64(int q, int a, int e0, int nends, unsigned big,
+                                                 EndRecord<double>* srec, const unsigned* lost,
+                                                 unsigned& smax, const Dims& D,
+                                                 const RecordTarget<double>& to) {
+  if (FIXED) {
+    big = __reduce_max_sync(0xffffffffu, big);
+    if ((threadIdx.x & 31) == 0 && big) atomicMax(&smax, big);
+  }
+  __syncthreads();
+  if (a == 0 && e0 + q < nends) {
+    if (FIXED && lost[q]) {  // the force of a lost end is not a number
+      for (int c = 0; c < 3; ++c) srec[q].F[c] = bits_double(0x7ff8000000000000ull);
+      atomicMax(to.max_f, 0x7ff80000u);
+    }
+    if (BUCKETS && to.count) bucket_end<FT_CAP>(e0 + q, srec[q].o, D, to.G, to.count, to.list);
+  }
+  if (FIXED && threadIdx.x == 0) atomicMax(to.max_f, smax);
+  __syncthreads();
+  const int words = min(REC64_ENDS, nends - e0) * (int)(sizeof(EndRecord<double>) / 8);
+  const unsigned long long* src = reinterpret_cast<const unsigned long long*>(srec);
+  unsigned long long* dst = reinterpret_cast<unsigned long long*>(to.ends + e0);
+  for (int w = threadIdx.x; w < words; w += blockDim.x) dst[w] = src[w];
+}
+
+// One thread per (end, axis), 64 ends per block: the axes' chains of FP64
+// operations run side by side.  e = 2i is the tail, 2i + 1 the head.  FIXED
+// (record_axis64): *max_f takes the largest high word of |F|.
 template <bool FIXED>
 __global__ void __launch_bounds__(REC64_THREADS) k_end_records_f64(
     int nsw, const double* __restrict__ r, const double* __restrict__ nv, double P, double l,
@@ -486,49 +583,11 @@ __global__ void __launch_bounds__(REC64_THREADS) k_end_records_f64(
     const int i = e >> 1;
     const bool head = e & 1;
     const double na = nv[(long long)nsw * a + i], ra = r[(long long)nsw * a + i];
-    const double x = head ? ra : __dsub_rn(ra, __dmul_rn(na, l));
-    double F = -P * na;
-    if (head) F *= -1.0;
-    const double x0 = ceil(x - 2.);
-    EndRecord<double>& rec = srec[q];
-    rec.o[a] = wrap_any((int)x0, D.n[a]);
-    if (FIXED) {
-      long long w[4];
-      const double dr = x - x0;
-      if (dr >= 1.0 && dr <= 2.0) {
-        fixed_weights4(dr, w);
-      } else {  // a coordinate beyond 2^52, or not a number
-        for (int j = 0; j < 4; ++j) w[j] = (long long)(peskin_delta<double>(x - (x0 + j)) * 0x1p63);
-        if (!(dr >= -4.0 && dr <= 4.0)) lost[q] = 1u;
-      }
-#pragma unroll
-      for (int j = 0; j < 4; ++j) rec.phi[a][j] = bits_double((unsigned long long)w[j]);
-      big = hi_word(double_bits(F)) & 0x7fffffffu;
-    } else {
-#pragma unroll
-      for (int j = 0; j < 4; ++j) rec.phi[a][j] = peskin_delta<double>(x - (x0 + j));
-    }
-    rec.F[a] = F;
-    if (a == 0) rec.pad = 0;
+    big = record_axis64<FIXED>(ra, na, head, P, l, D, a, srec[q], lost[q]);
+    if (a == 0) srec[q].pad = 0;
   }
-  if (FIXED) {
-    big = __reduce_max_sync(0xffffffffu, big);
-    if ((threadIdx.x & 31) == 0 && big) atomicMax(&smax, big);
-  }
-  __syncthreads();
-  if (a == 0 && e < nends) {
-    if (FIXED && lost[q]) {  // the force of a lost end is not a number
-      for (int c = 0; c < 3; ++c) srec[q].F[c] = bits_double(0x7ff8000000000000ull);
-      atomicMax(max_f, 0x7ff80000u);
-    }
-    if (bucket_count) bucket_end<FT_CAP>(e, srec[q].o, D, G, bucket_count, bucket_list);
-  }
-  if (FIXED && threadIdx.x == 0) atomicMax(max_f, smax);
-  __syncthreads();
-  const int words = min(REC64_ENDS, nends - e0) * (int)(sizeof(EndRecord<double>) / 8);
-  const unsigned long long* src = reinterpret_cast<const unsigned long long*>(srec);
-  unsigned long long* dst = reinterpret_cast<unsigned long long*>(ends + e0);
-  for (int w = threadIdx.x; w < words; w += REC64_THREADS) dst[w] = src[w];
+  finish_records64<FIXED, true>(q, a, e0, nends, big, srec, lost, smax, D,
+                          RecordTarget<double>{ends, max_f, G, bucket_count, bucket_list});
 }
 static_assert(sizeof(EndRecord<double>) % 8 == 0, "records are copied as 64-bit words");
 
@@ -675,7 +734,8 @@ __global__ void __launch_bounds__(FT_THREADS) k_force_fixed(
   __shared__ int org[3][FF_CHUNK];
   const int tile = blockIdx.x, tid = threadIdx.x;
   const int kz = tile % G.nt[2], ky = (tile / G.nt[2]) % G.nt[1], kx = tile / (G.nt[1] * G.nt[2]);
-  const unsigned listed = count[tile];
+  // without buckets (DIRECT_ENDS_F64 ends at most) a tile goes through all of them
+  const unsigned listed = count ? count[tile] : (unsigned)nends;
   const unsigned fmax = *max_f;
   const int kf = (int)(fmax >> 20);  // |F| < 2^(kf - 1022)
   const int cnt = fmax ? (int)listed : 0;  // no force at all: nothing to add
@@ -684,7 +744,7 @@ __global__ void __launch_bounds__(FT_THREADS) k_force_fixed(
   for (int a = 0; a < 3; ++a) fold *= D.n[a] >= 4 ? 1 : (D.n[a] == 1 ? 4 : 2);
   __syncthreads();
   if (tid == 0) {
-    count[tile] = 0u;  // every thread has read it
+    if (count) count[tile] = 0u;  // every thread has read it
     if (tile == 0) *next_max_f = 0u;
   }
   const int z0 = kz * FT_Z, y0 = ky * FT_Y, x0 = kx * FT_X;
@@ -717,7 +777,7 @@ __global__ void __launch_bounds__(FT_THREADS) k_force_fixed(
     for (int t = tid; t < 18 * FF_CHUNK; t += FT_THREADS) {
       const int q = t % FF_CHUNK, w = t / FF_CHUNK;
       if (q >= m) continue;
-      const EndRecord<double>& e = ends[list[s0 + base + q]];
+      const EndRecord<double>& e = ends[count ? list[s0 + base + q] : base + q];
       if (w < 12) {
         dig[w][q] = digits((long long)double_bits(e.phi[w >> 2][w & 3]));
       } else if (w < 15) {
@@ -955,7 +1015,7 @@ struct Stencil64 {
 // Weights and wrapped origin of coordinate x of point p on axis a.
 __device__ __forceinline__ void point_axis64(const Dims& D, double x, int a, int p, Stencil64& st) {
   const double x0 = ceil(x - 2.);
-  st.o[a][p] = wrap_any((int)x0, D.n[a]);
+  st.o[a][p] = wrap_any((int)x0, dim_of(D, a));
   const double dr = x - x0;
   long long w[4];
   if (dr >= 1.0 && dr <= 2.0) {
@@ -1072,20 +1132,23 @@ __global__ void __launch_bounds__(MOVE64_BLOCK, 3) k_tracers_move_f64(
   if (!valid) return;
   const double w = st.vel[a][p];
   v[at] = w;
-  r[at] = wrap_position(x + w, D.n[a], status);
+  r[at] = wrap_position(x + w, dim_of(D, a), status);
   s[at] = sa + w;
 }
 
 // Points [0, 32) of a block are the swimmers, [32, 64) their rear points r - l n;
 // the threads (p < 32, axis) update them.
+// RECORD: the block then records the ends of the moved swimmers into `to`, for
+// the next step (thread (p, a): axis a of the tail, p < 32, or head of swimmer p % 32).
 constexpr int MOVE64_SWIMMERS = MOVE64_POINTS / 2;
-template <class I>
+static_assert(2 * MOVE64_SWIMMERS == REC64_ENDS, "the ends of a block's swimmers");
+template <bool RECORD, class I>
 __global__ void __launch_bounds__(MOVE64_BLOCK, 3) k_swimmers_move_f64(
     int nsw, double* __restrict__ swr, double* __restrict__ swv, double* __restrict__ swn,
     lbswim_common_params c, unsigned long long seed, unsigned long long step, Dims D,
-    const double* __restrict__ u, unsigned* status) {
+    const double* __restrict__ u, unsigned* status, RecordTarget<double> to) {
   __shared__ Stencil64 st;
-  __shared__ double turned[3][MOVE64_SWIMMERS];
+  __shared__ double turned[3][MOVE64_SWIMMERS], moved[3][MOVE64_SWIMMERS];
   const int p = threadIdx.x % MOVE64_POINTS, a = threadIdx.x / MOVE64_POINTS;
   const int q = p % MOVE64_SWIMMERS, i = blockIdx.x * MOVE64_SWIMMERS + q;
   const long long at = (long long)nsw * a + i;
@@ -1107,7 +1170,9 @@ __global__ void __launch_bounds__(MOVE64_BLOCK, 3) k_swimmers_move_f64(
     double rDot = __dmul_rn(__dmul_rn(c.mobility, c.P), na);
     if (!c.translational_advection_off) rDot = __dadd_rn(rDot, va);
     swv[at] = rDot;
-    swr[at] = wrap_position(__dadd_rn(x, rDot), D.n[a], status);
+    const double xn = wrap_position(__dadd_rn(x, rDot), dim_of(D, a), status);
+    swr[at] = xn;
+    moved[a][q] = xn;
     if (tumble) {  // a direction uniform on the sphere
       double g[3];
       rng_normal3(seed, (uint32_t)i, step, g);
@@ -1117,11 +1182,30 @@ __global__ void __launch_bounds__(MOVE64_BLOCK, 3) k_swimmers_move_f64(
     }
   }
   __syncthreads();
-  if (!update || (!tumble && c.rotational_advection_off)) return;  // orientation unchanged
-  const double nx = turned[0][q], ny = turned[1][q], nz = turned[2][q];
-  const double norm =
-      __dsqrt_rn(__dadd_rn(__dadd_rn(__dmul_rn(nx, nx), __dmul_rn(ny, ny)), __dmul_rn(nz, nz)));
-  swn[at] = turned[a][q] / norm;
+  double nn = na;
+  if (update && (tumble || !c.rotational_advection_off)) {  // else the orientation is unchanged
+    const double nx = turned[0][q], ny = turned[1][q], nz = turned[2][q];
+    const double norm =
+        __dsqrt_rn(__dadd_rn(__dadd_rn(__dmul_rn(nx, nx), __dmul_rn(ny, ny)), __dmul_rn(nz, nz)));
+    nn = turned[a][q] / norm;
+    swn[at] = nn;
+  }
+  if constexpr (RECORD) {
+    __shared__ EndRecord<double> srec[REC64_ENDS];
+    __shared__ unsigned smax, lost[REC64_ENDS];
+    if (threadIdx.x == 0) smax = 0u;
+    if (a == 0) lost[p] = 0u;
+    __syncthreads();  // every axis of a swimmer has been normalised
+    if (update) turned[a][q] = nn;
+    __syncthreads();
+    const int e = 2 * q + (rear ? 1 : 0);  // of the block
+    unsigned big = 0u;
+    if (valid) {
+      big = record_axis64<true>(moved[a][q], turned[a][q], rear, c.P, c.l, D, a, srec[e], lost[e]);
+      if (a == 0) srec[e].pad = 0;
+    }
+    finish_records64<true, false>(e, a, blockIdx.x * REC64_ENDS, 2 * nsw, big, srec, lost, smax, D, to);
+  }
 }
 
 template <class U, class T>
@@ -1196,23 +1280,26 @@ __global__ void k_init_particles(int n, unsigned long long seed, Dims D, double*
 }
 
 // ---- FP32-path Move kernels ------------------------------------------------------
-// A block moves NP particles in three phases.  (1) One thread per particle forms
-// its stencil -- wrapped origin node and Peskin weights -- in shared memory.
-// (2) A group of 4 (or 8, 16) threads per interpolation point gathers the 4^3
-// nodes, lane k taking z node k & 3, and the partial sums are added with a
-// fixed shuffle tree, so the result does not depend on scheduling.  (3) One
-// thread per particle updates it.  GB300's FP64 pipe is narrow: the stencil
-// origin comes from the bits of the position by integer operations, positions
-// advance in Q44 fixed point, and orientations update in FP32.
+// A block interpolates 64 points in three phases.  (1) A thread per (point, axis)
+// forms the wrapped origin node and the Peskin weights in shared memory.  (2) Four
+// lanes per point, one per z node, gather its 4^3 nodes, and the partial sums are
+// added with a fixed shuffle tree, so the result does not depend on scheduling.
+// (3) A thread per (particle, axis) updates it.  GB300's FP64 pipe is narrow: the
+// stencil origin comes from the bits of the position by integer operations,
+// positions advance in Q44 fixed point, and orientations update in FP32.  With a
+// thread per particle in phases 1 and 3 a small array waited for one warp's chain
+// of three axes (and two points): 54 swimmers 11 -> 7 us, 3809 11.6 -> 7.9,
+// 65,536 the same.
+constexpr int MOVE_BLOCK = 256, MOVE_POINTS = MOVE_BLOCK / 4;
 
-// Stencils of NP interpolation points in shared memory, one array per field so
-// that one thread per point writes them without bank conflicts: wrapped origin
-// node, whether the point is gathered, Peskin weights per axis and node.
-template <int NP>
+// Stencils of a block's points, one array per field so that neighbouring threads
+// write them without bank conflicts: wrapped origin node, Peskin weights per axis
+// and node, whether the point is gathered, and its velocity.
 struct StencilSet {
-  int o[3][NP];
-  int active[NP];
-  float w[3][4][NP];
+  int o[3][MOVE_POINTS];
+  int active[MOVE_POINTS];
+  float w[3][4][MOVE_POINTS];
+  float vel[3][MOVE_POINTS];
 };
 
 // Exact FP64 value of a float, from its bits (no FP64 instruction).
@@ -1331,9 +1418,117 @@ __device__ __forceinline__ void rng_normal3_f(uint64_t seed, uint32_t swimmer, u
   g[2] = r2 * c2;
 }
 
-template <int NP>
-__device__ __forceinline__ void point_stencil(const Dims& D, const double r[3],
-                                              StencilSet<NP>& st, int p) {
+// Axis a of the stencil of point p at coordinate x.
+__device__ __forceinline__ void point_axis(const Dims& D, double x, int a, int p, StencilSet& st) {
+  int x0;
+  float dr;
+  stencil_axis(x, x0, dr);
+  st.o[a][p] = wrap_any(x0, dim_of(D, a));
+  float w[4];
+  peskin_weights4(dr, w);
+#pragma unroll
+  for (int j = 0; j < 4; ++j) st.w[a][j][p] = w[j];
+}
+
+// Lane k of a point's four takes z node k for the four y and x nodes.  I is the type
+// of the site offsets: int while N < 2^31.
+template <class Set, class I>
+__device__ __forceinline__ float3 gather_point(const float4* __restrict__ h, const Dims& D,
+                                               const Set& st, int p, int k) {
+  float vx = 0.f, vy = 0.f, vz = 0.f;
+  if (st.active[p]) {
+    const int nz = D.n[2];
+    const I nynz = (I)D.n[1] * D.n[2];
+    const int z = node_after(st.o[2][p], k, nz);
+    const float wz = st.w[2][k][p];
+    I xo[4];
+    float wx[4];
+#pragma unroll
+    for (int ix = 0; ix < 4; ++ix) {
+      xo[ix] = (I)node_after(st.o[0][p], ix, D.n[0]) * nynz;
+      wx[ix] = st.w[0][ix][p];
+    }
+#pragma unroll
+    for (int jy = 0; jy < 4; ++jy) {
+      const I yz = (I)node_after(st.o[1][p], jy, D.n[1]) * nz + z;
+      const float wyz = st.w[1][jy][p] * wz;
+#pragma unroll
+      for (int ix = 0; ix < 4; ++ix) {
+        const float4 q = __ldg(h + xo[ix] + yz);
+        const float w = wx[ix] * wyz;
+        vx += w * q.x;
+        vy += w * q.y;
+        vz += w * q.z;
+      }
+    }
+  }
+  return make_float3(vx, vy, vz);
+}
+// Sum over a point's four lanes (fixed shuffle tree).
+__device__ __forceinline__ float3 sum_lanes(float3 v) {
+#pragma unroll
+  for (int off = 2; off > 0; off >>= 1) {
+    v.x += __shfl_xor_sync(0xffffffffu, v.x, off);
+    v.y += __shfl_xor_sync(0xffffffffu, v.y, off);
+    v.z += __shfl_xor_sync(0xffffffffu, v.z, off);
+  }
+  return v;
+}
+
+// Phase 2 for a block's 64 points.
+template <class I>
+__device__ __forceinline__ void gather_points(const float4* __restrict__ h, const Dims& D,
+                                              StencilSet& st) {
+  const int p = threadIdx.x >> 2, k = threadIdx.x & 3;
+  const float3 v = sum_lanes(gather_point<StencilSet, I>(h, D, st, p, k));
+  if (k < 3) st.vel[k][p] = k == 0 ? v.x : (k == 1 ? v.y : v.z);
+}
+
+template <class I>
+__device__ __forceinline__ void tracers_move_block(int blk, int ntr, double* __restrict__ r,
+                                                   double* __restrict__ s,
+                                                   double* __restrict__ v, Dims D,
+                                                   const float4* __restrict__ h,
+                                                   unsigned* status) {
+  __shared__ StencilSet st;
+  const int p = threadIdx.x % MOVE_POINTS, a = threadIdx.x / MOVE_POINTS;
+  const int i = blk * MOVE_POINTS + p;
+  const long long at = (long long)ntr * a + i;
+  const bool valid = a < 3 && i < ntr;
+  // s is read with r, so the update at the end waits on no load of its own
+  double x = 0.0, sa = 0.0;
+  if (valid) {
+    x = r[at];
+    sa = s[at];
+    point_axis(D, x, a, p, st);
+  }
+  if (a == 3) st.active[p] = i < ntr;
+  __syncthreads();
+  gather_points<I>(h, D, st);
+  __syncthreads();
+  if (!valid) return;
+  const float w = st.vel[a][p];
+  const double vd = f2d_exact(w);
+  v[at] = vd;
+  r[at] = advance_position(x, w, dim_of(D, a), status);
+  s[at] = sa + vd;
+}
+
+// Large tracer arrays: a block takes 256 tracers, a thread forms the stencil of one
+// (all axes) and updates it, and four lanes gather two points at a time.  With
+// twice the loads in flight per thread 1,048,576 tracers take 118 us against 146 with
+// 64 per block; 60,938 take 15.6 us against 13.3, and 864 11 us against 5.4.
+constexpr int WIDE_TRACERS = 256;
+struct WideStencilSet {
+  int o[3][WIDE_TRACERS];
+  int active[WIDE_TRACERS];
+  float w[3][4][WIDE_TRACERS];
+  float3 vel[WIDE_TRACERS];
+};
+constexpr int TRACERS_WIDE_FROM = 65536;
+
+__device__ __forceinline__ void wide_stencil(const Dims& D, const double r[3],
+                                             WideStencilSet& st, int p) {
   float dr[3];
   for (int d = 0; d < 3; ++d) {
     int x0;
@@ -1350,103 +1545,39 @@ __device__ __forceinline__ void point_stencil(const Dims& D, const double r[3],
   }
 }
 
-// Sum over the L lanes of a point's group (fixed shuffle tree).
-template <int L>
-__device__ __forceinline__ void reduce_lanes(float& vx, float& vy, float& vz) {
-#pragma unroll
-  for (int off = L / 2; off > 0; off >>= 1) {
-    vx += __shfl_xor_sync(0xffffffffu, vx, off);
-    vy += __shfl_xor_sync(0xffffffffu, vy, off);
-    vz += __shfl_xor_sync(0xffffffffu, vz, off);
-  }
-}
-
-// Lane `sub` of the L lanes (4, 8 or 16) of a point gathers z node sub & 3 of
-// y nodes sub >> 2, sub >> 2 + L / 4, ... for the four x nodes.  I is the type
-// of the site offsets: int while N < 2^31.
-template <int L, int NP, class I = int>
-__device__ __forceinline__ void gather_point(const float4* __restrict__ h, const Dims& D,
-                                             const StencilSet<NP>& s, int p, int sub,
-                                             float& vx, float& vy, float& vz) {
-  vx = vy = vz = 0.f;
-  if (!s.active[p]) return;
-  const int nz = D.n[2];
-  const I nynz = (I)D.n[1] * D.n[2];
-  const int kz = sub & 3;
-  const int z = node_after(s.o[2][p], kz, nz);
-  const float wz = s.w[2][kz][p];
-  I xo[4];
-  float wx[4];
-#pragma unroll
-  for (int ix = 0; ix < 4; ++ix) {
-    xo[ix] = (I)node_after(s.o[0][p], ix, D.n[0]) * nynz;
-    wx[ix] = s.w[0][ix][p];
-  }
-#pragma unroll
-  for (int jy = sub >> 2; jy < 4; jy += L / 4) {
-    const I yz = (I)node_after(s.o[1][p], jy, D.n[1]) * nz + z;
-    const float wyz = s.w[1][jy][p] * wz;
-#pragma unroll
-    for (int ix = 0; ix < 4; ++ix) {
-      const float4 q = __ldg(h + xo[ix] + yz);
-      const float w = wx[ix] * wyz;
-      vx += w * q.x;
-      vy += w * q.y;
-      vz += w * q.z;
-    }
-  }
-}
-
-// Phase 2: the block's threads, L per point and two points per group at a
-// time, gather the velocity of the NP stencils.  Every thread runs the same
-// number of iterations (NP * L is a multiple of 2 * blockDim).
-template <int L, int NP, class I = int>
-__device__ __forceinline__ void gather_block(const float4* __restrict__ h, const Dims& D,
-                                             const StencilSet<NP>& st, float3* vel) {
-  const int sub = threadIdx.x & (L - 1);
-  const int groups = blockDim.x / L;
-  for (int p = threadIdx.x / L; p < NP; p += 2 * groups) {
-    float ax, ay, az, bx, by, bz;
-    gather_point<L, NP, I>(h, D, st, p, sub, ax, ay, az);
-    gather_point<L, NP, I>(h, D, st, p + groups, sub, bx, by, bz);
-    reduce_lanes<L>(ax, ay, az);
-    reduce_lanes<L>(bx, by, bz);
-    if (sub == 0) {
-      vel[p] = make_float3(ax, ay, az);
-      vel[p + groups] = make_float3(bx, by, bz);
-    }
-  }
-}
-
-constexpr int TRACER_MOVE_BLOCK = 256;
-constexpr int TRACER_LANES = 4;  // lanes per interpolation point
-
 template <class I = int>
-__device__ __forceinline__ void tracers_move_block(int blk, int ntr, double* __restrict__ r,
-                                                   double* __restrict__ s,
-                                                   double* __restrict__ v, Dims D,
-                                                   const float4* __restrict__ h,
-                                                   unsigned* status) {
-  __shared__ StencilSet<TRACER_MOVE_BLOCK> st;
-  __shared__ float3 vel[TRACER_MOVE_BLOCK];
-  const int i = blk * TRACER_MOVE_BLOCK + threadIdx.x;
+__device__ __forceinline__ void tracers_move_wide_block(int blk, int ntr, double* __restrict__ r,
+                                                        double* __restrict__ s,
+                                                        double* __restrict__ v, const Dims& D,
+                                                        const float4* __restrict__ h,
+                                                        unsigned* status) {
+  __shared__ WideStencilSet st;
+  const int i = blk * WIDE_TRACERS + threadIdx.x;
   const bool valid = i < ntr;
-  // s is read with r, so the update at the end waits on no load of its own
   double rr[3] = {0.0, 0.0, 0.0}, ss[3] = {0.0, 0.0, 0.0};
   if (valid) {
     for (int d = 0; d < 3; ++d) {
       rr[d] = r[(long long)ntr * d + i];
       ss[d] = s[(long long)ntr * d + i];
     }
-    point_stencil(D, rr, st, threadIdx.x);
+    wide_stencil(D, rr, st, threadIdx.x);
   } else {
     st.active[threadIdx.x] = 0;
   }
   __syncthreads();
-  gather_block<TRACER_LANES, TRACER_MOVE_BLOCK, I>(h, D, st, vel);
+  const int k = threadIdx.x & 3;
+  for (int p = threadIdx.x >> 2; p < WIDE_TRACERS; p += 2 * MOVE_POINTS) {
+    const float3 a = gather_point<WideStencilSet, I>(h, D, st, p, k);
+    const float3 b = gather_point<WideStencilSet, I>(h, D, st, p + MOVE_POINTS, k);
+    const float3 sa = sum_lanes(a), sb = sum_lanes(b);
+    if (k == 0) {
+      st.vel[p] = sa;
+      st.vel[p + MOVE_POINTS] = sb;
+    }
+  }
   __syncthreads();
   if (!valid) return;
-  const float3 w = vel[threadIdx.x];
+  const float3 w = st.vel[threadIdx.x];
   const float vv[3] = {w.x, w.y, w.z};
   for (int d = 0; d < 3; ++d) {
     const double vd = f2d_exact(vv[d]);
@@ -1456,112 +1587,109 @@ __device__ __forceinline__ void tracers_move_block(int blk, int ntr, double* __r
   }
 }
 
-template <class I>
-__global__ void __launch_bounds__(TRACER_MOVE_BLOCK) k_tracers_move_f32(
+template <bool WIDE, class I>
+__global__ void __launch_bounds__(MOVE_BLOCK) k_tracers_move_f32(
     int ntr, double* __restrict__ r, double* __restrict__ s, double* __restrict__ v, Dims D,
     const float4* __restrict__ h, unsigned* status) {
-  tracers_move_block<I>(blockIdx.x, ntr, r, s, v, D, h, status);
+  if constexpr (WIDE)
+    tracers_move_wide_block<I>(blockIdx.x, ntr, r, s, v, D, h, status);
+  else
+    tracers_move_block<I>(blockIdx.x, ntr, r, s, v, D, h, status);
 }
 
-// A block takes SWIMMERS_PER_BLOCK swimmers: two stencils (front and rear
-// point) per swimmer, SWIMMER_LANES threads per stencil.
-constexpr int SWIMMERS_PER_BLOCK = 64;
-constexpr int SWIMMER_LANES = 4;  // lanes per interpolation point
-constexpr int SWIMMER_MOVE_BLOCK = SWIMMERS_PER_BLOCK * SWIMMER_LANES;
-
-// The update of swimmer i from the fluid velocity at its front point r (v)
-// and at its rear point r - l n (vm): SwimmerArray.cu:151-209, with the FP32
-// path's arithmetic (Q44 positions, FP32 turn added to the FP64 orientation,
-// FP32 tumble normals).
-__device__ __forceinline__ void swimmer_update(int i, int nsw, double* __restrict__ swr,
-                                               double* __restrict__ swv, double* __restrict__ swn,
-                                               const lbswim_common_params& c,
-                                               unsigned long long seed, unsigned long long step,
-                                               const Dims& D, const double r[3],
-                                               const double nd[3], bool tumble, bool rotate,
-                                               const float v[3], const float vm[3],
-                                               unsigned* status) {
-  const float mP = (float)(c.mobility * c.P);
-  for (int d = 0; d < 3; ++d) {
-    float rDot = mP * (float)nd[d];
-    if (!c.translational_advection_off) rDot += v[d];
-    swv[nsw * d + i] = f2d_exact(rDot);
-    swr[nsw * d + i] = advance_position(r[d], rDot, D.n[d], status);
-  }
-  if (tumble) {
-    float nn[3];
-    rng_normal3_f(seed, (uint32_t)i, step, nn);
-    const float inv = 1.f / sqrtf(nn[0] * nn[0] + nn[1] * nn[1] + nn[2] * nn[2]);
-    for (int d = 0; d < 3; ++d) swn[nsw * d + i] = f2d_exact(nn[d] * inv);
-  } else if (rotate) {
-    // the small turn (v - v_rear) / l is formed in FP32 and added to the FP64
-    // orientation, which keeps its direction; the FP32 norm only rescales it
-    const float inv_l = 1.f / (float)c.l;
-    double nn[3];
-    float sq = 0.f;
-    for (int d = 0; d < 3; ++d) {
-      nn[d] = __dadd_rn(nd[d], f2d_exact((v[d] - vm[d]) * inv_l));
-      const float q = (float)nn[d];
-      sq += q * q;
-    }
-    const double inv = f2d_exact(1.f / sqrtf(sq));
-    for (int d = 0; d < 3; ++d) swn[nsw * d + i] = __dmul_rn(nn[d], inv);
-  }
-}
-
-// The rear point r - l n of a swimmer, as the dipole-end records compute it.
-__device__ __forceinline__ void rear_point(const double r[3], const double nd[3], double l,
-                                           double out[3]) {
-  for (int d = 0; d < 3; ++d) out[d] = __dsub_rn(r[d], __dmul_rn(nd[d], l));
-}
-
-template <class I = int>
+// Points [0, 32) of a block are its swimmers, [32, 64) their rear points r - l n; the
+// threads (p < 32, axis) update them: SwimmerArray.cu:151-209 with the FP32 path's
+// arithmetic (Q44 positions, FP32 turn added to the FP64 orientation, FP32 tumble
+// normals).  RECORD: the block also records the ends of the moved swimmers into
+// `to`, for the next step (thread (p, a): axis a of the tail, p < 32, or head of
+// swimmer p % 32).
+constexpr int MOVE_SWIMMERS = MOVE_POINTS / 2;
+static_assert(2 * MOVE_SWIMMERS == REC_ENDS, "the ends of a block's swimmers");
+template <bool RECORD, class I = int>
 __device__ __forceinline__ void swimmers_move_block(
     int blk, int nsw, double* __restrict__ swr, double* __restrict__ swv,
-    double* __restrict__ swn, lbswim_common_params c, unsigned long long seed,
-    unsigned long long step, Dims D, const float4* __restrict__ h, unsigned* status) {
-  constexpr int B = SWIMMERS_PER_BLOCK;
-  // stencils [0, B) at the swimmers, [B, 2B) at their rear points r - l n
-  __shared__ StencilSet<2 * B> st;
-  __shared__ float3 vel[2 * B];
-  const int t = threadIdx.x, i = blk * B + t;
-  const bool mine = t < B, valid = mine && i < nsw;
-  double r[3] = {0.0, 0.0, 0.0}, nd[3] = {0.0, 0.0, 0.0};
-  bool tumble = false, rotate = false;
+    double* __restrict__ swn, const lbswim_common_params& c, unsigned long long seed,
+    unsigned long long step, const Dims& D, const float4* __restrict__ h, unsigned* status,
+    const RecordTarget<float>& to = RecordTarget<float>{}) {
+  __shared__ StencilSet st;
+  __shared__ float turned[3][MOVE_SWIMMERS];
+  const int p = threadIdx.x % MOVE_POINTS, a = threadIdx.x / MOVE_POINTS;
+  const int q = p % MOVE_SWIMMERS, i = blk * MOVE_SWIMMERS + q;
+  const long long at = (long long)nsw * a + i;
+  const bool rear = p >= MOVE_SWIMMERS, valid = a < 3 && i < nsw, update = valid && !rear;
+  double x = 0.0, na = 0.0;
   if (valid) {
-    double rMinus[3];
-    for (int d = 0; d < 3; ++d) {
-      r[d] = swr[nsw * d + i];
-      nd[d] = swn[nsw * d + i];
-    }
+    x = swr[at];
+    na = swn[at];
+  }
+  bool tumble = false, rotate = false;
+  if (i < nsw) {
     tumble = rng_uniform(seed, (uint32_t)i, step) < c.alpha;
     rotate = !tumble && !c.rotational_advection_off;
-    point_stencil(D, r, st, t);
-    if (rotate) {
-      rear_point(r, nd, c.l, rMinus);
-      point_stencil(D, rMinus, st, B + t);
-    } else {
-      st.active[B + t] = 0;
+  }
+  // the rear point as the dipole-end records compute it
+  if (valid && (!rear || rotate))
+    point_axis(D, rear ? __dsub_rn(x, __dmul_rn(na, c.l)) : x, a, p, st);
+  if (a == 3) st.active[p] = i < nsw && (!rear || rotate);
+  __syncthreads();
+  gather_points<I>(h, D, st);
+  __syncthreads();
+  double xn = 0.0, nn = na;
+  float inv = 0.f;
+  if (update) {
+    const float va = st.vel[a][q];
+    float rDot = (float)(c.mobility * c.P) * (float)na;
+    if (!c.translational_advection_off) rDot += va;
+    swv[at] = f2d_exact(rDot);
+    xn = advance_position(x, rDot, dim_of(D, a), status);
+    swr[at] = xn;
+    if (tumble) {
+      float g[3];
+      rng_normal3_f(seed, (uint32_t)i, step, g);
+      inv = 1.f / sqrtf(g[0] * g[0] + g[1] * g[1] + g[2] * g[2]);
+      nn = f2d_exact((a == 0 ? g[0] : (a == 1 ? g[1] : g[2])) * inv);
+    } else if (rotate) {
+      // the small turn (v - v_rear) / l is formed in FP32 and added to the FP64
+      // orientation, which keeps its direction; the FP32 norm only rescales it
+      const float inv_l = 1.f / (float)c.l;
+      nn = __dadd_rn(na, f2d_exact((va - st.vel[a][MOVE_SWIMMERS + q]) * inv_l));
+      turned[a][q] = (float)nn;
     }
-  } else if (mine) {
-    st.active[t] = 0;
-    st.active[B + t] = 0;
   }
   __syncthreads();
-  gather_block<SWIMMER_LANES, 2 * SWIMMERS_PER_BLOCK, I>(h, D, st, vel);
-  __syncthreads();
-  if (!valid) return;
-  const float3 w = vel[t], wm = vel[B + t];
-  const float v[3] = {w.x, w.y, w.z}, vm[3] = {wm.x, wm.y, wm.z};
-  swimmer_update(i, nsw, swr, swv, swn, c, seed, step, D, r, nd, tumble, rotate, v, vm, status);
+  if (update && rotate) {
+    const float tx = turned[0][q], ty = turned[1][q], tz = turned[2][q];
+    float sq = 0.f;
+    sq += tx * tx;
+    sq += ty * ty;
+    sq += tz * tz;
+    nn = __dmul_rn(nn, f2d_exact(1.f / sqrtf(sq)));
+  }
+  if (update && (tumble || rotate)) swn[at] = nn;
+  if constexpr (RECORD) {
+    __shared__ double moved[2][3][MOVE_SWIMMERS];
+    __shared__ EndRecord<float> srec[REC_ENDS];
+    __shared__ unsigned smax;
+    if (threadIdx.x == 0) smax = 0u;
+    if (update) {
+      moved[0][a][q] = xn;
+      moved[1][a][q] = nn;
+    }
+    __syncthreads();
+    const int e = 2 * q + (rear ? 1 : 0);  // of the block
+    unsigned big = 0u;
+    if (valid)
+      big = record_axis32(moved[0][a][q], moved[1][a][q], rear, c.P, c.l, D, a, srec[e]);
+    finish_records32<false>(e, a, blk * REC_ENDS, 2 * nsw, 0, big, srec, smax, D, to);
+  }
 }
 
-template <class I>
-__global__ void __launch_bounds__(SWIMMER_MOVE_BLOCK) k_swimmers_move_f32(
+template <bool RECORD, class I>
+__global__ void __launch_bounds__(MOVE_BLOCK) k_swimmers_move_f32(
     int nsw, double* __restrict__ swr, double* __restrict__ swv, double* __restrict__ swn,
     lbswim_common_params c, unsigned long long seed, unsigned long long step, Dims D,
-    const float4* __restrict__ h, unsigned* status) {
-  swimmers_move_block<I>(blockIdx.x, nsw, swr, swv, swn, c, seed, step, D, h, status);
+    const float4* __restrict__ h, unsigned* status, RecordTarget<float> to) {
+  swimmers_move_block<RECORD, I>(blockIdx.x, nsw, swr, swv, swn, c, seed, step, D, h, status, to);
 }
 
 // ---- batched ensembles: per-step reset, end records, moves --------------------
@@ -1624,19 +1752,19 @@ __global__ void __launch_bounds__(REC_THREADS) k_ens_records(EnsTable t) {
       G.nt[a] = M.nt[a];
       if (a) G.by[a] = FastDiv{1u, (unsigned)__ffs(G.T[a]) - 1u};  // powers of two
     }
-    end_records_block(vb - t.rec_prefix[m], M.nsw, M.sw_r, M.sw_n, M.common.P,
-                             M.common.l, ens_dims(M), (EndRecord<float>*)M.ends, 0, M.max_abs_f,
-                             G, M.bucket_count, M.bucket_list);
+    end_records_block(vb - t.rec_prefix[m], M.nsw, M.sw_r, M.sw_n, M.common.P, M.common.l,
+                      ens_dims(M), 0,
+                      RecordTarget<float>{(EndRecord<float>*)M.ends, M.max_abs_f, G,
+                                          M.bucket_count, M.bucket_list});
     __syncthreads();
   }
 }
 
-static_assert(SWIMMER_MOVE_BLOCK == TRACER_MOVE_BLOCK, "one block size for both moves");
-static_assert(ENS_ENDS_PER_BLOCK == REC_THREADS && ENS_SWIMMERS_PER_BLOCK == SWIMMERS_PER_BLOCK &&
-                  ENS_TRACERS_PER_BLOCK == TRACER_MOVE_BLOCK,
+static_assert(ENS_ENDS_PER_BLOCK == REC_ENDS && ENS_SWIMMERS_PER_BLOCK == MOVE_SWIMMERS &&
+                  ENS_TRACERS_PER_BLOCK == WIDE_TRACERS,
               "batched work items per block");
 
-__global__ void __launch_bounds__(TRACER_MOVE_BLOCK) k_ens_move(EnsTable t, int parity) {
+__global__ void __launch_bounds__(MOVE_BLOCK) k_ens_move(EnsTable t, int parity) {
   const int nmem = *t.nmem;
   const int nsb = t.sw_prefix[nmem], total = nsb + t.tr_prefix[nmem];
   const unsigned long long g = (unsigned long long)*t.g_step;
@@ -1645,13 +1773,13 @@ __global__ void __launch_bounds__(TRACER_MOVE_BLOCK) k_ens_move(EnsTable t, int 
       const int m = ens_find(t.sw_prefix, nmem, vb);
       const EnsMember& M = t.mem[m];
       if ((long long)g >= M.limit) continue;  // uniform in the block: no barrier skipped
-      swimmers_move_block(vb - t.sw_prefix[m], M.nsw, M.sw_r, M.sw_v, M.sw_n, M.common, M.seed,
+      swimmers_move_block<false>(vb - t.sw_prefix[m], M.nsw, M.sw_r, M.sw_v, M.sw_n, M.common, M.seed,
                           M.step0 + g, ens_dims(M), (const float4*)M.hyd[parity], M.status);
     } else {
       const int m = ens_find(t.tr_prefix, nmem, vb - nsb);
       const EnsMember& M = t.mem[m];
       if ((long long)g >= M.limit) continue;
-      tracers_move_block(vb - nsb - t.tr_prefix[m], M.ntr, M.tr_r, M.tr_s, M.tr_v, ens_dims(M),
+      tracers_move_wide_block(vb - nsb - t.tr_prefix[m], M.ntr, M.tr_r, M.tr_s, M.tr_v, ens_dims(M),
                          (const float4*)M.hyd[parity], M.status);
     }
     __syncthreads();
@@ -1668,7 +1796,7 @@ void ens_launch_records(const EnsTable& t, int grid, cudaStream_t s) {
   LB_CHECK_LAUNCH(1);
 }
 void ens_launch_move(const EnsTable& t, int parity, int grid, cudaStream_t s) {
-  k_ens_move<<<grid, TRACER_MOVE_BLOCK, 0, s>>>(t, parity);
+  k_ens_move<<<grid, MOVE_BLOCK, 0, s>>>(t, parity);
   LB_CHECK_LAUNCH(1);
 }
 
@@ -1682,6 +1810,8 @@ static Dims make_dims(const Lattice* L) {
   D.N = L->n;
   return D;
 }
+
+static int slabs_of(const TileGrid& G) { return G.nt[0] * G.nt[1] * G.nt[2]; }
 
 static TileGrid force_tiles(const Lattice* L) {
   TileGrid G;
@@ -1823,11 +1953,33 @@ static void ensure_tile_buckets(Lattice* L, int ntiles) {
   LB_CUDA(cudaMemsetAsync(count, 0, sizeof(unsigned) * (ntiles + 2), L->stream));
 }
 
-// force = base + the spread of W's dipole ends on an FP64 lattice.  Buckets
-// while the average tile lists at most half of one (each end touches 2.6 tiles
-// of 1024 sites on average): two launches in place of eight, which at 16^3 took
-// 36 us of device time together and take 13 us.  Denser suspensions list their
-// ends by a counting sort (k_force_tile orders long lists in global scratch).
+// Buckets while the average tile lists at most half of one (an end touches 2.6
+// tiles of 1024 sites on average).
+static bool tiles_take_buckets(const TileGrid& G, long long nends) {
+  return nends <= 48ll * G.nt[0] * G.nt[1] * G.nt[2];
+}
+
+// force = base + the spread of the nends ends recorded (and listed in buckets); the
+// two words for the largest force alternate.
+static void spread_fixed(Lattice* L, int nends) {
+  SpreadScratch& S = L->spread;
+  const TileGrid G = force_tiles(L);
+  const int ntiles = G.nt[0] * G.nt[1] * G.nt[2];
+  unsigned* max_f = S.bucket_count + ntiles;
+  k_force_fixed<<<ntiles, FT_THREADS, 0, L->stream>>>(
+      make_dims(L), G, (const EndRecord<double>*)S.ends, nends,
+      nends > DIRECT_ENDS_F64 ? S.bucket_count : nullptr, S.bucket_list,
+      max_f + S.max_slot, max_f + (S.max_slot ^ 1), (double*)L->force,
+      L->force_zero_pending ? 0 : 1);
+  LB_CHECK_LAUNCH(1);
+  S.max_slot ^= 1;
+  L->force_zero_pending = false;
+}
+
+// force = base + the spread of W's dipole ends on an FP64 lattice.  With buckets it
+// takes two launches in place of eight, which at 16^3 took 36 us of device time
+// together and take 13 us.  Denser suspensions list their ends by a counting
+// sort (k_force_tile orders long lists in global scratch).
 static void add_forces_f64(Swimmers* W, Lattice* L) {
   SpreadScratch& S = L->spread;
   const int nends = 2 * W->n;
@@ -1838,36 +1990,35 @@ static void add_forces_f64(Swimmers* W, Lattice* L) {
   const bool exact = L->compat & LBSWIM_COMPAT_EXACT_F64;
   const Dims D = make_dims(L);
   const TileGrid G = force_tiles(L);
-  const long long ntiles = (long long)G.nt[0] * G.nt[1] * G.nt[2];
-  const bool buckets = nends <= 48 * ntiles;
+  const int ntiles = G.nt[0] * G.nt[1] * G.nt[2];
+  const bool buckets = tiles_take_buckets(G, nends);
   ensure_ends(L, nends);
-  if (buckets) ensure_tile_buckets(L, (int)ntiles);
-  EndRecord<double>* ends = (EndRecord<double>*)S.ends;
-  unsigned* max_f = buckets ? S.bucket_count + ntiles : nullptr;
-  const int grid = (nends + REC64_ENDS - 1) / REC64_ENDS;
-  const int accumulate = L->force_zero_pending ? 0 : 1;
-  double* force = (double*)L->force;
-  if (buckets && !exact) {
-    unsigned* now = max_f + S.max_slot;
-    S.max_slot ^= 1;
-    k_end_records_f64<true><<<grid, REC64_THREADS, 0, L->stream>>>(
-        W->n, W->r, W->nv, W->common.P, W->common.l, D, ends, now, G, S.bucket_count,
-        S.bucket_list);
-    k_force_fixed<<<(int)ntiles, FT_THREADS, 0, L->stream>>>(
-        D, G, ends, nends, S.bucket_count, S.bucket_list, now, max_f + S.max_slot, force,
-        accumulate);
-    LB_CHECK_LAUNCH(2);
-  } else {
-    k_end_records_f64<false><<<grid, REC64_THREADS, 0, L->stream>>>(
-        W->n, W->r, W->nv, W->common.P, W->common.l, D, ends, nullptr, G,
-        buckets ? S.bucket_count : nullptr, S.bucket_list);
-    LB_CHECK_LAUNCH(1);
-    if (!buckets) bin_ends(L, S.ftiles, G, nends);
-    k_force_tile<<<(int)ntiles, FT_THREADS, 0, L->stream>>>(
-        D, G, ends, nends, buckets ? nullptr : S.ftiles.start, S.bucket_count,
-        buckets ? S.bucket_list : S.ftiles.list, S.ftiles.sorted, force, accumulate);
-    LB_CHECK_LAUNCH(1);
+  if (buckets) ensure_tile_buckets(L, ntiles);
+  if (S.prep.dirty) {  // records of a move that no step took
+    LB_CUDA(cudaMemsetAsync(S.bucket_count, 0, sizeof(unsigned) * (ntiles + 2), L->stream));
+    S.prep.dirty = S.prep.valid = false;
   }
+  EndRecord<double>* ends = (EndRecord<double>*)S.ends;
+  const int grid = (nends + REC64_ENDS - 1) / REC64_ENDS;
+  if (buckets && !exact) {
+    k_end_records_f64<true><<<grid, REC64_THREADS, 0, L->stream>>>(
+        W->n, W->r, W->nv, W->common.P, W->common.l, D, ends,
+        S.bucket_count + ntiles + S.max_slot, G,
+        nends > DIRECT_ENDS_F64 ? S.bucket_count : nullptr, S.bucket_list);
+    LB_CHECK_LAUNCH(1);
+    spread_fixed(L, nends);
+    return;
+  }
+  k_end_records_f64<false><<<grid, REC64_THREADS, 0, L->stream>>>(
+      W->n, W->r, W->nv, W->common.P, W->common.l, D, ends, nullptr, G,
+      buckets ? S.bucket_count : nullptr, S.bucket_list);
+  LB_CHECK_LAUNCH(1);
+  if (!buckets) bin_ends(L, S.ftiles, G, nends);
+  k_force_tile<<<ntiles, FT_THREADS, 0, L->stream>>>(
+      D, G, ends, nends, buckets ? nullptr : S.ftiles.start, S.bucket_count,
+      buckets ? S.bucket_list : S.ftiles.list, S.ftiles.sorted, (double*)L->force,
+      L->force_zero_pending ? 0 : 1);
+  LB_CHECK_LAUNCH(1);
   L->force_zero_pending = false;
 }
 
@@ -1893,8 +2044,6 @@ static TileGrid slab_grid(const Lattice* L, int lx) {
   }
   return G;
 }
-
-static int slabs_of(const TileGrid& G) { return G.nt[0] * G.nt[1] * G.nt[2]; }
 
 // Buckets (count and list) for at least nslabs slabs; replacing them waits for
 // the lattice's work.
@@ -1931,7 +2080,11 @@ static void clear_buckets(Lattice* L) {
 SlabSpread spread_prepare_slabs(Lattice* L) {
   SpreadScratch& S = L->spread;
   S.last_pending = S.pending;
-  if (S.bucket_tile != L->fused_tile) {
+  const bool direct = S.pending <= DIRECT_ENDS;
+  if (direct) {
+    S.lx = choose_slab_lx(L->size, L->fused_tile, S.pending);
+    S.bucket_tile = -1;
+  } else if (S.bucket_tile != L->fused_tile) {
     S.lx = choose_slab_lx(L->size, L->fused_tile, S.pending);
     clear_buckets(L);
     if (S.pending > 0) {
@@ -1943,7 +2096,7 @@ SlabSpread spread_prepare_slabs(Lattice* L) {
   }
   SlabSpread out;
   out.ends = S.ends;
-  out.count = S.bucket_count;
+  out.count = direct ? nullptr : S.bucket_count;
   out.list = S.bucket_list;
   out.npending = S.pending;
   out.max_abs_force = S.max_abs_force;
@@ -1959,16 +2112,21 @@ static void append_ends(Swimmers* W, Lattice* L) {
   ensure_ends(L, S.pending + nends);
   if (!S.max_abs_force) LB_CUDA(cudaMalloc(&S.max_abs_force, sizeof(unsigned)));
   if (S.pending == 0) {
-    S.lx = choose_slab_lx(L->size, L->fused_tile, std::max(nends, S.last_pending));
-    clear_buckets(L);
+    S.bucket_tile = -1;
+    const int expected = std::max(nends, S.last_pending);
+    if (expected > DIRECT_ENDS) {
+      S.lx = choose_slab_lx(L->size, L->fused_tile, expected);
+      clear_buckets(L);
+    }
   }
   const bool fill = S.bucket_tile == L->fused_tile;
   if (S.pending == 0) LB_CUDA(cudaMemsetAsync(S.max_abs_force, 0, sizeof(unsigned), L->stream));
   if (nends > 0) {
-    k_end_records<<<(nends + REC_THREADS - 1) / REC_THREADS, REC_THREADS, 0, L->stream>>>(
-        W->n, W->r, W->nv, W->common.P, W->common.l, make_dims(L),
-        (EndRecord<float>*)S.ends + S.pending, S.pending, S.max_abs_force, slab_grid(L, S.lx),
-        fill ? S.bucket_count : nullptr, fill ? S.bucket_list : nullptr);
+    k_end_records<<<(nends + REC_ENDS - 1) / REC_ENDS, REC_THREADS, 0, L->stream>>>(
+        W->n, W->r, W->nv, W->common.P, W->common.l, make_dims(L), S.pending,
+        RecordTarget<float>{(EndRecord<float>*)S.ends + S.pending, S.max_abs_force,
+                            fill ? slab_grid(L, S.lx) : TileGrid{},
+                            fill ? S.bucket_count : nullptr, S.bucket_list});
     LB_CHECK_LAUNCH(1);
   }
   S.pending += nends;
@@ -1983,6 +2141,52 @@ static bool wide_particle_index(const Lattice* L) {
 static void swimmers_mark(Swimmers* W, cudaStream_t stream) {
   if (!W->done) LB_CUDA(cudaEventCreateWithFlags(&W->done, cudaEventDisableTiming));
   LB_CUDA(cudaEventRecord(W->done, stream));
+}
+
+// Swimmer fields into page-locked host buffers by the kernel itself: one launch in
+// place of three copies, whose starts cost more than the bytes of a small array.
+__global__ void k_swimmers_to_host(int n3, const double* __restrict__ r,
+                                   const double* __restrict__ v, const double* __restrict__ nv,
+                                   double* __restrict__ hr, double* __restrict__ hv,
+                                   double* __restrict__ hn) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n3) return;
+  if (hr) hr[i] = r[i];
+  if (hv) hv[i] = v[i];
+  if (hn) hn[i] = nv[i];
+}
+
+// Swimmers whose fields a kernel writes to the host (D2H_NOTE).
+constexpr int DIRECT_READ_SWIMMERS = 4096;
+
+void swimmers_read(Swimmers* W, double* r, double* v, double* n) {
+  if (!W->copy) {
+    // ahead of the blocks of queued tracer moves
+    int least = 0, greatest = 0;
+    LB_CUDA(cudaDeviceGetStreamPriorityRange(&least, &greatest));
+    LB_CUDA(cudaStreamCreateWithPriority(&W->copy, cudaStreamNonBlocking, greatest));
+  }
+  if (W->done) LB_CUDA(cudaStreamWaitEvent(W->copy, W->done, 0));
+  double* dst[3] = {r, v, n};
+  const double* src[3] = {W->r, W->v, W->nv};
+  double* mapped[3] = {nullptr, nullptr, nullptr};
+  bool direct = W->n > 0 && W->n <= DIRECT_READ_SWIMMERS;
+  for (int f = 0; f < 3 && direct; ++f)
+    if (dst[f]) {
+      mapped[f] = (double*)mapped_host(dst[f]);
+      direct = mapped[f] != nullptr;
+    }
+  const size_t bytes = sizeof(double) * 3 * (size_t)W->n;
+  if (direct) {
+    k_swimmers_to_host<<<(3 * W->n + 255) / 256, 256, 0, W->copy>>>(
+        3 * W->n, W->r, W->v, W->nv, mapped[0], mapped[1], mapped[2]);
+    LB_CHECK_LAUNCH(1);
+  } else {
+    for (int f = 0; f < 3; ++f)
+      if (dst[f] && bytes)
+        LB_CUDA(cudaMemcpyAsync(dst[f], src[f], bytes, cudaMemcpyDeviceToHost, W->copy));
+  }
+  LB_CUDA(cudaStreamSynchronize(W->copy));
 }
 
 void swimmers_wait(Swimmers* W) {
@@ -2001,55 +2205,50 @@ void swimmers_add_forces(Swimmers* W, Lattice* L) {
   L->force_version++;
 }
 
-void swimmers_move(Swimmers* W, Lattice* L) {
+// The move, recording the moved swimmers' ends into `to32` or `to64` when given.
+static void launch_swimmers_move(Swimmers* W, Lattice* L, const RecordTarget<float>* to32,
+                                 const RecordTarget<double>* to64) {
   const Dims D = make_dims(L);
-  if (W->n > 0) {
-    if (L->precision == LBSWIM_F64) {
-      const double* u = (const double*)L->u;
-      const int grid = (W->n + MOVE64_SWIMMERS - 1) / MOVE64_SWIMMERS;
-      if (L->compat & LBSWIM_COMPAT_EXACT_F64)
-        k_swimmers_move_exact<<<(int)((2ll * W->n + EXACT_MOVE_BLOCK - 1) / EXACT_MOVE_BLOCK),
-                                EXACT_MOVE_BLOCK, 0, L->stream>>>(
-            W->n, W->r, W->v, W->nv, W->common, W->seed, W->step, D, u, L->status);
-      else if (wide_particle_index(L))
-        k_swimmers_move_f64<long long><<<grid, MOVE64_BLOCK, 0, L->stream>>>(
-            W->n, W->r, W->v, W->nv, W->common, W->seed, W->step, D, u, L->status);
-      else
-        k_swimmers_move_f64<int><<<grid, MOVE64_BLOCK, 0, L->stream>>>(
-            W->n, W->r, W->v, W->nv, W->common, W->seed, W->step, D, u, L->status);
+  const bool wide = wide_particle_index(L);
+  if (L->precision == LBSWIM_F64) {
+    const double* u = (const double*)L->u;
+    if (L->compat & LBSWIM_COMPAT_EXACT_F64) {
+      k_swimmers_move_exact<<<(int)((2ll * W->n + EXACT_MOVE_BLOCK - 1) / EXACT_MOVE_BLOCK),
+                              EXACT_MOVE_BLOCK, 0, L->stream>>>(
+          W->n, W->r, W->v, W->nv, W->common, W->seed, W->step, D, u, L->status);
+    } else {
+      auto k = to64 ? (wide ? k_swimmers_move_f64<true, long long> : k_swimmers_move_f64<true, int>)
+                    : (wide ? k_swimmers_move_f64<false, long long> : k_swimmers_move_f64<false, int>);
+      k<<<(W->n + MOVE64_SWIMMERS - 1) / MOVE64_SWIMMERS, MOVE64_BLOCK, 0, L->stream>>>(
+          W->n, W->r, W->v, W->nv, W->common, W->seed, W->step, D, u, L->status,
+          to64 ? *to64 : RecordTarget<double>{});
     }
-    else if (wide_particle_index(L))
-      k_swimmers_move_f32<long long><<<(W->n + SWIMMERS_PER_BLOCK - 1) / SWIMMERS_PER_BLOCK,
-                                       SWIMMER_MOVE_BLOCK, 0, L->stream>>>(
-          W->n, W->r, W->v, W->nv, W->common, W->seed, W->step, D, (const float4*)L->hydro,
-          L->status);
-    else
-      k_swimmers_move_f32<int><<<(W->n + SWIMMERS_PER_BLOCK - 1) / SWIMMERS_PER_BLOCK,
-                                 SWIMMER_MOVE_BLOCK, 0, L->stream>>>(
-          W->n, W->r, W->v, W->nv, W->common, W->seed, W->step, D, (const float4*)L->hydro,
-          L->status);
-    LB_CHECK_LAUNCH(1);
-    swimmers_mark(W, L->stream);
+  } else {
+    auto k = to32 ? (wide ? k_swimmers_move_f32<true, long long> : k_swimmers_move_f32<true, int>)
+                  : (wide ? k_swimmers_move_f32<false, long long> : k_swimmers_move_f32<false, int>);
+    k<<<(W->n + MOVE_SWIMMERS - 1) / MOVE_SWIMMERS, MOVE_BLOCK, 0, L->stream>>>(
+        W->n, W->r, W->v, W->nv, W->common, W->seed, W->step, D, (const float4*)L->hydro,
+        L->status, to32 ? *to32 : RecordTarget<float>{});
   }
+  LB_CHECK_LAUNCH(1);
+  swimmers_mark(W, L->stream);
+}
+
+void swimmers_move(Swimmers* W, Lattice* L) {
+  if (W->n > 0) launch_swimmers_move(W, L, nullptr, nullptr);
   W->step++;
 }
 
-// The move of lbswim_system_step with one swimmer array: on reduced-precision
-// lattices it is followed by the records and slab buckets of the moved
-// swimmers' ends, made into the lattice's prepared set, which the next step's
-// AddForces takes if nothing changed in between (swimmers_add_forces_prepared).
-// A read-back of the swimmers waits for the move only; an upload also waits
-// for these records.
-void swimmers_move_preparing(Swimmers* W, Lattice* L, unsigned long long epoch) {
+// Before the step of a system step with one swimmer array: room for the records
+// that its move will make for the next step (reduced precision: in buffers of
+// their own, whose counts the step kernel clears).
+void swimmers_prepare_room(Swimmers* W, Lattice* L) {
   SpreadScratch::Prepared& P = L->spread.prep;
   P.valid = false;
-  swimmers_move(W, L);
+  P.clear = 0;
+  P.clear_max = false;
   if (W->n <= 0 || L->precision == LBSWIM_F64) return;
   const int nends = 2 * W->n;
-  const int lx = choose_slab_lx(L->size, L->fused_tile, nends);
-  const TileGrid G = slab_grid(L, lx);
-  const int nslabs = slabs_of(G);
-  const size_t rec = sizeof(EndRecord<float>);
   if (P.capacity_ends < nends) {
     // the buffers may still be read by earlier work on the stream
     LB_CUDA(cudaStreamSynchronize(L->stream));
@@ -2057,48 +2256,95 @@ void swimmers_move_preparing(Swimmers* W, Lattice* L, unsigned long long epoch) 
     P.ends = nullptr;
     P.capacity_ends = 0;
     const int cap = std::max(nends + nends / 2, 64);
-    LB_CUDA(cudaMalloc(&P.ends, rec * cap));
+    LB_CUDA(cudaMalloc(&P.ends, sizeof(EndRecord<float>) * cap));
     P.capacity_ends = cap;
-    P.ends_bytes = rec * cap;
+    P.ends_bytes = sizeof(EndRecord<float>) * cap;
   }
-  grow_buckets(L, nslabs, P.bucket_count, P.bucket_list, P.bucket_slabs);
   if (!P.max_abs_force) LB_CUDA(cudaMalloc(&P.max_abs_force, sizeof(unsigned)));
-  LB_CUDA(cudaMemsetAsync(P.bucket_count, 0, sizeof(unsigned) * nslabs, L->stream));
-  LB_CUDA(cudaMemsetAsync(P.max_abs_force, 0, sizeof(unsigned), L->stream));
-  k_end_records<<<(nends + REC_THREADS - 1) / REC_THREADS, REC_THREADS, 0, L->stream>>>(
-      W->n, W->r, W->nv, W->common.P, W->common.l, make_dims(L), (EndRecord<float>*)P.ends, 0,
-      P.max_abs_force, G, P.bucket_count, P.bucket_list);
-  LB_CHECK_LAUNCH(1);
-  if (!W->recorded) LB_CUDA(cudaEventCreateWithFlags(&W->recorded, cudaEventDisableTiming));
-  LB_CUDA(cudaEventRecord(W->recorded, L->stream));
+  P.clear_max = true;
+  if (nends > DIRECT_ENDS) {
+    P.lx = choose_slab_lx(L->size, L->fused_tile, nends);
+    P.clear = slabs_of(slab_grid(L, P.lx));
+    grow_buckets(L, P.clear, P.bucket_count, P.bucket_list, P.bucket_slabs);
+  }
+}
+
+// The move of lbswim_system_step with one swimmer array (after
+// swimmers_prepare_room and the step): the moved swimmers' ends are also recorded,
+// and the next step's AddForces takes them if nothing changed in between
+// (swimmers_add_forces_prepared).  A small array's move records them itself, one
+// launch on the critical path less; a larger one's are recorded, and listed under
+// their slabs, by a kernel after it, so that a read-back of the swimmers waits for
+// the move only (an upload for both) and one wave of blocks pays the bucket
+// atomics once.
+void swimmers_move_preparing(Swimmers* W, Lattice* L, unsigned long long epoch) {
+  SpreadScratch& S = L->spread;
+  SpreadScratch::Prepared& P = S.prep;
+  P.valid = false;
+  const int nends = 2 * W->n;
+  if (W->n <= 0) {
+    swimmers_move(W, L);
+    return;
+  }
+  if (L->precision == LBSWIM_F64) {
+    if ((L->compat & LBSWIM_COMPAT_EXACT_F64) || nends > DIRECT_ENDS_F64 || !S.bucket_count ||
+        S.capacity_ends < nends || P.dirty) {
+      swimmers_move(W, L);
+      return;
+    }
+    const TileGrid G = force_tiles(L);
+    const RecordTarget<double> to{(EndRecord<double>*)S.ends,
+                                  S.bucket_count + slabs_of(G) + S.max_slot, G, nullptr, nullptr};
+    P.dirty = true;
+    launch_swimmers_move(W, L, nullptr, &to);
+  } else if (nends <= DIRECT_ENDS) {
+    const RecordTarget<float> to{(EndRecord<float>*)P.ends, P.max_abs_force, TileGrid{}, nullptr,
+                                 nullptr};
+    launch_swimmers_move(W, L, &to, nullptr);
+    P.tile = -1;
+  } else {
+    launch_swimmers_move(W, L, nullptr, nullptr);
+    k_end_records<<<(nends + REC_ENDS - 1) / REC_ENDS, REC_THREADS, 0, L->stream>>>(
+        W->n, W->r, W->nv, W->common.P, W->common.l, make_dims(L), 0,
+        RecordTarget<float>{(EndRecord<float>*)P.ends, P.max_abs_force, slab_grid(L, P.lx),
+                            P.bucket_count, P.bucket_list});
+    LB_CHECK_LAUNCH(1);
+    if (!W->recorded) LB_CUDA(cudaEventCreateWithFlags(&W->recorded, cudaEventDisableTiming));
+    LB_CUDA(cudaEventRecord(W->recorded, L->stream));
+    P.tile = L->fused_tile;
+  }
+  W->step++;
   P.valid = true;
   P.owner = W;
   P.owner_step = W->step;
   P.epoch = epoch;
-  P.tile = L->fused_tile;
-  P.lx = lx;
   P.nends = nends;
 }
 
-// AddForces of W (right after ZeroForce) from the prepared set, when the last
+// AddForces of W (right after ZeroForce) from the prepared records, when the last
 // thing that happened to W and to this lattice was that preparing move.
 bool swimmers_add_forces_prepared(Swimmers* W, Lattice* L, unsigned long long epoch) {
   SpreadScratch& S = L->spread;
   SpreadScratch::Prepared& P = S.prep;
   if (!P.valid || P.owner != W || P.owner_step != W->step || P.epoch != epoch ||
-      P.tile != L->fused_tile || L->precision == LBSWIM_F64 || S.pending != 0 || S.stepped ||
-      P.nends != 2 * W->n)
+      S.pending != 0 || S.stepped || P.nends != 2 * W->n)
     return false;
-  std::swap(S.ends, P.ends);
-  std::swap(S.ends_bytes, P.ends_bytes);
-  std::swap(S.capacity_ends, P.capacity_ends);
-  std::swap(S.bucket_count, P.bucket_count);
-  std::swap(S.bucket_list, P.bucket_list);
-  std::swap(S.bucket_slabs, P.bucket_slabs);
-  std::swap(S.max_abs_force, P.max_abs_force);
-  S.bucket_tile = L->fused_tile;
-  S.lx = P.lx;
-  S.pending = P.nends;
+  if (L->precision == LBSWIM_F64) {
+    spread_fixed(L, P.nends);
+    P.dirty = false;
+  } else {
+    if (P.tile >= 0 && P.tile != L->fused_tile) return false;
+    std::swap(S.ends, P.ends);
+    std::swap(S.ends_bytes, P.ends_bytes);
+    std::swap(S.capacity_ends, P.capacity_ends);
+    std::swap(S.bucket_count, P.bucket_count);
+    std::swap(S.bucket_list, P.bucket_list);
+    std::swap(S.bucket_slabs, P.bucket_slabs);
+    std::swap(S.max_abs_force, P.max_abs_force);
+    S.bucket_tile = P.tile;  // -1: no buckets
+    S.lx = P.lx;
+    S.pending = P.nends;
+  }
   P.valid = false;
   swimmers_mark(W, L->stream);
   L->force_version++;
@@ -2313,14 +2559,14 @@ static void tracers_move_on(Tracers* T, Lattice* L, cudaStream_t stream) {
       k_tracers_move_f64<int><<<grid, MOVE64_BLOCK, 0, stream>>>(T->n, T->r, T->s, T->v, D, u,
                                                                  L->status);
   }
-  else if (wide_particle_index(L))
-    k_tracers_move_f32<long long><<<(T->n + TRACER_MOVE_BLOCK - 1) / TRACER_MOVE_BLOCK,
-                                    TRACER_MOVE_BLOCK, 0, stream>>>(T->n, T->r, T->s, T->v, D,
-                                                                    L->hydro, L->status);
-  else
-    k_tracers_move_f32<int><<<(T->n + TRACER_MOVE_BLOCK - 1) / TRACER_MOVE_BLOCK,
-                              TRACER_MOVE_BLOCK, 0, stream>>>(T->n, T->r, T->s, T->v, D,
-                                                              L->hydro, L->status);
+  else {
+    const bool far = wide_particle_index(L), wide = T->n >= TRACERS_WIDE_FROM;
+    const int per = wide ? WIDE_TRACERS : MOVE_POINTS;
+    auto k = wide ? (far ? k_tracers_move_f32<true, long long> : k_tracers_move_f32<true, int>)
+                  : (far ? k_tracers_move_f32<false, long long> : k_tracers_move_f32<false, int>);
+    k<<<(T->n + per - 1) / per, MOVE_BLOCK, 0, stream>>>(T->n, T->r, T->s, T->v, D, L->hydro,
+                                                         L->status);
+  }
   LB_CHECK_LAUNCH(1);
 }
 

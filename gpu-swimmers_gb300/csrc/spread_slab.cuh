@@ -62,8 +62,9 @@ struct SpreadLayout {
   static constexpr int total = align16(plist + SPREAD_CAP * SPREAD_PLANES_PER_END * 2);
 };
 
-// Where the ends of slab `slab` are: its bucket, or every pending end when the
-// bucket overflowed.
+// Where the ends of slab `slab` are: its bucket; every pending end when the bucket
+// overflowed, or when there are no buckets (count null: DIRECT_ENDS ends at most,
+// of which a slab picks its own).
 struct SlabEnds {
   const EndRecord<float>* ends;
   const unsigned* count;  // [slabs]
@@ -79,7 +80,7 @@ struct SlabEnds {
 // the same choice.
 __device__ __forceinline__ bool slab_sums_split(const SlabEnds& se, int slab, int nx, int ny,
                                                 int nz) {
-  const unsigned c = se.count[slab];
+  const unsigned c = se.count ? se.count[slab] : ~0u;
   const long long cnt = c > (unsigned)SLAB_BUCKET_CAP ? se.npending : (long long)c;
   return cnt * (nx < 4 || ny < 4 || nz < 4 ? 16 : 1) <= 65535ll;
 }
@@ -97,7 +98,7 @@ struct SlabSpreader {
   const int* list;
   long long s0;
   int cnt;
-  bool in_smem, overflow;
+  bool in_smem, overflow, direct;
   float fx_scale, fx_inv;
   // shared-memory arrays at fixed offsets from smem
   __device__ unsigned* fq() const { return reinterpret_cast<unsigned*>(smem + SL::fq); }
@@ -120,8 +121,9 @@ struct SlabSpreader {
     fx_inv = exp2_int(-e);
     ends = se.ends;
     list = se.list;
-    const unsigned c = se.count[slab];
-    overflow = c > (unsigned)SLAB_BUCKET_CAP;
+    direct = se.count == nullptr;
+    const unsigned c = direct ? 0u : se.count[slab];
+    overflow = direct || c > (unsigned)SLAB_BUCKET_CAP;
     cnt = overflow ? se.npending : (int)c;
     s0 = (long long)slab * SLAB_BUCKET_CAP;
     in_smem = !overflow && cnt <= SPREAD_CAP;
@@ -129,41 +131,70 @@ struct SlabSpreader {
 
   __device__ int planes() const { return ex + 2 * H; }
 
+  // Local planes holding one of the x nodes of the end with origin o (bit kk: plane
+  // x0 - H + kk), and the local row / column of its other nodes (-1: outside); bit
+  // 63 marks nodes that appear twice in the cross-section.
+  __device__ unsigned long long cover(const EndRecord<float>& g, NodeLocal& nl) const {
+    unsigned long long m = 0ull;  // one bit per plane: SLAB_LX_MAX + 2 < 63
+    if (nx >= 4) {
+      for (int i = 0; i < 4; ++i)
+        for (int d = wrap_small(g.o[0] + i - x0 + H, nx); d < planes(); d += nx) m |= 1ull << d;
+    } else {
+      float w;
+      for (int kk = 0; kk < planes(); ++kk)
+        if (cover_weight(wrap_once(x0 - H + kk, nx), g.o[0], nx, g.phi[0], w)) m |= 1ull << kk;
+    }
+    for (int j = 0; j < 4; ++j) {
+      const int ly2 = wrap_small(g.o[1] + j - y0 + H, ny);
+      const int lz2 = wrap_small(g.o[2] + j - z0 + H, nz);
+      nl.y[j] = (signed char)(ly2 <= ey - 1 + 2 * H ? ly2 : -1);
+      nl.z[j] = (signed char)(lz2 <= ez - 1 + 2 * H ? lz2 : -1);
+      if (ly2 + ny <= ey - 1 + 2 * H || lz2 + nz <= ez - 1 + 2 * H) m |= 1ull << 63;
+    }
+    return m;
+  }
+  __device__ void keep(int q, const EndRecord<float>& g, unsigned long long m,
+                       const NodeLocal& nl) const {
+    SlabEnd e;
+    e.ox = g.o[0];
+    for (int c = 0; c < 3; ++c) {
+      e.F[c] = g.F[c];
+      for (int j = 0; j < 4; ++j) e.phi[c][j] = g.phi[c][j];
+    }
+    srec()[q] = e;
+    nodes()[q] = nl;
+    xmask()[q] = m;
+  }
+
   // Records, coverage masks, local node rows and per-plane lists of the slab's
   // ends; zeroes the sums.  Every thread of the block calls it.
   __device__ void prologue(int tid, int nthreads) {
     if (in_smem) {
       for (int q = tid; q < cnt; q += nthreads) {
         const EndRecord<float>& g = ends[list[s0 + q]];
-        SlabEnd e;
-        e.ox = g.o[0];
-        for (int c = 0; c < 3; ++c) {
-          e.F[c] = g.F[c];
-          for (int j = 0; j < 4; ++j) e.phi[c][j] = g.phi[c][j];
-        }
-        // local planes kk (x = x0 - H + kk) holding one of the x nodes
-        unsigned long long m = 0ull;  // one bit per plane: SLAB_LX_MAX + 2 < 63
-        if (nx >= 4) {
-          for (int i = 0; i < 4; ++i)
-            for (int d = wrap_small(e.ox + i - x0 + H, nx); d < planes(); d += nx) m |= 1ull << d;
-        } else {
-          float w;
-          for (int kk = 0; kk < planes(); ++kk)
-            if (cover_weight(wrap_once(x0 - H + kk, nx), e.ox, nx, e.phi[0], w)) m |= 1ull << kk;
-        }
-        // local row / column of each stencil node (-1: outside); bit 63 marks
-        // nodes that appear twice in the cross-section
         NodeLocal nl;
-        for (int j = 0; j < 4; ++j) {
-          const int ly2 = wrap_small(g.o[1] + j - y0 + H, ny);
-          const int lz2 = wrap_small(g.o[2] + j - z0 + H, nz);
-          nl.y[j] = (signed char)(ly2 <= ey - 1 + 2 * H ? ly2 : -1);
-          nl.z[j] = (signed char)(lz2 <= ez - 1 + 2 * H ? lz2 : -1);
-          if (ly2 + ny <= ey - 1 + 2 * H || lz2 + nz <= ez - 1 + 2 * H) m |= 1ull << 63;
-        }
-        srec()[q] = e;
-        nodes()[q] = nl;
-        xmask()[q] = m;
+        const unsigned long long m = cover(g, nl);
+        keep(q, g, m, nl);
+      }
+    } else if (direct) {
+      // the slab's own of all pending ends (their order does not matter)
+      __shared__ int picked;
+      if (tid == 0) picked = 0;
+      __syncthreads();
+      for (int q = tid; q < cnt; q += nthreads) {
+        const EndRecord<float>& g = ends[q];
+        NodeLocal nl;
+        const unsigned long long m = cover(g, nl);
+        const bool in_y = (nl.y[0] & nl.y[1] & nl.y[2] & nl.y[3]) >= 0;
+        const bool in_z = (nl.z[0] & nl.z[1] & nl.z[2] & nl.z[3]) >= 0;
+        if ((m & ~(1ull << 63)) == 0ull || !in_y || !in_z) continue;
+        const int at = atomicAdd(&picked, 1);
+        if (at < SPREAD_CAP) keep(at, g, m, nl);
+      }
+      __syncthreads();
+      if (picked <= SPREAD_CAP) {
+        in_smem = true;
+        cnt = picked;
       }
     }
     for (int i = tid; i < 3 * 2 * PLANE; i += nthreads) fq()[i] = 0u;
