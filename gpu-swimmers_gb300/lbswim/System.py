@@ -21,17 +21,15 @@ class System:
         self.things.append(th)
 
     def _native(self):
-        sw = [t for t in self.things if type(t) is _sw.Array]
-        tr = [t for t in self.things if type(t) is _tr.Array]
-        if len(sw) + len(tr) != len(self.things):
-            return None
         # AddForces of tracers is a no-op and swimmers move before tracers only
         # if they come first in the list; keep the reference's order exactly.
-        seen_tracer = False
+        sw, tr = [], []
         for t in self.things:
             if type(t) is _tr.Array:
-                seen_tracer = True
-            elif seen_tracer:
+                tr.append(t._h)
+            elif type(t) is _sw.Array and not tr:
+                sw.append(t._h)
+            else:
                 return None
         return sw, tr
 
@@ -39,10 +37,9 @@ class System:
         native = self._native()
         if native is not None:
             sw, tr = native
-            swa = (C.c_void_p * max(len(sw), 1))(*[t._h for t in sw])
-            tra = (C.c_void_p * max(len(tr), 1))(*[t._h for t in tr])
-            _lib.check(_lib.lib.lbswim_system_step(self.lat._h, swa, len(sw), tra, len(tr),
-                                                   int(nsteps)))
+            _lib.check(_lib.lib.lbswim_system_step(
+                self.lat._h, (C.c_void_p * max(len(sw), 1))(*sw), len(sw),
+                (C.c_void_p * max(len(tr), 1))(*tr), len(tr), int(nsteps)))
             return
         for _ in range(int(nsteps)):
             self.lat.ZeroForce()

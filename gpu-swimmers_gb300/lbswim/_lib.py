@@ -162,7 +162,10 @@ def dptr(a):
     """Pointer to the data of a C-contiguous float64 numpy array."""
     if a.dtype.char != "d" or not a.flags.c_contiguous:
         raise TypeError("expected a C-contiguous float64 array")
-    return a.ctypes.data_as(_D)
+    try:  # a fraction of the time of ctypes.data_as
+        return C.byref(C.c_double.from_buffer(a))
+    except (TypeError, ValueError):  # read-only or empty
+        return a.ctypes.data_as(_D)
 
 
 class _PinnedBlock:

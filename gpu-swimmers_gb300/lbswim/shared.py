@@ -82,7 +82,8 @@ class PrngArray:
         seed, step = _lib.C.c_ulonglong(), _lib.C.c_ulonglong()
         _lib.check(_lib.lib.lbswim_swimmers_get_rng(self.owner._h, _lib.C.byref(seed),
                                                     _lib.C.byref(step)))
-        self.view[:] = (seed.value, step.value)
+        self.view[0] = seed.value
+        self.view[1] = step.value
 
     def H2D(self):
         _lib.check(_lib.lib.lbswim_swimmers_set_rng(self.owner._h, int(self.view[0]),

@@ -121,8 +121,9 @@ class Array:
 
     def D2H(self):
         # r, v and n in one call (one wait for the device), then the stream state
-        bufs = [a.view.reshape(-1) for a in (self._r, self._v, self._n)]
-        _lib.check(_lib.lib.lbswim_swimmers_d2h_all(self._h, *[_lib.dptr(b) for b in bufs]))
+        _lib.check(_lib.lib.lbswim_swimmers_d2h_all(
+            self._h, _lib.dptr(self._r.view.reshape(-1)), _lib.dptr(self._v.view.reshape(-1)),
+            _lib.dptr(self._n.view.reshape(-1))))
         self.prng.D2H()
 
     @property
