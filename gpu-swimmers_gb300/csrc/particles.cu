@@ -1646,7 +1646,7 @@ __device__ __forceinline__ void swimmers_move_block(
     if (tumble) {
       float g[3];
       rng_normal3_f(seed, (uint32_t)i, step, g);
-      inv = 1.f / sqrtf(g[0] * g[0] + g[1] * g[1] + g[2] * g[2]);
+      inv = 1.f / sqrtf(__fmaf_rn(g[2], g[2], __fmaf_rn(g[1], g[1], __fmul_rn(g[0], g[0]))));
       nn = f2d_exact((a == 0 ? g[0] : (a == 1 ? g[1] : g[2])) * inv);
     } else if (rotate) {
       // the small turn (v - v_rear) / l is formed in FP32 and added to the FP64
@@ -1659,10 +1659,8 @@ __device__ __forceinline__ void swimmers_move_block(
   __syncthreads();
   if (update && rotate) {
     const float tx = turned[0][q], ty = turned[1][q], tz = turned[2][q];
-    float sq = 0.f;
-    sq += tx * tx;
-    sq += ty * ty;
-    sq += tz * tz;
+    // the roundings are spelt out: every instance of this code gives the same bits
+    const float sq = __fmaf_rn(tz, tz, __fmaf_rn(ty, ty, __fmul_rn(tx, tx)));
     nn = __dmul_rn(nn, f2d_exact(1.f / sqrtf(sq)));
   }
   if (update && (tumble || rotate)) swn[at] = nn;
