@@ -33,7 +33,7 @@ struct NodeLocal {
 // What the scatter needs of a pending dipole end, kept in shared memory.
 struct SlabEnd {
   int ox;           // wrapped x origin of the stencil
-  float F[3];       // force carried by the end
+  float F[3];       // force carried by the end, in units of the sums
   float phi[3][4];  // Peskin weights of the 4 nodes per axis
 };
 
@@ -158,7 +158,7 @@ struct SlabSpreader {
     SlabEnd e;
     e.ox = g.o[0];
     for (int c = 0; c < 3; ++c) {
-      e.F[c] = g.F[c];
+      e.F[c] = g.F[c] * fx_scale;  // exact: a power of two
       for (int j = 0; j < 4; ++j) e.phi[c][j] = g.phi[c][j];
     }
     srec()[q] = e;
@@ -276,9 +276,9 @@ struct SlabSpreader {
         else
           wx = e.phi[0][(ent >> 8) & 3u];
         const float py = e.phi[1][jy], pz = e.phi[2][jz];
-        const int q0 = fx_quant32(node_contrib(py, pz, wx, e.F[0]), fx_scale);
-        const int q1 = fx_quant32(node_contrib(py, pz, wx, e.F[1]), fx_scale);
-        const int q2 = fx_quant32(node_contrib(py, pz, wx, e.F[2]), fx_scale);
+        const int q0 = __float2int_rn(node_contrib(py, pz, wx, e.F[0]));
+        const int q1 = __float2int_rn(node_contrib(py, pz, wx, e.F[1]));
+        const int q2 = __float2int_rn(node_contrib(py, pz, wx, e.F[2]));
         if (!(ent & PL_DUP)) {
           add3(ly2 * HZ + lz2, q0, q1, q2);
         } else {
@@ -307,14 +307,30 @@ struct SlabSpreader {
     }
   }
 
-  // The sum of component c at local site `at` as a float, and zero it.
-  __device__ float take(int at, int c) const {
-    uint2* p = reinterpret_cast<uint2*>(fq()) + c * PLANE + at;
-    const uint2 w = *p;
-    *p = make_uint2(0u, 0u);
-    const long long q = SPLIT ? (long long)(int)w.y * 65536ll + (long long)w.x
-                              : (long long)(((unsigned long long)w.y << 32) | w.x);
-    return fx_value(q, fx_inv);
+  // The sums of the three components at local site `at` as floats, zeroed behind.  A
+  // sum of 32 bits, as nearly all are, converts in one step: split words make one
+  // when the high word with the low one's upper half fits 16 bits.  One branch
+  // for the three, after all of their loads.
+  __device__ void take(int at, float v[3]) const {
+    uint2* p = reinterpret_cast<uint2*>(fq()) + at;
+    const uint2 w[3] = {p[0], p[PLANE], p[2 * PLANE]};
+    bool fits = true;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      p[c * PLANE] = make_uint2(0u, 0u);
+      const int h = SPLIT ? (int)w[c].y + (int)(w[c].x >> 16) : (int)w[c].y;
+      const int q = SPLIT ? (int)(((unsigned)h << 16) | (w[c].x & 0xffffu)) : (int)w[c].x;
+      fits = fits && (SPLIT ? q >> 16 : q >> 31) == h;
+      v[c] = __int2float_rn(q) * fx_inv;
+    }
+    if (!fits) {
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        const long long q = SPLIT ? (long long)(int)w[c].y * 65536ll + (long long)w[c].x
+                                  : (long long)(((unsigned long long)w[c].y << 32) | w[c].x);
+        v[c] = fx_value(q, fx_inv);
+      }
+    }
   }
 };
 
