@@ -713,15 +713,17 @@ int lbswim_system_step(lbswim_lattice* lat, lbswim_swimmers* const* swimmers, in
   for (int i = 0; i < n_swimmers; ++i) REQUIRE(swimmers[i], "swimmer handle is NULL");
   for (int i = 0; i < n_tracers; ++i) REQUIRE(tracers[i], "tracer handle is NULL");
   Lattice* L = LAT(lat);
-  // With one swimmer array, each move also records the moved swimmers' ends
-  // for the next step; that step's AddForces takes them unless another call
-  // changed something in between.
+  // With one swimmer array (or a few, in reduced precision), each move also records
+  // the moved swimmers' ends for the next step; that step's AddForces takes them
+  // unless another call changed something in between.
+  Swimmers* const* w = reinterpret_cast<Swimmers* const*>(swimmers);
+  const bool together = swimmers_move_together(w, n_swimmers, L);
   const unsigned long long calls = g_calls.load(std::memory_order_relaxed);
   for (int t = 0; t < nsteps; ++t) {
     lattice_zero_force(L);  // ZeroForce
-    if (n_swimmers != 1 || !swimmers_add_forces_prepared(SW(swimmers[0]), L, calls))
-      for (int i = 0; i < n_swimmers; ++i) swimmers_add_forces(SW(swimmers[i]), L);
-    if (n_swimmers == 1) swimmers_prepare_room(SW(swimmers[0]), L);
+    if (!together || !swimmers_add_forces_prepared(w, n_swimmers, L, calls))
+      for (int i = 0; i < n_swimmers; ++i) swimmers_add_forces(w[i], L);
+    if (together) swimmers_prepare_room(w, n_swimmers, L);
     lattice_step(L);
     lattice_calc_hydro(L);
     // Tracers move on their own streams while the swimmers move and the next
@@ -733,10 +735,10 @@ int lbswim_system_step(lbswim_lattice* lat, lbswim_swimmers* const* swimmers, in
       LB_CUDA(cudaEventRecord(L->hydro_ready, L->stream));
       for (int i = 0; i < n_tracers; ++i) tracers_move_async(TR(tracers[i]), L);
     }
-    if (n_swimmers == 1)
-      swimmers_move_preparing(SW(swimmers[0]), L, calls);
+    if (together)
+      swimmers_move_preparing(w, n_swimmers, L, calls);
     else
-      for (int i = 0; i < n_swimmers; ++i) swimmers_move(SW(swimmers[i]), L);
+      for (int i = 0; i < n_swimmers; ++i) swimmers_move(w[i], L);
   }
   API_END
 }

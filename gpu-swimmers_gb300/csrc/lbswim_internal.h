@@ -110,8 +110,9 @@ struct SpreadScratch {
     bool clear_max = false;  // ... and the largest force
     bool dirty = false;  // FP64: the buckets hold records that no step has taken
     bool valid = false;
-    const void* owner = nullptr;          // the Swimmers moved
-    unsigned long long owner_step = 0;    // its move counter after that move
+    int owners = 0;                         // the arrays moved ...
+    const void* owner[8] = {};
+    unsigned long long owner_step[8] = {};  // ... and their move counters after it
     unsigned long long epoch = 0;         // API-call count then
     int tile = -1;
     int lx = 0;
@@ -337,13 +338,16 @@ void spread_free(SpreadScratch& S);
 // particles.cu
 void swimmers_add_forces(Swimmers* S, Lattice* L);
 void swimmers_move(Swimmers* S, Lattice* L);
-// lbswim_system_step with one swimmer array: AddForces from the records the
-// last move prepared (false: nothing prepared that still holds), and the move
-// that prepares them for the next step (swimmers_prepare_room before the step
-// between them).  epoch counts the API calls made.
-bool swimmers_add_forces_prepared(Swimmers* S, Lattice* L, unsigned long long epoch);
-void swimmers_prepare_room(Swimmers* S, Lattice* L);
-void swimmers_move_preparing(Swimmers* S, Lattice* L, unsigned long long epoch);
+// lbswim_system_step with arrays that can move together (reduced precision: up to 8
+// of them): AddForces from the records the last moves prepared (false: nothing
+// prepared that still holds), and the moves that prepare them for the next step
+// (swimmers_prepare_room before the step between them).  epoch counts the API
+// calls made.
+bool swimmers_move_together(Swimmers* const* w, int nw, const Lattice* L);
+bool swimmers_add_forces_prepared(Swimmers* const* w, int nw, Lattice* L,
+                                  unsigned long long epoch);
+void swimmers_prepare_room(Swimmers* const* w, int nw, Lattice* L);
+void swimmers_move_preparing(Swimmers* const* w, int nw, Lattice* L, unsigned long long epoch);
 // Wait on the host for the last kernel that used the swimmer arrays.
 void swimmers_wait(Swimmers* S);
 // Host copies (null: none) of the fields, after that kernel; waits for them.

@@ -360,6 +360,25 @@ __device__ __forceinline__ unsigned record_axis32(double r, double n, bool head,
   return __float_as_uint(fmaxf(0.f, fabsf((float)F)));  // 0 for a NaN
 }
 
+// The swimmer arrays of one launch, each with its first block (of MOVE_SWIMMERS
+// swimmers, or REC_ENDS ends) and its first end among all of the lattice's.
+constexpr int LIST_ARRAYS = 8;
+struct SwimmerPart {
+  int n, block0, end0;
+  double *r, *v, *nv;
+  lbswim_common_params common;
+  unsigned long long seed, step;
+};
+struct SwimmerList {
+  int count;
+  SwimmerPart part[LIST_ARRAYS];
+};
+__device__ __forceinline__ int part_of_block(const SwimmerList& w) {
+  int m = 0;
+  while (m + 1 < w.count && (int)blockIdx.x >= w.part[m + 1].block0) ++m;
+  return m;
+}
+
 // Where the end records of a swimmer array go: the records, the largest |F|, and
 // the buckets of the tiles of G.
 template <class T>
@@ -417,12 +436,11 @@ __device__ __forceinline__ void end_records_block(int blk, int nsw, const double
   finish_records32<true>(q, a, e0, nends, e_base, big, srec, smax, D, to);
 }
 
-__global__ void __launch_bounds__(REC_THREADS) k_end_records(int nsw,
-                                                             const double* __restrict__ r,
-                                                             const double* __restrict__ nv,
-                                                             double P, double l, Dims D,
-                                                             int e_base, RecordTarget<float> to) {
-  end_records_block(blockIdx.x, nsw, r, nv, P, l, D, e_base, to);
+__global__ void __launch_bounds__(REC_THREADS) k_end_records(const __grid_constant__ SwimmerList w,
+                                                             Dims D, RecordTarget<float> to) {
+  const SwimmerPart& p = w.part[part_of_block(w)];
+  to.ends += p.end0;
+  end_records_block(blockIdx.x - p.block0, p.n, p.r, p.nv, p.common.P, p.common.l, D, p.end0, to);
 }
 
 // Slab buckets of recorded ends (the slab shape changed since they were recorded).
@@ -1684,10 +1702,12 @@ __device__ __forceinline__ void swimmers_move_block(
 
 template <bool RECORD, class I>
 __global__ void __launch_bounds__(MOVE_BLOCK) k_swimmers_move_f32(
-    int nsw, double* __restrict__ swr, double* __restrict__ swv, double* __restrict__ swn,
-    lbswim_common_params c, unsigned long long seed, unsigned long long step, Dims D,
-    const float4* __restrict__ h, unsigned* status, RecordTarget<float> to) {
-  swimmers_move_block<RECORD, I>(blockIdx.x, nsw, swr, swv, swn, c, seed, step, D, h, status, to);
+    const __grid_constant__ SwimmerList w, Dims D, const float4* __restrict__ h, unsigned* status,
+    RecordTarget<float> to) {
+  const SwimmerPart& p = w.part[part_of_block(w)];
+  to.ends += p.end0;
+  swimmers_move_block<RECORD, I>(blockIdx.x - p.block0, p.n, p.r, p.v, p.nv, p.common, p.seed,
+                                 p.step, D, h, status, to);
 }
 
 // ---- batched ensembles: per-step reset, end records, moves --------------------
@@ -2102,6 +2122,30 @@ SlabSpread spread_prepare_slabs(Lattice* L) {
   return out;
 }
 
+// The parts of nw arrays, `per` items of 1 / `scale` of a swimmer a block, their ends
+// counted from end0; returns the number of blocks.
+static int list_parts(Swimmers* const* w, int nw, int per, int scale, int end0, SwimmerList& out) {
+  int blocks = 0;
+  out.count = nw;
+  for (int i = 0; i < nw; ++i) {
+    const Swimmers* W = w[i];
+    out.part[i] = SwimmerPart{W->n, blocks, end0, W->r, W->v, W->nv, W->common, W->seed, W->step};
+    blocks += (int)(((long long)scale * W->n + per - 1) / per);
+    end0 += 2 * W->n;
+  }
+  return blocks;
+}
+
+// FP32 records of the arrays' ends, the first of them end0 of the lattice's.
+static void launch_end_records(Swimmers* const* w, int nw, Lattice* L, int end0,
+                               const RecordTarget<float>& to) {
+  SwimmerList list;
+  const int blocks = list_parts(w, nw, REC_ENDS, 2, end0, list);
+  if (blocks == 0) return;
+  k_end_records<<<blocks, REC_THREADS, 0, L->stream>>>(list, make_dims(L), to);
+  LB_CHECK_LAUNCH(1);
+}
+
 // Records W's ends after the pending ones of a reduced-precision lattice, listed
 // under the step kernel's slabs.
 static void append_ends(Swimmers* W, Lattice* L) {
@@ -2119,14 +2163,10 @@ static void append_ends(Swimmers* W, Lattice* L) {
   }
   const bool fill = S.bucket_tile == L->fused_tile;
   if (S.pending == 0) LB_CUDA(cudaMemsetAsync(S.max_abs_force, 0, sizeof(unsigned), L->stream));
-  if (nends > 0) {
-    k_end_records<<<(nends + REC_ENDS - 1) / REC_ENDS, REC_THREADS, 0, L->stream>>>(
-        W->n, W->r, W->nv, W->common.P, W->common.l, make_dims(L), S.pending,
-        RecordTarget<float>{(EndRecord<float>*)S.ends + S.pending, S.max_abs_force,
-                            fill ? slab_grid(L, S.lx) : TileGrid{},
-                            fill ? S.bucket_count : nullptr, S.bucket_list});
-    LB_CHECK_LAUNCH(1);
-  }
+  launch_end_records(&W, 1, L, S.pending,
+                     RecordTarget<float>{(EndRecord<float>*)S.ends, S.max_abs_force,
+                                         fill ? slab_grid(L, S.lx) : TileGrid{},
+                                         fill ? S.bucket_count : nullptr, S.bucket_list});
   S.pending += nends;
 }
 
@@ -2203,50 +2243,79 @@ void swimmers_add_forces(Swimmers* W, Lattice* L) {
   L->force_version++;
 }
 
-// The move, recording the moved swimmers' ends into `to32` or `to64` when given.
-static void launch_swimmers_move(Swimmers* W, Lattice* L, const RecordTarget<float>* to32,
-                                 const RecordTarget<double>* to64) {
+// FP64 move of an array, recording the moved swimmers' ends into `to` when given.
+static void launch_move_f64(Swimmers* W, Lattice* L, const RecordTarget<double>* to) {
   const Dims D = make_dims(L);
-  const bool wide = wide_particle_index(L);
-  if (L->precision == LBSWIM_F64) {
-    const double* u = (const double*)L->u;
-    if (L->compat & LBSWIM_COMPAT_EXACT_F64) {
-      k_swimmers_move_exact<<<(int)((2ll * W->n + EXACT_MOVE_BLOCK - 1) / EXACT_MOVE_BLOCK),
-                              EXACT_MOVE_BLOCK, 0, L->stream>>>(
-          W->n, W->r, W->v, W->nv, W->common, W->seed, W->step, D, u, L->status);
-    } else {
-      auto k = to64 ? (wide ? k_swimmers_move_f64<true, long long> : k_swimmers_move_f64<true, int>)
-                    : (wide ? k_swimmers_move_f64<false, long long> : k_swimmers_move_f64<false, int>);
-      k<<<(W->n + MOVE64_SWIMMERS - 1) / MOVE64_SWIMMERS, MOVE64_BLOCK, 0, L->stream>>>(
-          W->n, W->r, W->v, W->nv, W->common, W->seed, W->step, D, u, L->status,
-          to64 ? *to64 : RecordTarget<double>{});
-    }
+  const double* u = (const double*)L->u;
+  if (L->compat & LBSWIM_COMPAT_EXACT_F64) {
+    k_swimmers_move_exact<<<(int)((2ll * W->n + EXACT_MOVE_BLOCK - 1) / EXACT_MOVE_BLOCK),
+                            EXACT_MOVE_BLOCK, 0, L->stream>>>(
+        W->n, W->r, W->v, W->nv, W->common, W->seed, W->step, D, u, L->status);
   } else {
-    auto k = to32 ? (wide ? k_swimmers_move_f32<true, long long> : k_swimmers_move_f32<true, int>)
-                  : (wide ? k_swimmers_move_f32<false, long long> : k_swimmers_move_f32<false, int>);
-    k<<<(W->n + MOVE_SWIMMERS - 1) / MOVE_SWIMMERS, MOVE_BLOCK, 0, L->stream>>>(
-        W->n, W->r, W->v, W->nv, W->common, W->seed, W->step, D, (const float4*)L->hydro,
-        L->status, to32 ? *to32 : RecordTarget<float>{});
+    const bool wide = wide_particle_index(L);
+    auto k = to ? (wide ? k_swimmers_move_f64<true, long long> : k_swimmers_move_f64<true, int>)
+                : (wide ? k_swimmers_move_f64<false, long long> : k_swimmers_move_f64<false, int>);
+    k<<<(W->n + MOVE64_SWIMMERS - 1) / MOVE64_SWIMMERS, MOVE64_BLOCK, 0, L->stream>>>(
+        W->n, W->r, W->v, W->nv, W->common, W->seed, W->step, D, u, L->status,
+        to ? *to : RecordTarget<double>{});
   }
   LB_CHECK_LAUNCH(1);
   swimmers_mark(W, L->stream);
 }
 
+// FP32 move of nw arrays in one launch, recording the moved swimmers' ends into `to`
+// when given.
+static void launch_move_f32(Swimmers* const* w, int nw, Lattice* L,
+                            const RecordTarget<float>* to) {
+  SwimmerList list;
+  const int blocks = list_parts(w, nw, MOVE_SWIMMERS, 1, 0, list);
+  if (blocks == 0) return;
+  const bool wide = wide_particle_index(L);
+  auto k = to ? (wide ? k_swimmers_move_f32<true, long long> : k_swimmers_move_f32<true, int>)
+              : (wide ? k_swimmers_move_f32<false, long long> : k_swimmers_move_f32<false, int>);
+  k<<<blocks, MOVE_BLOCK, 0, L->stream>>>(list, make_dims(L), (const float4*)L->hydro, L->status,
+                                          to ? *to : RecordTarget<float>{});
+  LB_CHECK_LAUNCH(1);
+  for (int i = 0; i < nw; ++i) swimmers_mark(w[i], L->stream);
+}
+
 void swimmers_move(Swimmers* W, Lattice* L) {
-  if (W->n > 0) launch_swimmers_move(W, L, nullptr, nullptr);
+  if (W->n > 0) {
+    if (L->precision == LBSWIM_F64)
+      launch_move_f64(W, L, nullptr);
+    else
+      launch_move_f32(&W, 1, L, nullptr);
+  }
   W->step++;
 }
 
-// Before the step of a system step with one swimmer array: room for the records
-// that its move will make for the next step (reduced precision: in buffers of
-// their own, whose counts the step kernel clears).
-void swimmers_prepare_room(Swimmers* W, Lattice* L) {
+bool swimmers_move_together(Swimmers* const* w, int nw, const Lattice* L) {
+  if (nw < 1 || nw > (L->precision == LBSWIM_F64 ? 1 : LIST_ARRAYS)) return false;
+  for (int i = 0; i < nw; ++i) {
+    if (w[i]->n <= 0) return false;
+    for (int j = 0; j < i; ++j)
+      if (w[j] == w[i]) return false;
+  }
+  return true;
+}
+
+static int ends_of(Swimmers* const* w, int nw) {
+  long long n = 0;
+  for (int i = 0; i < nw; ++i) n += 2ll * w[i]->n;
+  if (n > 0x7fffffffll) throw LbswimError{LBSWIM_ENOTSUP, "more than 2^30 swimmers on a lattice"};
+  return (int)n;
+}
+
+// Before the step of a system step: room for the records that its moves will make
+// for the next step (reduced precision: in buffers of their own, whose counts
+// the step kernel clears).
+void swimmers_prepare_room(Swimmers* const* w, int nw, Lattice* L) {
   SpreadScratch::Prepared& P = L->spread.prep;
   P.valid = false;
   P.clear = 0;
   P.clear_max = false;
-  if (W->n <= 0 || L->precision == LBSWIM_F64) return;
-  const int nends = 2 * W->n;
+  if (L->precision == LBSWIM_F64) return;
+  const int nends = ends_of(w, nw);
   if (P.capacity_ends < nends) {
     // the buffers may still be read by earlier work on the stream
     LB_CUDA(cudaStreamSynchronize(L->stream));
@@ -2267,66 +2336,70 @@ void swimmers_prepare_room(Swimmers* W, Lattice* L) {
   }
 }
 
-// The move of lbswim_system_step with one swimmer array (after
-// swimmers_prepare_room and the step): the moved swimmers' ends are also recorded,
-// and the next step's AddForces takes them if nothing changed in between
-// (swimmers_add_forces_prepared).  A small array's move records them itself, one
-// launch on the critical path less; a larger one's are recorded, and listed under
-// their slabs, by a kernel after it, so that a read-back of the swimmers waits for
-// the move only (an upload for both) and one wave of blocks pays the bucket
-// atomics once.
-void swimmers_move_preparing(Swimmers* W, Lattice* L, unsigned long long epoch) {
+// The moves of lbswim_system_step (after swimmers_prepare_room and the step): the
+// moved swimmers' ends are also recorded, and the next step's AddForces takes them
+// if nothing changed in between (swimmers_add_forces_prepared).  Several arrays move
+// in one launch and are recorded in one: four of 7,800 in a 192x200x208 lattice
+// 50 us a step less.  A small suspension's move records it itself, one launch on the
+// critical path less; a larger one's ends are recorded, and listed under their
+// slabs, by a kernel after it, so that a read-back of the swimmers waits for the
+// move only (an upload for both) and one wave of blocks pays the bucket atomics
+// once.
+void swimmers_move_preparing(Swimmers* const* w, int nw, Lattice* L, unsigned long long epoch) {
   SpreadScratch& S = L->spread;
   SpreadScratch::Prepared& P = S.prep;
   P.valid = false;
-  const int nends = 2 * W->n;
-  if (W->n <= 0) {
-    swimmers_move(W, L);
-    return;
-  }
+  const int nends = ends_of(w, nw);
   if (L->precision == LBSWIM_F64) {
     if ((L->compat & LBSWIM_COMPAT_EXACT_F64) || nends > DIRECT_ENDS_F64 || !S.bucket_count ||
         S.capacity_ends < nends || P.dirty) {
-      swimmers_move(W, L);
+      swimmers_move(w[0], L);
       return;
     }
     const TileGrid G = force_tiles(L);
     const RecordTarget<double> to{(EndRecord<double>*)S.ends,
                                   S.bucket_count + slabs_of(G) + S.max_slot, G, nullptr, nullptr};
     P.dirty = true;
-    launch_swimmers_move(W, L, nullptr, &to);
+    launch_move_f64(w[0], L, &to);
   } else if (nends <= DIRECT_ENDS) {
     const RecordTarget<float> to{(EndRecord<float>*)P.ends, P.max_abs_force, TileGrid{}, nullptr,
                                  nullptr};
-    launch_swimmers_move(W, L, &to, nullptr);
+    launch_move_f32(w, nw, L, &to);
     P.tile = -1;
   } else {
-    launch_swimmers_move(W, L, nullptr, nullptr);
-    k_end_records<<<(nends + REC_ENDS - 1) / REC_ENDS, REC_THREADS, 0, L->stream>>>(
-        W->n, W->r, W->nv, W->common.P, W->common.l, make_dims(L), 0,
-        RecordTarget<float>{(EndRecord<float>*)P.ends, P.max_abs_force, slab_grid(L, P.lx),
-                            P.bucket_count, P.bucket_list});
-    LB_CHECK_LAUNCH(1);
-    if (!W->recorded) LB_CUDA(cudaEventCreateWithFlags(&W->recorded, cudaEventDisableTiming));
-    LB_CUDA(cudaEventRecord(W->recorded, L->stream));
+    launch_move_f32(w, nw, L, nullptr);
+    launch_end_records(w, nw, L, 0,
+                       RecordTarget<float>{(EndRecord<float>*)P.ends, P.max_abs_force,
+                                           slab_grid(L, P.lx), P.bucket_count, P.bucket_list});
+    for (int i = 0; i < nw; ++i) {
+      if (!w[i]->recorded)
+        LB_CUDA(cudaEventCreateWithFlags(&w[i]->recorded, cudaEventDisableTiming));
+      LB_CUDA(cudaEventRecord(w[i]->recorded, L->stream));
+    }
     P.tile = L->fused_tile;
   }
-  W->step++;
+  P.owners = nw;
+  for (int i = 0; i < nw; ++i) {
+    w[i]->step++;
+    P.owner[i] = w[i];
+    P.owner_step[i] = w[i]->step;
+  }
   P.valid = true;
-  P.owner = W;
-  P.owner_step = W->step;
   P.epoch = epoch;
   P.nends = nends;
 }
 
-// AddForces of W (right after ZeroForce) from the prepared records, when the last
-// thing that happened to W and to this lattice was that preparing move.
-bool swimmers_add_forces_prepared(Swimmers* W, Lattice* L, unsigned long long epoch) {
+// AddForces of the arrays (right after ZeroForce) from the prepared records, when
+// the last thing that happened to them and to this lattice was that preparing move.
+bool swimmers_add_forces_prepared(Swimmers* const* w, int nw, Lattice* L,
+                                  unsigned long long epoch) {
   SpreadScratch& S = L->spread;
   SpreadScratch::Prepared& P = S.prep;
-  if (!P.valid || P.owner != W || P.owner_step != W->step || P.epoch != epoch ||
-      S.pending != 0 || S.stepped || P.nends != 2 * W->n)
+  if (!P.valid || P.owners != nw || P.epoch != epoch || S.pending != 0 || S.stepped ||
+      P.nends != ends_of(w, nw))
     return false;
+  for (int i = 0; i < nw; ++i)
+    if (P.owner[i] != w[i] || P.owner_step[i] != w[i]->step) return false;
   if (L->precision == LBSWIM_F64) {
     spread_fixed(L, P.nends);
     P.dirty = false;
@@ -2344,7 +2417,7 @@ bool swimmers_add_forces_prepared(Swimmers* W, Lattice* L, unsigned long long ep
     S.pending = P.nends;
   }
   P.valid = false;
-  swimmers_mark(W, L->stream);
+  for (int i = 0; i < nw; ++i) swimmers_mark(w[i], L->stream);
   L->force_version++;
   return true;
 }
