@@ -552,11 +552,11 @@ __device__ __forceinline__ unsigned record_axis64(double r, double n, bool head,
   return hi_word(double_bits(F)) & 0x7fffffffu;
 }
 
-// The rest of a block's records e0, e0 + 1, ... (REC64_ENDS of them, thread (q, a)
+// The rest of a block's records e0, e0 + 1, ... (ENDS of them, thread (q, a)
 // for axis a of record q, a <= 2): the force of lost ends, the largest force, the
 // buckets and the copy to global memory.  Every thread of the block calls it.
 constexpr int REC64_ENDS = 64, REC64_THREADS = 3 * REC64_ENDS;
-template <bool FIXED, bool BUCKETS>
+template <bool FIXED, bool BUCKETS, int ENDS>
 __device__ __forceinline__ void finish_records64(int q, int a, int e0, int nends, unsigned big,
                                                  EndRecord<double>* srec, const unsigned* lost,
                                                  unsigned& smax, const Dims& D,
@@ -575,7 +575,7 @@ __device__ __forceinline__ void finish_records64(int q, int a, int e0, int nends
   }
   if (FIXED && threadIdx.x == 0) atomicMax(to.max_f, smax);
   __syncthreads();
-  const int words = min(REC64_ENDS, nends - e0) * (int)(sizeof(EndRecord<double>) / 8);
+  const int words = min(ENDS, nends - e0) * (int)(sizeof(EndRecord<double>) / 8);
   const unsigned long long* src = reinterpret_cast<const unsigned long long*>(srec);
   unsigned long long* dst = reinterpret_cast<unsigned long long*>(to.ends + e0);
   for (int w = threadIdx.x; w < words; w += blockDim.x) dst[w] = src[w];
@@ -604,7 +604,7 @@ __global__ void __launch_bounds__(REC64_THREADS) k_end_records_f64(
     big = record_axis64<FIXED>(ra, na, head, P, l, D, a, srec[q], lost[q]);
     if (a == 0) srec[q].pad = 0;
   }
-  finish_records64<FIXED, true>(q, a, e0, nends, big, srec, lost, smax, D,
+  finish_records64<FIXED, true, REC64_ENDS>(q, a, e0, nends, big, srec, lost, smax, D,
                           RecordTarget<double>{ends, max_f, G, bucket_count, bucket_list});
 }
 static_assert(sizeof(EndRecord<double>) % 8 == 0, "records are copied as 64-bit words");
@@ -1012,7 +1012,7 @@ __global__ void __launch_bounds__(EXACT_MOVE_BLOCK) k_tracers_move_exact(
 }
 
 // ---- FP64 moves (default) ------------------------------------------------------
-// A block interpolates 64 points, four lanes each (one per z node), from integer
+// A block interpolates its points, four lanes each (one per z node), from integer
 // weights (fixed_weights4), in three phases: a thread per (point, axis) forms the
 // weights, a lane sums its 16 nodes a component, a thread per (particle, axis)
 // updates it.  A lane's 16 velocities become integers below 2^60 under the
@@ -1022,16 +1022,26 @@ __global__ void __launch_bounds__(EXACT_MOVE_BLOCK) k_tracers_move_exact(
 // point took before ran on two lanes per clock and SM.  1,048,576 tracers at
 // 256^3: 748 -> 430 us (2400 instructions per warp, the integer pipe 64% busy);
 // 65,536 swimmers 204 -> 104 us, one swimmer 50 -> 11 us.
-constexpr int MOVE64_BLOCK = 256, MOVE64_POINTS = 64;
+//
+// A small array's blocks take 16 points and give each component lanes of its own,
+// so that their chains run side by side (one swimmer 10.9 -> 7.6 us, 1074 18.3 ->
+// 15.2, 4096 tracers 8.6 -> 5.9); a lane of a large one's, of 64 points, takes the
+// three in turn and forms the nodes' offsets once (1,048,576 tracers 470 -> 430).
+constexpr int MOVE64_FEW = 16, MOVE64_MANY = 64;
+constexpr int MOVE64_MANY_FROM = 16384;  // points
+constexpr int move64_block(int points) { return points == MOVE64_FEW ? 12 * points : 4 * points; }
 
+template <int POINTS>
 struct Stencil64 {
-  Digits w[3][4][MOVE64_POINTS];
-  int o[3][MOVE64_POINTS];
-  double vel[3][MOVE64_POINTS];
+  Digits w[3][4][POINTS];
+  int o[3][POINTS];
+  double vel[3][POINTS];
 };
 
 // Weights and wrapped origin of coordinate x of point p on axis a.
-__device__ __forceinline__ void point_axis64(const Dims& D, double x, int a, int p, Stencil64& st) {
+template <int POINTS>
+__device__ __forceinline__ void point_axis64(const Dims& D, double x, int a, int p,
+                                             Stencil64<POINTS>& st) {
   const double x0 = ceil(x - 2.);
   st.o[a][p] = wrap_any((int)x0, dim_of(D, a));
   const double dr = x - x0;
@@ -1066,11 +1076,11 @@ __device__ __forceinline__ long long sum_of(long long acc, long long t) {
   return acc + ((t + 0x80000000ll) >> 32);
 }
 
-// Velocity of the block's 64 points; I: the type of the site offsets.
-template <class I>
+// Velocity of the block's points; I: the type of the site offsets.
+template <int POINTS, class I>
 __device__ __forceinline__ void gather64(const double* __restrict__ u, const Dims& D,
-                                         Stencil64& st) {
-  const int p = threadIdx.x >> 2, k = threadIdx.x & 3;
+                                         Stencil64<POINTS>& st) {
+  const int p = (threadIdx.x >> 2) % POINTS, k = threadIdx.x & 3;
   const I nynz = (I)D.n[1] * D.n[2];
   I xo[4];
   int yo[4];
@@ -1080,8 +1090,9 @@ __device__ __forceinline__ void gather64(const double* __restrict__ u, const Dim
     yo[i] = node_after(st.o[1][p], i, D.n[1]) * D.n[2];
   }
   const int z = node_after(st.o[2][p], k, D.n[2]);
+  const int c0 = POINTS == MOVE64_FEW ? threadIdx.x / (4 * POINTS) : 0;
 #pragma unroll 1
-  for (int c = 0; c < 3; ++c) {
+  for (int c = c0; c < (POINTS == MOVE64_FEW ? c0 + 1 : 3); ++c) {
     const double* __restrict__ uc = u + c * D.N + z;
     unsigned long long b[16];
     unsigned top = 0u;
@@ -1129,13 +1140,13 @@ __device__ __forceinline__ void gather64(const double* __restrict__ u, const Dim
   }
 }
 
-template <class I>
-__global__ void __launch_bounds__(MOVE64_BLOCK, 3) k_tracers_move_f64(
+template <int POINTS, class I>
+__global__ void __launch_bounds__(move64_block(POINTS)) k_tracers_move_f64(
     int ntr, double* __restrict__ r, double* __restrict__ s, double* __restrict__ v, Dims D,
     const double* __restrict__ u, unsigned* status) {
-  __shared__ Stencil64 st;
-  const int p = threadIdx.x % MOVE64_POINTS, a = threadIdx.x / MOVE64_POINTS;
-  const int i = blockIdx.x * MOVE64_POINTS + p;
+  __shared__ Stencil64<POINTS> st;
+  const int p = threadIdx.x % POINTS, a = threadIdx.x / POINTS;
+  const int i = blockIdx.x * POINTS + p;
   const long long at = (long long)ntr * a + i;
   const bool mine = a < 3, valid = mine && i < ntr;
   double x = 0.0, sa = 0.0;
@@ -1145,7 +1156,7 @@ __global__ void __launch_bounds__(MOVE64_BLOCK, 3) k_tracers_move_f64(
   }
   if (mine) point_axis64(D, x, a, p, st);
   __syncthreads();
-  gather64<I>(u, D, st);
+  gather64<POINTS, I>(u, D, st);
   __syncthreads();
   if (!valid) return;
   const double w = st.vel[a][p];
@@ -1154,23 +1165,22 @@ __global__ void __launch_bounds__(MOVE64_BLOCK, 3) k_tracers_move_f64(
   s[at] = sa + w;
 }
 
-// Points [0, 32) of a block are the swimmers, [32, 64) their rear points r - l n;
-// the threads (p < 32, axis) update them.
+// The first half of a block's points are its swimmers, the others their rear points
+// r - l n; the threads (p < half, axis) update them.
 // RECORD: the block then records the ends of the moved swimmers into `to`, for
-// the next step (thread (p, a): axis a of the tail, p < 32, or head of swimmer p % 32).
-constexpr int MOVE64_SWIMMERS = MOVE64_POINTS / 2;
-static_assert(2 * MOVE64_SWIMMERS == REC64_ENDS, "the ends of a block's swimmers");
-template <bool RECORD, class I>
-__global__ void __launch_bounds__(MOVE64_BLOCK, 3) k_swimmers_move_f64(
+// the next step (thread (p, a): axis a of the tail, p < half, or head of its swimmer).
+template <bool RECORD, int POINTS, class I>
+__global__ void __launch_bounds__(move64_block(POINTS)) k_swimmers_move_f64(
     int nsw, double* __restrict__ swr, double* __restrict__ swv, double* __restrict__ swn,
     lbswim_common_params c, unsigned long long seed, unsigned long long step, Dims D,
     const double* __restrict__ u, unsigned* status, RecordTarget<double> to) {
-  __shared__ Stencil64 st;
-  __shared__ double turned[3][MOVE64_SWIMMERS], moved[3][MOVE64_SWIMMERS];
-  const int p = threadIdx.x % MOVE64_POINTS, a = threadIdx.x / MOVE64_POINTS;
-  const int q = p % MOVE64_SWIMMERS, i = blockIdx.x * MOVE64_SWIMMERS + q;
+  __shared__ Stencil64<POINTS> st;
+  constexpr int HALF = POINTS / 2;
+  __shared__ double turned[3][HALF], moved[3][HALF];
+  const int p = threadIdx.x % POINTS, a = threadIdx.x / POINTS;
+  const int q = p % HALF, i = blockIdx.x * HALF + q;
   const long long at = (long long)nsw * a + i;
-  const bool rear = p >= MOVE64_SWIMMERS, mine = a < 3, valid = mine && i < nsw;
+  const bool rear = p >= HALF, mine = a < 3, valid = mine && i < nsw;
   double x = 0.0, na = 0.0;
   if (valid) {
     x = swr[at];
@@ -1178,7 +1188,7 @@ __global__ void __launch_bounds__(MOVE64_BLOCK, 3) k_swimmers_move_f64(
   }
   if (mine) point_axis64(D, rear ? __dsub_rn(x, __dmul_rn(na, c.l)) : x, a, p, st);
   __syncthreads();
-  gather64<I>(u, D, st);
+  gather64<POINTS, I>(u, D, st);
   __syncthreads();
   const bool update = valid && !rear;
   bool tumble = false;
@@ -1196,7 +1206,7 @@ __global__ void __launch_bounds__(MOVE64_BLOCK, 3) k_swimmers_move_f64(
       rng_normal3(seed, (uint32_t)i, step, g);
       turned[a][q] = a == 0 ? g[0] : (a == 1 ? g[1] : g[2]);
     } else {  // rotate with the local shear
-      turned[a][q] = na + (va - st.vel[a][MOVE64_SWIMMERS + q]) / c.l;
+      turned[a][q] = na + (va - st.vel[a][HALF + q]) / c.l;
     }
   }
   __syncthreads();
@@ -1209,8 +1219,8 @@ __global__ void __launch_bounds__(MOVE64_BLOCK, 3) k_swimmers_move_f64(
     swn[at] = nn;
   }
   if constexpr (RECORD) {
-    __shared__ EndRecord<double> srec[REC64_ENDS];
-    __shared__ unsigned smax, lost[REC64_ENDS];
+    __shared__ EndRecord<double> srec[POINTS];
+    __shared__ unsigned smax, lost[POINTS];
     if (threadIdx.x == 0) smax = 0u;
     if (a == 0) lost[p] = 0u;
     __syncthreads();  // every axis of a swimmer has been normalised
@@ -1222,7 +1232,7 @@ __global__ void __launch_bounds__(MOVE64_BLOCK, 3) k_swimmers_move_f64(
       big = record_axis64<true>(moved[a][q], turned[a][q], rear, c.P, c.l, D, a, srec[e], lost[e]);
       if (a == 0) srec[e].pad = 0;
     }
-    finish_records64<true, false>(e, a, blockIdx.x * REC64_ENDS, 2 * nsw, big, srec, lost, smax, D, to);
+    finish_records64<true, false, POINTS>(e, a, blockIdx.x * POINTS, 2 * nsw, big, srec, lost, smax, D, to);
   }
 }
 
@@ -2252,10 +2262,16 @@ static void launch_move_f64(Swimmers* W, Lattice* L, const RecordTarget<double>*
                             EXACT_MOVE_BLOCK, 0, L->stream>>>(
         W->n, W->r, W->v, W->nv, W->common, W->seed, W->step, D, u, L->status);
   } else {
-    const bool wide = wide_particle_index(L);
-    auto k = to ? (wide ? k_swimmers_move_f64<true, long long> : k_swimmers_move_f64<true, int>)
-                : (wide ? k_swimmers_move_f64<false, long long> : k_swimmers_move_f64<false, int>);
-    k<<<(W->n + MOVE64_SWIMMERS - 1) / MOVE64_SWIMMERS, MOVE64_BLOCK, 0, L->stream>>>(
+    const bool wide = wide_particle_index(L), many = 2ll * W->n >= MOVE64_MANY_FROM;
+    constexpr int FEW = MOVE64_FEW, MANY = MOVE64_MANY;
+    auto k = to     ? (wide ? k_swimmers_move_f64<true, FEW, long long>
+                            : k_swimmers_move_f64<true, FEW, int>)
+             : many ? (wide ? k_swimmers_move_f64<false, MANY, long long>
+                            : k_swimmers_move_f64<false, MANY, int>)
+                    : (wide ? k_swimmers_move_f64<false, FEW, long long>
+                            : k_swimmers_move_f64<false, FEW, int>);
+    const int points = !to && many ? MANY : FEW;
+    k<<<(int)((2ll * W->n + points - 1) / points), move64_block(points), 0, L->stream>>>(
         W->n, W->r, W->v, W->nv, W->common, W->seed, W->step, D, u, L->status,
         to ? *to : RecordTarget<double>{});
   }
@@ -2619,16 +2635,19 @@ static void tracers_move_on(Tracers* T, Lattice* L, cudaStream_t stream) {
   const Dims D = make_dims(L);
   if (L->precision == LBSWIM_F64) {
     const double* u = (const double*)L->u;
-    const int grid = (T->n + MOVE64_POINTS - 1) / MOVE64_POINTS;
-    if (L->compat & LBSWIM_COMPAT_EXACT_F64)
+    if (L->compat & LBSWIM_COMPAT_EXACT_F64) {
       k_tracers_move_exact<<<(T->n + EXACT_MOVE_BLOCK - 1) / EXACT_MOVE_BLOCK, EXACT_MOVE_BLOCK,
                              0, stream>>>(T->n, T->r, T->s, T->v, D, u, L->status);
-    else if (wide_particle_index(L))
-      k_tracers_move_f64<long long><<<grid, MOVE64_BLOCK, 0, stream>>>(T->n, T->r, T->s, T->v, D,
-                                                                       u, L->status);
-    else
-      k_tracers_move_f64<int><<<grid, MOVE64_BLOCK, 0, stream>>>(T->n, T->r, T->s, T->v, D, u,
-                                                                 L->status);
+    } else {
+      const bool far = wide_particle_index(L), many = T->n >= MOVE64_MANY_FROM;
+      const int points = many ? MOVE64_MANY : MOVE64_FEW;
+      auto k = many ? (far ? k_tracers_move_f64<MOVE64_MANY, long long>
+                           : k_tracers_move_f64<MOVE64_MANY, int>)
+                    : (far ? k_tracers_move_f64<MOVE64_FEW, long long>
+                           : k_tracers_move_f64<MOVE64_FEW, int>);
+      k<<<(T->n + points - 1) / points, move64_block(points), 0, stream>>>(T->n, T->r, T->s, T->v,
+                                                                           D, u, L->status);
+    }
   }
   else {
     const bool far = wide_particle_index(L), wide = T->n >= TRACERS_WIDE_FROM;

@@ -54,8 +54,9 @@ TOL = (3 * 4 * 2.0 ** -54 + 70 * 2.0 ** -53)
 
 
 @pytest.mark.parametrize("kind", ["plain", "rest", "mixed", "tiny", "small"])
+# one point a block or many, and both block shapes
 @pytest.mark.parametrize("size,n", [((8, 9, 33), 130), ((16, 5, 7), 64), ((1, 2, 3), 33),
-                                    ((4, 1, 40), 1)])
+                                    ((4, 1, 40), 1), ((12, 16, 40), 17001)])
 @pytest.mark.parametrize("compat", [0, _lib.COMPAT_WIDE_INDEX, _lib.COMPAT_EXACT_F64])
 def test_moves(kind, size, n, compat):
     rng = np.random.default_rng([n, len(kind)])
