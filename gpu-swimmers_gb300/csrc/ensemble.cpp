@@ -1,15 +1,15 @@
 // ensemble.cpp -- batched ensembles: many independent FP32 solves (each a
 // lattice with its swimmers and tracers) advanced together.
 //
-// One batched step is five launches over all members: the step counter, a
-// reset of the slab counts, the dipole-end records of every swimmer array (listed under the
-// slabs they touch), one persistent step kernel that takes the slabs of every
-// member from a shared counter, and one move kernel over every swimmer and
-// tracer array.  Everything the kernels need comes from device tables, so the
-// launches of two consecutive steps are captured once into a CUDA graph and
-// replayed; a change of membership rewrites the tables only.  Members keep
-// their buffers: the run starts from, and leaves, each member's state exactly
-// as the single-lattice calls would.
+// One batched step is two launches over all members: one persistent step kernel
+// that takes the slabs of every member from a shared counter, and one move kernel
+// over every swimmer and tracer array, which also makes the dipole-end records of
+// the next step (listed under the slabs they touch).  A run begins with a reset of
+// the slab counts and the records of its first step.  Everything the kernels need
+// comes from device tables, so the launches of two consecutive steps are captured
+// once into a CUDA graph and replayed; a change of membership rewrites the tables
+// only.  Members keep their buffers: the run starts from, and leaves, each
+// member's state exactly as the single-lattice calls would.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -30,7 +30,8 @@ struct Ensemble {
   int capacity = 0;
   void* tables = nullptr;  // one device allocation for all tables
   EnsTable t{};
-  std::vector<EnsMember> hmem;
+  std::vector<EnsMember> hmem;  // by position in the run: longest slabs first
+  std::vector<int> order;       // the member at a position
   std::vector<int> pre[4];
   cudaStream_t stream = nullptr;
   cudaEvent_t done = nullptr;
@@ -86,7 +87,7 @@ static void ensure_tables(Ensemble* E, int cap) {
   const size_t o_n = take(sizeof(int)), o_mem = take(sizeof(EnsMember) * cap);
   size_t o_pre[4];
   for (int i = 0; i < 4; ++i) o_pre[i] = take(sizeof(int) * (cap + 1));
-  const size_t o_cnt = take(2 * sizeof(unsigned)), o_step = take(sizeof(long long));
+  const size_t o_cnt = take(2 * sizeof(unsigned)), o_step = take(2 * sizeof(long long));
   LB_CUDA(cudaMalloc(&E->tables, off));
   LB_CUDA(cudaMemset(E->tables, 0, off));
   char* b = (char*)E->tables;
@@ -133,8 +134,6 @@ static void capture(Ensemble* E, int nsteps_in_graph, cudaGraphExec_t* out) {
   cudaGraph_t g = nullptr;
   LB_CUDA(cudaStreamBeginCapture(E->stream, cudaStreamCaptureModeThreadLocal));
   for (int p = 0; p < nsteps_in_graph; ++p) {
-    ens_launch_reset(E->t, p, E->stream);
-    ens_launch_records(E->t, E->grid_rec, E->stream);
     ens_launch_step(E->t, p, E->grid_step, E->stream);
     ens_launch_move(E->t, p, E->grid_move, E->stream);
   }
@@ -181,13 +180,18 @@ static void build_tables(Ensemble* E) {
   E->hmem.assign(n, EnsMember{});
   for (auto& p : E->pre) p.assign(n + 1, 0);
   const std::vector<int> lx = slab_lengths(E);
+  // the queue hands out slabs by position: the short ones last, to level the CTAs
+  E->order.resize(n);
+  for (int i = 0; i < n; ++i) E->order[i] = i;
+  std::stable_sort(E->order.begin(), E->order.end(), [&](int a, int b) { return lx[a] > lx[b]; });
   for (int m = 0; m < n; ++m) {
-    Lattice* L = E->lat[m];
-    Swimmers* W = E->sw[m];
-    Tracers* T = E->tr[m];
+    const int i = E->order[m];
+    Lattice* L = E->lat[i];
+    Swimmers* W = E->sw[i];
+    Tracers* T = E->tr[i];
     EnsMember& M = E->hmem[m];
     const int nsw = W ? W->n : 0, ntr = T ? T->n : 0;
-    M.lx = lx[m];
+    M.lx = lx[i];
     spread_reserve(L, 2 * nsw, M.lx);
     for (int a = 0; a < 3; ++a) M.size[a] = L->size[a];
     M.n = L->n;
@@ -234,6 +238,21 @@ static void build_tables(Ensemble* E) {
   }
 }
 
+// The tables of the run to the device, and what precedes its first step.
+static void begin_run(Ensemble* E) {
+  const int n = (int)E->hmem.size();
+  LB_CUDA(cudaMemcpyAsync(E->t.nmem, &n, sizeof(int), cudaMemcpyHostToDevice, E->stream));
+  LB_CUDA(cudaMemcpyAsync(E->t.mem, E->hmem.data(), sizeof(EnsMember) * n,
+                          cudaMemcpyHostToDevice, E->stream));
+  int* pre_dev[4] = {E->t.tile_prefix, E->t.rec_prefix, E->t.sw_prefix, E->t.tr_prefix};
+  for (int i = 0; i < 4; ++i)
+    LB_CUDA(cudaMemcpyAsync(pre_dev[i], E->pre[i].data(), sizeof(int) * (n + 1),
+                            cudaMemcpyHostToDevice, E->stream));
+  LB_CUDA(cudaMemsetAsync(E->t.g_step, 0, 2 * sizeof(long long), E->stream));
+  ens_launch_reset(E->t, E->stream);
+  ens_launch_records(E->t, E->grid_rec, E->stream);
+}
+
 void ensemble_step(Ensemble* E, int nsteps, const int* limits) {
   const int n = (int)E->lat.size();
   if (n == 0 || nsteps <= 0) return;
@@ -243,28 +262,22 @@ void ensemble_step(Ensemble* E, int nsteps, const int* limits) {
   build_tables(E);
   std::vector<int> took(n);
   for (int m = 0; m < n; ++m) {
-    took[m] = limits ? std::max(0, std::min(nsteps, limits[m])) : nsteps;
+    const int i = E->order[m];
+    took[m] = limits ? std::max(0, std::min(nsteps, limits[i])) : nsteps;
     E->hmem[m].limit = took[m];
   }
-  LB_CUDA(cudaMemcpyAsync(E->t.nmem, &n, sizeof(int), cudaMemcpyHostToDevice, E->stream));
-  LB_CUDA(cudaMemcpyAsync(E->t.mem, E->hmem.data(), sizeof(EnsMember) * n,
-                          cudaMemcpyHostToDevice, E->stream));
-  int* pre_dev[4] = {E->t.tile_prefix, E->t.rec_prefix, E->t.sw_prefix, E->t.tr_prefix};
-  for (int i = 0; i < 4; ++i)
-    LB_CUDA(cudaMemcpyAsync(pre_dev[i], E->pre[i].data(), sizeof(int) * (n + 1),
-                            cudaMemcpyHostToDevice, E->stream));
-  const long long start = -1;
-  LB_CUDA(cudaMemcpyAsync(E->t.g_step, &start, sizeof(start), cudaMemcpyHostToDevice,
-                          E->stream));
+  begin_run(E);
   if (!E->g2) capture(E, 2, &E->g2);
   if (!E->g1) capture(E, 1, &E->g1);
   for (int i = 0; i < nsteps / 2; ++i) LB_CUDA(cudaGraphLaunch(E->g2, E->stream));
   if (nsteps & 1) LB_CUDA(cudaGraphLaunch(E->g1, E->stream));
-  count_launches(5ull * nsteps);
+  count_launches(2ull * nsteps);
+  ens_launch_finish(E->t, n, E->stream);
   // the host copies above must outlive the copies: wait for the run
   LB_CUDA(cudaStreamSynchronize(E->stream));
   for (int m = 0; m < n; ++m) {
-    Lattice* L = E->lat[m];
+    const int i = E->order[m];
+    Lattice* L = E->lat[i];
     const int k = took[m];
     if (k == 0) continue;
     if (k & 1) {
@@ -276,12 +289,11 @@ void ensemble_step(Ensemble* E, int nsteps, const int* limits) {
     L->shadow_f_version = 0;  // rho, u of the last step are published
     L->force_version++;
     L->force_zero_pending = true;
-    L->spread.pending = 2 * (E->sw[m] ? E->sw[m]->n : 0);
+    L->spread.pending = 2 * (E->sw[i] ? E->sw[i]->n : 0);
     L->spread.stepped = true;
-    L->spread.bucket_tile = L->fused_tile;
-    L->spread.lx = E->hmem[m].lx;
-    if (E->sw[m]) E->sw[m]->step += k;
-    if (E->tr[m]) E->tr[m]->moves_since_sort += k;
+    L->spread.bucket_tile = -1;  // the step kernel has emptied the buckets
+    if (E->sw[i]) E->sw[i]->step += k;
+    if (E->tr[i]) E->tr[i]->moves_since_sort += k;
   }
 }
 
@@ -336,8 +348,7 @@ static float time_shape(int nx, int ny, int nz, int tile, int copies) {
     ensemble_step(E, 2);  // warm-up, graphs
     // the timed replays below run past that call's step count: no member limit
     for (auto& M : E->hmem) M.limit = 1 << 30;
-    LB_CUDA(cudaMemcpyAsync(E->t.mem, E->hmem.data(), sizeof(EnsMember) * E->hmem.size(),
-                            cudaMemcpyHostToDevice, E->stream));
+    begin_run(E);
     LB_CUDA(cudaEventCreate(&e0));
     LB_CUDA(cudaEventCreate(&e1));
     LB_CUDA(cudaEventRecord(e0, E->stream));

@@ -758,10 +758,17 @@ constexpr int ENS_STEP_SMEM =
         : fused_smem_bytes<16, 16, true>();
 static_assert(8 * 32 == 16 * 16, "both slab shapes use the same block");
 
+// The kernel leaves the counts at zero, and the words of the other parity, for the
+// records that the move makes for the next step.  (A quarter of the slabs of a
+// batch of 96 members has no ends; the code of a step without forces for those,
+// compiled in beside the rest, took the registers of both: 432 against 386 us a
+// step.)
 __global__ void __launch_bounds__(8 * 32 + FUSED_RING_THREADS, 2) k_ens_step(EnsTable t, int parity) {
   __shared__ int s_tile;
   const int nmem = *t.nmem;
   const int total = t.tile_prefix[nmem];
+  const long long g = t.g_step[parity];
+  if (blockIdx.x == 0 && threadIdx.x == 0) t.counters[parity ^ 1] = 0u;
   for (;;) {
     if (threadIdx.x == 0) s_tile = (int)atomicAdd(&t.counters[parity], 1u);
     __syncthreads();
@@ -770,12 +777,13 @@ __global__ void __launch_bounds__(8 * 32 + FUSED_RING_THREADS, 2) k_ens_step(Ens
     if (tile >= total) break;
     const int m = ens_member_of(t.tile_prefix, nmem, tile);
     const EnsMember& M = t.mem[m];
-    if (*t.g_step >= M.limit) {  // the member has taken its steps of this run
+    if (g >= M.limit) {  // the member has taken its steps of this run
       __syncthreads();
       continue;
     }
     const int lt = tile - t.tile_prefix[m];
     const int tz = lt % M.nt[2], ty = (lt / M.nt[2]) % M.nt[1], tx = lt / (M.nt[2] * M.nt[1]);
+    if (lt == 0 && threadIdx.x == 0) M.max_abs_f[parity ^ 1] = 0u;
     FusedArgs a{};
     a.f_old = M.f[parity];
     a.f_new = M.f[parity ^ 1];
@@ -789,7 +797,7 @@ __global__ void __launch_bounds__(8 * 32 + FUSED_RING_THREADS, 2) k_ens_step(Ens
     a.rho0 = M.rho0;
     a.k = Relax<float>{M.omega_s, M.omega_b, M.force_s, M.force_b};
     a.spread = SlabEnds{(const EndRecord<float>*)M.ends, M.bucket_count, M.bucket_list,
-                        2 * M.nsw, M.max_abs_f};
+                        2 * M.nsw, M.max_abs_f + parity};
     a.status = M.status;
     // members have few enough swimmers for split force sums on every slab
     // (checked when the members are set)
@@ -798,6 +806,7 @@ __global__ void __launch_bounds__(8 * 32 + FUSED_RING_THREADS, 2) k_ens_step(Ens
     else
       fused_slab<float, 32, 8, true, int, true>(a, tz, ty, tx, lt);
     __syncthreads();
+    if (threadIdx.x == 0) M.bucket_count[lt] = 0u;  // every thread has read it
   }
 }
 

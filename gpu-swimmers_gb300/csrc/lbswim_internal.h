@@ -81,7 +81,9 @@ struct SpreadScratch {
   size_t ends_bytes = 0;
   int pending = 0;
   bool stepped = false;  // a Step already consumed the pending ends
-  unsigned* max_abs_force = nullptr;  // device: largest |F| component of the pending ends
+  // device: largest |F| component of the pending ends, and a second word that a
+  // batched run alternates with
+  unsigned* max_abs_force = nullptr;
   TileLists ftiles;      // force tiles of a dense FP64 suspension
   int max_slot = 0;      // FP64: which of the two max-force words is in use
   // slab buckets of the pending ends, filled as the ends are recorded; an FP64
@@ -238,7 +240,7 @@ struct EnsMember {
   void* ends;           // EndRecord<float>[2 nsw]
   unsigned* bucket_count;
   int* bucket_list;
-  unsigned* max_abs_f;
+  unsigned* max_abs_f;  // [2] by the parity of the step that reads it
   int nsw;
   double* sw_r;
   double* sw_v;
@@ -263,16 +265,17 @@ struct EnsTable {
   int* sw_prefix;      // [capacity + 1] first swimmer-move block
   int* tr_prefix;      // [capacity + 1] first tracer-move block
   unsigned* counters;  // [2] slab counters of the two relative parities
-  long long* g_step;   // steps of the current run, -1 before its first
+  long long* g_step;   // [2] step of the current run, by its parity
 };
 
 // Work items per block of the batched kernels (particles.cu checks them).
 constexpr int ENS_ENDS_PER_BLOCK = 64;
 constexpr int ENS_SWIMMERS_PER_BLOCK = 32;
-constexpr int ENS_TRACERS_PER_BLOCK = 256;
+constexpr int ENS_TRACERS_PER_BLOCK = 64;
 
 // Launches of the batched step (lattice.cu, particles.cu).
-void ens_launch_reset(const EnsTable& t, int parity, cudaStream_t s);
+void ens_launch_reset(const EnsTable& t, cudaStream_t s);
+void ens_launch_finish(const EnsTable& t, int members, cudaStream_t s);
 void ens_launch_records(const EnsTable& t, int grid, cudaStream_t s);
 void ens_launch_step(const EnsTable& t, int parity, int grid, cudaStream_t s);
 void ens_launch_move(const EnsTable& t, int parity, int grid, cudaStream_t s);

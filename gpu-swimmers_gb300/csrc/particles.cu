@@ -1633,7 +1633,7 @@ __global__ void __launch_bounds__(MOVE_BLOCK) k_tracers_move_f32(
 // swimmer p % 32).
 constexpr int MOVE_SWIMMERS = MOVE_POINTS / 2;
 static_assert(2 * MOVE_SWIMMERS == REC_ENDS, "the ends of a block's swimmers");
-template <bool RECORD, class I = int>
+template <bool RECORD, class I = int, bool BUCKETS = false>
 __device__ __forceinline__ void swimmers_move_block(
     int blk, int nsw, double* __restrict__ swr, double* __restrict__ swv,
     double* __restrict__ swn, const lbswim_common_params& c, unsigned long long seed,
@@ -1692,7 +1692,7 @@ __device__ __forceinline__ void swimmers_move_block(
     nn = __dmul_rn(nn, f2d_exact(1.f / sqrtf(sq)));
   }
   if (update && (tumble || rotate)) swn[at] = nn;
-  if constexpr (RECORD) {
+  if (RECORD && to.ends) {  // uniform in the block
     __shared__ double moved[2][3][MOVE_SWIMMERS];
     __shared__ EndRecord<float> srec[REC_ENDS];
     __shared__ unsigned smax;
@@ -1706,7 +1706,7 @@ __device__ __forceinline__ void swimmers_move_block(
     unsigned big = 0u;
     if (valid)
       big = record_axis32(moved[0][a][q], moved[1][a][q], rear, c.P, c.l, D, a, srec[e]);
-    finish_records32<false>(e, a, blk * REC_ENDS, 2 * nsw, 0, big, srec, smax, D, to);
+    finish_records32<BUCKETS>(e, a, blk * REC_ENDS, 2 * nsw, 0, big, srec, smax, D, to);
   }
 }
 
@@ -1743,81 +1743,100 @@ __device__ __forceinline__ Dims ens_dims(const EnsMember& M) {
   return D;
 }
 
-// Advance the run's step counter (its own launch, so that every block of the
-// step's kernels reads the same step index).
-__global__ void k_ens_tick(EnsTable t) { *t.g_step += 1; }
+__device__ __forceinline__ TileGrid ens_grid(const EnsMember& M) {
+  TileGrid G;
+  G.T[0] = M.lx;
+  G.T[1] = M.tile == 1 ? 16 : 8;  // as slab_section_of
+  G.T[2] = M.tile == 1 ? 16 : 32;
+  G.h = 1;
+  G.by[0] = FastDiv{M.by_lx[0], M.by_lx[1]};
+  for (int a = 0; a < 3; ++a) {
+    G.nt[a] = M.nt[a];
+    if (a) G.by[a] = FastDiv{1u, (unsigned)__ffs(G.T[a]) - 1u};  // powers of two
+  }
+  return G;
+}
 
-// Zero the slab counts and largest |F| of every member still stepping, and
-// the slab counter of this parity.
-
-__global__ void k_ens_reset(EnsTable t, int parity) {
+// Before a run: zero the slab counts and largest |F| of every member that steps,
+// and the slab counters.
+__global__ void k_ens_reset(EnsTable t) {
   const int nmem = *t.nmem;
-  if (blockIdx.x == 0 && threadIdx.x == 0) t.counters[parity] = 0u;
-  const long long g = *t.g_step;
+  if (blockIdx.x == 0 && threadIdx.x < 2) t.counters[threadIdx.x] = 0u;
   for (int m = blockIdx.x; m < nmem; m += gridDim.x) {
     const EnsMember& M = t.mem[m];
-    if (g >= M.limit) continue;
+    if (M.limit <= 0) continue;
     const int nslabs = M.nt[0] * M.nt[1] * M.nt[2];
     for (int i = threadIdx.x; i < nslabs; i += blockDim.x) M.bucket_count[i] = 0u;
-    if (threadIdx.x == 0) *M.max_abs_f = 0u;
+    if (threadIdx.x < 2) M.max_abs_f[threadIdx.x] = 0u;
   }
 }
 
+// After a run: the largest |F| of a member's last step to the first word, beside
+// its records (a member's last move makes none).
+__global__ void k_ens_finish(EnsTable t) {
+  const int m = blockIdx.x * blockDim.x + threadIdx.x;
+  if (m >= *t.nmem) return;
+  const EnsMember& M = t.mem[m];
+  if (M.limit > 0) M.max_abs_f[0] = M.max_abs_f[(M.limit - 1) & 1];
+}
+
+// The records of a run's first step; the later ones' are made by the moves.
 __global__ void __launch_bounds__(REC_THREADS) k_ens_records(EnsTable t) {
   const int nmem = *t.nmem;
   const int total = t.rec_prefix[nmem];
   for (int vb = blockIdx.x; vb < total; vb += gridDim.x) {
     const int m = ens_find(t.rec_prefix, nmem, vb);
     const EnsMember& M = t.mem[m];
-    if (*t.g_step >= M.limit) continue;
-    TileGrid G;
-    G.T[0] = M.lx;
-    G.T[1] = M.tile == 1 ? 16 : 8;  // as slab_section_of
-    G.T[2] = M.tile == 1 ? 16 : 32;
-    G.h = 1;
-    G.by[0] = FastDiv{M.by_lx[0], M.by_lx[1]};
-    for (int a = 0; a < 3; ++a) {
-      G.nt[a] = M.nt[a];
-      if (a) G.by[a] = FastDiv{1u, (unsigned)__ffs(G.T[a]) - 1u};  // powers of two
-    }
+    if (M.limit <= 0) continue;
     end_records_block(vb - t.rec_prefix[m], M.nsw, M.sw_r, M.sw_n, M.common.P, M.common.l,
                       ens_dims(M), 0,
-                      RecordTarget<float>{(EndRecord<float>*)M.ends, M.max_abs_f, G,
+                      RecordTarget<float>{(EndRecord<float>*)M.ends, M.max_abs_f, ens_grid(M),
                                           M.bucket_count, M.bucket_list});
     __syncthreads();
   }
 }
 
 static_assert(ENS_ENDS_PER_BLOCK == REC_ENDS && ENS_SWIMMERS_PER_BLOCK == MOVE_SWIMMERS &&
-                  ENS_TRACERS_PER_BLOCK == WIDE_TRACERS,
+                  ENS_TRACERS_PER_BLOCK == MOVE_POINTS,
               "batched work items per block");
 
+// The moves of a step, and the records of the next one (none by a member's last
+// move, so that its records stay those of the forces of its last step).
 __global__ void __launch_bounds__(MOVE_BLOCK) k_ens_move(EnsTable t, int parity) {
   const int nmem = *t.nmem;
   const int nsb = t.sw_prefix[nmem], total = nsb + t.tr_prefix[nmem];
-  const unsigned long long g = (unsigned long long)*t.g_step;
+  const unsigned long long g = (unsigned long long)t.g_step[parity];
+  if (blockIdx.x == 0 && threadIdx.x == 0) t.g_step[parity ^ 1] = (long long)g + 1;
   for (int vb = blockIdx.x; vb < total; vb += gridDim.x) {
     if (vb < nsb) {
       const int m = ens_find(t.sw_prefix, nmem, vb);
       const EnsMember& M = t.mem[m];
       if ((long long)g >= M.limit) continue;  // uniform in the block: no barrier skipped
-      swimmers_move_block<false>(vb - t.sw_prefix[m], M.nsw, M.sw_r, M.sw_v, M.sw_n, M.common, M.seed,
-                          M.step0 + g, ens_dims(M), (const float4*)M.hyd[parity], M.status);
+      const bool more = (long long)g + 1 < M.limit;
+      swimmers_move_block<true, int, true>(
+          vb - t.sw_prefix[m], M.nsw, M.sw_r, M.sw_v, M.sw_n, M.common, M.seed, M.step0 + g,
+          ens_dims(M), (const float4*)M.hyd[parity], M.status,
+          RecordTarget<float>{more ? (EndRecord<float>*)M.ends : nullptr,
+                              M.max_abs_f + (parity ^ 1), ens_grid(M), M.bucket_count,
+                              M.bucket_list});
     } else {
       const int m = ens_find(t.tr_prefix, nmem, vb - nsb);
       const EnsMember& M = t.mem[m];
       if ((long long)g >= M.limit) continue;
-      tracers_move_wide_block(vb - nsb - t.tr_prefix[m], M.ntr, M.tr_r, M.tr_s, M.tr_v, ens_dims(M),
-                         (const float4*)M.hyd[parity], M.status);
+      tracers_move_block<int>(vb - nsb - t.tr_prefix[m], M.ntr, M.tr_r, M.tr_s, M.tr_v,
+                              ens_dims(M), (const float4*)M.hyd[parity], M.status);
     }
     __syncthreads();
   }
 }
 
-void ens_launch_reset(const EnsTable& t, int parity, cudaStream_t s) {
-  k_ens_tick<<<1, 1, 0, s>>>(t);
-  k_ens_reset<<<152, 256, 0, s>>>(t, parity);
-  LB_CHECK_LAUNCH(2);
+void ens_launch_reset(const EnsTable& t, cudaStream_t s) {
+  k_ens_reset<<<152, 256, 0, s>>>(t);
+  LB_CHECK_LAUNCH(1);
+}
+void ens_launch_finish(const EnsTable& t, int members, cudaStream_t s) {
+  k_ens_finish<<<(members + 255) / 256, 256, 0, s>>>(t);
+  LB_CHECK_LAUNCH(1);
 }
 void ens_launch_records(const EnsTable& t, int grid, cudaStream_t s) {
   k_ens_records<<<grid, REC_THREADS, 0, s>>>(t);
@@ -2091,7 +2110,7 @@ static void grow_buckets(Lattice* L, int nslabs, unsigned*& count, int*& list, i
 void spread_reserve(Lattice* L, int nends, int lx) {
   ensure_ends(L, nends);
   SpreadScratch& S = L->spread;
-  if (!S.max_abs_force) LB_CUDA(cudaMalloc(&S.max_abs_force, sizeof(unsigned)));
+  if (!S.max_abs_force) LB_CUDA(cudaMalloc(&S.max_abs_force, 2 * sizeof(unsigned)));
   grow_buckets(L, slabs_of(slab_grid(L, lx)), S.bucket_count, S.bucket_list, S.bucket_slabs);
   S.bucket_tile = -1;
 }
@@ -2162,7 +2181,7 @@ static void append_ends(Swimmers* W, Lattice* L) {
   SpreadScratch& S = L->spread;
   const int nends = 2 * W->n;
   ensure_ends(L, S.pending + nends);
-  if (!S.max_abs_force) LB_CUDA(cudaMalloc(&S.max_abs_force, sizeof(unsigned)));
+  if (!S.max_abs_force) LB_CUDA(cudaMalloc(&S.max_abs_force, 2 * sizeof(unsigned)));
   if (S.pending == 0) {
     S.bucket_tile = -1;
     const int expected = std::max(nends, S.last_pending);
@@ -2343,7 +2362,7 @@ void swimmers_prepare_room(Swimmers* const* w, int nw, Lattice* L) {
     P.capacity_ends = cap;
     P.ends_bytes = sizeof(EndRecord<float>) * cap;
   }
-  if (!P.max_abs_force) LB_CUDA(cudaMalloc(&P.max_abs_force, sizeof(unsigned)));
+  if (!P.max_abs_force) LB_CUDA(cudaMalloc(&P.max_abs_force, 2 * sizeof(unsigned)));
   P.clear_max = true;
   if (nends > DIRECT_ENDS) {
     P.lx = choose_slab_lx(L->size, L->fused_tile, nends);
