@@ -492,6 +492,17 @@ static_assert(2 * (fused_smem_total<float, 32, 8, true, true>() + 1024) <= 228 *
 static_assert(2 * (fused_smem_bytes<32, 8, true>() + 1024) <= 132 * 1024, "SPREAD slab smem");
 static_assert(2 * (fused_smem_bytes<16, 16, true>() + 1024) <= 132 * 1024, "SPREAD slab smem");
 
+// CTAs per SM.  The kernels wait on the chain between their barriers, and a third
+// CTA fills in for 16-bit storage, whose loads in flight fit the L1 cache that is
+// left (BF16 192x200x208: 304 -> 274 us with ends, 217 -> 183 without); FP32's do
+// not (256^3 with ends: 514 -> 561, or 520 with 144 ends held per slab in place
+// of 256).
+template <class S, bool TMA>
+constexpr int fused_ctas() { return sizeof(S) == 2 && !TMA ? 3 : 2; }
+// Whether the next plane's loads follow the collision (see fused_slab).
+template <class S, bool SPREAD, bool TMA>
+constexpr bool fused_late_loads() { return (SPREAD || sizeof(S) == 2) && !TMA; }
+
 // One slab: tile (tz, ty, tx) of the lattice in units of (TZ, TY, a.lx)
 // sites; `slab` indexes its bucket of pending ends.  Called by one CTA.
 // I is the site-index type: int when 15 N fits it (one multiply-add per
@@ -614,14 +625,15 @@ __device__ __forceinline__ void fused_slab(const FusedArgs& a, int tz, int ty, i
   float keep0 = 0.f, keep1a = 0.f, keep1b = 0.f;
   int k3 = 0;  // k % 3
   for (int k = 0; k < ex + 2; ++k) {
-    // The SPREAD instances, bound by the chain between their barriers rather than by
-    // DRAM, load the next plane into the registers that the collision has just
-    // freed (256^3 521 -> 516 us, BF16 314 -> 307, 100x75x130 51.7 -> 49.5); the
-    // others issue the loads first, to have them in flight for the whole plane, and
-    // copy.
+    // The instances bound by the chain between their barriers rather than by DRAM load
+    // the next plane into the registers that the collision has just freed (256^3
+    // with ends 521 -> 516 us, 100x75x130 51.7 -> 49.5; it leaves 56 registers a
+    // thread, which 16-bit storage's third CTA needs); the others issue the loads
+    // first, to have them in flight for the whole plane, and copy.
+    constexpr bool LATE = fused_late_loads<S, SPREAD, TMA>();
     float held[18];
-    float(&cur)[18] = SPREAD && !TMA ? pre : held;
-    if (!SPREAD || TMA) {
+    float(&cur)[18] = LATE ? pre : held;
+    if (!LATE) {
 #pragma unroll
       for (int i = 0; i < 18; ++i) held[i] = pre[i];
       if (active && k + 1 < ex + 2) load(wrap_once(x0 + k, nx));
@@ -666,7 +678,7 @@ __device__ __forceinline__ void fused_slab(const FusedArgs& a, int tz, int ty, i
       new2 = d[2];
     }
     const float Fn0 = cur[15], Fn1 = cur[16], Fn2 = cur[17];
-    if (SPREAD && !TMA && active && k + 1 < ex + 2) load(wrap_once(x0 + k, nx));
+    if (LATE && active && k + 1 < ex + 2) load(wrap_once(x0 + k, nx));
     __syncthreads();
     if constexpr (TMA) {
       // every thread has read stage k % 2: it takes plane k + 2
@@ -722,7 +734,8 @@ __device__ __forceinline__ void fused_slab(const FusedArgs& a, int tz, int ty, i
 }
 
 template <class S, int TZ, int TY, bool SPREAD, class I, bool TMA>
-__global__ void __launch_bounds__(TY * TZ + FUSED_RING_THREADS, 2) k_fused_step(FusedArgs a) {
+__global__ void __launch_bounds__(TY * TZ + FUSED_RING_THREADS, fused_ctas<S, TMA>())
+    k_fused_step(FusedArgs a) {
   const int slab = (blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
   for (int i = slab * blockDim.x + threadIdx.x; i < a.nclear;
        i += gridDim.x * gridDim.y * gridDim.z * blockDim.x)
@@ -1189,7 +1202,7 @@ static void fused_step_tile(Lattice* L, FusedArgs& a) {
     a.lx = sp.lx;
     launch_fused<S, TZ, TY, true>(L, a);
   } else {
-    a.lx = choose_slab_lx(L->size, L->fused_tile, 0);
+    a.lx = choose_slab_lx(L->size, L->fused_tile, 0, L->precision);
     launch_fused<S, TZ, TY, false>(L, a);
   }
 }
@@ -1228,17 +1241,17 @@ int slab_lx_within(const int size[3], int tile, long long nends, int cap) {
 
 // x planes per slab of a lattice stepped with nends pending ends, by the time
 // its slabs take: a slab takes lx + 2 planes (the ring) and a start that costs
-// about 3 more planes when it lists ends, 1 when not; 304 run at a time, and
+// about 3 more planes when it lists ends, 1 when not; 304 (or 456) run at a time, and
 // with half of them or fewer each has an SM to itself and takes about 0.65 of
 // the time a plane takes with two.  Ends listed in buckets cost an atomic per
 // slab they touch, about 1 + 5 / lx of them along x.  A small lattice then has
 // enough slabs for the SMs, and a large one wastes less of its last wave.
-int choose_slab_lx(const int size[3], int tile, long long nends) {
+int choose_slab_lx(const int size[3], int tile, long long nends, int precision) {
   int ty, tz;
   slab_section_of(tile, &ty, &tz);
   const long long section = (long long)((size[1] + ty - 1) / ty) * ((size[2] + tz - 1) / tz);
   const int longest = longest_slab(size, tile, nends);
-  constexpr int SLOTS = 304;
+  const int SLOTS = elem_bytes(precision) == 2 ? 456 : 304;  // fused_ctas
   int best = 1;
   double least = 0.0;
   for (int lx = 1; lx <= longest; ++lx) {

@@ -283,7 +283,7 @@ int ens_step_ctas_per_sm();
 // Cross-section (rows, columns) of the slabs of a tile choice, and the x planes
 // per slab of a lattice stepped with nends pending ends.
 void slab_section_of(int tile, int* ty, int* tz);
-int choose_slab_lx(const int size[3], int tile, long long nends);
+int choose_slab_lx(const int size[3], int tile, long long nends, int precision);
 // The same with slabs of at most `cap` planes, as even as they come.
 int slab_lx_within(const int size[3], int tile, long long nends, int cap);
 // Multiplier and shift of a division by lx (FastDiv).
