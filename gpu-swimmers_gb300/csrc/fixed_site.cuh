@@ -4,8 +4,8 @@
 // FP64 collision of a site (165 FP64 instructions and a division) took 5.16 ms
 // per step at 256^3, 8 times what its bytes take, with the FP64 pipe busy 86%
 // of the time; CalcHydro took 1.55 ms, 3.6 times its bytes'.  In integers they
-// take 0.73 ms (0.82 of the copy bandwidth; 0.88 ms with a force, 1350
-// instructions per warp, the integer pipe 74% busy) and 0.435 ms (the copy
+// take 0.73 ms (0.82 of the copy bandwidth; 0.86 ms with a force, 1330
+// instructions per warp, the integer pipe 73% busy) and 0.435 ms (the copy
 // bandwidth).
 // Here a site's 15 distributions become integers in units of 2^-59 of the
 // binade of its rest population (2^-62 at density 1, 8 units to the last bit
@@ -109,17 +109,23 @@ __host__ __device__ __forceinline__ bool site_to_fixed(const double d[15],
                                                        unsigned long long X[15], int& k) {
   const unsigned long long b0 = double_bits(d[0]);
   k = (int)(hi_word(b0) >> 20);  // with the sign: a negative d[0] gives k >= 2048
-  unsigned worst = 0u;
+  unsigned any = 0u;
 #pragma unroll
   for (int p = 0; p < 15; ++p) {
     const unsigned long long b = double_bits(d[p]);
-    // MAX_DROP less the binades below the rest population's; sign, zero, inf
-    // and nan wrap to a large value
+    // MAX_DROP less the binades below the rest population's, 0 to 7 when it fits;
+    // sign, zero, inf and nan wrap to a large value
     const unsigned up = (hi_word(b) >> 20) - (unsigned)(k - FIXED_MAX_DROP);
-    worst = up > worst ? up : worst;
-    X[p] = ((b & 0xfffffffffffffull) | 0x10000000000000ull) << (up & 31u);
+    any |= up;
+    const unsigned h = (hi_word(b) & 0xfffffu) | 0x100000u, l = (unsigned)b;
+#ifdef __CUDA_ARCH__
+    X[p] = ((unsigned long long)__funnelshift_l(l, h, up) << 32) | __funnelshift_l(0u, l, up);
+#else
+    X[p] = (((unsigned long long)h << 32) | l) << (up & 31u);
+#endif
   }
-  return worst <= (unsigned)FIXED_MAX_DROP && k >= FIXED_MIN_K && k <= FIXED_MAX_K;
+  static_assert((FIXED_MAX_DROP & (FIXED_MAX_DROP + 1)) == 0, "a mask tests the drops");
+  return any <= (unsigned)FIXED_MAX_DROP && k >= FIXED_MIN_K && k <= FIXED_MAX_K;
 }
 
 // x in the units of k, toward zero; false when |x| >= 2^56 units (a sixteenth

@@ -134,7 +134,9 @@ __device__ __forceinline__ void load_force(const T* F, long long N, long long s,
 // F64_THREADS + threadIdx.x of x plane blockIdx.y, so that a ragged nz idles
 // no lanes.  The collision runs on integers (fixed_site.cuh); the sites that do
 // not fit, and every site of a lattice whose relaxation constants do not, take
-// FP64 arithmetic.
+// FP64 arithmetic.  Bound by the integer pipe with a force: 32-bit offsets from
+// uniform bases and funnel shifts took the forced step at 256^3 from 878 to 861 us
+// (without a force 728 -> 734, by the bytes; CalcHydro at 65x47x90 10.5 -> 9.5).
 constexpr int F64_THREADS = 128;
 template <bool FORCED>
 __global__ void __launch_bounds__(F64_THREADS, 4) k_step_push_f64(const double* __restrict__ f,
@@ -147,14 +149,16 @@ __global__ void __launch_bounds__(F64_THREADS, 4) k_step_push_f64(const double* 
   const unsigned t = blockIdx.x * F64_THREADS + threadIdx.x;
   if (t >= nynz) return;
   const int x = blockIdx.y, y = (int)div_by(t, by_nz), z = (int)(t - (unsigned)y * nz);
-  const long long s = (long long)x * nynz + t;
+  // the plane's bases are uniform, the offsets 32 bits
+  f += (long long)x * nynz;
+  F += (long long)x * nynz;
   double d[15];
 #pragma unroll
-  for (int p = 0; p < 15; ++p) d[p] = f[p * N + s];
+  for (int p = 0; p < 15; ++p) d[p] = (f + p * N)[t];
   double Fa[3] = {0.0, 0.0, 0.0};
   if (FORCED) {
 #pragma unroll
-    for (int a = 0; a < 3; ++a) Fa[a] = F[a * N + s];
+    for (int a = 0; a < 3; ++a) Fa[a] = (F + a * N)[t];
   }
   unsigned long long X[15];
   int e;
@@ -171,18 +175,18 @@ __global__ void __launch_bounds__(F64_THREADS, 4) k_step_push_f64(const double* 
   } else {
     // read again, so that the distributions need no registers meanwhile
 #pragma unroll
-    for (int p = 0; p < 15; ++p) d[p] = f[p * N + s];
+    for (int p = 0; p < 15; ++p) d[p] = (f + p * N)[t];
     collide(d, Fa[0], Fa[1], Fa[2], 0.0, k, d);
   }
   const int xm = wrap_once(x - 1, nx), xp = wrap_once(x + 1, nx);
-  const int ym = wrap_once(y - 1, ny) * nz, yp = wrap_once(y + 1, ny) * nz, y0 = y * nz;
-  const int zm = wrap_once(z - 1, nz), zp = wrap_once(z + 1, nz);
+  const unsigned ym = wrap_once(y - 1, ny) * nz, yp = wrap_once(y + 1, ny) * nz, y0 = y * nz;
+  const unsigned zm = wrap_once(z - 1, nz), zp = wrap_once(z + 1, nz), zc = z;
 #pragma unroll
   for (int p = 0; p < 15; ++p) {
     const int dx = cx_of(p), dy = cy_of(p), dz = cz_of(p);
     const int X1 = dx > 0 ? xp : (dx < 0 ? xm : x);
-    const int Y1 = dy > 0 ? yp : (dy < 0 ? ym : y0);
-    const int Z1 = dz > 0 ? zp : (dz < 0 ? zm : z);
+    const unsigned Y1 = dy > 0 ? yp : (dy < 0 ? ym : y0);
+    const unsigned Z1 = dz > 0 ? zp : (dz < 0 ? zm : zc);
     (fn + p * N + (long long)X1 * nynz)[Y1 + Z1] = d[p];
   }
 }
