@@ -511,8 +511,8 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan_apply_total(
 //    in units of 2^-60 of the largest force, added as three words of 22, 22 and
 //    20 bits with shared-memory atomics that return nothing, and converted
 //    once.  All 32 lanes work on the nodes of an end.  Integer sums do not
-//    depend on their order.  256^3, 65,536 swimmers: 0.24 ms, against 0.71 ms
-//    in FP64 by site; 65x47x90: 12 us against 29.
+//    depend on their order.  256^3, 65,536 swimmers: 0.21 ms, against 0.71 ms
+//    in FP64 by site; 65x47x90: 10 us against 29.
 //  * k_force_tile (LBSWIM_COMPAT_EXACT_F64, and suspensions too dense for
 //    buckets): every site adds the ends that cover it in end order,
 //    ((phi_x phi_y) phi_z) F as the reference does (SwimmerArray.cu:64-73).  A
@@ -623,7 +623,7 @@ __device__ __forceinline__ void force_gather(const Dims& D, int kx, int ky, int 
   const bool zval = z < D.n[2];
   // no axis shorter than a stencil: one node of an end lands on a site
   const bool single = D.n[0] >= 4 && D.n[1] >= 4 && D.n[2] >= 4;
-  for (int row = warp; row < FT_X * FT_Y; row += FT_THREADS / 32) {
+  for (int row = warp; row < FT_X * FT_Y; row += blockDim.x / 32) {
     const int x = kx * FT_X + row / FT_Y, y = ky * FT_Y + row % FT_Y;
     if (x >= D.n[0] || y >= D.n[1]) continue;
     const long long s = (long long)x * D.n[1] * D.n[2] + (long long)y * D.n[2] + z;
@@ -742,7 +742,18 @@ static_assert(FF_ROW % 32 == 4 && FF_PLANE % 32 == 16 && FF_SITES % 4 == 0, "ban
 // a tile the units grow so that a site's sum stays within 62 bits.  Tiles whose
 // words could overflow (more than 1024 contributions a site), and forces that
 // are not finite or below 2^-894, take FP64 arithmetic in end order.
-__global__ void __launch_bounds__(FT_THREADS) k_force_fixed(
+// Issue-bound where most tiles have ends (64% of the slots; the scatter and the
+// conversions take 4500 warp instructions each of a tile's 10,000), so a thread's
+// sites differ in x alone and the record loads run under the zeroing: AddForces at
+// 256^3 255 -> 224 us, 128^3 with 40,000 swimmers 103 -> 92.  Up to FT_WIDE_TILES,
+// two to an SM, the chain of a block's phases bounds the launch: 512 threads
+// shorten each, and the list is read with its count: onto a force 64^3 (256
+// tiles) 20.0 -> 18.7 us and 24^3 18.6 -> 15.6, alone 16.8 and 15.2 either way;
+// with more tiles they cost occupancy (64x64x80, 384 tiles, 20.7 -> 21.9; 80^3
+// 18.8 -> 23.2; 256^3 224 -> 320).
+constexpr int FT_WIDE_TILES = 2 * 152;
+template <int THREADS>
+__global__ void __launch_bounds__(THREADS) k_force_fixed(
     Dims D, TileGrid G, const EndRecord<double>* __restrict__ ends, int nends,
     unsigned* __restrict__ count, const int* __restrict__ list,
     const unsigned* __restrict__ max_f, unsigned* __restrict__ next_max_f,
@@ -750,10 +761,18 @@ __global__ void __launch_bounds__(FT_THREADS) k_force_fixed(
   __shared__ __align__(16) unsigned sums[9 * FF_SITES];
   __shared__ Digits dig[15][FF_CHUNK];  // 12 weights, 3 force components per end
   __shared__ int org[3][FF_CHUNK];
-  const int tile = blockIdx.x, tid = threadIdx.x;
+  constexpr int WARPS = THREADS / 32;
+  static_assert(WARPS % FT_Y == 0 && FF_CHUNK == 32, "the mappings below");
+  const int tile = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int kz = tile % G.nt[2], ky = (tile / G.nt[2]) % G.nt[1], kx = tile / (G.nt[1] * G.nt[2]);
   // without buckets (DIRECT_ENDS_F64 ends at most) a tile goes through all of them
   const unsigned listed = count ? count[tile] : (unsigned)nends;
+  const long long s0 = (long long)tile * FT_CAP;
+  // entry of a chunk that this lane stages; few tiles read it before the count is
+  // known (the bucket has FT_CAP > lane of them), many tiles are mostly empty
+  constexpr bool EARLY = THREADS > FT_THREADS;
+  int mine = lane;
+  if (EARLY && count) mine = list[s0 + lane];
   const unsigned fmax = *max_f;
   const int kf = (int)(fmax >> 20);  // |F| < 2^(kf - 1022)
   const int cnt = fmax ? (int)listed : 0;  // no force at all: nothing to add
@@ -768,7 +787,7 @@ __global__ void __launch_bounds__(FT_THREADS) k_force_fixed(
   const int z0 = kz * FT_Z, y0 = ky * FT_Y, x0 = kx * FT_X;
   if (cnt == 0) {
     if (!accumulate)
-      for (int t = tid; t < FT_X * FT_Y * FT_Z; t += FT_THREADS) {
+      for (int t = tid; t < FT_X * FT_Y * FT_Z; t += THREADS) {
         const int z = z0 + t % FT_Z, y = y0 + (t / FT_Z) % FT_Y, x = x0 + t / (FT_Z * FT_Y);
         if (x >= D.n[0] || y >= D.n[1] || z >= D.n[2]) continue;
         const long long s = ((long long)x * D.n[1] + y) * D.n[2] + z;
@@ -781,37 +800,56 @@ __global__ void __launch_bounds__(FT_THREADS) k_force_fixed(
     force_gather<true>(D, kx, ky, kz, nends, rec, force, accumulate);
     return;
   }
-  for (int i = tid; i < 9 * FF_SITES / 4; i += FT_THREADS)
+  // the words of a chunk's records: lane q has end q, a warp every WARPS-th word;
+  // their way here is covered by the zeroing, or by the chunk before
+  constexpr int WORDS = (18 + WARPS - 1) / WARPS;
+  unsigned long long word[WORDS];
+  auto fetch = [&](int m) {
+    if (lane >= m) return;
+    const EndRecord<double>& e = ends[mine];
+#pragma unroll
+    for (int i = 0; i < WORDS; ++i) {
+      const int w = warp + i * WARPS;
+      if (w < 12) word[i] = double_bits(e.phi[w >> 2][w & 3]);
+      else if (w < 15) word[i] = double_bits(e.F[w - 12]);
+      else if (w < 18) word[i] = (unsigned)e.o[w - 15];
+    }
+  };
+  if (!EARLY && count && lane < cnt) mine = list[s0 + lane];
+  fetch(min(FF_CHUNK, cnt));
+  for (int i = tid; i < 9 * FF_SITES / 4; i += THREADS)
     reinterpret_cast<uint4*>(sums)[i] = make_uint4(0u, 0u, 0u, 0u);
   // coarser units by the doublings of the largest sum over 32 unfolded ends
   const int most = cnt * (fold > 1 ? 8 : 1);
   const int coarse = most > 32 ? 32 - __clz((most - 1) >> 5) : 0;
-  const int lane = tid & 31, warp = tid >> 5;
   const int jy = (lane >> 2) & 3, jz = lane & 3;
-  const long long s0 = (long long)tile * FT_CAP;
   for (int base = 0; base < cnt; base += FF_CHUNK) {
     const int m = min(FF_CHUNK, cnt - base);
-    __syncthreads();
-    for (int t = tid; t < 18 * FF_CHUNK; t += FT_THREADS) {
-      const int q = t % FF_CHUNK, w = t / FF_CHUNK;
-      if (q >= m) continue;
-      const EndRecord<double>& e = ends[count ? list[s0 + base + q] : base + q];
-      if (w < 12) {
-        dig[w][q] = digits((long long)double_bits(e.phi[w >> 2][w & 3]));
-      } else if (w < 15) {
-        // F in units of 2^(kf - 1022 - 62), to nearest
-        const unsigned long long b = double_bits(e.F[w - 12]);
-        const int drop = kf - (int)((hi_word(b) >> 20) & 0x7ffu);
-        const unsigned long long mant = ((b << 11) | 0x8000000000000000ull);
-        const unsigned long long v = drop > 61 ? 0ull : ((mant >> (drop + 1)) + 1) >> 1;
-        const long long sg = (long long)b >> 63;
-        dig[w][q] = digits(((long long)v ^ sg) - sg);
-      } else {
-        org[w - 15][q] = e.o[w - 15];
+    const int next = base + FF_CHUNK + lane;
+    if (next < cnt) mine = count ? list[s0 + next] : next;
+    if (base) __syncthreads();  // the chunk before has been added
+    if (lane < m) {
+#pragma unroll
+      for (int i = 0; i < WORDS; ++i) {
+        const int w = warp + i * WARPS;
+        const unsigned long long b = word[i];
+        if (w < 12) {
+          dig[w][lane] = digits((long long)b);
+        } else if (w < 15) {
+          // F in units of 2^(kf - 1022 - 62), to nearest
+          const int drop = kf - (int)((hi_word(b) >> 20) & 0x7ffu);
+          const unsigned long long mant = ((b << 11) | 0x8000000000000000ull);
+          const unsigned long long v = drop > 61 ? 0ull : ((mant >> (drop + 1)) + 1) >> 1;
+          const long long sg = (long long)b >> 63;
+          dig[w][lane] = digits(((long long)v ^ sg) - sg);
+        } else if (w < 18) {
+          org[w - 15][lane] = (int)b;
+        }
       }
     }
+    fetch(min(FF_CHUNK, cnt - base - FF_CHUNK));
     __syncthreads();
-    for (int q = warp; q < m; q += FT_THREADS / 32) {
+    for (int q = warp; q < m; q += WARPS) {
       const int ly = node_after(org[1][q], jy, D.n[1]) - y0;
       const int lz = node_after(org[2][q], jz, D.n[2]) - z0;
       const bool in_yz = (unsigned)ly < (unsigned)FT_Y && (unsigned)lz < (unsigned)FT_Z;
@@ -835,11 +873,14 @@ __global__ void __launch_bounds__(FT_THREADS) k_force_fixed(
     }
   }
   __syncthreads();
-  for (int t = tid; t < FT_X * FT_Y * FT_Z; t += FT_THREADS) {
-    const int lz = t % FT_Z, ly = (t / FT_Z) % FT_Y, lx = t / (FT_Z * FT_Y);
-    const int z = z0 + lz, y = y0 + ly, x = x0 + lx;
-    if (x >= D.n[0] || y >= D.n[1] || z >= D.n[2]) continue;
-    const unsigned* at = sums + lx * FF_PLANE + ly * FF_ROW + lz;
+  // a warp has one row of sites in every (WARPS / FT_Y)-th plane
+  const int ly = warp % FT_Y, y = y0 + ly, z = z0 + lane;
+  if (y >= D.n[1] || z >= D.n[2]) return;
+#pragma unroll
+  for (int i = 0; i < FT_X * FT_Y / WARPS; ++i) {
+    const int lx = warp / FT_Y + i * (WARPS / FT_Y), x = x0 + lx;
+    if (x >= D.n[0]) break;
+    const unsigned* at = sums + lx * FF_PLANE + ly * FF_ROW + lane;
     const long long s = ((long long)x * D.n[1] + y) * D.n[2] + z;
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
@@ -2013,7 +2054,9 @@ static void spread_fixed(Lattice* L, int nends) {
   const TileGrid G = force_tiles(L);
   const int ntiles = G.nt[0] * G.nt[1] * G.nt[2];
   unsigned* max_f = S.bucket_count + ntiles;
-  k_force_fixed<<<ntiles, FT_THREADS, 0, L->stream>>>(
+  const int threads = ntiles <= FT_WIDE_TILES ? 2 * FT_THREADS : FT_THREADS;
+  auto kernel = threads > FT_THREADS ? k_force_fixed<2 * FT_THREADS> : k_force_fixed<FT_THREADS>;
+  kernel<<<ntiles, threads, 0, L->stream>>>(
       make_dims(L), G, (const EndRecord<double>*)S.ends, nends,
       nends > DIRECT_ENDS_F64 ? S.bucket_count : nullptr, S.bucket_list,
       max_f + S.max_slot, max_f + (S.max_slot ^ 1), (double*)L->force,

@@ -96,3 +96,29 @@ def test_force_scales(P):
     largest = float(np.abs(X(P) * sw.n.data).max())
     tol = (count + 1) * 2.0 ** -52 * largest
     assert np.all(np.abs(lat.force.data.reshape(3, N) - force) <= tol)
+
+
+@pytest.mark.parametrize("size", [(75, 60, 50), (77, 60, 50)])  # 304 and 320 tiles
+@pytest.mark.parametrize("n,box", [(40, 1.0), (4000, 1.0), (100, 0.02), (190, 0.01)])
+def test_force_of_either_block_size(size, n, box):
+    rng = np.random.default_rng([n, size[0]])
+    lat = lb.Lattice(*size, 0.8, 0.8)
+    cp = swimmers.CommonParams()
+    cp.P, cp.l, cp.alpha, cp.mobility, cp.seed = 0.3, 0.4, 0.0, 1.0, 1
+    sw = swimmers.Array(n, cp)
+    sw.r[:] = rng.random((3, n)) * (box * np.array(size)[:, None])
+    nv = rng.standard_normal((3, n))
+    sw.n[:] = nv / np.linalg.norm(nv, axis=0)
+    sw.H2D()
+    lat.ZeroForce()
+    sw.AddForces(lat)
+    sw.AddForces(lat)
+    lat.force.D2H()
+    N = size[0] * size[1] * size[2]
+    force, count = np.zeros((3, N), X), np.zeros(N)
+    nv = sw.n.data
+    spread(force, count, size, sw.r.data - nv * 0.4, -0.3 * nv.astype(X))
+    spread(force, count, size, sw.r.data, 0.3 * nv.astype(X))
+    # as above, twice
+    tol = (2 * count + 1) * 2.0 ** -52 * 0.3
+    assert np.all(np.abs(lat.force.data.reshape(3, N) - 2 * force) <= tol)
