@@ -36,6 +36,7 @@ struct Ensemble {
   cudaStream_t stream = nullptr;
   cudaEvent_t done = nullptr;
   cudaGraphExec_t g2 = nullptr, g1 = nullptr;
+  bool longest_slabs = false;  // as in a run of many members (autotuner)
   int grid_step = 0, grid_rec = 0, grid_move = 0;
 };
 
@@ -146,11 +147,12 @@ static void capture(Ensemble* E, int nsteps_in_graph, cudaGraphExec_t* out) {
 // x planes per slab of every member.  304 CTAs take the slabs from one queue,
 // so a run lasts about the sum of their lx + 5 planes (ring and start) over 304
 // and half a slab more: long slabs for many members, short ones where few
-// members would leave CTAs without a slab.
+// members would leave CTAs without a slab.  (512 members of 16^3 to 48x48x96: 2.07 ms a
+// step with up to 60 planes, 2.12 with up to 32; 12 members want 2 to 8.)
 static std::vector<int> slab_lengths(const Ensemble* E) {
   std::vector<int> best;
   double least = 0.0;
-  for (int cap = 32; cap >= 2; cap /= 2) {
+  for (int cap = SLAB_LX_MAX; cap >= 2; cap = cap > 32 ? 32 : cap / 2) {
     std::vector<int> lx(E->lat.size());
     double planes = 0.0, longest = 0.0;
     for (size_t m = 0; m < lx.size(); ++m) {
@@ -168,6 +170,7 @@ static std::vector<int> slab_lengths(const Ensemble* E) {
       best = lx;
       least = cost;
     }
+    if (E->longest_slabs) break;
   }
   return best;
 }
@@ -299,9 +302,25 @@ void ensemble_step(Ensemble* E, int nsteps, const int* limits) {
 
 // ---- tile autotuner ---------------------------------------------------------
 // For each lattice shape among the members, time a batched run of scratch
-// copies with each slab shape and keep the faster one (cached per shape).
+// copies with each slab shape and keep the one with more slabs a second for the
+// slabs it takes (cached per shape).  The slabs are as long as in a run of many
+// members, and a part of a wave counts as that part: by the plain time of copies in
+// short slabs, 16^3 and 24^3 were given the slower shape and 48^3 not the faster
+// one (512 members 2.24 ms a step, 2.07 with this and the longer slabs).  A square
+// section as wide as the lattice meets its ends twice: 16^3 stays with 8 x 32 (53 of
+// the 512 members in 16 x 16: 2.12 ms).
 static std::mutex g_tune_mu;
 static std::map<std::tuple<int, int, int>, int> g_tuned;
+
+constexpr int TUNE_SWIMMERS = 64;
+
+static long long slabs_per_lattice(const int size[3], int tile, long long nends) {
+  int ty, tz;
+  slab_section_of(tile, &ty, &tz);
+  const int lx = slab_lx_within(size, tile, nends, SLAB_LX_MAX);
+  return (long long)((size[0] + lx - 1) / lx) * ((size[1] + ty - 1) / ty) *
+         ((size[2] + tz - 1) / tz);
+}
 
 static float time_shape(int nx, int ny, int nz, int tile, int copies) {
   std::vector<lbswim_lattice*> lats(copies, nullptr);
@@ -321,7 +340,7 @@ static float time_shape(int nx, int ny, int nz, int tile, int copies) {
         throw LbswimError{LBSWIM_ECUDA, lbswim_last_error()};
       Lattice* L = reinterpret_cast<Lattice*>(lats[i]);
       L->fused_tile = tile;
-      const int nsw = 64;
+      const int nsw = TUNE_SWIMMERS;
       if (lbswim_swimmers_create(nsw, &cp, &sws[i]) != LBSWIM_OK)
         throw LbswimError{LBSWIM_ECUDA, lbswim_last_error()};
       std::vector<double> r(3 * nsw), nv(3 * nsw, 0.0);
@@ -345,6 +364,7 @@ static float time_shape(int nx, int ny, int nz, int tile, int copies) {
       W[i] = reinterpret_cast<Swimmers*>(sws[i]);
     }
     ensemble_set_members(E, L.data(), W.data(), nullptr, copies);
+    E->longest_slabs = true;
     ensemble_step(E, 2);  // warm-up, graphs
     // the timed replays below run past that call's step count: no member limit
     for (auto& M : E->hmem) M.limit = 1 << 30;
@@ -375,10 +395,13 @@ void ensemble_autotune(Ensemble* E) {
     if (it == g_tuned.end()) {
       // enough copies to fill the GPU a few times over
       const int copies = (int)std::max<long long>(2, std::min<long long>(64, (1 << 22) / L->n));
-      const float a = time_shape(L->size[0], L->size[1], L->size[2], 0, copies);
-      const float b = L->size[2] >= 16 && L->size[1] >= 16
-                          ? time_shape(L->size[0], L->size[1], L->size[2], 1, copies)
-                          : -1.f;
+      auto cost = [&](int tile) {
+        const float ms = time_shape(L->size[0], L->size[1], L->size[2], tile, copies);
+        const long long slabs = copies * slabs_per_lattice(L->size, tile, 2 * TUNE_SWIMMERS);
+        return ms * (float)slabs / (float)((slabs + E->grid_step - 1) / E->grid_step);
+      };
+      const float a = cost(0);
+      const float b = L->size[2] > 16 && L->size[1] > 16 ? cost(1) : -1.f;
       const int best = (b > 0.f && (a <= 0.f || b < a)) ? 1 : 0;
       it = g_tuned.emplace(key, best).first;
     }
