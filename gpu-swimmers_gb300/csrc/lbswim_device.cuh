@@ -259,18 +259,6 @@ __device__ __forceinline__ void peskin_weights4(float dr, float w[4]) {
   w[3] = 0.125f * (q - s);
 }
 
-// The same four weights in FP64 (the default FP64 particle moves; exact mode
-// keeps the reference's delta per node, below).
-__device__ __forceinline__ void peskin_weights4(double dr, double w[4]) {
-  const double a = dr - 1.0;
-  const double s = sqrt(fma(4.0 * a, 1.0 - a, 1.0));
-  const double p = 3.0 - 2.0 * a, q = 1.0 + 2.0 * a;
-  w[0] = 0.125 * (p - s);
-  w[1] = 0.125 * (p + s);
-  w[2] = 0.125 * (q + s);
-  w[3] = 0.125 * (q - s);
-}
-
 // FP64: the reference's operations in its order, each rounded on its own (no
 // fused multiply-add), so that FP64 lattices can reproduce the oracle bit for bit.
 template <>
@@ -562,16 +550,11 @@ __device__ __forceinline__ bool cover_weight(int x, int o, int n, const T phi[4]
   return true;
 }
 
-// One end's contribution to one force component at a site.  FP64 keeps the
-// reference's order ((phi_x phi_y) phi_z) F (SwimmerArray.cu:64-73); FP32
-// evaluates (phi_y phi_z)(phi_x F) so that phi_x F can be formed once per x
-// plane.  Every FP32 kernel that spreads uses this one expression, so the
-// step kernel's own spreading and the materialised force agree bit for bit.
+// One end's contribution to one force component at a site, in the reference's
+// order ((phi_x phi_y) phi_z) F (SwimmerArray.cu:64-73).  (FP32: node_contrib,
+// spread_slab.cuh.)
 __device__ __forceinline__ double end_contrib(double wx, double wy, double wz, double F) {
   return __dmul_rn(__dmul_rn(__dmul_rn(wx, wy), wz), F);
-}
-__device__ __forceinline__ float end_contrib_f(float wy, float wz, float wxF) {
-  return (wy * wz) * wxF;
 }
 
 // ---- fixed-point force accumulation (FP32 lattices) ---------------------------

@@ -74,9 +74,10 @@ extern "C" {
 /* FP64 lattices only: Step, CalcHydro and InitFromHydro use the reference's
  * dense 15x15 transforms in its operation order (lb.cu:72-218, 250-295,
  * 314-371), every operation rounded on its own, so that results are bit for
- * bit those of the reference's host build (about 3x the FP64 work of the
- * default butterfly transform).  The particle kernels of FP64 lattices always
- * follow the reference's operation order. */
+ * bit those of the reference's host build.  The force spreading and the particle
+ * moves follow its operation order too.  The default FP64 arithmetic works on
+ * 64-bit integers, with errors no larger than the reference's rounding; the exact
+ * step takes 1.58 ms at 128^3 and its CalcHydro 0.31, against 0.11 and 0.06. */
 #define LBSWIM_COMPAT_EXACT_F64 4
 /* FP32/BF16/FP16 lattices: the step and the particle moves use 64-bit site
  * offsets whatever the lattice size; the results are the same bits.  Without
@@ -322,7 +323,7 @@ int lbswim_lattice_set_tau(lbswim_lattice* lat, double tau_s, double tau_b);
  * ensemble advances many independent FP32 solves -- each an FP32 lattice with
  * an optional swimmer array and an optional tracer array, all created and
  * initialised with the calls above -- by the same coupled step as
- * lbswim_system_step, in four batched launches per step replayed from a CUDA
+ * lbswim_system_step, in two batched launches per step replayed from a CUDA
  * graph.  Each member ends exactly where lbswim_system_step would have taken
  * it (bit for bit, with the same slab shape).  Membership can change between
  * calls to lbswim_ensemble_step; members stay owned by the caller and must
