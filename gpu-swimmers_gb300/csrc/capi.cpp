@@ -261,6 +261,10 @@ int lbswim_lattice_set_stream(lbswim_lattice* lat, void* stream) {
   lattice_join(L);
   LB_CUDA(cudaStreamSynchronize(L->stream));
   L->stream = (cudaStream_t)stream;
+  int least = 0, greatest = 0, mine = 0;
+  LB_CUDA(cudaDeviceGetStreamPriorityRange(&least, &greatest));
+  LB_CUDA(cudaStreamGetPriority(L->stream, &mine));
+  L->outranks_tracers = mine < least;
   API_END
 }
 
@@ -725,6 +729,8 @@ int lbswim_system_step(lbswim_lattice* lat, lbswim_swimmers* const* swimmers, in
   Swimmers* const* w = reinterpret_cast<Swimmers* const*>(swimmers);
   const bool together = swimmers_move_together(w, n_swimmers, L);
   const unsigned long long calls = g_calls.load(std::memory_order_relaxed);
+  if (n_tracers > 0 && !L->hydro_ready)
+    LB_CUDA(cudaEventCreateWithFlags(&L->hydro_ready, cudaEventDisableTiming));
   for (int t = 0; t < nsteps; ++t) {
     lattice_zero_force(L);  // ZeroForce
     if (!together || !swimmers_add_forces_prepared(w, n_swimmers, L, calls))
@@ -736,8 +742,6 @@ int lbswim_system_step(lbswim_lattice* lat, lbswim_swimmers* const* swimmers, in
     // step spreads forces; the step after that waits before overwriting the
     // velocities they read.
     if (n_tracers > 0) {
-      if (!L->hydro_ready)
-        LB_CUDA(cudaEventCreateWithFlags(&L->hydro_ready, cudaEventDisableTiming));
       LB_CUDA(cudaEventRecord(L->hydro_ready, L->stream));
       for (int i = 0; i < n_tracers; ++i) tracers_move_async(TR(tracers[i]), L);
     }

@@ -164,7 +164,8 @@ struct Lattice {
   // recorded after them).  Work that writes the buffer waits for the events.
   std::vector<std::pair<const void*, cudaEvent_t>> readers;
   std::vector<cudaEvent_t> reader_pool;
-  cudaEvent_t hydro_ready = nullptr;  // recorded on stream after CalcHydro
+  cudaEvent_t hydro_ready = nullptr;  // recorded on stream after CalcHydro, for tracers
+  bool outranks_tracers = false;      // stream has a higher priority than theirs
   // CUDA-event timing of the LB step kernel (lbswim_lattice_set_timing)
   bool timing = false;
   std::vector<std::pair<cudaEvent_t, cudaEvent_t>> timed;  // recorded, not yet read
@@ -283,7 +284,7 @@ int ens_step_ctas_per_sm();
 // Cross-section (rows, columns) of the slabs of a tile choice, and the x planes
 // per slab of a lattice stepped with nends pending ends.
 void slab_section_of(int tile, int* ty, int* tz);
-int choose_slab_lx(const int size[3], int tile, long long nends, int precision);
+int choose_slab_lx(const Lattice* L, long long nends);
 // The same with slabs of at most `cap` planes, as even as they come.
 int slab_lx_within(const int size[3], int tile, long long nends, int cap);
 // Multiplier and shift of a division by lx (FastDiv).

@@ -2174,10 +2174,10 @@ SlabSpread spread_prepare_slabs(Lattice* L) {
   S.last_pending = S.pending;
   const bool direct = S.pending <= DIRECT_ENDS;
   if (direct) {
-    S.lx = choose_slab_lx(L->size, L->fused_tile, S.pending, L->precision);
+    S.lx = choose_slab_lx(L, S.pending);
     S.bucket_tile = -1;
   } else if (S.bucket_tile != L->fused_tile) {
-    S.lx = choose_slab_lx(L->size, L->fused_tile, S.pending, L->precision);
+    S.lx = choose_slab_lx(L, S.pending);
     clear_buckets(L);
     if (S.pending > 0) {
       k_bucket_ends<<<(S.pending + 255) / 256, 256, 0, L->stream>>>(
@@ -2231,7 +2231,7 @@ static void append_ends(Swimmers* W, Lattice* L) {
     S.bucket_tile = -1;
     const int expected = std::max(nends, S.last_pending);
     if (expected > DIRECT_ENDS) {
-      S.lx = choose_slab_lx(L->size, L->fused_tile, expected, L->precision);
+      S.lx = choose_slab_lx(L, expected);
       clear_buckets(L);
     }
   }
@@ -2412,7 +2412,7 @@ void swimmers_prepare_room(Swimmers* const* w, int nw, Lattice* L) {
   if (!P.max_abs_force) LB_CUDA(cudaMalloc(&P.max_abs_force, 2 * sizeof(unsigned)));
   P.clear_max = true;
   if (nends > DIRECT_ENDS) {
-    P.lx = choose_slab_lx(L->size, L->fused_tile, nends, L->precision);
+    P.lx = choose_slab_lx(L, nends);
     P.clear = slabs_of(slab_grid(L, P.lx));
     grow_buckets(L, P.clear, P.bucket_count, P.bucket_list, P.bucket_slabs);
   }

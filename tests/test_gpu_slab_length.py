@@ -96,3 +96,25 @@ def _with(lat, arrays):
     for sw in arrays:
         system.AddThing(sw)
     return system
+
+
+def test_priority_stream_gives_the_same_bits():
+    """Tracers at a lower priority than the lattice's stream: slabs of another length
+    (13 planes in place of 26)."""
+    torch = pytest.importorskip("torch")
+    from lbswim import tracers
+    got = []
+    for priority in (0, -5):
+        for n in (15578, 1):
+            lat, system, arrays = build((52, 271, 283), (n,), 0)
+            stream = torch.cuda.Stream(priority=priority)
+            lat.set_stream(stream.cuda_stream)
+            tr = tracers.Array(500)
+            tr.init_random(lat, 5)
+            system.AddThing(tr)
+            system.Step(4)
+            lat.join()
+            tr.D2H()
+            got.append(state(lat, arrays) + [tr.r.data.copy()])
+            del system, tr, arrays, lat
+    assert same(got[0], got[2]) and same(got[1], got[3])
