@@ -503,7 +503,9 @@ static_assert(2 * (fused_smem_bytes<16, 16, true>() + 1024) <= 132 * 1024, "SPRE
 // of 256).
 template <class S, bool TMA>
 constexpr int fused_ctas() { return sizeof(S) == 2 && !TMA ? 3 : 2; }
-// Whether the next plane's loads follow the collision (see fused_slab).
+// Whether the next plane's loads follow the collision (see fused_slab).  The batched
+// step loads first: its members have few ends a slab (512 members 2.07 -> 1.93 ms a
+// step, 96 345 -> 324 us, 12 108 -> 101).
 template <class S, bool SPREAD, bool TMA>
 constexpr bool fused_late_loads() { return (SPREAD || sizeof(S) == 2) && !TMA; }
 
@@ -514,7 +516,8 @@ constexpr bool fused_late_loads() { return (SPREAD || sizeof(S) == 2) && !TMA; }
 // SPLIT: the form of the slab's force sums (slab_sums_split); SPREAD only.
 // TMA: the distributions of the cross-section's rows arrive by bulk copies
 // into shared memory (tma_* above); the lattice has nz a multiple of 32.
-template <class S, int TZ, int TY, bool SPREAD, class I, bool SPLIT, bool TMA = false>
+template <class S, int TZ, int TY, bool SPREAD, class I, bool SPLIT, bool TMA = false,
+          bool LATE = fused_late_loads<S, SPREAD, TMA>()>
 __device__ __forceinline__ void fused_slab(const FusedArgs& a, int tz, int ty, int tx, int slab) {
   static_assert(sizeof(S) < 8, "the fused step serves the reduced-precision layouts");
   static_assert(!TMA || TZ == 32, "bulk-copied rows are whole 32-site blocks");
@@ -634,7 +637,6 @@ __device__ __forceinline__ void fused_slab(const FusedArgs& a, int tz, int ty, i
     // with ends 521 -> 516 us, 100x75x130 51.7 -> 49.5; it leaves 56 registers a
     // thread, which 16-bit storage's third CTA needs); the others issue the loads
     // first, to have them in flight for the whole plane, and copy.
-    constexpr bool LATE = fused_late_loads<S, SPREAD, TMA>();
     float held[18];
     float(&cur)[18] = LATE ? pre : held;
     if (!LATE) {
@@ -819,9 +821,9 @@ __global__ void __launch_bounds__(8 * 32 + FUSED_RING_THREADS, 2) k_ens_step(Ens
     // members have few enough swimmers for split force sums on every slab
     // (checked when the members are set)
     if (M.tile == 1)
-      fused_slab<float, 16, 16, true, int, true>(a, tz, ty, tx, lt);
+      fused_slab<float, 16, 16, true, int, true, false, false>(a, tz, ty, tx, lt);
     else
-      fused_slab<float, 32, 8, true, int, true>(a, tz, ty, tx, lt);
+      fused_slab<float, 32, 8, true, int, true, false, false>(a, tz, ty, tx, lt);
     __syncthreads();
     if (threadIdx.x == 0) M.bucket_count[lt] = 0u;  // every thread has read it
   }
