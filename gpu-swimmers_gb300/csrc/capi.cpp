@@ -725,7 +725,10 @@ int lbswim_system_step(lbswim_lattice* lat, lbswim_swimmers* const* swimmers, in
   Lattice* L = LAT(lat);
   // With one swimmer array (or a few, in reduced precision), each move also records
   // the moved swimmers' ends for the next step; that step's AddForces takes them
-  // unless another call changed something in between.
+  // unless another call changed something in between, or may have: the caller of a
+  // device pointer writes without one, so its arrays' first step of a call records anew.
+  for (int i = 0; i < n_swimmers; ++i)
+    if (SW(swimmers[i])->exposed) L->spread.prep.valid = false;
   Swimmers* const* w = reinterpret_cast<Swimmers* const*>(swimmers);
   const bool together = swimmers_move_together(w, n_swimmers, L);
   const unsigned long long calls = g_calls.load(std::memory_order_relaxed);
@@ -806,7 +809,9 @@ int lbswim_lattice_device_buffers(const lbswim_lattice* lat, void* out[5]) {
 int lbswim_swimmers_device_ptr(const lbswim_swimmers* sw, int field, void** out) {
   API_BEGIN_READ
   REQUIRE(sw && out, "NULL argument");
-  *out = sw_field(const_cast<Swimmers*>(reinterpret_cast<const Swimmers*>(sw)), field);
+  Swimmers* W = const_cast<Swimmers*>(reinterpret_cast<const Swimmers*>(sw));
+  *out = sw_field(W, field);
+  if (field != LBSWIM_SW_V) W->exposed = true;
   API_END
 }
 

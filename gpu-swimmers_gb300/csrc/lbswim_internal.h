@@ -189,6 +189,9 @@ struct Swimmers {
   cudaStream_t copy = nullptr;  // host copies of several fields in one wait
   double* stage = nullptr;      // [3][n] upload checked before it replaces a field
   unsigned* flag = nullptr;     // result of the upload check
+  // r or n was handed out (lbswim_swimmers_device_ptr): the caller may write it on the
+  // device between any two calls, unseen
+  bool exposed = false;
 };
 
 // Tracers live on the device in a work order binned by position (8^3-site

@@ -366,7 +366,10 @@ int lbswim_lbparams_fill(lbswim_lbparams* p);
  * layouts).  fOld and fNew swap on every Step (lb.cu:241-244); the packed
  * rho/u buffer of a reduced-precision lattice swaps on CalcHydro. */
 int lbswim_lattice_device_buffers(const lbswim_lattice* lat, void* out[5]);
-/* SwimmerArray::r/v/n.device (SwimmerArray.h:25-27): [3][n] doubles. */
+/* SwimmerArray::r/v/n.device (SwimmerArray.h:25-27): [3][n] doubles.  The caller may
+ * write r and n on the device between calls, while no queued work of the library uses
+ * the array; every later call reads what is there then.  (From the first request of r
+ * or n on, lbswim_system_step does not take end records made by the call before.) */
 int lbswim_swimmers_device_ptr(const lbswim_swimmers* sw, int field, void** out);
 /* TracerArray::r/s/v.device (TracerArray.h:13-15): [3][n] doubles, in the
  * library's binned work order (a permutation of the user's order, which the
