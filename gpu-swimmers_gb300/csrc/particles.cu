@@ -1076,6 +1076,7 @@ template <int POINTS>
 struct Stencil64 {
   Digits w[3][4][POINTS];
   int o[3][POINTS];
+  bool lost[3][POINTS];  // the coordinate is not a finite number
   double vel[3][POINTS];
 };
 
@@ -1086,10 +1087,11 @@ __device__ __forceinline__ void point_axis64(const Dims& D, double x, int a, int
   const double x0 = ceil(x - 2.);
   st.o[a][p] = wrap_any((int)x0, dim_of(D, a));
   const double dr = x - x0;
+  st.lost[a][p] = !finite_d(x);
   long long w[4];
   if (dr >= 1.0 && dr <= 2.0) {
     fixed_weights4(dr, w);
-  } else {  // a coordinate beyond 2^52 (or not a number, whose position stays one)
+  } else {  // a coordinate beyond 2^52, or a lost one
 #pragma unroll
     for (int j = 0; j < 4; ++j) w[j] = (long long)(peskin_delta<double>(x - (x0 + j)) * 0x1p63);
   }
@@ -1158,6 +1160,7 @@ __device__ __forceinline__ void gather64(const double* __restrict__ u, const Dim
     v += __shfl_xor_sync(0xffffffffu, v, 1);
     v += __shfl_xor_sync(0xffffffffu, v, 2);
     const bool fits = ke >= FIXED_MIN_K && ke <= FIXED_MAX_K;
+    const bool lost = st.lost[0][p] | st.lost[1][p] | st.lost[2][p];
     if (k == 0 && fits) st.vel[c][p] = signed_fixed_to_double(v, ke + 3);
     // velocities of 0 (a fluid at rest), beyond the integers' range or not
     // finite: in FP64
@@ -1178,6 +1181,8 @@ __device__ __forceinline__ void gather64(const double* __restrict__ u, const Dim
     } else if (k == 0 && !fits) {
       st.vel[c][p] = 0.0;
     }
+    // no weights: no velocity
+    if (k == 0 && lost) st.vel[c][p] = bits_double(0x7ff8000000000000ull);
   }
 }
 
