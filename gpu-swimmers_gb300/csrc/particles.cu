@@ -2438,12 +2438,13 @@ void swimmers_move_preparing(Swimmers* const* w, int nw, Lattice* L, unsigned lo
   P.valid = false;
   const int nends = ends_of(w, nw);
   if (L->precision == LBSWIM_F64) {
-    if ((L->compat & LBSWIM_COMPAT_EXACT_F64) || nends > DIRECT_ENDS_F64 || !S.bucket_count ||
-        S.capacity_ends < nends || P.dirty) {
+    // records for the kernel that add_forces_f64 would choose, which has run before
+    const TileGrid G = force_tiles(L);
+    if ((L->compat & LBSWIM_COMPAT_EXACT_F64) || nends > DIRECT_ENDS_F64 ||
+        !tiles_take_buckets(G, nends) || !S.bucket_count || S.capacity_ends < nends || P.dirty) {
       swimmers_move(w[0], L);
       return;
     }
-    const TileGrid G = force_tiles(L);
     const RecordTarget<double> to{(EndRecord<double>*)S.ends,
                                   S.bucket_count + slabs_of(G) + S.max_slot, G, nullptr, nullptr};
     P.dirty = true;

@@ -129,3 +129,31 @@ def test_f64_calls_between_system_steps(n, exact):
     (lat, sw, seen), (ref, rsw, want) = got
     assert all(np.array_equal(x, y) for x, y in zip(seen, want))
     same(lat, [sw], ref, [rsw])
+
+
+@pytest.mark.parametrize("first", [0, 10])
+def test_f64_step_of_a_one_tile_lattice(first):
+    """Thirty swimmers on 4 x 8 x 32 sites, more than the tile's bucket rule admits: System.Step
+    gives the bits of the single calls, whatever smaller array the lattice has seen."""
+    def make():
+        lat = lb.Lattice(4, 8, 32, 0.7, 0.9)
+        lat.init_random(5)
+        out = []
+        for n in (first, 30):
+            cp = swimmers.CommonParams()
+            cp.P, cp.l, cp.alpha, cp.mobility, cp.seed = 2e-3, 0.4, 0.0, 1.0, 7
+            sw = swimmers.Array(n, cp) if n else None
+            if sw:
+                sw.init_random(lat, 31 + n)
+            out.append(sw)
+        return lat, out
+    lat, (small, sw) = make()
+    ref, (rsmall, rsw) = make()
+    if first:
+        lat.ZeroForce()
+        small.AddForces(lat)  # the lattice has buckets from here on
+    system = System(lat)
+    system.AddThing(sw)
+    system.Step(4)
+    single(ref, [rsw], 4)
+    same(lat, [sw], ref, [rsw])
