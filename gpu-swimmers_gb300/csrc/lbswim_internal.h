@@ -85,10 +85,8 @@ struct SpreadScratch {
   // batched run alternates with
   unsigned* max_abs_force = nullptr;
   TileLists ftiles;      // force tiles of a dense FP64 suspension
-  int max_slot = 0;      // FP64: which of the two max-force words is in use
   // slab buckets of the pending ends, filled as the ends are recorded; an FP64
-  // lattice's force-tile buckets (its bucket_count ends with two words for the
-  // largest force)
+  // lattice's force-tile buckets
   unsigned* bucket_count = nullptr;  // [bucket_slabs]
   int* bucket_list = nullptr;        // [bucket_slabs][SLAB_BUCKET_CAP], FP64: [][FT_CAP]
   int bucket_slabs = 0;  // slabs (or tiles) the buckets have room for
@@ -110,7 +108,6 @@ struct SpreadScratch {
     unsigned* max_abs_force = nullptr;
     int clear = 0;       // counts that the next step kernel clears ...
     bool clear_max = false;  // ... and the largest force
-    bool dirty = false;  // FP64: the buckets hold records that no step has taken
     bool valid = false;
     int owners = 0;                         // the arrays moved ...
     const void* owner[8] = {};

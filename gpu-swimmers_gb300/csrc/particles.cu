@@ -379,8 +379,8 @@ __device__ __forceinline__ int part_of_block(const SwimmerList& w) {
   return m;
 }
 
-// Where the end records of a swimmer array go: the records, the largest |F|, and
-// the buckets of the tiles of G.
+// Where the end records of a swimmer array go: the records, the largest |F| (FP32),
+// and the buckets of the tiles of G.
 template <class T>
 struct RecordTarget {
   EndRecord<T>* ends;
@@ -507,12 +507,10 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan_apply_total(
 // Force tiles of 4 (x) x 8 (y) x 32 (z) sites.  The end records list every end
 // under the tiles its stencil touches, in buckets of FT_CAP (a tile with more
 // takes all pending ends).  Two kernels sum them:
-//  * k_force_fixed (default): the (end, node) contributions are 64-bit integers
-//    in units of 2^-60 of the largest force, added as three words of 22, 22 and
-//    20 bits with shared-memory atomics that return nothing, and converted
-//    once.  All 32 lanes work on the nodes of an end.  Integer sums do not
-//    depend on their order.  256^3, 65,536 swimmers: 0.21 ms, against 0.71 ms
-//    in FP64 by site; 65x47x90: 10 us against 29.
+//  * k_force_fixed (default): the (end, node) contributions are integers of 72 to 84
+//    bits below the tile's largest force, added as three words with shared-memory
+//    atomics that return nothing, and converted once.  All 32 lanes work on the nodes of
+//    an end.  Integer sums do not depend on their order.
 //  * k_force_tile (LBSWIM_COMPAT_EXACT_F64, and suspensions too dense for
 //    buckets): every site adds the ends that cover it in end order,
 //    ((phi_x phi_y) phi_z) F as the reference does (SwimmerArray.cu:64-73).  A
@@ -521,11 +519,11 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan_apply_total(
 constexpr int FT_X = 4, FT_Y = 8, FT_Z = 32, FT_THREADS = 256, FT_CAP = 256;
 
 // Axis a of the record of an end (tail or head) of a swimmer at r, n.  FIXED: the
-// weights are integers in units of 2^-63 (fixed_weights4) in place of doubles, the
-// result is the high word of |F|, and `lost` is set when the coordinate is not a
-// number; otherwise they are the reference's delta per node.
+// weights are integers in units of 2^-63 (fixed_weights4) in place of doubles, and
+// `lost` is set when the coordinate is not a number; otherwise they are the
+// reference's delta per node.
 template <bool FIXED>
-__device__ __forceinline__ unsigned record_axis64(double r, double n, bool head, double P,
+__device__ __forceinline__ void record_axis64(double r, double n, bool head, double P,
                                                   double l, const Dims& D, int a,
                                                   EndRecord<double>& rec, unsigned& lost) {
   const double x = head ? r : __dsub_rn(r, __dmul_rn(n, l));
@@ -537,7 +535,7 @@ __device__ __forceinline__ unsigned record_axis64(double r, double n, bool head,
   if (!FIXED) {
 #pragma unroll
     for (int j = 0; j < 4; ++j) rec.phi[a][j] = peskin_delta<double>(x - (x0 + j));
-    return 0u;
+    return;
   }
   long long w[4];
   const double dr = x - x0;
@@ -549,31 +547,22 @@ __device__ __forceinline__ unsigned record_axis64(double r, double n, bool head,
   }
 #pragma unroll
   for (int j = 0; j < 4; ++j) rec.phi[a][j] = bits_double((unsigned long long)w[j]);
-  return hi_word(double_bits(F)) & 0x7fffffffu;
 }
 
 // The rest of a block's records e0, e0 + 1, ... (ENDS of them, thread (q, a)
-// for axis a of record q, a <= 2): the force of lost ends, the largest force, the
-// buckets and the copy to global memory.  Every thread of the block calls it.
+// for axis a of record q, a <= 2): the force of lost ends, the buckets and the copy to
+// global memory.  Every thread of the block calls it.
 constexpr int REC64_ENDS = 64, REC64_THREADS = 3 * REC64_ENDS;
 template <bool FIXED, bool BUCKETS, int ENDS>
-__device__ __forceinline__ void finish_records64(int q, int a, int e0, int nends, unsigned big,
+__device__ __forceinline__ void finish_records64(int q, int a, int e0, int nends,
                                                  EndRecord<double>* srec, const unsigned* lost,
-                                                 unsigned& smax, const Dims& D,
-                                                 const RecordTarget<double>& to) {
-  if (FIXED) {
-    big = __reduce_max_sync(0xffffffffu, big);
-    if ((threadIdx.x & 31) == 0 && big) atomicMax(&smax, big);
-  }
+                                                 const Dims& D, const RecordTarget<double>& to) {
   __syncthreads();
   if (a == 0 && e0 + q < nends) {
-    if (FIXED && lost[q]) {  // the force of a lost end is not a number
+    if (FIXED && lost[q])  // the force of a lost end is not a number
       for (int c = 0; c < 3; ++c) srec[q].F[c] = bits_double(0x7ff8000000000000ull);
-      atomicMax(to.max_f, 0x7ff80000u);
-    }
     if (BUCKETS && to.count) bucket_end<FT_CAP>(e0 + q, srec[q].o, D, to.G, to.count, to.list);
   }
-  if (FIXED && threadIdx.x == 0) atomicMax(to.max_f, smax);
   __syncthreads();
   const int words = min(ENDS, nends - e0) * (int)(sizeof(EndRecord<double>) / 8);
   const unsigned long long* src = reinterpret_cast<const unsigned long long*>(srec);
@@ -582,30 +571,25 @@ __device__ __forceinline__ void finish_records64(int q, int a, int e0, int nends
 }
 
 // One thread per (end, axis), 64 ends per block: the axes' chains of FP64
-// operations run side by side.  e = 2i is the tail, 2i + 1 the head.  FIXED
-// (record_axis64): *max_f takes the largest high word of |F|.
+// operations run side by side.  e = 2i is the tail, 2i + 1 the head.
 template <bool FIXED>
 __global__ void __launch_bounds__(REC64_THREADS) k_end_records_f64(
     int nsw, const double* __restrict__ r, const double* __restrict__ nv, double P, double l,
-    Dims D, EndRecord<double>* __restrict__ ends, unsigned* __restrict__ max_f, TileGrid G,
-    unsigned* __restrict__ bucket_count, int* __restrict__ bucket_list) {
+    Dims D, RecordTarget<double> to) {
   __shared__ EndRecord<double> srec[REC64_ENDS];
-  __shared__ unsigned smax, lost[REC64_ENDS];
+  __shared__ unsigned lost[REC64_ENDS];
   const int q = threadIdx.x % REC64_ENDS, a = threadIdx.x / REC64_ENDS;
   const int nends = 2 * nsw, e0 = blockIdx.x * REC64_ENDS, e = e0 + q;
-  if (threadIdx.x == 0) smax = 0u;
   if (a == 0) lost[q] = 0u;
   __syncthreads();
-  unsigned big = 0u;
   if (e < nends) {
     const int i = e >> 1;
     const bool head = e & 1;
     const double na = nv[(long long)nsw * a + i], ra = r[(long long)nsw * a + i];
-    big = record_axis64<FIXED>(ra, na, head, P, l, D, a, srec[q], lost[q]);
+    record_axis64<FIXED>(ra, na, head, P, l, D, a, srec[q], lost[q]);
     if (a == 0) srec[q].pad = 0;
   }
-  finish_records64<FIXED, true, REC64_ENDS>(q, a, e0, nends, big, srec, lost, smax, D,
-                          RecordTarget<double>{ends, max_f, G, bucket_count, bucket_list});
+  finish_records64<FIXED, true, REC64_ENDS>(q, a, e0, nends, srec, lost, D, to);
 }
 static_assert(sizeof(EndRecord<double>) % 8 == 0, "records are copied as 64-bit words");
 
@@ -733,57 +717,128 @@ __global__ void __launch_bounds__(FT_THREADS) k_force_tile(
 // are padded by 4 and planes by 16 words, so that the 32 nodes that a warp adds
 // at once (2 planes x 4 rows x 4 columns) fall into 32 banks.
 constexpr int FF_ROW = FT_Z + 4, FF_PLANE = FT_Y * FF_ROW + 16, FF_SITES = FT_X * FF_PLANE;
-constexpr int FF_CHUNK = 32;  // ends staged at a time
+constexpr int FF_CHUNK = 32;  // ends staged at a time, at most
 static_assert(FF_ROW % 32 == 4 && FF_PLANE % 32 == 16 && FF_SITES % 4 == 0, "bank layout");
 
-// Default FP64 spreading (see above).  max_f: the largest high word of |F|;
-// next_max_f is zeroed for the next call.  A contribution is below 2^57 of the
-// units (2^60 where stencil nodes fold); with more than 32 ends, or folds, in
-// a tile the units grow so that a site's sum stays within 62 bits.  Tiles whose
-// words could overflow (more than 1024 contributions a site), and forces that
-// are not finite or below 2^-894, take FP64 arithmetic in end order.
-// Issue-bound where most tiles have ends (64% of the slots; the scatter and the
-// conversions take 4500 warp instructions each of a tile's 10,000), so a thread's
-// sites differ in x alone and the record loads run under the zeroing: AddForces at
-// 256^3 255 -> 224 us, 128^3 with 40,000 swimmers 103 -> 92.  Up to FT_WIDE_TILES,
-// two to an SM, the chain of a block's phases bounds the launch: 512 threads
-// shorten each, and the list is read with its count: onto a force 64^3 (256
-// tiles) 20.0 -> 18.7 us and 24^3 18.6 -> 15.6, alone 16.8 and 15.2 either way;
-// with more tiles they cost occupancy (64x64x80, 384 tiles, 20.7 -> 21.9; 80^3
-// 18.8 -> 23.2; 256^3 224 -> 320).
+// The sums of a tile are numbers hi 2^(2 low) + mid 2^low + lo, hi signed.  A contribution
+// is cut into two unsigned digits of `low` bits and a signed top, small enough that all
+// contributions to a site, `most` of them, keep each word within 32 bits: 84 bits in all
+// for 16 of them, 81 for 32, 72 for 256.  Past 256 the digits have the 24 bits that a
+// chunk of 128 leaves room for, and their carries move up after each chunk; 57 bits
+// for 2^23.  (Stencil nodes of an end can meet on a site, 2^log2_fold of them.)
+struct SumWords {
+  int low, bits;
+};
+__device__ __forceinline__ SumWords sum_words(long long most) {
+  const int n = most > 1 ? 64 - __clzll(most - 1) : 0;  // most <= 2^n
+  const int top = min(28, 32 - n), low = max(top, 24);
+  return SumWords{low, 2 * low + top};
+}
+// The digits of v 2^32 / 2^m, |v| < 2^60 and m < 96, toward minus infinity.
+__device__ __forceinline__ void cut_words(long long v, int m, int low, unsigned mask, unsigned& lo,
+                                          unsigned& mid, int& hi) {
+  const unsigned v0 = (unsigned)v, v1 = (unsigned)(v >> 32), sg = (unsigned)((int)v1 >> 31);
+  const bool one = m >= 32, two = m >= 64;  // whole words of the shift
+  const unsigned a0 = two ? v1 : (one ? v0 : 0u), a1 = two ? sg : (one ? v1 : v0),
+                 a2 = one ? sg : v1;
+  const unsigned x0 = __funnelshift_r(a0, a1, m), x1 = __funnelshift_r(a1, a2, m),
+                 x2 = __funnelshift_r(a2, sg, m);
+  lo = x0 & mask;
+  mid = __funnelshift_r(x0, x1, low) & mask;
+  hi = (int)__funnelshift_r(x1, x2, 2 * low);  // 2 low is 48 to 56
+}
+// The double nearest to a sum in the units of k (2^(k - 1082), fixed_site.cuh).
+__device__ __forceinline__ double words_to_double(unsigned lo, unsigned mid, int hi, int low,
+                                                  int k) {
+  const unsigned long long l = (unsigned long long)mid * (1u << low) + lo;
+  const long long t = (long long)hi * (1 << (2 * low - 32)) + hi_word(l);  // the sum / 2^32
+  const unsigned long long sg = (unsigned long long)(t >> 63);
+  const unsigned c0 = ((unsigned)l ^ (unsigned)sg) + ((unsigned)sg & 1u);
+  const unsigned long long a = ((unsigned long long)t ^ sg) + (c0 == 0u ? sg & 1u : 0u);
+  // the top word that is not zero, and the two after it
+  const bool b1 = hi_word(a) == 0u, b2 = a == 0ull;
+  const unsigned a1 = (unsigned)a;
+  const unsigned u2 = b2 ? c0 : (b1 ? a1 : hi_word(a)), u1 = b2 ? 0u : (b1 ? c0 : a1),
+                 u0 = b1 ? 0u : c0;
+  const int lz = leading_zeros(u2);
+  const unsigned h = __funnelshift_l(u1, u2, lz), g = __funnelshift_l(u0, u1, lz);
+  const unsigned long long m = (((unsigned long long)h << 32) | g) >> 1;
+  const bool below = ((u0 << (lz & 31)) | (g & 1u)) != 0u;
+  const double r = round_to_double(m | (below ? 1u : 0u), lz + (b2 ? 32 : (b1 ? 0 : -32)), k);
+  return u2 == 0u ? 0.0 : bits_double(double_bits(r) | (sg & 0x8000000000000000ull));
+}
+
+// Default FP64 spreading (see above).  A record's weights and force components are
+// taken as 62-bit mantissas with exponents of their own, so a contribution keeps its
+// digits however small its factors; the unit of a component's sums lies 74 bits below
+// the largest such component among a tile's 256 ends, 83 below 32 ends' (sum_words).
+// In a unit that all components and tiles shared, 60 bits below the largest force,
+// swimmers aligned with an axis lost the digits of the other components.  Tiles with
+// forces that are not finite, or below 2^-894, take FP64 arithmetic in end order.
+// Bound by the integer pipe where most tiles have ends (16,000 warp instructions a
+// tile, a quarter of them in the conversions), so a thread's sites differ in x alone and
+// the record loads run under the zeroing: AddForces at 256^3 with 65,536 swimmers 313 us,
+// against 840 in FP64 by site; 65x47x90 with 1074 20 against 76.  Up to FT_WIDE_TILES,
+// two to an SM, the chain of a block's phases bounds the launch: 512 threads shorten
+// each, and the list is read with its count (onto a force 24^3 18.6 -> 15.6 us); with
+// more tiles they cost occupancy (80^3 18.8 -> 23.2; 256^3 224 -> 320), and of a few ends
+// without buckets each tile first picks its own (256^3 with 32 swimmers 199 -> 88 us).
 constexpr int FT_WIDE_TILES = 2 * 152;
 template <int THREADS>
 __global__ void __launch_bounds__(THREADS) k_force_fixed(
     Dims D, TileGrid G, const EndRecord<double>* __restrict__ ends, int nends,
-    unsigned* __restrict__ count, const int* __restrict__ list,
-    const unsigned* __restrict__ max_f, unsigned* __restrict__ next_max_f,
-    double* __restrict__ force, int accumulate) {
+    unsigned* __restrict__ count, const int* __restrict__ list, double* __restrict__ force,
+    int accumulate) {
   __shared__ __align__(16) unsigned sums[9 * FF_SITES];
-  __shared__ Digits dig[15][FF_CHUNK];  // 12 weights, 3 force components per end
+  __shared__ Digits dig[15][FF_CHUNK];  // mantissas of 12 weights, 3 force components per end
+  __shared__ unsigned char shift[12][FF_CHUNK];       // binades of a weight below 1/2 ...
+  __shared__ unsigned short exponent[3][FF_CHUNK];    // ... and the force's biased exponent
   __shared__ int org[3][FF_CHUNK];
+  __shared__ unsigned top_f[3];  // largest high word of |F| (1 for what has none)
   constexpr int WARPS = THREADS / 32;
   static_assert(WARPS % FT_Y == 0 && FF_CHUNK == 32, "the mappings below");
   const int tile = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int kz = tile % G.nt[2], ky = (tile / G.nt[2]) % G.nt[1], kx = tile / (G.nt[1] * G.nt[2]);
-  // without buckets (DIRECT_ENDS_F64 ends at most) a tile goes through all of them
-  const unsigned listed = count ? count[tile] : (unsigned)nends;
+  // without buckets (DIRECT_ENDS_F64 ends at most) a tile goes through all of them, or,
+  // where many tiles have none, picks its own
+  constexpr bool PICK = THREADS == FT_THREADS;
+  __shared__ int own[DIRECT_ENDS_F64 + 1];
+  int cnt = count ? (int)count[tile] : nends;
   const long long s0 = (long long)tile * FT_CAP;
   // entry of a chunk that this lane stages; few tiles read it before the count is
   // known (the bucket has FT_CAP > lane of them), many tiles are mostly empty
   constexpr bool EARLY = THREADS > FT_THREADS;
   int mine = lane;
   if (EARLY && count) mine = list[s0 + lane];
-  const unsigned fmax = *max_f;
-  const int kf = (int)(fmax >> 20);  // |F| < 2^(kf - 1022)
-  const int cnt = fmax ? (int)listed : 0;  // no force at all: nothing to add
-  // contributions an end can make to one site: stencil nodes that fold onto it
-  int fold = 1;
-  for (int a = 0; a < 3; ++a) fold *= D.n[a] >= 4 ? 1 : (D.n[a] == 1 ? 4 : 2);
-  __syncthreads();
-  if (tid == 0) {
-    if (count) count[tile] = 0u;  // every thread has read it
-    if (tile == 0) *next_max_f = 0u;
+  if (tid < 3) top_f[tid] = 0u;
+  if (PICK && !count && warp == 0) {
+    int n = 0;
+    for (int base = 0; base < DIRECT_ENDS_F64; base += 32) {
+      const int e = base + lane;
+      bool in = e < nends;
+      if (in)
+        for (int a = 0; a < 3; ++a) {
+          int f, c;
+          touched_range(ends[e].o[a], D.n[a], G.by[a], 0, G.nt[a], f, c);
+          int k = (a == 0 ? kx : (a == 1 ? ky : kz)) - f;
+          in = in && (k < 0 ? k + G.nt[a] : k) < c;
+        }
+      const unsigned m = __ballot_sync(0xffffffffu, in);
+      if (in) own[n + __popc(m & ((1u << lane) - 1u))] = e;
+      n += __popc(m);
+    }
+    if (lane == 0) own[DIRECT_ENDS_F64] = n;
   }
+  // contributions an end can make to one site: stencil nodes that fold onto it
+  int log2_fold = 0;
+  for (int a = 0; a < 3; ++a) log2_fold += D.n[a] >= 4 ? 0 : (D.n[a] == 1 ? 2 : 1);
+  const int chunk = FF_CHUNK >> max(log2_fold - 2, 0);
+  __syncthreads();
+  if (tid == 0 && count) count[tile] = 0u;  // every thread has read it
+  const bool picked = PICK && !count;
+  if (picked) cnt = own[DIRECT_ENDS_F64];
+  // the q-th end of the tile
+  auto entry = [&](int q) { return count ? list[s0 + q] : (picked ? own[q] : q); };
   const int z0 = kz * FT_Z, y0 = ky * FT_Y, x0 = kx * FT_X;
   if (cnt == 0) {
     if (!accumulate)
@@ -795,11 +850,18 @@ __global__ void __launch_bounds__(THREADS) k_force_fixed(
       }
     return;
   }
-  if (listed > (unsigned)FT_CAP || cnt * fold > 1024 || kf < FIXED_MIN_K || kf > FIXED_MAX_K) {
+  auto in_order = [&]() {
     auto rec = [&](int q) -> const EndRecord<double>& { return ends[q]; };
     force_gather<true>(D, kx, ky, kz, nends, rec, force, accumulate);
+  };
+  if (cnt > FT_CAP) {
+    in_order();
     return;
   }
+  auto f_word = [](double F) {
+    const unsigned long long b = double_bits(F);
+    return (hi_word(b) & 0x7fffffffu) | ((unsigned)b != 0u ? 1u : 0u);
+  };
   // the words of a chunk's records: lane q has end q, a warp every WARPS-th word;
   // their way here is covered by the zeroing, or by the chunk before
   constexpr int WORDS = (18 + WARPS - 1) / WARPS;
@@ -815,61 +877,106 @@ __global__ void __launch_bounds__(THREADS) k_force_fixed(
       else if (w < 18) word[i] = (unsigned)e.o[w - 15];
     }
   };
-  if (!EARLY && count && lane < cnt) mine = list[s0 + lane];
-  fetch(min(FF_CHUNK, cnt));
+  if (!EARLY && lane < cnt) mine = entry(lane);
+  fetch(min(chunk, cnt));
+  for (int q = chunk + tid; q < cnt; q += THREADS) {  // the later chunks' forces
+    const EndRecord<double>& e = ends[entry(q)];
+    for (int c = 0; c < 3; ++c) atomicMax(top_f + c, f_word(e.F[c]));
+  }
   for (int i = tid; i < 9 * FF_SITES / 4; i += THREADS)
     reinterpret_cast<uint4*>(sums)[i] = make_uint4(0u, 0u, 0u, 0u);
-  // coarser units by the doublings of the largest sum over 32 unfolded ends
-  const int most = cnt * (fold > 1 ? 8 : 1);
-  const int coarse = most > 32 ? 32 - __clz((most - 1) >> 5) : 0;
+  const long long most = (long long)cnt << log2_fold;
+  const SumWords sw = sum_words(most);
+  const unsigned mask = (1u << sw.low) - 1u;
   const int jy = (lane >> 2) & 3, jz = lane & 3;
-  for (int base = 0; base < cnt; base += FF_CHUNK) {
-    const int m = min(FF_CHUNK, cnt - base);
-    const int next = base + FF_CHUNK + lane;
-    if (next < cnt) mine = count ? list[s0 + next] : next;
+  int kf[3];  // |F_c| < 2^(kf[c] - 1022)
+  for (int base = 0; base < cnt; base += chunk) {
+    const int m = min(chunk, cnt - base);
+    const int next = base + chunk + lane;
+    if (next < cnt) mine = entry(next);
     if (base) __syncthreads();  // the chunk before has been added
-    if (lane < m) {
 #pragma unroll
-      for (int i = 0; i < WORDS; ++i) {
-        const int w = warp + i * WARPS;
-        const unsigned long long b = word[i];
-        if (w < 12) {
-          dig[w][lane] = digits((long long)b);
-        } else if (w < 15) {
-          // F in units of 2^(kf - 1022 - 62), to nearest
-          const int drop = kf - (int)((hi_word(b) >> 20) & 0x7ffu);
-          const unsigned long long mant = ((b << 11) | 0x8000000000000000ull);
-          const unsigned long long v = drop > 61 ? 0ull : ((mant >> (drop + 1)) + 1) >> 1;
-          const long long sg = (long long)b >> 63;
-          dig[w][lane] = digits(((long long)v ^ sg) - sg);
-        } else if (w < 18) {
-          org[w - 15][lane] = (int)b;
+    for (int i = 0; i < WORDS; ++i) {
+      const int w = warp + i * WARPS;  // uniform in the warp
+      const unsigned long long b = lane < m ? word[i] : 0ull;
+      if (w < 12) {
+        // weights are not negative but for rounding
+        const unsigned long long p = (long long)b > 0 ? b : 0ull;
+        const int e = p ? max(__clzll((long long)p) - 2, 0) : 0;
+        dig[w][lane] = digits((long long)(p << e));
+        shift[w][lane] = (unsigned char)e;
+      } else if (w < 15) {
+        const int e = (int)((hi_word(b) >> 20) & 0x7ffu);
+        const long long v =
+            e ? (long long)(((b << 11) | 0x8000000000000000ull) >> 2) : 0ll;
+        const long long sg = (long long)b >> 63;
+        dig[w][lane] = digits((v ^ sg) - sg);
+        exponent[w - 12][lane] = (unsigned short)e;
+        if (base == 0) {
+          const unsigned f = __reduce_max_sync(0xffffffffu, f_word(bits_double(b)));
+          if (lane == 0) atomicMax(top_f + (w - 12), f);
         }
+      } else if (w < 18) {
+        org[w - 15][lane] = (int)b;
       }
     }
-    fetch(min(FF_CHUNK, cnt - base - FF_CHUNK));
+    fetch(min(chunk, cnt - base - chunk));
     __syncthreads();
+    if (base == 0) {
+      bool range = true;
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        kf[c] = (int)(top_f[c] >> 20);
+        range = range && (top_f[c] == 0u || (kf[c] >= FIXED_MIN_K && kf[c] <= FIXED_MAX_K));
+      }
+      if (!range) {  // uniform in the block
+        in_order();
+        return;
+      }
+    }
     for (int q = warp; q < m; q += WARPS) {
       const int ly = node_after(org[1][q], jy, D.n[1]) - y0;
       const int lz = node_after(org[2][q], jz, D.n[2]) - z0;
       const bool in_yz = (unsigned)ly < (unsigned)FT_Y && (unsigned)lz < (unsigned)FT_Z;
       if (!in_yz) continue;
-      const Digits wyz = digits(2 * mul_hi(dig[4 + jy][q], dig[8 + jz][q]));
+      const Digits wyz = digits(mul_hi(dig[4 + jy][q], dig[8 + jz][q]) << 2);
+      const int eyz = 93 - sw.bits + shift[4 + jy][q] + shift[8 + jz][q];
+      Digits F[3];  // (the sums' atomics would have them read again for each node)
+      int eF[3];
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        F[c] = dig[12 + c][q];
+        eF[c] = kf[c] - exponent[c][q] + eyz;
+      }
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
         const int ix = (lane >> 4) + 2 * h;
         const int lx = node_after(org[0][q], ix, D.n[0]) - x0;
         if ((unsigned)lx >= (unsigned)FT_X) continue;
-        const Digits w = digits(mul_hi(dig[ix][q], wyz));
+        const Digits w = digits(mul_hi(dig[ix][q], wyz) << 2);
+        const int ew = shift[ix][q];
         unsigned* at = sums + lx * FF_PLANE + ly * FF_ROW + lz;
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
-          const long long v = mul_hi(w, dig[12 + c][q]) >> coarse;
-          atomicAdd(at + (3 * c) * FF_SITES, (unsigned)v & 0x3fffffu);
-          atomicAdd(at + (3 * c + 1) * FF_SITES, (unsigned)(v >> 22) & 0x3fffffu);
-          atomicAdd(reinterpret_cast<int*>(at + (3 * c + 2) * FF_SITES), (int)(v >> 44));
+          unsigned lo, mid;
+          int hi;
+          cut_words(mul_hi(w, F[c]), min(ew + eF[c], 95), sw.low, mask, lo, mid, hi);
+          atomicAdd(at + (3 * c) * FF_SITES, lo);
+          atomicAdd(at + (3 * c + 1) * FF_SITES, mid);
+          atomicAdd(reinterpret_cast<int*>(at + (3 * c + 2) * FF_SITES), hi);
         }
       }
+    }
+    if (most > 256 && base + chunk < cnt) {
+      __syncthreads();
+      for (int i = tid; i < FF_SITES; i += THREADS)
+        for (int c = 0; c < 3; ++c) {
+          unsigned* at = sums + 3 * c * FF_SITES + i;
+          const unsigned mid = at[FF_SITES] + (at[0] >> sw.low);
+          at[0] &= mask;
+          at[FF_SITES] = mid & mask;
+          at[2 * FF_SITES] += mid >> sw.low;
+        }
     }
   }
   __syncthreads();
@@ -882,13 +989,17 @@ __global__ void __launch_bounds__(THREADS) k_force_fixed(
     if (x >= D.n[0]) break;
     const unsigned* at = sums + lx * FF_PLANE + ly * FF_ROW + lane;
     const long long s = ((long long)x * D.n[1] + y) * D.n[2] + z;
+    unsigned w[9], any = 0u;
+#pragma unroll
+    for (int j = 0; j < 9; ++j) any |= w[j] = at[j * FF_SITES];
+    const bool some = __any_sync(__activemask(), any != 0u);  // else the row is empty
+    if (accumulate && !some) continue;
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
-      const long long v = (long long)at[(3 * c) * FF_SITES] +
-                          ((long long)at[(3 * c + 1) * FF_SITES] << 22) +
-                          (long long)((unsigned long long)at[(3 * c + 2) * FF_SITES] << 44);
-      if (accumulate && v == 0) continue;
-      const double f = signed_fixed_to_double(v, kf + coarse);
+      double f = 0.0;
+      if (some)
+        f = words_to_double(w[3 * c], w[3 * c + 1], (int)w[3 * c + 2], sw.low, kf[c] + 58 - sw.bits);
+      if (accumulate && f == 0.0) continue;
       force[c * D.N + s] = accumulate ? force[c * D.N + s] + f : f;
     }
   }
@@ -1266,19 +1377,17 @@ __global__ void __launch_bounds__(move64_block(POINTS)) k_swimmers_move_f64(
   }
   if constexpr (RECORD) {
     __shared__ EndRecord<double> srec[POINTS];
-    __shared__ unsigned smax, lost[POINTS];
-    if (threadIdx.x == 0) smax = 0u;
+    __shared__ unsigned lost[POINTS];
     if (a == 0) lost[p] = 0u;
     __syncthreads();  // every axis of a swimmer has been normalised
     if (update) turned[a][q] = nn;
     __syncthreads();
     const int e = 2 * q + (rear ? 1 : 0);  // of the block
-    unsigned big = 0u;
     if (valid) {
-      big = record_axis64<true>(moved[a][q], turned[a][q], rear, c.P, c.l, D, a, srec[e], lost[e]);
+      record_axis64<true>(moved[a][q], turned[a][q], rear, c.P, c.l, D, a, srec[e], lost[e]);
       if (a == 0) srec[e].pad = 0;
     }
-    finish_records64<true, false, POINTS>(e, a, blockIdx.x * POINTS, 2 * nsw, big, srec, lost, smax, D, to);
+    finish_records64<true, false, POINTS>(e, a, blockIdx.x * POINTS, 2 * nsw, srec, lost, D, to);
   }
 }
 
@@ -2030,13 +2139,12 @@ static void bin_ends(Lattice* L, TileLists& TL, const TileGrid& G, int nends) {
   LB_CHECK_LAUNCH(5);
 }
 
-// Buckets of FT_CAP ends per force tile, counts zero between calls, and the two
-// alternating words for the largest force.
+// Buckets of FT_CAP ends per force tile, counts zero between calls.
 static void ensure_tile_buckets(Lattice* L, int ntiles) {
   SpreadScratch& S = L->spread;
   if (S.bucket_count) return;  // the tiles of an FP64 lattice never change
   unsigned* count = nullptr;
-  LB_CUDA(cudaMalloc(&count, sizeof(unsigned) * (ntiles + 2)));
+  LB_CUDA(cudaMalloc(&count, sizeof(unsigned) * ntiles));
   const cudaError_t e = cudaMalloc(&S.bucket_list, sizeof(int) * (size_t)ntiles * FT_CAP);
   if (e != cudaSuccess) {
     cudaFree(count);
@@ -2045,7 +2153,7 @@ static void ensure_tile_buckets(Lattice* L, int ntiles) {
   }
   S.bucket_count = count;
   S.bucket_slabs = ntiles;
-  LB_CUDA(cudaMemsetAsync(count, 0, sizeof(unsigned) * (ntiles + 2), L->stream));
+  LB_CUDA(cudaMemsetAsync(count, 0, sizeof(unsigned) * ntiles, L->stream));
 }
 
 // Buckets while the average tile lists at most half of one (an end touches 2.6
@@ -2054,22 +2162,18 @@ static bool tiles_take_buckets(const TileGrid& G, long long nends) {
   return nends <= 48ll * G.nt[0] * G.nt[1] * G.nt[2];
 }
 
-// force = base + the spread of the nends ends recorded (and listed in buckets); the
-// two words for the largest force alternate.
+// force = base + the spread of the nends ends recorded (and listed in buckets).
 static void spread_fixed(Lattice* L, int nends) {
   SpreadScratch& S = L->spread;
   const TileGrid G = force_tiles(L);
-  const int ntiles = G.nt[0] * G.nt[1] * G.nt[2];
-  unsigned* max_f = S.bucket_count + ntiles;
+  const int ntiles = slabs_of(G);
   const int threads = ntiles <= FT_WIDE_TILES ? 2 * FT_THREADS : FT_THREADS;
   auto kernel = threads > FT_THREADS ? k_force_fixed<2 * FT_THREADS> : k_force_fixed<FT_THREADS>;
   kernel<<<ntiles, threads, 0, L->stream>>>(
       make_dims(L), G, (const EndRecord<double>*)S.ends, nends,
-      nends > DIRECT_ENDS_F64 ? S.bucket_count : nullptr, S.bucket_list,
-      max_f + S.max_slot, max_f + (S.max_slot ^ 1), (double*)L->force,
+      nends > DIRECT_ENDS_F64 ? S.bucket_count : nullptr, S.bucket_list, (double*)L->force,
       L->force_zero_pending ? 0 : 1);
   LB_CHECK_LAUNCH(1);
-  S.max_slot ^= 1;
   L->force_zero_pending = false;
 }
 
@@ -2091,24 +2195,21 @@ static void add_forces_f64(Swimmers* W, Lattice* L) {
   const bool buckets = tiles_take_buckets(G, nends);
   ensure_ends(L, nends);
   if (buckets) ensure_tile_buckets(L, ntiles);
-  if (S.prep.dirty) {  // records of a move that no step took
-    LB_CUDA(cudaMemsetAsync(S.bucket_count, 0, sizeof(unsigned) * (ntiles + 2), L->stream));
-    S.prep.dirty = S.prep.valid = false;
-  }
+  S.prep.valid = false;  // its records share the buffer
   EndRecord<double>* ends = (EndRecord<double>*)S.ends;
   const int grid = (nends + REC64_ENDS - 1) / REC64_ENDS;
   if (buckets && !exact) {
     k_end_records_f64<true><<<grid, REC64_THREADS, 0, L->stream>>>(
-        W->n, W->r, W->nv, W->common.P, W->common.l, D, ends,
-        S.bucket_count + ntiles + S.max_slot, G,
-        nends > DIRECT_ENDS_F64 ? S.bucket_count : nullptr, S.bucket_list);
+        W->n, W->r, W->nv, W->common.P, W->common.l, D,
+        RecordTarget<double>{ends, nullptr, G,
+                             nends > DIRECT_ENDS_F64 ? S.bucket_count : nullptr, S.bucket_list});
     LB_CHECK_LAUNCH(1);
     spread_fixed(L, nends);
     return;
   }
   k_end_records_f64<false><<<grid, REC64_THREADS, 0, L->stream>>>(
-      W->n, W->r, W->nv, W->common.P, W->common.l, D, ends, nullptr, G,
-      buckets ? S.bucket_count : nullptr, S.bucket_list);
+      W->n, W->r, W->nv, W->common.P, W->common.l, D,
+      RecordTarget<double>{ends, nullptr, G, buckets ? S.bucket_count : nullptr, S.bucket_list});
   LB_CHECK_LAUNCH(1);
   if (!buckets) bin_ends(L, S.ftiles, G, nends);
   k_force_tile<<<ntiles, FT_THREADS, 0, L->stream>>>(
@@ -2441,13 +2542,11 @@ void swimmers_move_preparing(Swimmers* const* w, int nw, Lattice* L, unsigned lo
     // records for the kernel that add_forces_f64 would choose, which has run before
     const TileGrid G = force_tiles(L);
     if ((L->compat & LBSWIM_COMPAT_EXACT_F64) || nends > DIRECT_ENDS_F64 ||
-        !tiles_take_buckets(G, nends) || !S.bucket_count || S.capacity_ends < nends || P.dirty) {
+        !tiles_take_buckets(G, nends) || S.capacity_ends < nends) {
       swimmers_move(w[0], L);
       return;
     }
-    const RecordTarget<double> to{(EndRecord<double>*)S.ends,
-                                  S.bucket_count + slabs_of(G) + S.max_slot, G, nullptr, nullptr};
-    P.dirty = true;
+    const RecordTarget<double> to{(EndRecord<double>*)S.ends, nullptr, G, nullptr, nullptr};
     launch_move_f64(w[0], L, &to);
   } else if (nends <= DIRECT_ENDS) {
     const RecordTarget<float> to{(EndRecord<float>*)P.ends, P.max_abs_force, TileGrid{}, nullptr,
@@ -2490,7 +2589,6 @@ bool swimmers_add_forces_prepared(Swimmers* const* w, int nw, Lattice* L,
     if (P.owner[i] != w[i] || P.owner_step[i] != w[i]->step) return false;
   if (L->precision == LBSWIM_F64) {
     spread_fixed(L, P.nends);
-    P.dirty = false;
   } else {
     if (P.tile >= 0 && P.tile != L->fused_tile) return false;
     std::swap(S.ends, P.ends);
