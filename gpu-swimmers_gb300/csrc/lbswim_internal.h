@@ -85,6 +85,11 @@ struct SpreadScratch {
   // batched run alternates with
   unsigned* max_abs_force = nullptr;
   TileLists ftiles;      // force tiles of a dense FP64 suspension
+  // chains of the ends past the buckets of FP64 force tiles (particles.cu: TileChains)
+  int* chain_head = nullptr;
+  int* chain_next = nullptr;
+  int* chain_ids = nullptr;  // exact mode
+  long long chain_room = 0;  // entries
   // slab buckets of the pending ends, filled as the ends are recorded; an FP64
   // lattice's force-tile buckets
   unsigned* bucket_count = nullptr;  // [bucket_slabs]

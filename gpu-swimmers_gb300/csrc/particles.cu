@@ -300,11 +300,15 @@ __device__ __forceinline__ int node_after(int o, int j, int n) {
 constexpr int REC_ENDS = 64, REC_THREADS = 3 * REC_ENDS;  // records of a block
 
 // List end e under every tile of grid G whose extended region its stencil
-// touches (at most CAP ends are kept per tile; the count goes on).
-template <int CAP>
+// touches.  At most CAP ends are kept per tile; the count goes on, and `over` takes the
+// later ones: (tile, the end's place among the tile's, number of the tile among the end's).
+struct DropEnd {
+  __device__ void operator()(int, unsigned, int) const {}
+};
+template <int CAP, class Over = DropEnd>
 __device__ __forceinline__ void bucket_end(int e, const int o[3], const Dims& D, const TileGrid& G,
-                                           unsigned* __restrict__ count,
-                                           int* __restrict__ list) {
+                                           unsigned* __restrict__ count, int* __restrict__ list,
+                                           Over over = Over()) {
   int f[3], c[3];
   for (int a = 0; a < 3; ++a) touched_range(o[a], D.n[a], G.by[a], G.h, G.nt[a], f[a], c[a]);
   auto tile = [&](int i, int j, int k) {
@@ -324,16 +328,23 @@ __device__ __forceinline__ void bucket_end(int e, const int o[3], const Dims& D,
           slot[q] = atomicAdd(count + tile(i0 + (q >> 2), (q >> 1) & 1, q & 1), 1u);
 #pragma unroll
       for (int q = 0; q < 8; ++q)
-        if (i0 + (q >> 2) < c[0] && ((q >> 1) & 1) < c[1] && (q & 1) < c[2] &&
-            slot[q] < (unsigned)CAP)
-          list[(long long)tile(i0 + (q >> 2), (q >> 1) & 1, q & 1) * CAP + slot[q]] = e;
+        if (i0 + (q >> 2) < c[0] && ((q >> 1) & 1) < c[1] && (q & 1) < c[2]) {
+          const int i = i0 + (q >> 2), j = (q >> 1) & 1, k = q & 1, t = tile(i, j, k);
+          if (slot[q] < (unsigned)CAP)
+            list[(long long)t * CAP + slot[q]] = e;
+          else
+            over(t, slot[q], (i * c[1] + j) * c[2] + k);
+        }
     } else {
       for (int i = i0; i < min(i0 + 2, c[0]); ++i)
         for (int j = 0; j < c[1]; ++j)
           for (int k = 0; k < c[2]; ++k) {
             const int t = tile(i, j, k);
             const unsigned slot = atomicAdd(count + t, 1u);
-            if (slot < (unsigned)CAP) list[(long long)t * CAP + slot] = e;
+            if (slot < (unsigned)CAP)
+              list[(long long)t * CAP + slot] = e;
+            else
+              over(t, slot, (i * c[1] + j) * c[2] + k);
           }
     }
   }
@@ -505,8 +516,8 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan_apply_total(
 
 // ---- force spreading of FP64 lattices -------------------------------------------
 // Force tiles of 4 (x) x 8 (y) x 32 (z) sites.  The end records list every end
-// under the tiles its stencil touches, in buckets of FT_CAP (a tile with more
-// takes all pending ends).  Two kernels sum them:
+// under the tiles its stencil touches, in buckets of FT_CAP and, past those, chains
+// (TileChains).  Two kernels sum them:
 //  * k_force_fixed (default): the (end, node) contributions are integers of 72 to 84
 //    bits below the tile's largest force, added as three words with shared-memory
 //    atomics that return nothing, and converted once.  All 32 lanes work on the nodes of
@@ -517,6 +528,38 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan_apply_total(
 //    row's 32 lanes have half an end each on average and run as long as the one
 //    with most, on the narrow FP64 pipe.
 constexpr int FT_X = 4, FT_Y = 8, FT_Z = 32, FT_THREADS = 256, FT_CAP = 256;
+
+// Entries FT_CAP, FT_CAP + 1, ... of a tile hang on its 32 chains in turn, so that the
+// lanes of a warp walk them side by side and a tile with many ends (swimmers in a
+// cluster) takes its own and no others: 256^3 with 65,536 swimmers in a sixteenth of the
+// box, where some tiles hold 500 ends, took 24 ms while such a tile went through all
+// 131,072, and 950 us when every tile's ends were listed by a counting sort.  An entry is
+// end * touch + the tile's number among the end's; chain c has
+// (count - FT_CAP + 31 - c) / 32 of them, so heads left over from before do not matter.
+struct TileChains {
+  int* head;  // [tiles][32]; null: no tile can have more than FT_CAP ends
+  int* next;  // [ends * touch]
+  int touch;  // tiles an end can touch
+  FastDiv by_touch;
+  int* ids;  // exact mode: [2][half] the ends of tiles with more, and in order
+  long long half;
+  unsigned long long* id_end;  // ids in use
+};
+struct ChainEnd {
+  TileChains ch;
+  int e;
+  __device__ void operator()(int t, unsigned slot, int i) const {
+    const int entry = e * ch.touch + i;
+    ch.next[entry] = atomicExch(ch.head + 32 * t + (int)(slot & 31u), entry);
+  }
+};
+static_assert(FT_CAP % 32 == 0, "entry FT_CAP hangs on chain 0");
+// The end of the entry after `at` on this lane's chain (at < 0: the first one), which
+// becomes `at`.
+__device__ __forceinline__ int chain_step(const TileChains& ch, int tile, int& at) {
+  at = at < 0 ? ch.head[32 * tile + (threadIdx.x & 31)] : ch.next[at];
+  return (int)div_by((unsigned)at, ch.by_touch);
+}
 
 // Axis a of the record of an end (tail or head) of a swimmer at r, n.  FIXED: the
 // weights are integers in units of 2^-63 (fixed_weights4) in place of doubles, and
@@ -556,12 +599,14 @@ constexpr int REC64_ENDS = 64, REC64_THREADS = 3 * REC64_ENDS;
 template <bool FIXED, bool BUCKETS, int ENDS>
 __device__ __forceinline__ void finish_records64(int q, int a, int e0, int nends,
                                                  EndRecord<double>* srec, const unsigned* lost,
-                                                 const Dims& D, const RecordTarget<double>& to) {
+                                                 const Dims& D, const RecordTarget<double>& to,
+                                                 const TileChains& ch) {
   __syncthreads();
   if (a == 0 && e0 + q < nends) {
     if (FIXED && lost[q])  // the force of a lost end is not a number
       for (int c = 0; c < 3; ++c) srec[q].F[c] = bits_double(0x7ff8000000000000ull);
-    if (BUCKETS && to.count) bucket_end<FT_CAP>(e0 + q, srec[q].o, D, to.G, to.count, to.list);
+    if (BUCKETS && to.count)
+      bucket_end<FT_CAP>(e0 + q, srec[q].o, D, to.G, to.count, to.list, ChainEnd{ch, e0 + q});
   }
   __syncthreads();
   const int words = min(ENDS, nends - e0) * (int)(sizeof(EndRecord<double>) / 8);
@@ -575,9 +620,10 @@ __device__ __forceinline__ void finish_records64(int q, int a, int e0, int nends
 template <bool FIXED>
 __global__ void __launch_bounds__(REC64_THREADS) k_end_records_f64(
     int nsw, const double* __restrict__ r, const double* __restrict__ nv, double P, double l,
-    Dims D, RecordTarget<double> to) {
+    Dims D, RecordTarget<double> to, TileChains ch) {
   __shared__ EndRecord<double> srec[REC64_ENDS];
   __shared__ unsigned lost[REC64_ENDS];
+  if (ch.id_end && blockIdx.x == 0 && threadIdx.x == 0) *ch.id_end = 0ull;
   const int q = threadIdx.x % REC64_ENDS, a = threadIdx.x / REC64_ENDS;
   const int nends = 2 * nsw, e0 = blockIdx.x * REC64_ENDS, e = e0 + q;
   if (a == 0) lost[q] = 0u;
@@ -589,7 +635,7 @@ __global__ void __launch_bounds__(REC64_THREADS) k_end_records_f64(
     record_axis64<FIXED>(ra, na, head, P, l, D, a, srec[q], lost[q]);
     if (a == 0) srec[q].pad = 0;
   }
-  finish_records64<FIXED, true, REC64_ENDS>(q, a, e0, nends, srec, lost, D, to);
+  finish_records64<FIXED, true, REC64_ENDS>(q, a, e0, nends, srec, lost, D, to, ch);
 }
 static_assert(sizeof(EndRecord<double>) % 8 == 0, "records are copied as 64-bit words");
 
@@ -675,40 +721,50 @@ __device__ __forceinline__ void force_gather(const Dims& D, int kx, int ky, int 
 
 // The ends of a tile in end order, by rank, then force_gather.  start: counting-
 // sorted lists [start[tile], start[tile + 1]) (with `sorted` as scratch for the
-// long ones); null: buckets, whose count is zeroed for the next call.
+// long ones); null: buckets, whose count is zeroed for the next call, and chains.
 __global__ void __launch_bounds__(FT_THREADS) k_force_tile(
-    Dims D, TileGrid G, const EndRecord<double>* __restrict__ ends, int nends,
+    Dims D, TileGrid G, const EndRecord<double>* __restrict__ ends,
     const unsigned* __restrict__ start, unsigned* __restrict__ count,
-    const int* __restrict__ list, int* __restrict__ sorted, double* __restrict__ force,
-    int accumulate) {
+    const int* __restrict__ list, int* __restrict__ sorted, TileChains ch,
+    double* __restrict__ force, int accumulate) {
   __shared__ EndRecord<double> srec[FT_CAP];
   __shared__ int skey[FT_CAP];
+  __shared__ unsigned long long place;
   const int tile = blockIdx.x;
   const int kz = tile % G.nt[2], ky = (tile / G.nt[2]) % G.nt[1], kx = tile / (G.nt[1] * G.nt[2]);
   const int tid = threadIdx.x;
-  const long long s0 = start ? (long long)start[tile] : (long long)tile * FT_CAP;
-  int cnt = (int)(start ? start[tile + 1] - start[tile] : count[tile]);
+  const int cnt = (int)(start ? start[tile + 1] - start[tile] : count[tile]);
+  const int* ids = list + (start ? (long long)start[tile] : (long long)tile * FT_CAP);
+  int* in_order = start ? sorted + start[tile] : nullptr;
   const bool in_smem = cnt <= FT_CAP;
   if (in_smem) {
-    for (int q = tid; q < cnt; q += FT_THREADS) skey[q] = list[s0 + q];
+    for (int q = tid; q < cnt; q += FT_THREADS) skey[q] = ids[q];
     __syncthreads();
     for (int q = tid; q < cnt; q += FT_THREADS) srec[rank_of(skey[q], skey, cnt)] = ends[skey[q]];
-  } else if (start) {
+  } else {
     // more ends than fit: order them in global scratch and read records from there
+    if (!start) {
+      if (tid == 0) place = atomicAdd(ch.id_end, (unsigned long long)cnt);
+      __syncthreads();
+      int* all = ch.ids + place;
+      in_order = all + ch.half;
+      for (int q = tid; q < FT_CAP; q += FT_THREADS) all[q] = ids[q];
+      if (tid < 32)
+        for (int q = FT_CAP + tid, at = -1; q < cnt; q += 32) all[q] = chain_step(ch, tile, at);
+      __syncthreads();
+      ids = all;
+    }
     for (int q = tid; q < cnt; q += FT_THREADS) {
-      const int k = list[s0 + q];
+      const int k = ids[q];
       int r = 0;
-      for (int j = 0; j < cnt; ++j) r += list[s0 + j] < k;
-      sorted[s0 + r] = k;
+      for (int j = 0; j < cnt; ++j) r += ids[j] < k;
+      in_order[r] = k;
     }
   }
   __syncthreads();
-  if (!start) {
-    if (tid == 0) count[tile] = 0u;  // every thread has read it
-    if (!in_smem) cnt = nends;
-  }
+  if (!start && tid == 0) count[tile] = 0u;  // every thread has read it
   auto rec = [&](int q) -> const EndRecord<double>& {
-    return in_smem ? srec[q] : ends[start ? sorted[s0 + q] : q];
+    return in_smem ? srec[q] : ends[in_order[q]];
   };
   force_gather<false>(D, kx, ky, kz, cnt, rec, force, accumulate);
 }
@@ -723,15 +779,16 @@ static_assert(FF_ROW % 32 == 4 && FF_PLANE % 32 == 16 && FF_SITES % 4 == 0, "ban
 // The sums of a tile are numbers hi 2^(2 low) + mid 2^low + lo, hi signed.  A contribution
 // is cut into two unsigned digits of `low` bits and a signed top, small enough that all
 // contributions to a site, `most` of them, keep each word within 32 bits: 84 bits in all
-// for 16 of them, 81 for 32, 72 for 256.  Past 256 the digits have the 24 bits that a
-// chunk of 128 leaves room for, and their carries move up after each chunk; 57 bits
-// for 2^23.  (Stencil nodes of an end can meet on a site, 2^log2_fold of them.)
+// for 16 of them, 81 for 32, 72 for 256.  Past 256 the digits have the 26 bits that
+// 32 contributions and a carried rest leave room for, and their carries move up after
+// each batch of ends: 73 bits for 2048, 61 for 2^23.  (Stencil nodes of an end can meet on
+// a site, 2^log2_fold of them: 64 on a lattice of one site, which has 25 bits.)
 struct SumWords {
   int low, bits;
 };
-__device__ __forceinline__ SumWords sum_words(long long most) {
+__device__ __forceinline__ SumWords sum_words(long long most, int log2_fold) {
   const int n = most > 1 ? 64 - __clzll(most - 1) : 0;  // most <= 2^n
-  const int top = min(28, 32 - n), low = max(top, 24);
+  const int top = max(min(28, 32 - n), 2), low = n <= 8 ? top : (log2_fold == 6 ? 25 : 26);
   return SumWords{low, 2 * low + top};
 }
 // The digits of v 2^32 / 2^m, |v| < 2^60 and m < 96, toward minus infinity.
@@ -787,8 +844,8 @@ constexpr int FT_WIDE_TILES = 2 * 152;
 template <int THREADS>
 __global__ void __launch_bounds__(THREADS) k_force_fixed(
     Dims D, TileGrid G, const EndRecord<double>* __restrict__ ends, int nends,
-    unsigned* __restrict__ count, const int* __restrict__ list, double* __restrict__ force,
-    int accumulate) {
+    unsigned* __restrict__ count, const int* __restrict__ list, TileChains ch,
+    double* __restrict__ force, int accumulate) {
   __shared__ __align__(16) unsigned sums[9 * FF_SITES];
   __shared__ Digits dig[15][FF_CHUNK];  // mantissas of 12 weights, 3 force components per end
   __shared__ unsigned char shift[12][FF_CHUNK];       // binades of a weight below 1/2 ...
@@ -832,13 +889,17 @@ __global__ void __launch_bounds__(THREADS) k_force_fixed(
   // contributions an end can make to one site: stencil nodes that fold onto it
   int log2_fold = 0;
   for (int a = 0; a < 3; ++a) log2_fold += D.n[a] >= 4 ? 0 : (D.n[a] == 1 ? 2 : 1);
-  const int chunk = FF_CHUNK >> max(log2_fold - 2, 0);
+  const int batch = max(FF_CHUNK >> log2_fold, 1);
   __syncthreads();
   if (tid == 0 && count) count[tile] = 0u;  // every thread has read it
   const bool picked = PICK && !count;
   if (picked) cnt = own[DIRECT_ENDS_F64];
-  // the q-th end of the tile
-  auto entry = [&](int q) { return count ? list[s0 + q] : (picked ? own[q] : q); };
+  // the q-th end of the tile; those past the bucket one after another, from `at` = -1 on
+  auto entry = [&](int q, int& at) {
+    if (q >= FT_CAP) return chain_step(ch, tile, at);
+    return count ? list[s0 + q] : (picked ? own[q] : q);
+  };
+  int at = -1;
   const int z0 = kz * FT_Z, y0 = ky * FT_Y, x0 = kx * FT_X;
   if (cnt == 0) {
     if (!accumulate)
@@ -854,10 +915,6 @@ __global__ void __launch_bounds__(THREADS) k_force_fixed(
     auto rec = [&](int q) -> const EndRecord<double>& { return ends[q]; };
     force_gather<true>(D, kx, ky, kz, nends, rec, force, accumulate);
   };
-  if (cnt > FT_CAP) {
-    in_order();
-    return;
-  }
   auto f_word = [](double F) {
     const unsigned long long b = double_bits(F);
     return (hi_word(b) & 0x7fffffffu) | ((unsigned)b != 0u ? 1u : 0u);
@@ -877,23 +934,27 @@ __global__ void __launch_bounds__(THREADS) k_force_fixed(
       else if (w < 18) word[i] = (unsigned)e.o[w - 15];
     }
   };
-  if (!EARLY && lane < cnt) mine = entry(lane);
-  fetch(min(chunk, cnt));
-  for (int q = chunk + tid; q < cnt; q += THREADS) {  // the later chunks' forces
-    const EndRecord<double>& e = ends[entry(q)];
-    for (int c = 0; c < 3; ++c) atomicMax(top_f + c, f_word(e.F[c]));
+  if (!EARLY && lane < cnt) mine = entry(lane, at);
+  fetch(min(FF_CHUNK, cnt));
+  // the later chunks' forces; every warp walks the chains
+  for (int q = FF_CHUNK + lane, ahead = -1; q < cnt; q += FF_CHUNK) {
+    const bool turn = (q / FF_CHUNK) % WARPS == warp;
+    if (q < FT_CAP && !turn) continue;
+    const EndRecord<double>& e = ends[entry(q, ahead)];
+    if (turn)
+      for (int c = 0; c < 3; ++c) atomicMax(top_f + c, f_word(e.F[c]));
   }
   for (int i = tid; i < 9 * FF_SITES / 4; i += THREADS)
     reinterpret_cast<uint4*>(sums)[i] = make_uint4(0u, 0u, 0u, 0u);
   const long long most = (long long)cnt << log2_fold;
-  const SumWords sw = sum_words(most);
+  const SumWords sw = sum_words(most, log2_fold);
   const unsigned mask = (1u << sw.low) - 1u;
   const int jy = (lane >> 2) & 3, jz = lane & 3;
   int kf[3];  // |F_c| < 2^(kf[c] - 1022)
-  for (int base = 0; base < cnt; base += chunk) {
-    const int m = min(chunk, cnt - base);
-    const int next = base + chunk + lane;
-    if (next < cnt) mine = entry(next);
+  for (int base = 0; base < cnt; base += FF_CHUNK) {
+    const int m = min(FF_CHUNK, cnt - base);
+    const int next = base + FF_CHUNK + lane;
+    if (next < cnt) mine = entry(next, at);
     if (base) __syncthreads();  // the chunk before has been added
 #pragma unroll
     for (int i = 0; i < WORDS; ++i) {
@@ -920,7 +981,7 @@ __global__ void __launch_bounds__(THREADS) k_force_fixed(
         org[w - 15][lane] = (int)b;
       }
     }
-    fetch(min(chunk, cnt - base - chunk));
+    fetch(min(FF_CHUNK, cnt - base - FF_CHUNK));
     __syncthreads();
     if (base == 0) {
       bool range = true;
@@ -934,49 +995,52 @@ __global__ void __launch_bounds__(THREADS) k_force_fixed(
         return;
       }
     }
-    for (int q = warp; q < m; q += WARPS) {
-      const int ly = node_after(org[1][q], jy, D.n[1]) - y0;
-      const int lz = node_after(org[2][q], jz, D.n[2]) - z0;
-      const bool in_yz = (unsigned)ly < (unsigned)FT_Y && (unsigned)lz < (unsigned)FT_Z;
-      if (!in_yz) continue;
-      const Digits wyz = digits(mul_hi(dig[4 + jy][q], dig[8 + jz][q]) << 2);
-      const int eyz = 93 - sw.bits + shift[4 + jy][q] + shift[8 + jz][q];
-      Digits F[3];  // (the sums' atomics would have them read again for each node)
-      int eF[3];
-#pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        F[c] = dig[12 + c][q];
-        eF[c] = kf[c] - exponent[c][q] + eyz;
-      }
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int ix = (lane >> 4) + 2 * h;
-        const int lx = node_after(org[0][q], ix, D.n[0]) - x0;
-        if ((unsigned)lx >= (unsigned)FT_X) continue;
-        const Digits w = digits(mul_hi(dig[ix][q], wyz) << 2);
-        const int ew = shift[ix][q];
-        unsigned* at = sums + lx * FF_PLANE + ly * FF_ROW + lz;
+    for (int first = 0; first < m; first += batch) {
+      for (int q = first + warp; q < min(m, first + batch); q += WARPS) {
+        const int ly = node_after(org[1][q], jy, D.n[1]) - y0;
+        const int lz = node_after(org[2][q], jz, D.n[2]) - z0;
+        const bool in_yz = (unsigned)ly < (unsigned)FT_Y && (unsigned)lz < (unsigned)FT_Z;
+        if (!in_yz) continue;
+        const Digits wyz = digits(mul_hi(dig[4 + jy][q], dig[8 + jz][q]) << 2);
+        const int eyz = 93 - sw.bits + shift[4 + jy][q] + shift[8 + jz][q];
+        Digits F[3];  // (the sums' atomics would have them read again for each node)
+        int eF[3];
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
-          unsigned lo, mid;
-          int hi;
-          cut_words(mul_hi(w, F[c]), min(ew + eF[c], 95), sw.low, mask, lo, mid, hi);
-          atomicAdd(at + (3 * c) * FF_SITES, lo);
-          atomicAdd(at + (3 * c + 1) * FF_SITES, mid);
-          atomicAdd(reinterpret_cast<int*>(at + (3 * c + 2) * FF_SITES), hi);
+          F[c] = dig[12 + c][q];
+          eF[c] = kf[c] - exponent[c][q] + eyz;
+        }
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int ix = (lane >> 4) + 2 * h;
+          const int lx = node_after(org[0][q], ix, D.n[0]) - x0;
+          if ((unsigned)lx >= (unsigned)FT_X) continue;
+          const Digits w = digits(mul_hi(dig[ix][q], wyz) << 2);
+          const int ew = shift[ix][q];
+          unsigned* sum = sums + lx * FF_PLANE + ly * FF_ROW + lz;
+#pragma unroll
+          for (int c = 0; c < 3; ++c) {
+            unsigned lo, mid;
+            int hi;
+            cut_words(mul_hi(w, F[c]), min(ew + eF[c], 95), sw.low, mask, lo, mid, hi);
+            atomicAdd(sum + (3 * c) * FF_SITES, lo);
+            atomicAdd(sum + (3 * c + 1) * FF_SITES, mid);
+            atomicAdd(reinterpret_cast<int*>(sum + (3 * c + 2) * FF_SITES), hi);
+          }
         }
       }
-    }
-    if (most > 256 && base + chunk < cnt) {
-      __syncthreads();
-      for (int i = tid; i < FF_SITES; i += THREADS)
-        for (int c = 0; c < 3; ++c) {
-          unsigned* at = sums + 3 * c * FF_SITES + i;
-          const unsigned mid = at[FF_SITES] + (at[0] >> sw.low);
-          at[0] &= mask;
-          at[FF_SITES] = mid & mask;
-          at[2 * FF_SITES] += mid >> sw.low;
-        }
+      if (most > 256 && (first + batch < m || base + FF_CHUNK < cnt)) {
+        __syncthreads();
+        for (int i = tid; i < FF_SITES; i += THREADS)
+          for (int c = 0; c < 3; ++c) {
+            unsigned* w = sums + 3 * c * FF_SITES + i;
+            const unsigned mid = w[FF_SITES] + (w[0] >> sw.low);
+            w[0] &= mask;
+            w[FF_SITES] = mid & mask;
+            w[2 * FF_SITES] += mid >> sw.low;
+          }
+        if (first + batch < m) __syncthreads();
+      }
     }
   }
   __syncthreads();
@@ -987,11 +1051,11 @@ __global__ void __launch_bounds__(THREADS) k_force_fixed(
   for (int i = 0; i < FT_X * FT_Y / WARPS; ++i) {
     const int lx = warp / FT_Y + i * (WARPS / FT_Y), x = x0 + lx;
     if (x >= D.n[0]) break;
-    const unsigned* at = sums + lx * FF_PLANE + ly * FF_ROW + lane;
+    const unsigned* sum = sums + lx * FF_PLANE + ly * FF_ROW + lane;
     const long long s = ((long long)x * D.n[1] + y) * D.n[2] + z;
     unsigned w[9], any = 0u;
 #pragma unroll
-    for (int j = 0; j < 9; ++j) any |= w[j] = at[j * FF_SITES];
+    for (int j = 0; j < 9; ++j) any |= w[j] = sum[j * FF_SITES];
     const bool some = __any_sync(__activemask(), any != 0u);  // else the row is empty
     if (accumulate && !some) continue;
 #pragma unroll
@@ -1387,7 +1451,8 @@ __global__ void __launch_bounds__(move64_block(POINTS)) k_swimmers_move_f64(
       record_axis64<true>(moved[a][q], turned[a][q], rear, c.P, c.l, D, a, srec[e], lost[e]);
       if (a == 0) srec[e].pad = 0;
     }
-    finish_records64<true, false, POINTS>(e, a, blockIdx.x * POINTS, 2 * nsw, srec, lost, D, to);
+    finish_records64<true, false, POINTS>(e, a, blockIdx.x * POINTS, 2 * nsw, srec, lost, D, to,
+                                          TileChains{});
   }
 }
 
@@ -2040,6 +2105,14 @@ static long long touches_per_end(const TileGrid& G) {
   return m;
 }
 
+static void free_chains(SpreadScratch& S) {
+  void* ptrs[] = {S.chain_head, S.chain_next, S.chain_ids};
+  for (void* p : ptrs)
+    if (p) cudaFree(p);
+  S.chain_head = S.chain_next = S.chain_ids = nullptr;
+  S.chain_room = 0;
+}
+
 static void free_lists(TileLists& TL) {
   void* ptrs[] = {TL.count, TL.start, TL.scan_tmp, TL.list, TL.sorted};
   for (void* p : ptrs)
@@ -2066,6 +2139,7 @@ void spread_free(SpreadScratch& S) {
   S.bucket_slabs = 0;
   S.bucket_tile = -1;
   free_lists(S.ftiles);
+  free_chains(S);
 }
 
 static size_t record_bytes(const Lattice* L) {
@@ -2159,11 +2233,39 @@ static void ensure_tile_buckets(Lattice* L, int ntiles) {
 // Buckets while the average tile lists at most half of one (an end touches 2.6
 // tiles of 1024 sites on average).
 static bool tiles_take_buckets(const TileGrid& G, long long nends) {
-  return nends <= 48ll * G.nt[0] * G.nt[1] * G.nt[2];
+  return nends <= 48ll * G.nt[0] * G.nt[1] * G.nt[2] &&
+         nends * touches_per_end(G) <= 0x7fffffffll;  // a chain's entries
 }
 
-// force = base + the spread of the nends ends recorded (and listed in buckets).
-static void spread_fixed(Lattice* L, int nends) {
+// Chains for the tiles that may list more of nends ends than a bucket holds.
+static TileChains tile_chains(Lattice* L, const TileGrid& G, int nends, bool exact) {
+  TileChains ch{};
+  if (nends <= FT_CAP) return ch;
+  SpreadScratch& S = L->spread;
+  ch.touch = (int)touches_per_end(G);
+  ch.by_touch = fast_div((unsigned)ch.touch);
+  ch.half = (long long)nends * ch.touch;
+  if (S.chain_room < ch.half || (exact && !S.chain_ids)) {
+    LB_CUDA(cudaStreamSynchronize(L->stream));
+    free_chains(S);
+    // the ids' counter after the heads
+    LB_CUDA(cudaMalloc(&S.chain_head, sizeof(int) * 32 * (size_t)slabs_of(G) + 8));
+    LB_CUDA(cudaMalloc(&S.chain_next, sizeof(int) * ch.half));
+    if (exact) LB_CUDA(cudaMalloc(&S.chain_ids, sizeof(int) * 2 * ch.half));
+    S.chain_room = ch.half;
+  }
+  ch.head = S.chain_head;
+  ch.next = S.chain_next;
+  if (exact) {
+    ch.ids = S.chain_ids;
+    ch.half = S.chain_room;
+    ch.id_end = reinterpret_cast<unsigned long long*>(S.chain_head + 32 * (size_t)slabs_of(G));
+  }
+  return ch;
+}
+
+// force = base + the spread of the nends ends recorded (and listed in buckets and chains).
+static void spread_fixed(Lattice* L, int nends, const TileChains& ch) {
   SpreadScratch& S = L->spread;
   const TileGrid G = force_tiles(L);
   const int ntiles = slabs_of(G);
@@ -2171,7 +2273,7 @@ static void spread_fixed(Lattice* L, int nends) {
   auto kernel = threads > FT_THREADS ? k_force_fixed<2 * FT_THREADS> : k_force_fixed<FT_THREADS>;
   kernel<<<ntiles, threads, 0, L->stream>>>(
       make_dims(L), G, (const EndRecord<double>*)S.ends, nends,
-      nends > DIRECT_ENDS_F64 ? S.bucket_count : nullptr, S.bucket_list, (double*)L->force,
+      nends > DIRECT_ENDS_F64 ? S.bucket_count : nullptr, S.bucket_list, ch, (double*)L->force,
       L->force_zero_pending ? 0 : 1);
   LB_CHECK_LAUNCH(1);
   L->force_zero_pending = false;
@@ -2195,6 +2297,7 @@ static void add_forces_f64(Swimmers* W, Lattice* L) {
   const bool buckets = tiles_take_buckets(G, nends);
   ensure_ends(L, nends);
   if (buckets) ensure_tile_buckets(L, ntiles);
+  const TileChains ch = buckets ? tile_chains(L, G, nends, exact) : TileChains{};
   S.prep.valid = false;  // its records share the buffer
   EndRecord<double>* ends = (EndRecord<double>*)S.ends;
   const int grid = (nends + REC64_ENDS - 1) / REC64_ENDS;
@@ -2202,19 +2305,21 @@ static void add_forces_f64(Swimmers* W, Lattice* L) {
     k_end_records_f64<true><<<grid, REC64_THREADS, 0, L->stream>>>(
         W->n, W->r, W->nv, W->common.P, W->common.l, D,
         RecordTarget<double>{ends, nullptr, G,
-                             nends > DIRECT_ENDS_F64 ? S.bucket_count : nullptr, S.bucket_list});
+                             nends > DIRECT_ENDS_F64 ? S.bucket_count : nullptr, S.bucket_list},
+        ch);
     LB_CHECK_LAUNCH(1);
-    spread_fixed(L, nends);
+    spread_fixed(L, nends, ch);
     return;
   }
   k_end_records_f64<false><<<grid, REC64_THREADS, 0, L->stream>>>(
       W->n, W->r, W->nv, W->common.P, W->common.l, D,
-      RecordTarget<double>{ends, nullptr, G, buckets ? S.bucket_count : nullptr, S.bucket_list});
+      RecordTarget<double>{ends, nullptr, G, buckets ? S.bucket_count : nullptr, S.bucket_list},
+      ch);
   LB_CHECK_LAUNCH(1);
   if (!buckets) bin_ends(L, S.ftiles, G, nends);
   k_force_tile<<<ntiles, FT_THREADS, 0, L->stream>>>(
-      D, G, ends, nends, buckets ? nullptr : S.ftiles.start, S.bucket_count,
-      buckets ? S.bucket_list : S.ftiles.list, S.ftiles.sorted, (double*)L->force,
+      D, G, ends, buckets ? nullptr : S.ftiles.start, S.bucket_count,
+      buckets ? S.bucket_list : S.ftiles.list, S.ftiles.sorted, ch, (double*)L->force,
       L->force_zero_pending ? 0 : 1);
   LB_CHECK_LAUNCH(1);
   L->force_zero_pending = false;
@@ -2588,7 +2693,7 @@ bool swimmers_add_forces_prepared(Swimmers* const* w, int nw, Lattice* L,
   for (int i = 0; i < nw; ++i)
     if (P.owner[i] != w[i] || P.owner_step[i] != w[i]->step) return false;
   if (L->precision == LBSWIM_F64) {
-    spread_fixed(L, P.nends);
+    spread_fixed(L, P.nends, TileChains{});  // DIRECT_ENDS_F64 at most
   } else {
     if (P.tile >= 0 && P.tile != L->fused_tile) return false;
     std::swap(S.ends, P.ends);
