@@ -128,16 +128,17 @@ __host__ __device__ __forceinline__ bool site_to_fixed(const double d[15],
   return any <= (unsigned)FIXED_MAX_DROP && k >= FIXED_MIN_K && k <= FIXED_MAX_K;
 }
 
-// x in the units of k, toward zero; false when |x| >= 2^56 units (a sixteenth
-// of the top of the rest population's binade) or not finite.  Below one unit
-// it is 0.
+// x in the units of k, to nearest (a force of 1e-8 has 36 bits of units at density 1, and
+// a steady one cut toward zero would lose momentum at every step); false when
+// |x| >= 2^56 units (a sixteenth of the top of the rest population's binade) or not
+// finite.
 __host__ __device__ __forceinline__ bool value_to_fixed(double x, int k, long long& v) {
   const unsigned long long b = double_bits(x);
   const int e = (int)((hi_word(b) >> 20) & 0x7ffu);
   const int drop = k - e;
-  const int s = drop + 4 < 64 ? drop + 4 : 64;  // 8 .. 64 when it fits
+  const int s = drop + 4 < 65 ? drop + 4 : 65;  // 8 .. 65 when it fits
   const unsigned long long m = (b << 11) | 0x8000000000000000ull;
-  const long long a = (long long)((m >> 1) >> ((s - 1) & 63));
+  const long long a = (long long)((((m >> 1) >> ((s - 2) & 63)) + 1) >> 1);
   const long long sg = (long long)b >> 63;
   v = (a ^ sg) - sg;
   return drop >= 4;
