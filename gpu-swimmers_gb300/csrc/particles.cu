@@ -1233,16 +1233,20 @@ __global__ void __launch_bounds__(EXACT_MOVE_BLOCK) k_tracers_move_exact(
 // weights, a lane sums its 16 nodes a component, a thread per (particle, axis)
 // updates it.  A lane's 16 velocities become integers below 2^60 under the
 // largest exponent of the point's 64, and are summed over y, x and z with three
-// 32-bit multiply-adds a product: within 2^-57 of the largest velocity in all,
-// where FP64 sums are within 2^-53 of their terms.  The 400 FP64 operations a
-// point took before ran on two lanes per clock and SM.  1,048,576 tracers at
-// 256^3: 748 -> 430 us (2400 instructions per warp, the integer pipe 64% busy);
-// 65,536 swimmers 204 -> 104 us, one swimmer 50 -> 11 us.
+// 32-bit multiply-adds a product: within 2^-57 of the largest velocity in all (rms
+// 2^-59), where FP64 sums are within 2^-53 of their terms.  Where the largest velocity
+// has hardly any weight (a front in a fluid at rest) that is the coarser one: the sum of
+// weight times size, in FP32 beside the integers, sends such points to FP64 (7% of the
+// time).  The 400 FP64 operations a point took before ran on two lanes per clock and SM.
+// 1,048,576 tracers at 256^3: 748 -> 450 us; 65,536 swimmers 204 -> 107 us, one
+// swimmer 50 -> 8 us.
 //
 // A small array's blocks take 16 points and give each component lanes of its own,
 // so that their chains run side by side (one swimmer 10.9 -> 7.6 us, 1074 18.3 ->
 // 15.2, 4096 tracers 8.6 -> 5.9); a lane of a large one's, of 64 points, takes the
-// three in turn and forms the nodes' offsets once (1,048,576 tracers 470 -> 430).
+// three in turn and forms the nodes' offsets once (1,048,576 tracers 470 -> 430).  80
+// registers a thread keep three of the large blocks to an SM (65,536 swimmers 123 us in
+// 102 registers, 109 in 80).
 constexpr int MOVE64_FEW = 16, MOVE64_MANY = 64;
 constexpr int MOVE64_MANY_FROM = 16384;  // points
 constexpr int move64_block(int points) { return points == MOVE64_FEW ? 12 * points : 4 * points; }
@@ -1274,10 +1278,9 @@ __device__ __forceinline__ void point_axis64(const Dims& D, double x, int a, int
   for (int j = 0; j < 4; ++j) st.w[a][j][p] = digits(w[j]);
 }
 
-// b as digits of an integer below 2^60 in units of 2^(ke - 1082), toward zero,
-// for a double of biased exponent at most ke.
-__device__ __forceinline__ Digits velocity_digits(unsigned long long b, int ke) {
-  const int drop = ke - (int)((hi_word(b) >> 20) & 0x7ffu);
+// b as digits of an integer below 2^60 in units of 2^(ke - 1082), toward zero, for a
+// double of biased exponent ke - drop.
+__device__ __forceinline__ Digits velocity_digits(unsigned long long b, int drop) {
   const unsigned long long m =
       ((b & 0xfffffffffffffull) | 0x10000000000000ull) << 10;  // bit 62
   const long long v = (long long)(m >> min(drop + 3, 63));
@@ -1308,6 +1311,10 @@ __device__ __forceinline__ void gather64(const double* __restrict__ u, const Dim
     yo[i] = node_after(st.o[1][p], i, D.n[1]) * D.n[2];
   }
   const int z = node_after(st.o[2][p], k, D.n[2]);
+  float wyz[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j)
+    wyz[j] = (float)st.w[1][j][p].h * (float)st.w[2][k][p].h * 0x1p-62f;
   const int c0 = POINTS == MOVE64_FEW ? threadIdx.x / (4 * POINTS) : 0;
 #pragma unroll 1
   for (int c = c0; c < (POINTS == MOVE64_FEW ? c0 + 1 : 3); ++c) {
@@ -1323,23 +1330,33 @@ __device__ __forceinline__ void gather64(const double* __restrict__ u, const Dim
     top = max(top, __shfl_xor_sync(0xffffffffu, top, 2));
     const int ke = (int)(top >> 20);
     long long xa = 0, xt = 0;
+    float sizes = 0.f;  // sum of weight times size, the binade below, in units of 2^(ke - 1022)
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       long long ya = 0, yt = 0;
+      float part = 0.f;
 #pragma unroll
-      for (int j = 0; j < 4; ++j)
-        mul_add(st.w[1][j][p], velocity_digits(b[4 * i + j], ke), ya, yt);
-      mul_add(st.w[0][i][p], digits(sum_of(ya, yt)), xa, xt);
+      for (int j = 0; j < 4; ++j) {
+        const int drop = ke - (int)((hi_word(b[4 * i + j]) >> 20) & 0x7ffu);
+        mul_add(st.w[1][j][p], velocity_digits(b[4 * i + j], drop), ya, yt);
+        part = __fmaf_rn(wyz[j], __uint_as_float((unsigned)max(126 - drop, 0) << 23), part);
+      }
+      sizes = __fmaf_rn(part, (float)st.w[0][i][p].h * 0x1p-31f, sizes);
+      // a product with a weight halves; the sums come back below 2^60
+      mul_add(st.w[0][i][p], digits(2 * sum_of(ya, yt)), xa, xt);
     }
-    long long v = mul_hi(digits(sum_of(xa, xt)), st.w[2][k][p]);
+    long long v = mul_hi(digits(8 * sum_of(xa, xt)), st.w[2][k][p]);
     v += __shfl_xor_sync(0xffffffffu, v, 1);
     v += __shfl_xor_sync(0xffffffffu, v, 2);
     const bool fits = ke >= FIXED_MIN_K && ke <= FIXED_MAX_K;
     const bool lost = st.lost[0][p] | st.lost[1][p] | st.lost[2][p];
-    if (k == 0 && fits) st.vel[c][p] = signed_fixed_to_double(v, ke + 3);
-    // velocities of 0 (a fluid at rest), beyond the integers' range or not
-    // finite: in FP64
-    if (__any_sync(0xffffffffu, !fits && top != 0u)) {
+    if (k == 0 && fits) st.vel[c][p] = signed_fixed_to_double(v, ke - 1);
+    // in FP64: velocities beyond the integers' range or not finite, and stencils whose
+    // largest velocity has so little weight that its units are too coarse for the rest
+    sizes += __shfl_xor_sync(0xffffffffu, sizes, 1);
+    sizes += __shfl_xor_sync(0xffffffffu, sizes, 2);
+    const bool redo = top != 0u && (!fits || sizes < 0x1p-6f);
+    if (__any_sync(0xffffffffu, redo)) {
       double s = 0.0;
 #pragma unroll 1
       for (int q = 0; q < 16; ++q) {
@@ -1352,17 +1369,16 @@ __device__ __forceinline__ void gather64(const double* __restrict__ u, const Dim
       }
       s += __shfl_xor_sync(0xffffffffu, s, 1);
       s += __shfl_xor_sync(0xffffffffu, s, 2);
-      if (k == 0 && !fits) st.vel[c][p] = s;
-    } else if (k == 0 && !fits) {
-      st.vel[c][p] = 0.0;
+      if (k == 0 && redo) st.vel[c][p] = s;
     }
+    if (k == 0 && !fits && !redo) st.vel[c][p] = 0.0;  // a fluid at rest
     // no weights: no velocity
     if (k == 0 && lost) st.vel[c][p] = bits_double(0x7ff8000000000000ull);
   }
 }
 
 template <int POINTS, class I>
-__global__ void __launch_bounds__(move64_block(POINTS)) k_tracers_move_f64(
+__global__ void __launch_bounds__(move64_block(POINTS), POINTS == MOVE64_MANY ? 3 : 4) k_tracers_move_f64(
     int ntr, double* __restrict__ r, double* __restrict__ s, double* __restrict__ v, Dims D,
     const double* __restrict__ u, unsigned* status) {
   __shared__ Stencil64<POINTS> st;
@@ -1391,7 +1407,7 @@ __global__ void __launch_bounds__(move64_block(POINTS)) k_tracers_move_f64(
 // RECORD: the block then records the ends of the moved swimmers into `to`, for
 // the next step (thread (p, a): axis a of the tail, p < half, or head of its swimmer).
 template <bool RECORD, int POINTS, class I>
-__global__ void __launch_bounds__(move64_block(POINTS)) k_swimmers_move_f64(
+__global__ void __launch_bounds__(move64_block(POINTS), POINTS == MOVE64_MANY ? 3 : 4) k_swimmers_move_f64(
     int nsw, double* __restrict__ swr, double* __restrict__ swv, double* __restrict__ swn,
     lbswim_common_params c, unsigned long long seed, unsigned long long step, Dims D,
     const double* __restrict__ u, unsigned* status, RecordTarget<double> to) {
