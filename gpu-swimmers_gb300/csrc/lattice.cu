@@ -12,6 +12,7 @@
 #include <cuda_fp16.h>
 
 #include <algorithm>
+#include <cstdint>
 #include <cstring>
 
 #include "bulk_copy.cuh"
@@ -991,18 +992,31 @@ static double* staging(Lattice* L, size_t elems) {
 // is mapped into the device's address space, so a conversion kernel can read
 // or write the caller's buffer itself over the host link: one pass, with no
 // staging copy and no serialisation of copy and conversion.  Returns the
-// buffer's device address, or null for pageable memory (which goes through
-// the staging buffer).
-const void* mapped_host(const void* host) {
-  cudaPointerAttributes at;
+// buffer's device address; null for pageable memory, also at its end only, and for
+// addresses that a kernel cannot take as doubles (these go through copies).
+const void* mapped_host(const void* host, size_t bytes) {
+  if (bytes == 0 || ((uintptr_t)host & (alignof(double) - 1)) != 0) return nullptr;
   int dev = -1;
-  if (cudaPointerGetAttributes(&at, host) != cudaSuccess || cudaGetDevice(&dev) != cudaSuccess) {
+  if (cudaGetDevice(&dev) != cudaSuccess) {
     (void)cudaGetLastError();
     return nullptr;
   }
-  // page-locked by this device's context (memory pinned under another
-  // device takes the staging path)
-  return at.type == cudaMemoryTypeHost && at.device == dev ? at.devicePointer : nullptr;
+  const char* first = nullptr;
+  for (const size_t off : {(size_t)0, bytes - 1}) {
+    cudaPointerAttributes at;
+    if (cudaPointerGetAttributes(&at, (const char*)host + off) != cudaSuccess) {
+      (void)cudaGetLastError();
+      return nullptr;
+    }
+    // page-locked by this device's context (memory pinned under another
+    // device takes the staging path)
+    if (at.type != cudaMemoryTypeHost || at.device != dev || !at.devicePointer) return nullptr;
+    if (off == 0)
+      first = (const char*)at.devicePointer;
+    else if ((const char*)at.devicePointer != first + off)
+      return nullptr;
+  }
+  return first;
 }
 
 void lattice_zero_force_now(Lattice* L) {
@@ -1438,7 +1452,7 @@ static long long field_count(const Lattice* L, int field) {
 template <class S>
 static void f_h2d_t(Lattice* L, void* dst, const double* host) {
   const long long total = 15 * L->n;
-  if (const double* mh = (const double*)mapped_host(host)) {
+  if (const double* mh = (const double*)mapped_host(host, 8 * total)) {
     k_f_from_f64<S><<<grid_for(total, 256), 256, 0, L->stream>>>(mh, (S*)dst, 0, total, L->n,
                                                                   L->rho0);
     LB_CHECK_LAUNCH(1);
@@ -1459,7 +1473,7 @@ static void f_h2d_t(Lattice* L, void* dst, const double* host) {
 template <class S>
 static void f_d2h_t(Lattice* L, const void* src, double* host) {
   const long long total = 15 * L->n;
-  if (double* mh = (double*)mapped_host(host)) {
+  if (double* mh = (double*)mapped_host(host, 8 * total)) {
     k_f_to_f64<S><<<grid_for(total, 256), 256, 0, L->stream>>>((const S*)src, mh, 0, total,
                                                                 L->n, L->rho0);
     LB_CHECK_LAUNCH(1);
@@ -1510,7 +1524,7 @@ void lattice_h2d(Lattice* L, int field, const double* host) {
       case LBSWIM_BF16: f_h2d_t<__nv_bfloat16>(L, dst, host); break;
       default: f_h2d_t<__half>(L, dst, host); break;
     }
-  } else if (const double* mh = (const double*)mapped_host(host)) {
+  } else if (const double* mh = (const double*)mapped_host(host, 8 * cnt)) {
     const long long N = L->n;
     if (field == LBSWIM_FIELD_FORCE)
       k_f64_to_f32<<<grid_for(cnt, 256), 256, 0, L->stream>>>(mh, (float*)dst, cnt);
@@ -1554,7 +1568,7 @@ void lattice_d2h(Lattice* L, int field, double* host) {
     }
     return;
   }
-  if (double* mh = (double*)mapped_host(host)) {
+  if (double* mh = (double*)mapped_host(host, 8 * cnt)) {
     const long long N = L->n;
     if (field == LBSWIM_FIELD_FORCE)
       k_f32_to_f64<<<grid_for(cnt, 256), 256, 0, L->stream>>>((const float*)src, mh, cnt);

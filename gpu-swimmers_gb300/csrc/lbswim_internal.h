@@ -361,8 +361,9 @@ void swimmers_move_preparing(Swimmers* const* w, int nw, Lattice* L, unsigned lo
 void swimmers_wait(Swimmers* S);
 // Host copies (null: none) of the fields, after that kernel; waits for them.
 void swimmers_read(Swimmers* S, double* r, double* v, double* n);
-// Device address of a page-locked host buffer, null for pageable memory (lattice.cu).
-const void* mapped_host(const void* host);
+// Device address of a buffer of page-locked host memory, null where a kernel cannot use it
+// (lattice.cu).
+const void* mapped_host(const void* host, size_t bytes);
 void tracers_move(Tracers* T, Lattice* L);
 // Move on the tracers' own stream after the point of the lattice stream where
 // L->hydro_ready was last recorded.

@@ -2511,13 +2511,13 @@ void swimmers_read(Swimmers* W, double* r, double* v, double* n) {
   double* dst[3] = {r, v, n};
   const double* src[3] = {W->r, W->v, W->nv};
   double* mapped[3] = {nullptr, nullptr, nullptr};
+  const size_t bytes = sizeof(double) * 3 * (size_t)W->n;
   bool direct = W->n > 0 && W->n <= DIRECT_READ_SWIMMERS;
   for (int f = 0; f < 3 && direct; ++f)
     if (dst[f]) {
-      mapped[f] = (double*)mapped_host(dst[f]);
+      mapped[f] = (double*)mapped_host(dst[f], bytes);
       direct = mapped[f] != nullptr;
     }
-  const size_t bytes = sizeof(double) * 3 * (size_t)W->n;
   if (direct) {
     k_swimmers_to_host<<<(3 * W->n + 255) / 256, 256, 0, W->copy>>>(
         3 * W->n, W->r, W->v, W->nv, mapped[0], mapped[1], mapped[2]);
