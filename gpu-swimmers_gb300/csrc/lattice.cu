@@ -1259,10 +1259,20 @@ int slab_lx_within(const int size[3], int tile, long long nends, int cap) {
   return even_slab(size[0], std::min(cap, longest_slab(size, tile, nends)));
 }
 
+int sm_count() {
+  static const int n = [] {
+    int dev = 0, v = 0;
+    LB_CUDA(cudaGetDevice(&dev));
+    LB_CUDA(cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev));
+    return v;
+  }();
+  return n;
+}
+
 // x planes per slab of a lattice stepped with nends pending ends, by the time
 // its slabs take: a slab takes lx + 2 planes (the ring) and a start that costs
-// about 3 more planes when it lists ends, 1 when not; 304 (or 456) run at a time, and
-// with half of them or fewer each has an SM to itself and takes about 0.65 of
+// about 3 more planes when it lists ends, 1 when not; two an SM (or three) run at a time,
+// and with half of them or fewer each has an SM to itself and takes about 0.65 of
 // the time a plane takes with two.  Ends listed in buckets cost an atomic per
 // slab they touch, about 1 + 5 / lx of them along x.  A small lattice then has
 // enough slabs for the SMs, and a large one wastes less of its last wave.
@@ -1278,16 +1288,20 @@ int choose_slab_lx(const Lattice* L, long long nends) {
   slab_section_of(tile, &ty, &tz);
   const long long section = (long long)((size[1] + ty - 1) / ty) * ((size[2] + tz - 1) / tz);
   const int longest = longest_slab(size, tile, nends);
-  const int SLOTS = elem_bytes(L->precision) == 2 ? 456 : 304;  // fused_ctas
+  const bool copied = fused_uses_tma(L, tz);
+  const int ctas = elem_bytes(L->precision) == 2
+                       ? (copied ? fused_ctas<__nv_bfloat16, true>() : fused_ctas<__nv_bfloat16, false>())
+                       : (copied ? fused_ctas<float, true>() : fused_ctas<float, false>());
+  const int slots = ctas * sm_count();
   int best = 1;
   double least = 0.0;
   for (int lx = 1; lx <= longest; ++lx) {
     if (even_slab(size[0], lx) != lx) continue;  // a shorter slab gives as many
-    const long long slabs = (size[0] + lx - 1) / lx * section, rest = slabs % SLOTS;
+    const long long slabs = (size[0] + lx - 1) / lx * section, rest = slabs % slots;
     const double waves =
-        filled && slabs > 4 * SLOTS
-            ? (double)slabs / SLOTS + 0.5
-            : (double)(slabs / SLOTS) + (rest == 0 ? 0.0 : rest <= SLOTS / 2 ? 0.65 : 1.0);
+        filled && slabs > 4 * slots
+            ? (double)slabs / slots + 0.5
+            : (double)(slabs / slots) + (rest == 0 ? 0.0 : rest <= slots / 2 ? 0.65 : 1.0);
     const double cost = waves * (lx + 2 + (nends > 0 ? 3 : 1)) +
                         (nends > DIRECT_ENDS ? 1.75 * (1 + 5.0 / lx) : 0.0);
     if (least == 0.0 || cost < least) {

@@ -289,6 +289,7 @@ int ens_step_ctas_per_sm();
 // Cross-section (rows, columns) of the slabs of a tile choice, and the x planes
 // per slab of a lattice stepped with nends pending ends.
 void slab_section_of(int tile, int* ty, int* tz);
+int sm_count();
 int choose_slab_lx(const Lattice* L, long long nends);
 // The same with slabs of at most `cap` planes, as even as they come.
 int slab_lx_within(const int size[3], int tile, long long nends, int cap);

@@ -835,12 +835,11 @@ __device__ __forceinline__ double words_to_double(unsigned lo, unsigned mid, int
 // Bound by the integer pipe where most tiles have ends (16,000 warp instructions a
 // tile, a quarter of them in the conversions), so a thread's sites differ in x alone and
 // the record loads run under the zeroing: AddForces at 256^3 with 65,536 swimmers 313 us,
-// against 840 in FP64 by site; 65x47x90 with 1074 20 against 76.  Up to FT_WIDE_TILES,
-// two to an SM, the chain of a block's phases bounds the launch: 512 threads shorten
+// against 840 in FP64 by site; 65x47x90 with 1074 20 against 76.  Up to two tiles
+// to an SM, the chain of a block's phases bounds the launch: 512 threads shorten
 // each, and the list is read with its count (onto a force 24^3 18.6 -> 15.6 us); with
 // more tiles they cost occupancy (80^3 18.8 -> 23.2; 256^3 224 -> 320), and of a few ends
 // without buckets each tile first picks its own (256^3 with 32 swimmers 199 -> 88 us).
-constexpr int FT_WIDE_TILES = 2 * 152;
 template <int THREADS>
 __global__ void __launch_bounds__(THREADS) k_force_fixed(
     Dims D, TileGrid G, const EndRecord<double>* __restrict__ ends, int nends,
@@ -2285,7 +2284,7 @@ static void spread_fixed(Lattice* L, int nends, const TileChains& ch) {
   SpreadScratch& S = L->spread;
   const TileGrid G = force_tiles(L);
   const int ntiles = slabs_of(G);
-  const int threads = ntiles <= FT_WIDE_TILES ? 2 * FT_THREADS : FT_THREADS;
+  const int threads = ntiles <= 2 * sm_count() ? 2 * FT_THREADS : FT_THREADS;
   auto kernel = threads > FT_THREADS ? k_force_fixed<2 * FT_THREADS> : k_force_fixed<FT_THREADS>;
   kernel<<<ntiles, threads, 0, L->stream>>>(
       make_dims(L), G, (const EndRecord<double>*)S.ends, nends,
