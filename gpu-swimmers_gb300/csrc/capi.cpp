@@ -262,9 +262,10 @@ int lbswim_lattice_set_stream(lbswim_lattice* lat, void* stream) {
   LB_CUDA(cudaStreamSynchronize(L->stream));
   L->stream = (cudaStream_t)stream;
   int least = 0, greatest = 0, mine = 0;
-  LB_CUDA(cudaDeviceGetStreamPriorityRange(&least, &greatest));
-  LB_CUDA(cudaStreamGetPriority(L->stream, &mine));
-  L->outranks_tracers = mine < least;
+  L->outranks_tracers =
+      cudaDeviceGetStreamPriorityRange(&least, &greatest) == cudaSuccess &&
+      cudaStreamGetPriority(L->stream, &mine) == cudaSuccess && mine < least;
+  (void)cudaGetLastError();
   API_END
 }
 
@@ -732,6 +733,12 @@ int lbswim_system_step(lbswim_lattice* lat, lbswim_swimmers* const* swimmers, in
   Swimmers* const* w = reinterpret_cast<Swimmers* const*>(swimmers);
   const bool together = swimmers_move_together(w, n_swimmers, L);
   const unsigned long long calls = g_calls.load(std::memory_order_relaxed);
+  struct Beside {  // for the length of the call
+    Lattice* L;
+    ~Beside() { L->tracers_beside = 0; }
+  } beside{L};
+  for (int i = 0; i < n_tracers && L->outranks_tracers; ++i)
+    L->tracers_beside += TR(tracers[i])->n;
   if (n_tracers > 0 && !L->hydro_ready)
     LB_CUDA(cudaEventCreateWithFlags(&L->hydro_ready, cudaEventDisableTiming));
   for (int t = 0; t < nsteps; ++t) {

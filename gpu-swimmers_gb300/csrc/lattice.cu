@@ -1275,15 +1275,15 @@ int sm_count() {
 // and with half of them or fewer each has an SM to itself and takes about 0.65 of
 // the time a plane takes with two.  Ends listed in buckets cost an atomic per
 // slab they touch, about 1 + 5 / lx of them along x.  A small lattice then has
-// enough slabs for the SMs, and a large one wastes less of its last wave.
-// Where tracers move beside the steps at a lower priority they fill the last wave of
-// several, and the slabs take their share of the slots and half a slab more: 256^3
-// with a million tracers 658 us a step in 37 planes, 653 in 32; at equal priority 684
-// and 690, without tracers 586 and 596.
+// enough slabs for the SMs, and a large one wastes less of its last wave.  Tracers that move
+// beside the steps of the present call at a lower priority fill what the last waves
+// leave, as far as they go (a million take about as long as 50 planes of all slots), and then
+// add to the time, with up to half a slab for the slots that wait for one: 256^3 with a
+// million tracers and 65,536 swimmers 663 us a step in 37 planes, 657 in 32, with
+// 8192 swimmers 565 in 37 and 554 in 43; with 500 tracers 588 and 598, 481 and 501.
 int choose_slab_lx(const Lattice* L, long long nends) {
   const int* size = L->size;
   const int tile = L->fused_tile;
-  const bool filled = L->outranks_tracers && L->hydro_ready;
   int ty, tz;
   slab_section_of(tile, &ty, &tz);
   const long long section = (long long)((size[1] + ty - 1) / ty) * ((size[2] + tz - 1) / tz);
@@ -1293,16 +1293,18 @@ int choose_slab_lx(const Lattice* L, long long nends) {
                        ? (copied ? fused_ctas<__nv_bfloat16, true>() : fused_ctas<__nv_bfloat16, false>())
                        : (copied ? fused_ctas<float, true>() : fused_ctas<float, false>());
   const int slots = ctas * sm_count();
+  const double beside = (double)L->tracers_beside / 21000.0;
   int best = 1;
   double least = 0.0;
   for (int lx = 1; lx <= longest; ++lx) {
     if (even_slab(size[0], lx) != lx) continue;  // a shorter slab gives as many
     const long long slabs = (size[0] + lx - 1) / lx * section, rest = slabs % slots;
     const double waves =
-        filled && slabs > 4 * slots
-            ? (double)slabs / slots + 0.5
-            : (double)(slabs / slots) + (rest == 0 ? 0.0 : rest <= slots / 2 ? 0.65 : 1.0);
-    const double cost = waves * (lx + 2 + (nends > 0 ? 3 : 1)) +
+        (double)(slabs / slots) + (rest == 0 ? 0.0 : rest <= slots / 2 ? 0.65 : 1.0);
+    const int planes = lx + 2 + (nends > 0 ? 3 : 1);
+    const double filled =
+        (double)slabs / slots * planes + beside + std::min(beside, 0.5 * planes);
+    const double cost = std::max(waves * planes, filled) +
                         (nends > DIRECT_ENDS ? 1.75 * (1 + 5.0 / lx) : 0.0);
     if (least == 0.0 || cost < least) {
       best = lx;

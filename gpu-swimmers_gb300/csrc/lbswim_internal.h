@@ -168,6 +168,7 @@ struct Lattice {
   std::vector<cudaEvent_t> reader_pool;
   cudaEvent_t hydro_ready = nullptr;  // recorded on stream after CalcHydro, for tracers
   bool outranks_tracers = false;      // stream has a higher priority than theirs
+  long long tracers_beside = 0;       // of the present system step, if outranked
   // CUDA-event timing of the LB step kernel (lbswim_lattice_set_timing)
   bool timing = false;
   std::vector<std::pair<cudaEvent_t, cudaEvent_t>> timed;  // recorded, not yet read
