@@ -148,7 +148,9 @@ static void capture(Ensemble* E, int nsteps_in_graph, cudaGraphExec_t* out) {
 // so a run lasts about the sum of their lx + 5 planes (ring and start) over 304
 // and half a slab more: long slabs for many members, short ones where few
 // members would leave CTAs without a slab.  (512 members of 16^3 to 48x48x96: 2.07 ms a
-// step with up to 60 planes, 2.12 with up to 32; 12 members want 2 to 8.)
+// step with up to 60 planes, 2.12 with up to 32; 12 members want 2 to 8.)  Members whose
+// ends might not all fit one slab's shared memory stay at 32: of a cluster of
+// swimmers, every plane goes through all of the slab's ends.
 static std::vector<int> slab_lengths(const Ensemble* E) {
   std::vector<int> best;
   double least = 0.0;
@@ -159,7 +161,9 @@ static std::vector<int> slab_lengths(const Ensemble* E) {
       const Lattice* L = E->lat[m];
       int ty, tz;
       slab_section_of(L->fused_tile, &ty, &tz);
-      lx[m] = slab_lx_within(L->size, L->fused_tile, E->sw[m] ? 2ll * E->sw[m]->n : 0, cap);
+      const long long nends = E->sw[m] ? 2ll * E->sw[m]->n : 0;
+      lx[m] = slab_lx_within(L->size, L->fused_tile, nends,
+                             nends > SLAB_ENDS_HELD ? std::min(cap, 32) : cap);
       const double slabs = (double)((L->size[0] + lx[m] - 1) / lx[m]) *
                            ((L->size[1] + ty - 1) / ty) * ((L->size[2] + tz - 1) / tz);
       planes += slabs * (lx[m] + 5);

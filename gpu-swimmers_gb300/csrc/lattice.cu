@@ -504,11 +504,8 @@ static_assert(2 * (fused_smem_bytes<16, 16, true>() + 1024) <= 132 * 1024, "SPRE
 // of 256).
 template <class S, bool TMA>
 constexpr int fused_ctas() { return sizeof(S) == 2 && !TMA ? 3 : 2; }
-// Whether the next plane's loads follow the collision (see fused_slab).  The batched
-// step loads first: its members have few ends a slab (512 members 2.07 -> 1.93 ms a
-// step, 96 345 -> 324 us, 12 108 -> 101).
-template <class S, bool SPREAD, bool TMA>
-constexpr bool fused_late_loads() { return (SPREAD || sizeof(S) == 2) && !TMA; }
+// When the next plane's loads are issued (see fused_slab).
+enum class Loads { EARLY, LATE };
 
 // One slab: tile (tz, ty, tx) of the lattice in units of (TZ, TY, a.lx)
 // sites; `slab` indexes its bucket of pending ends.  Called by one CTA.
@@ -517,8 +514,9 @@ constexpr bool fused_late_loads() { return (SPREAD || sizeof(S) == 2) && !TMA; }
 // SPLIT: the form of the slab's force sums (slab_sums_split); SPREAD only.
 // TMA: the distributions of the cross-section's rows arrive by bulk copies
 // into shared memory (tma_* above); the lattice has nz a multiple of 32.
+// ENDS: whether the slab's ends fit shared memory (SlabSpreader).
 template <class S, int TZ, int TY, bool SPREAD, class I, bool SPLIT, bool TMA = false,
-          bool LATE = fused_late_loads<S, SPREAD, TMA>()>
+          Loads LOADS = Loads::EARLY, Ends ENDS = Ends::FEW>
 __device__ __forceinline__ void fused_slab(const FusedArgs& a, int tz, int ty, int tx, int slab) {
   static_assert(sizeof(S) < 8, "the fused step serves the reduced-precision layouts");
   static_assert(!TMA || TZ == 32, "bulk-copied rows are whole 32-site blocks");
@@ -599,7 +597,7 @@ __device__ __forceinline__ void fused_slab(const FusedArgs& a, int tz, int ty, i
   }
 
   // ---- this slab's pending dipole ends and the fixed-point force plane ----
-  SlabSpreader<TZ, TY, 1, spread_base<TZ, TY>(), SPLIT> sp;
+  SlabSpreader<TZ, TY, 1, spread_base<TZ, TY>(), SPLIT, ENDS> sp;
   // the ring threads, which write no output plane, take the first pairs
   const int rt = tid >= NI ? tid - NI : tid + (int)blockDim.x - NI;
   if (SPREAD) {
@@ -633,11 +631,10 @@ __device__ __forceinline__ void fused_slab(const FusedArgs& a, int tz, int ty, i
   float keep0 = 0.f, keep1a = 0.f, keep1b = 0.f;
   int k3 = 0;  // k % 3
   for (int k = 0; k < ex + 2; ++k) {
-    // The instances bound by the chain between their barriers rather than by DRAM load
-    // the next plane into the registers that the collision has just freed (256^3
-    // with ends 521 -> 516 us, 100x75x130 51.7 -> 49.5; it leaves 56 registers a
-    // thread, which 16-bit storage's third CTA needs); the others issue the loads
-    // first, to have them in flight for the whole plane, and copy.
+    // LATE loads the next plane into the registers that the collision has just freed, 56 a
+    // thread with 16-bit storage, as its third CTA needs; EARLY issues the loads first, to
+    // have them in flight for the whole plane, and copies (launch_fused chooses).
+    constexpr bool LATE = LOADS == Loads::LATE;
     float held[18];
     float(&cur)[18] = LATE ? pre : held;
     if (!LATE) {
@@ -740,18 +737,53 @@ __device__ __forceinline__ void fused_slab(const FusedArgs& a, int tz, int ty, i
   if (nonfinite != 0.f) raise_status(a.status, LBSWIM_STATUS_NONFINITE);
 }
 
-template <class S, int TZ, int TY, bool SPREAD, class I, bool TMA>
+// Slabs with more ends than shared memory holds go through the plane loop's other form, in a
+// function of its own, called where nothing else is live: the usual form (with split
+// sums, which its ends always allow) keeps the registers and the instruction cache.
+template <class S, int TZ, int TY, class I>
+__device__ __noinline__ void fused_slab_many(const FusedArgs& a, int tz, int ty, int tx, int slab) {
+  if (slab_sums_split(a.spread, slab, a.nx, a.ny, a.nz))
+    fused_slab<S, TZ, TY, true, I, true, false, Loads::LATE, Ends::MANY>(a, tz, ty, tx, slab);
+  else
+    fused_slab<S, TZ, TY, true, I, false, false, Loads::LATE, Ends::MANY>(a, tz, ty, tx, slab);
+}
+static_assert(SPREAD_CAP * 16 <= 65535, "the usual form's sums are split (slab_sums_split)");
+
+// Whether the ends of a slab without buckets, its own of all pending ones, fit.
+template <int TZ, int TY>
+__device__ __noinline__ bool own_ends_fit(const FusedArgs& a, int tz, int ty, int tx) {
+  const int z0 = tz * TZ, y0 = ty * TY, x0 = tx * a.lx;
+  SlabSpreader<TZ, TY, 1, 0, true> sp;
+  sp.bind(nullptr, a.spread, 0, a.nx, a.ny, a.nz, x0, y0, z0, min(a.lx, a.nx - x0),
+          min(TY, a.ny - y0), min(TZ, a.nz - z0));
+  int n = 0;
+  for (int q0 = 0; q0 < a.spread.npending; q0 += blockDim.x)
+    n += __syncthreads_count(q0 + (int)threadIdx.x < a.spread.npending &&
+                             sp.touches(a.spread.ends[q0 + threadIdx.x]));
+  return n <= SPREAD_CAP;
+}
+template <int TZ, int TY>
+__device__ __forceinline__ bool slab_ends_fit(const FusedArgs& a, int tz, int ty, int tx,
+                                              int slab) {
+  if (a.spread.count) return a.spread.count[slab] <= (unsigned)SPREAD_CAP;
+  return a.spread.npending <= SPREAD_CAP || own_ends_fit<TZ, TY>(a, tz, ty, tx);
+}
+
+template <class S, int TZ, int TY, bool SPREAD, class I, bool TMA, Loads LOADS>
 __global__ void __launch_bounds__(TY * TZ + FUSED_RING_THREADS, fused_ctas<S, TMA>())
-    k_fused_step(FusedArgs a) {
+    k_fused_step(const __grid_constant__ FusedArgs a) {
   const int slab = (blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
   for (int i = slab * blockDim.x + threadIdx.x; i < a.nclear;
        i += gridDim.x * gridDim.y * gridDim.z * blockDim.x)
     a.clear[i] = 0u;
   if (a.clear_max && slab == 0 && threadIdx.x == 0) *a.clear_max = 0u;
-  if (!SPREAD || slab_sums_split(a.spread, slab, a.nx, a.ny, a.nz))
-    fused_slab<S, TZ, TY, SPREAD, I, true, TMA>(a, blockIdx.x, blockIdx.y, blockIdx.z, slab);
-  else
-    fused_slab<S, TZ, TY, SPREAD, I, false, TMA>(a, blockIdx.x, blockIdx.y, blockIdx.z, slab);
+  if constexpr (SPREAD) {
+    if (!slab_ends_fit<TZ, TY>(a, blockIdx.x, blockIdx.y, blockIdx.z, slab)) {
+      fused_slab_many<S, TZ, TY, I>(a, blockIdx.x, blockIdx.y, blockIdx.z, slab);
+      return;
+    }
+  }
+  fused_slab<S, TZ, TY, SPREAD, I, true, TMA, LOADS>(a, blockIdx.x, blockIdx.y, blockIdx.z, slab);
 }
 
 // ---------------------------------------------------------------------------
@@ -777,6 +809,25 @@ constexpr int ENS_STEP_SMEM =
         ? fused_smem_bytes<32, 8, true>()
         : fused_smem_bytes<16, 16, true>();
 static_assert(8 * 32 == 16 * 16, "both slab shapes use the same block");
+
+__device__ __forceinline__ FusedArgs ens_args(const EnsMember& M, int parity) {
+  FusedArgs a{};
+  a.f_old = M.f[parity];
+  a.f_new = M.f[parity ^ 1];
+  a.force = nullptr;
+  a.hydro = (float4*)M.hyd[parity];
+  a.nx = M.size[0];
+  a.ny = M.size[1];
+  a.nz = M.size[2];
+  a.lx = M.lx;
+  a.n = M.n;
+  a.rho0 = M.rho0;
+  a.k = Relax<float>{M.omega_s, M.omega_b, M.force_s, M.force_b};
+  a.spread = SlabEnds{(const EndRecord<float>*)M.ends, M.bucket_count, M.bucket_list, 2 * M.nsw,
+                      M.max_abs_f + parity};
+  a.status = M.status;
+  return a;
+}
 
 // The kernel leaves the counts at zero, and the words of the other parity, for the
 // records that the move makes for the next step.  (A quarter of the slabs of a
@@ -804,27 +855,13 @@ __global__ void __launch_bounds__(8 * 32 + FUSED_RING_THREADS, 2) k_ens_step(Ens
     const int lt = tile - t.tile_prefix[m];
     const int tz = lt % M.nt[2], ty = (lt / M.nt[2]) % M.nt[1], tx = lt / (M.nt[2] * M.nt[1]);
     if (lt == 0 && threadIdx.x == 0) M.max_abs_f[parity ^ 1] = 0u;
-    FusedArgs a{};
-    a.f_old = M.f[parity];
-    a.f_new = M.f[parity ^ 1];
-    a.force = nullptr;
-    a.hydro = (float4*)M.hyd[parity];
-    a.nx = M.size[0];
-    a.ny = M.size[1];
-    a.nz = M.size[2];
-    a.lx = M.lx;
-    a.n = M.n;
-    a.rho0 = M.rho0;
-    a.k = Relax<float>{M.omega_s, M.omega_b, M.force_s, M.force_b};
-    a.spread = SlabEnds{(const EndRecord<float>*)M.ends, M.bucket_count, M.bucket_list,
-                        2 * M.nsw, M.max_abs_f + parity};
-    a.status = M.status;
+    const FusedArgs a = ens_args(M, parity);
     // members have few enough swimmers for split force sums on every slab
     // (checked when the members are set)
     if (M.tile == 1)
-      fused_slab<float, 16, 16, true, int, true, false, false>(a, tz, ty, tx, lt);
+      fused_slab<float, 16, 16, true, int, true, false, Loads::EARLY, Ends::ANY>(a, tz, ty, tx, lt);
     else
-      fused_slab<float, 32, 8, true, int, true, false, false>(a, tz, ty, tx, lt);
+      fused_slab<float, 32, 8, true, int, true, false, Loads::EARLY, Ends::ANY>(a, tz, ty, tx, lt);
     __syncthreads();
     if (threadIdx.x == 0) M.bucket_count[lt] = 0u;  // every thread has read it
   }
@@ -857,24 +894,30 @@ __device__ __forceinline__ void force_slab(const SlabEnds& se, float* __restrict
   const int tid = threadIdx.x;
   const int z0 = blockIdx.x * TZ, y0 = blockIdx.y * TY, x0 = blockIdx.z * lx;
   const int ez = min(TZ, nz - z0), ey = min(TY, ny - y0), ex = min(lx, nx - x0);
-  SlabSpreader<TZ, TY, 0, 0, SPLIT> sp;
-  sp.bind(smraw, se, slab, nx, ny, nz, x0, y0, z0, ex, ey, ez);
-  sp.prologue(tid, blockDim.x);
   const int ly = tid / TZ, lz = tid % TZ;
   const bool valid = ly < ey && lz < ez;
   const int my = ly * TZ + lz;
   const long long yz = (long long)(y0 + ly) * nz + (z0 + lz), nynz = (long long)ny * nz;
-  for (int kk = 0; kk < ex; ++kk) {
-    sp.scatter(kk, tid, blockDim.x);
-    __syncthreads();
-    if (valid) {
-      const long long s = (long long)(x0 + kk) * nynz + yz;
-      float v[3];
-      sp.take(my, v);
+  auto planes = [&](auto sp) {
+    sp.bind(smraw, se, slab, nx, ny, nz, x0, y0, z0, ex, ey, ez);
+    if (!sp.prologue(tid, blockDim.x)) return false;
+    for (int kk = 0; kk < ex; ++kk) {
+      sp.scatter(kk, tid, blockDim.x);
+      __syncthreads();
+      if (valid) {
+        const long long s = (long long)(x0 + kk) * nynz + yz;
+        float v[3];
+        sp.take(my, v);
 #pragma unroll
-      for (int c = 0; c < 3; ++c) force[c * N + s] = accumulate ? force[c * N + s] + v[c] : v[c];
+        for (int c = 0; c < 3; ++c) force[c * N + s] = accumulate ? force[c * N + s] + v[c] : v[c];
+      }
+      __syncthreads();
     }
+    return true;
+  };
+  if (!planes(SlabSpreader<TZ, TY, 0, 0, SPLIT>())) {
     __syncthreads();
+    planes(SlabSpreader<TZ, TY, 0, 0, SPLIT, Ends::MANY>());
   }
 }
 
@@ -1159,23 +1202,23 @@ void lattice_init_from_hydro(Lattice* L) {
   L->f_version++;
 }
 
-template <class S, int TZ, int TY, bool SPREAD, class I, bool TMA>
+template <class S, int TZ, int TY, bool SPREAD, class I, bool TMA, Loads LOADS>
 static void launch_fused_i(Lattice* L, const FusedArgs& a) {
   constexpr int smem = fused_smem_total<S, TZ, TY, SPREAD, TMA>();
   static bool configured = false;  // per template instance, per process
   if (!configured) {
-    LB_CUDA(cudaFuncSetAttribute(k_fused_step<S, TZ, TY, SPREAD, I, TMA>,
+    LB_CUDA(cudaFuncSetAttribute(k_fused_step<S, TZ, TY, SPREAD, I, TMA, LOADS>,
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     // the bulk-copied rows bypass L1: give shared memory the whole carveout so
     // that two CTAs fit an SM
     if (TMA)
-      LB_CUDA(cudaFuncSetAttribute(k_fused_step<S, TZ, TY, SPREAD, I, TMA>,
+      LB_CUDA(cudaFuncSetAttribute(k_fused_step<S, TZ, TY, SPREAD, I, TMA, LOADS>,
                                    cudaFuncAttributePreferredSharedMemoryCarveout,
                                    cudaSharedmemCarveoutMaxShared));
     configured = true;
   }
   dim3 grid((a.nz + TZ - 1) / TZ, (a.ny + TY - 1) / TY, (a.nx + a.lx - 1) / a.lx);
-  k_fused_step<S, TZ, TY, SPREAD, I, TMA>
+  k_fused_step<S, TZ, TY, SPREAD, I, TMA, LOADS>
       <<<grid, TY * TZ + FUSED_RING_THREADS, smem, L->stream>>>(a);
   LB_CHECK_LAUNCH(1);
 }
@@ -1191,22 +1234,38 @@ inline bool fused_uses_tma(const Lattice* L, int TZ) {
   return TZ == 32 && (L->size[2] & 31) == 0 && (L->compat & LBSWIM_COMPAT_BULK_COPY);
 }
 
+template <class S, int TZ, int TY, bool SPREAD, bool TMA, Loads LOADS>
+static void launch_fused_w(Lattice* L, const FusedArgs& a) {
+  if (!fits_int_index(a.n) || (L->compat & LBSWIM_COMPAT_WIDE_INDEX))
+    launch_fused_i<S, TZ, TY, SPREAD, long long, TMA, LOADS>(L, a);
+  else
+    launch_fused_i<S, TZ, TY, SPREAD, int, TMA, LOADS>(L, a);
+}
+
+// FP32 steps with ends load late up to three waves of slabs, where the chain of a plane
+// bounds them (us a step late and early: 100x75x130 71.2 and 73.3, 128^3 with 300 swimmers
+// 86.5 and 88.2), early beyond, where DRAM does (160^3, 4 waves, 167.1 and 166.4; 256^3
+// 587 and 578 with 65,536 swimmers, 480 and 469 with 8192); without ends early.
 template <class S, int TZ, int TY, bool SPREAD>
 static void launch_fused(Lattice* L, const FusedArgs& a) {
-  const bool wide = !fits_int_index(a.n) || (L->compat & LBSWIM_COMPAT_WIDE_INDEX);
   if constexpr (TZ == 32) {
     if (fused_uses_tma(L, TZ)) {
-      if (wide)
-        launch_fused_i<S, TZ, TY, SPREAD, long long, true>(L, a);
-      else
-        launch_fused_i<S, TZ, TY, SPREAD, int, true>(L, a);
+      launch_fused_w<S, TZ, TY, SPREAD, true, Loads::EARLY>(L, a);
       return;
     }
   }
-  if (wide)
-    launch_fused_i<S, TZ, TY, SPREAD, long long, false>(L, a);
-  else
-    launch_fused_i<S, TZ, TY, SPREAD, int, false>(L, a);
+  if constexpr (sizeof(S) == 2) {
+    launch_fused_w<S, TZ, TY, SPREAD, false, Loads::LATE>(L, a);
+  } else if constexpr (SPREAD) {
+    const long long slabs = (long long)((a.nz + TZ - 1) / TZ) * ((a.ny + TY - 1) / TY) *
+                            ((a.nx + a.lx - 1) / a.lx);
+    if (slabs <= 3ll * fused_ctas<S, false>() * sm_count())
+      launch_fused_w<S, TZ, TY, SPREAD, false, Loads::LATE>(L, a);
+    else
+      launch_fused_w<S, TZ, TY, SPREAD, false, Loads::EARLY>(L, a);
+  } else {
+    launch_fused_w<S, TZ, TY, SPREAD, false, Loads::EARLY>(L, a);
+  }
 }
 
 // Pending dipole ends are spread by the step kernel itself (true), or first

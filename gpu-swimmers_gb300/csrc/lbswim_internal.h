@@ -69,6 +69,7 @@ struct TileLists {
 // with more is spread from the whole list of pending ends).
 constexpr int SLAB_BUCKET_CAP = 1024;
 constexpr int SLAB_LX_MAX = 60;  // x planes of a slab at most
+constexpr int SLAB_ENDS_HELD = 256;  // ends of a slab that shared memory holds
 // Up to this many pending ends, every slab (and force tile of an FP64 lattice) picks
 // its own from all of them and no buckets are filled: their atomics, one after
 // another per end, took longer than the small steps that use them.  A

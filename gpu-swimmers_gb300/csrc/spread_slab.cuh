@@ -19,7 +19,7 @@
 
 namespace lbswim {
 
-constexpr int SPREAD_CAP = 256;            // ends of one slab held in shared memory
+constexpr int SPREAD_CAP = SLAB_ENDS_HELD;  // ends of one slab held in shared memory
 constexpr int SPREAD_PLANES_PER_END = 8;   // local planes one end can cover (6 at most)
 constexpr unsigned PL_FOLD = 1u << 10;     // nx < 4: several x nodes fold onto the plane
 constexpr unsigned PL_DUP = 1u << 11;      // a node appears twice in the cross-section
@@ -85,10 +85,37 @@ __device__ __forceinline__ bool slab_sums_split(const SlabEnds& se, int slab, in
   return cnt * (nx < 4 || ny < 4 || nz < 4 ? 16 : 1) <= 65535ll;
 }
 
+// Exact addition of q into the two words w[0], w[1] of a sum.  Split: the
+// low 16 bits (at most 65535 of them sum below 2^32) and q >> 16 (their sum
+// stays within 32 bits).  Otherwise a 64-bit sum: the high word takes the
+// sign of q and the low word's carry, when they do not cancel.
+template <bool SPLIT>
+__device__ __forceinline__ void add_to_sum(unsigned* w, int q) {
+  if (SPLIT) {
+    atomicAdd(w, (unsigned)q & 0xffffu);
+    atomicAdd(reinterpret_cast<int*>(w + 1), q >> 16);
+  } else {
+    const unsigned l = (unsigned)q;
+    const unsigned old = atomicAdd(w, l);
+    const int h = (q >> 31) + (old + l < old ? 1 : 0);
+    if (h != 0) atomicAdd(reinterpret_cast<int*>(w + 1), h);
+  }
+}
+template <int PLANE, bool SPLIT>
+__device__ __forceinline__ void add_to_sums(unsigned* fq, int at, int q0, int q1, int q2) {
+  add_to_sum<SPLIT>(fq + 2 * at, q0);
+  add_to_sum<SPLIT>(fq + 2 * (PLANE + at), q1);
+  add_to_sum<SPLIT>(fq + 2 * (2 * PLANE + at), q2);
+}
+
 // SPLIT: the sums are (sum of the low 16 bits, sum of q >> 16), each added
 // with an atomic that returns nothing; otherwise 64-bit sums whose high word
 // takes the low word's carries (slab_sums_split decides).
-template <int TZ, int TY, int H, int BASE, bool SPLIT>
+// FEW and MANY are the forms for slabs whose ends fit shared memory and for the others
+// (prologue() of FEW tells, by false), apart so that the usual one has the registers and the
+// instruction cache to itself; ANY decides at run time.
+enum class Ends { FEW, MANY, ANY };
+template <int TZ, int TY, int H, int BASE, bool SPLIT, Ends ENDS = Ends::FEW>
 struct SlabSpreader {
   static constexpr int HZ = TZ + 2 * H, PLANE = (TY + 2 * H) * HZ;
   using SL = SpreadLayout<TZ, TY, H, BASE>;
@@ -153,6 +180,17 @@ struct SlabSpreader {
     }
     return m;
   }
+  __device__ static bool reaches(unsigned long long m, const NodeLocal& nl) {
+    const bool in_y = (nl.y[0] & nl.y[1] & nl.y[2] & nl.y[3]) >= 0;
+    const bool in_z = (nl.z[0] & nl.z[1] & nl.z[2] & nl.z[3]) >= 0;
+    return (m & ~(1ull << 63)) != 0ull && in_y && in_z;
+  }
+  // Whether a node of the end lies in the slab or its surroundings.
+  __device__ bool touches(const EndRecord<float>& g) const {
+    NodeLocal nl;
+    const unsigned long long m = cover(g, nl);
+    return reaches(m, nl);
+  }
   __device__ void keep(int q, const EndRecord<float>& g, unsigned long long m,
                        const NodeLocal& nl) const {
     SlabEnd e;
@@ -166,9 +204,15 @@ struct SlabSpreader {
     xmask()[q] = m;
   }
 
-  // Records, coverage masks, local node rows and per-plane lists of the slab's
-  // ends; zeroes the sums.  Every thread of the block calls it.
-  __device__ void prologue(int tid, int nthreads) {
+  // Zeroes the sums and makes records, coverage masks, local node rows and per-plane lists
+  // of the slab's ends; FEW: false when they do not fit (MANY needs none of it).  Every thread
+  // of the block calls it, and all get the same answer.
+  __device__ bool prologue(int tid, int nthreads) {
+    if (ENDS == Ends::MANY) {
+      for (int i = tid; i < 3 * 2 * PLANE; i += nthreads) fq()[i] = 0u;
+      __syncthreads();
+      return true;
+    }
     if (in_smem) {
       for (int q = tid; q < cnt; q += nthreads) {
         const EndRecord<float>& g = ends[list[s0 + q]];
@@ -185,9 +229,7 @@ struct SlabSpreader {
         const EndRecord<float>& g = ends[q];
         NodeLocal nl;
         const unsigned long long m = cover(g, nl);
-        const bool in_y = (nl.y[0] & nl.y[1] & nl.y[2] & nl.y[3]) >= 0;
-        const bool in_z = (nl.z[0] & nl.z[1] & nl.z[2] & nl.z[3]) >= 0;
-        if ((m & ~(1ull << 63)) == 0ull || !in_y || !in_z) continue;
+        if (!reaches(m, nl)) continue;
         const int at = atomicAdd(&picked, 1);
         if (at < SPREAD_CAP) keep(at, g, m, nl);
       }
@@ -197,9 +239,10 @@ struct SlabSpreader {
         cnt = picked;
       }
     }
+    if (ENDS == Ends::FEW && !in_smem) return false;
     for (int i = tid; i < 3 * 2 * PLANE; i += nthreads) fq()[i] = 0u;
     __syncthreads();
-    if (in_smem) {
+    if (ENDS == Ends::FEW || in_smem) {
       // per-plane lists in increasing end position: count, offsets, fill
       const int lane = tid & 31, warp = tid >> 5, nwarps = nthreads >> 5;
       for (int kk = warp; kk < planes(); kk += nwarps) {
@@ -234,34 +277,30 @@ struct SlabSpreader {
       }
       __syncthreads();
     }
+    return true;
   }
 
-  // Exact addition of q into the two words w[0], w[1] of a sum.  Split: the
-  // low 16 bits (at most 65535 of them sum below 2^32) and q >> 16 (their sum
-  // stays within 32 bits).  Otherwise a 64-bit sum: the high word takes the
-  // sign of q and the low word's carry, when they do not cancel.
-  __device__ void add1(unsigned* w, int q) const {
-    if (SPLIT) {
-      atomicAdd(w, (unsigned)q & 0xffffu);
-      atomicAdd(reinterpret_cast<int*>(w + 1), q >> 16);
-    } else {
-      const unsigned l = (unsigned)q;
-      const unsigned old = atomicAdd(w, l);
-      const int h = (q >> 31) + (old + l < old ? 1 : 0);
-      if (h != 0) atomicAdd(reinterpret_cast<int*>(w + 1), h);
-    }
-  }
   __device__ void add3(int at, int q0, int q1, int q2) const {
-    add1(fq() + 2 * at, q0);
-    add1(fq() + 2 * (PLANE + at), q1);
-    add1(fq() + 2 * (2 * PLANE + at), q2);
+    add_to_sums<PLANE, SPLIT>(fq(), at, q0, q1, q2);
+  }
+
+  // Add node (jy, jz) of an end, of x weight wx.
+  __device__ void add_from_record(const EndRecord<float>& e, int jy, int jz, float wx) const {
+    const float py = e.phi[1][jy], pz = e.phi[2][jz];
+    const int q0 = fx_quant32(node_contrib(py, pz, wx, e.F[0]), fx_scale);
+    const int q1 = fx_quant32(node_contrib(py, pz, wx, e.F[1]), fx_scale);
+    const int q2 = fx_quant32(node_contrib(py, pz, wx, e.F[2]), fx_scale);
+    const int yg = wrap_any(e.o[1] + jy, ny), zg = wrap_any(e.o[2] + jz, nz);
+    for (int ly2 = wrap_any(yg - y0 + H, ny); ly2 <= ey - 1 + 2 * H; ly2 += ny)
+      for (int lz2 = wrap_any(zg - z0 + H, nz); lz2 <= ez - 1 + 2 * H; lz2 += nz)
+        add3(ly2 * HZ + lz2, q0, q1, q2);
   }
 
   // Add the contributions of local plane kk; this thread takes the pairs
   // t0, t0 + stride, ...
   __device__ void scatter(int kk, int t0, int stride) const {
     const int gx = wrap_once(x0 - H + kk, nx);
-    if (in_smem) {
+    if (ENDS == Ends::FEW || (ENDS == Ends::ANY && in_smem)) {
       const int p0 = poff()[kk], np = poff()[kk + 1] - p0;
       for (int t = t0; t < np * 16; t += stride) {
         const unsigned ent = plist()[p0 + (t >> 4)];
@@ -288,21 +327,40 @@ struct SlabSpreader {
               add3(a2 * HZ + b2, q0, q1, q2);
         }
       }
-    } else {
-      // more ends than shared memory holds: records from global memory
+    } else if (ENDS == Ends::ANY) {
+      // records from global memory
       for (int t = t0; t < cnt * 16; t += stride) {
         const EndRecord<float>& e = ends[overflow ? (t >> 4) : list[s0 + (t >> 4)]];
         float wx;
         if (!cover_weight(gx, e.o[0], nx, e.phi[0], wx)) continue;
-        const int jy = (t >> 2) & 3, jz = t & 3;
-        const float py = e.phi[1][jy], pz = e.phi[2][jz];
-        const int q0 = fx_quant32(node_contrib(py, pz, wx, e.F[0]), fx_scale);
-        const int q1 = fx_quant32(node_contrib(py, pz, wx, e.F[1]), fx_scale);
-        const int q2 = fx_quant32(node_contrib(py, pz, wx, e.F[2]), fx_scale);
-        const int yg = wrap_any(e.o[1] + jy, ny), zg = wrap_any(e.o[2] + jz, nz);
-        for (int ly2 = wrap_any(yg - y0 + H, ny); ly2 <= ey - 1 + 2 * H; ly2 += ny)
-          for (int lz2 = wrap_any(zg - z0 + H, nz); lz2 <= ez - 1 + 2 * H; lz2 += nz)
-            add3(ly2 * HZ + lz2, q0, q1, q2);
+        add_from_record(e, (t >> 2) & 3, t & 3, wx);
+      }
+    } else {
+      // records from global memory: a lane tests an end, then half a warp adds the nodes
+      // of each that covers the plane (with sixteen threads testing every end, 256^3 with
+      // 65,536 swimmers in 100^3 took 45 ms a step)
+      const int lane = t0 & 31, node = lane & 15;
+      const int jy = node >> 2, jz = node & 3;
+      for (int base = t0 - lane; base < cnt; base += stride) {
+        const int q = base + lane;
+        float w = 0.f;
+        bool covers = false;
+        int id = 0;
+        if (q < cnt) {
+          id = overflow ? q : list[s0 + q];
+          covers = cover_weight(gx, ends[id].o[0], nx, ends[id].phi[0], w);
+        }
+        for (unsigned m = __ballot_sync(0xffffffffu, covers); m;) {
+          const int first = __ffs(m) - 1;
+          m &= m - 1;
+          const int second = m ? __ffs(m) - 1 : first;
+          const bool waits = lane >= 16 && !m;  // no second end
+          m &= m - 1;
+          const int src = lane < 16 ? first : second;
+          const int end = __shfl_sync(0xffffffffu, id, src);
+          const float wx = __shfl_sync(0xffffffffu, w, src);
+          if (!waits) add_from_record(ends[end], jy, jz, wx);
+        }
       }
     }
   }
