@@ -4,7 +4,8 @@
 // One batched step is two launches over all members: one persistent step kernel
 // that takes the slabs of every member from a shared counter, and one move kernel
 // over every swimmer and tracer array, which also makes the dipole-end records of
-// the next step (listed under the slabs they touch).  A run begins with a reset of
+// the next step (listed under the slabs they touch); with members of more than 256
+// ends a third beside the first, for slabs that hold more.  A run begins with a reset of
 // the slab counts and the records of its first step.  Everything the kernels need
 // comes from device tables, so the launches of two consecutive steps are captured
 // once into a CUDA graph and replayed; a change of membership rewrites the tables
@@ -33,10 +34,11 @@ struct Ensemble {
   std::vector<EnsMember> hmem;  // by position in the run: longest slabs first
   std::vector<int> order;       // the member at a position
   std::vector<int> pre[4];
-  cudaStream_t stream = nullptr;
-  cudaEvent_t done = nullptr;
+  cudaStream_t stream = nullptr, side = nullptr;
+  cudaEvent_t done = nullptr, fork = nullptr;
   cudaGraphExec_t g2 = nullptr, g1 = nullptr;
   bool longest_slabs = false;  // as in a run of many members (autotuner)
+  bool many = false;  // a sparse member has more ends than a slab holds (as captured)
   int grid_step = 0, grid_rec = 0, grid_move = 0;
 };
 
@@ -49,7 +51,9 @@ static void drop_graphs(Ensemble* E) {
 Ensemble* ensemble_new() {
   Ensemble* E = new Ensemble();
   LB_CUDA(cudaStreamCreateWithFlags(&E->stream, cudaStreamNonBlocking));
+  LB_CUDA(cudaStreamCreateWithFlags(&E->side, cudaStreamNonBlocking));
   LB_CUDA(cudaEventCreateWithFlags(&E->done, cudaEventDisableTiming));
+  LB_CUDA(cudaEventCreateWithFlags(&E->fork, cudaEventDisableTiming));
   int dev = 0, sms = 0;
   LB_CUDA(cudaGetDevice(&dev));
   LB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
@@ -65,6 +69,8 @@ void ensemble_delete(Ensemble* E) {
   drop_graphs(E);
   if (E->tables) cudaFree(E->tables);
   cudaEventDestroy(E->done);
+  cudaEventDestroy(E->fork);
+  cudaStreamDestroy(E->side);
   cudaStreamDestroy(E->stream);
   delete E;
 }
@@ -135,7 +141,15 @@ static void capture(Ensemble* E, int nsteps_in_graph, cudaGraphExec_t* out) {
   cudaGraph_t g = nullptr;
   LB_CUDA(cudaStreamBeginCapture(E->stream, cudaStreamCaptureModeThreadLocal));
   for (int p = 0; p < nsteps_in_graph; ++p) {
+    // slabs past what shared memory holds, on a branch of their own
+    if (E->many) {
+      LB_CUDA(cudaEventRecord(E->fork, E->stream));
+      LB_CUDA(cudaStreamWaitEvent(E->side, E->fork, 0));
+      ens_launch_step_many(E->t, p, E->grid_step, E->side);
+      LB_CUDA(cudaEventRecord(E->fork, E->side));
+    }
     ens_launch_step(E->t, p, E->grid_step, E->stream);
+    if (E->many) LB_CUDA(cudaStreamWaitEvent(E->stream, E->fork, 0));
     ens_launch_move(E->t, p, E->grid_move, E->stream);
   }
   LB_CUDA(cudaStreamEndCapture(E->stream, &g));
@@ -148,9 +162,7 @@ static void capture(Ensemble* E, int nsteps_in_graph, cudaGraphExec_t* out) {
 // so a run lasts about the sum of their lx + 5 planes (ring and start) over 304
 // and half a slab more: long slabs for many members, short ones where few
 // members would leave CTAs without a slab.  (512 members of 16^3 to 48x48x96: 2.07 ms a
-// step with up to 60 planes, 2.12 with up to 32; 12 members want 2 to 8.)  Members whose
-// ends might not all fit one slab's shared memory stay at 32: of a cluster of
-// swimmers, every plane goes through all of the slab's ends.
+// step with up to 60 planes, 2.12 with up to 32; 12 members want 2 to 8.)
 static std::vector<int> slab_lengths(const Ensemble* E) {
   std::vector<int> best;
   double least = 0.0;
@@ -161,9 +173,7 @@ static std::vector<int> slab_lengths(const Ensemble* E) {
       const Lattice* L = E->lat[m];
       int ty, tz;
       slab_section_of(L->fused_tile, &ty, &tz);
-      const long long nends = E->sw[m] ? 2ll * E->sw[m]->n : 0;
-      lx[m] = slab_lx_within(L->size, L->fused_tile, nends,
-                             nends > SLAB_ENDS_HELD ? std::min(cap, 32) : cap);
+      lx[m] = slab_lx_within(L->size, L->fused_tile, E->sw[m] ? 2ll * E->sw[m]->n : 0, cap);
       const double slabs = (double)((L->size[0] + lx[m] - 1) / lx[m]) *
                            ((L->size[1] + ty - 1) / ty) * ((L->size[2] + tz - 1) / tz);
       planes += slabs * (lx[m] + 5);
@@ -199,6 +209,7 @@ static void build_tables(Ensemble* E) {
     EnsMember& M = E->hmem[m];
     const int nsw = W ? W->n : 0, ntr = T ? T->n : 0;
     M.lx = lx[i];
+    M.dense = slabs_overfull(L->size, L->fused_tile, 2ll * nsw, M.lx);
     spread_reserve(L, 2 * nsw, M.lx);
     for (int a = 0; a < 3; ++a) M.size[a] = L->size[a];
     M.n = L->n;
@@ -273,12 +284,18 @@ void ensemble_step(Ensemble* E, int nsteps, const int* limits) {
     took[m] = limits ? std::max(0, std::min(nsteps, limits[i])) : nsteps;
     E->hmem[m].limit = took[m];
   }
+  bool many = false;
+  for (const EnsMember& M : E->hmem) many = many || (2 * M.nsw > SLAB_ENDS_HELD && !M.dense);
+  if (many != E->many) {
+    drop_graphs(E);
+    E->many = many;
+  }
   begin_run(E);
   if (!E->g2) capture(E, 2, &E->g2);
   if (!E->g1) capture(E, 1, &E->g1);
   for (int i = 0; i < nsteps / 2; ++i) LB_CUDA(cudaGraphLaunch(E->g2, E->stream));
   if (nsteps & 1) LB_CUDA(cudaGraphLaunch(E->g1, E->stream));
-  count_launches(2ull * nsteps);
+  count_launches((many ? 3ull : 2ull) * nsteps);
   ens_launch_finish(E->t, n, E->stream);
   // the host copies above must outlive the copies: wait for the run
   LB_CUDA(cudaStreamSynchronize(E->stream));

@@ -514,10 +514,11 @@ enum class Loads { EARLY, LATE };
 // SPLIT: the form of the slab's force sums (slab_sums_split); SPREAD only.
 // TMA: the distributions of the cross-section's rows arrive by bulk copies
 // into shared memory (tma_* above); the lattice has nz a multiple of 32.
-// ENDS: whether the slab's ends fit shared memory (SlabSpreader).
+// ENDS: whether the slab's ends fit shared memory (SlabSpreader); FEW returns false, with
+// nothing done, for a slab whose ends do not.
 template <class S, int TZ, int TY, bool SPREAD, class I, bool SPLIT, bool TMA = false,
           Loads LOADS = Loads::EARLY, Ends ENDS = Ends::FEW>
-__device__ __forceinline__ void fused_slab(const FusedArgs& a, int tz, int ty, int tx, int slab) {
+__device__ __forceinline__ bool fused_slab(const FusedArgs& a, int tz, int ty, int tx, int slab) {
   static_assert(sizeof(S) < 8, "the fused step serves the reduced-precision layouts");
   static_assert(!TMA || TZ == 32, "bulk-copied rows are whole 32-site blocks");
   constexpr int NI = TY * TZ;
@@ -602,7 +603,13 @@ __device__ __forceinline__ void fused_slab(const FusedArgs& a, int tz, int ty, i
   const int rt = tid >= NI ? tid - NI : tid + (int)blockDim.x - NI;
   if (SPREAD) {
     sp.bind(smraw, a.spread, slab, nx, ny, nz, x0, y0, z0, ex, ey, ez);
-    sp.prologue(tid, blockDim.x);
+    if (!sp.prologue(tid, blockDim.x)) {
+      if constexpr (TMA) {  // the copies under way land in stages that nothing reads
+        for (int st = 0; st < TMA_STAGES; ++st)
+          mbar_wait(bars + st, 0u, a.status, LBSWIM_STATUS_COPY_TIMEOUT);
+      }
+      return false;
+    }
     sp.scatter(0, rt, blockDim.x);
     __syncthreads();
   }
@@ -735,11 +742,13 @@ __device__ __forceinline__ void fused_slab(const FusedArgs& a, int tz, int ty, i
     k3 = k3 == 2 ? 0 : k3 + 1;
   }
   if (nonfinite != 0.f) raise_status(a.status, LBSWIM_STATUS_NONFINITE);
+  return true;
 }
 
 // Slabs with more ends than shared memory holds go through the plane loop's other form, in a
-// function of its own, called where nothing else is live: the usual form (with split
-// sums, which its ends always allow) keeps the registers and the instruction cache.
+// function of its own, called where nothing else is live (a call, or the code itself,
+// in the plane loop cost the usual slabs 2 to 8%): the usual form, with split sums, which
+// its ends always allow, keeps the registers and the instruction cache.
 template <class S, int TZ, int TY, class I>
 __device__ __noinline__ void fused_slab_many(const FusedArgs& a, int tz, int ty, int tx, int slab) {
   if (slab_sums_split(a.spread, slab, a.nx, a.ny, a.nz))
@@ -749,26 +758,6 @@ __device__ __noinline__ void fused_slab_many(const FusedArgs& a, int tz, int ty,
 }
 static_assert(SPREAD_CAP * 16 <= 65535, "the usual form's sums are split (slab_sums_split)");
 
-// Whether the ends of a slab without buckets, its own of all pending ones, fit.
-template <int TZ, int TY>
-__device__ __noinline__ bool own_ends_fit(const FusedArgs& a, int tz, int ty, int tx) {
-  const int z0 = tz * TZ, y0 = ty * TY, x0 = tx * a.lx;
-  SlabSpreader<TZ, TY, 1, 0, true> sp;
-  sp.bind(nullptr, a.spread, 0, a.nx, a.ny, a.nz, x0, y0, z0, min(a.lx, a.nx - x0),
-          min(TY, a.ny - y0), min(TZ, a.nz - z0));
-  int n = 0;
-  for (int q0 = 0; q0 < a.spread.npending; q0 += blockDim.x)
-    n += __syncthreads_count(q0 + (int)threadIdx.x < a.spread.npending &&
-                             sp.touches(a.spread.ends[q0 + threadIdx.x]));
-  return n <= SPREAD_CAP;
-}
-template <int TZ, int TY>
-__device__ __forceinline__ bool slab_ends_fit(const FusedArgs& a, int tz, int ty, int tx,
-                                              int slab) {
-  if (a.spread.count) return a.spread.count[slab] <= (unsigned)SPREAD_CAP;
-  return a.spread.npending <= SPREAD_CAP || own_ends_fit<TZ, TY>(a, tz, ty, tx);
-}
-
 template <class S, int TZ, int TY, bool SPREAD, class I, bool TMA, Loads LOADS>
 __global__ void __launch_bounds__(TY * TZ + FUSED_RING_THREADS, fused_ctas<S, TMA>())
     k_fused_step(const __grid_constant__ FusedArgs a) {
@@ -777,13 +766,11 @@ __global__ void __launch_bounds__(TY * TZ + FUSED_RING_THREADS, fused_ctas<S, TM
        i += gridDim.x * gridDim.y * gridDim.z * blockDim.x)
     a.clear[i] = 0u;
   if (a.clear_max && slab == 0 && threadIdx.x == 0) *a.clear_max = 0u;
-  if constexpr (SPREAD) {
-    if (!slab_ends_fit<TZ, TY>(a, blockIdx.x, blockIdx.y, blockIdx.z, slab)) {
-      fused_slab_many<S, TZ, TY, I>(a, blockIdx.x, blockIdx.y, blockIdx.z, slab);
-      return;
-    }
+  const int tz = blockIdx.x, ty = blockIdx.y, tx = blockIdx.z;
+  if (!fused_slab<S, TZ, TY, SPREAD, I, true, TMA, LOADS>(a, tz, ty, tx, slab)) {
+    __syncthreads();
+    fused_slab_many<S, TZ, TY, I>(a, tz, ty, tx, slab);
   }
-  fused_slab<S, TZ, TY, SPREAD, I, true, TMA, LOADS>(a, blockIdx.x, blockIdx.y, blockIdx.z, slab);
 }
 
 // ---------------------------------------------------------------------------
@@ -824,17 +811,23 @@ __device__ __forceinline__ FusedArgs ens_args(const EnsMember& M, int parity) {
   a.rho0 = M.rho0;
   a.k = Relax<float>{M.omega_s, M.omega_b, M.force_s, M.force_b};
   a.spread = SlabEnds{(const EndRecord<float>*)M.ends, M.bucket_count, M.bucket_list, 2 * M.nsw,
-                      M.max_abs_f + parity};
+                      M.max_abs_f + parity, M.dense != 0};
   a.status = M.status;
   return a;
 }
 
+// A slab whose ends do not fit is passed over by k_ens_step, for k_ens_step_many; the later of the two clears its count, for the records
+// of the next step, the first one marks it (SLAB_COUNT).
+__device__ __forceinline__ void ens_release(unsigned* count) {
+  if (atomicOr(count, ~SLAB_COUNT) & ~SLAB_COUNT) *count = 0u;
+}
 // The kernel leaves the counts at zero, and the words of the other parity, for the
 // records that the move makes for the next step.  (A quarter of the slabs of a
 // batch of 96 members has no ends; the code of a step without forces for those,
 // compiled in beside the rest, took the registers of both: 432 against 386 us a
 // step.)
-__global__ void __launch_bounds__(8 * 32 + FUSED_RING_THREADS, 2) k_ens_step(EnsTable t, int parity) {
+__global__ void __launch_bounds__(8 * 32 + FUSED_RING_THREADS, 2)
+    k_ens_step(EnsTable t, int parity) {
   __shared__ int s_tile;
   const int nmem = *t.nmem;
   const int total = t.tile_prefix[nmem];
@@ -856,14 +849,61 @@ __global__ void __launch_bounds__(8 * 32 + FUSED_RING_THREADS, 2) k_ens_step(Ens
     const int tz = lt % M.nt[2], ty = (lt / M.nt[2]) % M.nt[1], tx = lt / (M.nt[2] * M.nt[1]);
     if (lt == 0 && threadIdx.x == 0) M.max_abs_f[parity ^ 1] = 0u;
     const FusedArgs a = ens_args(M, parity);
-    // members have few enough swimmers for split force sums on every slab
-    // (checked when the members are set)
-    if (M.tile == 1)
-      fused_slab<float, 16, 16, true, int, true, false, Loads::EARLY, Ends::ANY>(a, tz, ty, tx, lt);
-    else
-      fused_slab<float, 32, 8, true, int, true, false, Loads::EARLY, Ends::ANY>(a, tz, ty, tx, lt);
+    const bool done =
+        M.tile == 1
+            ? fused_slab<float, 16, 16, true, int, true, false, Loads::EARLY, Ends::ANY>(a, tz, ty,
+                                                                                        tx, lt)
+            : fused_slab<float, 32, 8, true, int, true, false, Loads::EARLY, Ends::ANY>(a, tz, ty,
+                                                                                       tx, lt);
+    __syncthreads();  // every thread has read the count
+    if (threadIdx.x == 0) {
+      if (done)
+        M.bucket_count[lt] = 0u;
+      else
+        ens_release(M.bucket_count + lt);
+    }
+  }
+}
+
+// The slabs with more ends than shared memory holds, beside k_ens_step (launched only for
+// batches with a member of so many ends): a block looks at every gridDim-th slab, a thread
+// each, and steps those it finds one after another.  In k_ens_step, as code or as a call,
+// this cost all slabs 2 to 20%; but small dense members, every slab of which has that
+// many, stay there in a plainer form (96 members with them here 395 us a step, there 375).
+__global__ void __launch_bounds__(8 * 32 + FUSED_RING_THREADS, 2)
+    k_ens_step_many(EnsTable t, int parity) {
+  __shared__ int2 found[8 * 32 + FUSED_RING_THREADS];  // member, slab
+  __shared__ int nfound;
+  const int nmem = *t.nmem;
+  const int total = t.tile_prefix[nmem];
+  const long long g = t.g_step[parity];
+  for (int base = blockIdx.x; base < total; base += (int)(gridDim.x * blockDim.x)) {
+    if (threadIdx.x == 0) nfound = 0;
     __syncthreads();
-    if (threadIdx.x == 0) M.bucket_count[lt] = 0u;  // every thread has read it
+    const long long mine = base + (long long)threadIdx.x * gridDim.x;
+    if (mine < total) {
+      const int m = ens_member_of(t.tile_prefix, nmem, (int)mine);
+      const EnsMember& M = t.mem[m];
+      const int lt = (int)mine - t.tile_prefix[m];
+      if (2 * M.nsw > SPREAD_CAP && !M.dense && g < M.limit &&
+          (M.bucket_count[lt] & SLAB_COUNT) > (unsigned)SPREAD_CAP)
+        found[atomicAdd(&nfound, 1)] = make_int2(m, lt);
+    }
+    __syncthreads();
+    const int n = nfound;
+    for (int i = 0; i < n; ++i) {
+      const EnsMember& M = t.mem[found[i].x];
+      const int lt = found[i].y;
+      const int tz = lt % M.nt[2], ty = (lt / M.nt[2]) % M.nt[1], tx = lt / (M.nt[2] * M.nt[1]);
+      const FusedArgs a = ens_args(M, parity);
+      if (M.tile == 1)
+        fused_slab_many<float, 16, 16, int>(a, tz, ty, tx, lt);
+      else
+        fused_slab_many<float, 32, 8, int>(a, tz, ty, tx, lt);
+      __syncthreads();
+      if (threadIdx.x == 0) ens_release(M.bucket_count + lt);
+    }
+    __syncthreads();
   }
 }
 
@@ -877,6 +917,17 @@ void ens_launch_step(const EnsTable& t, int parity, int grid, cudaStream_t s) {
     configured = true;
   }
   k_ens_step<<<grid, 8 * 32 + FUSED_RING_THREADS, ENS_STEP_SMEM, s>>>(t, parity);
+  LB_CHECK_LAUNCH(1);
+}
+
+void ens_launch_step_many(const EnsTable& t, int parity, int grid, cudaStream_t s) {
+  static bool configured = false;
+  if (!configured) {
+    LB_CUDA(cudaFuncSetAttribute(k_ens_step_many, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 ENS_STEP_SMEM));
+    configured = true;
+  }
+  k_ens_step_many<<<grid, 8 * 32 + FUSED_RING_THREADS, ENS_STEP_SMEM, s>>>(t, parity);
   LB_CHECK_LAUNCH(1);
 }
 
@@ -1312,6 +1363,14 @@ static int longest_slab(const int size[3], int tile, long long nends) {
 static int even_slab(int nx, int lx) {
   const int ns = (nx + lx - 1) / lx;
   return (nx + ns - 1) / ns;
+}
+
+bool slabs_overfull(const int size[3], int tile, long long nends, int lx) {
+  int ty, tz;
+  slab_section_of(tile, &ty, &tz);
+  return (double)nends / ((double)size[0] * size[1] * size[2]) * std::min(lx + 5, size[0]) *
+             std::min(ty + 5, size[1]) * std::min(tz + 5, size[2]) >
+         180.0;
 }
 
 int slab_lx_within(const int size[3], int tile, long long nends, int cap) {

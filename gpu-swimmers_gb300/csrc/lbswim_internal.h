@@ -241,6 +241,7 @@ struct EnsMember {
   float omega_s, omega_b, force_s, force_b;  // Relax<float>
   int tile;                                  // slab shape: 0 = 8 x 32, 1 = 16 x 16
   int lx;                                    // x planes per slab
+  int dense;                                 // every slab may have more ends than it holds
   unsigned by_lx[2];                         // FastDiv by it
   int nt[3];                                 // slabs per axis
   void* f[2];           // f(t) at the run's start, and the other buffer
@@ -286,6 +287,8 @@ void ens_launch_reset(const EnsTable& t, cudaStream_t s);
 void ens_launch_finish(const EnsTable& t, int members, cudaStream_t s);
 void ens_launch_records(const EnsTable& t, int grid, cudaStream_t s);
 void ens_launch_step(const EnsTable& t, int parity, int grid, cudaStream_t s);
+// Beside it, for members with more ends than a slab's shared memory holds.
+void ens_launch_step_many(const EnsTable& t, int parity, int grid, cudaStream_t s);
 void ens_launch_move(const EnsTable& t, int parity, int grid, cudaStream_t s);
 int ens_step_ctas_per_sm();
 // Cross-section (rows, columns) of the slabs of a tile choice, and the x planes
@@ -295,6 +298,8 @@ int sm_count();
 int choose_slab_lx(const Lattice* L, long long nends);
 // The same with slabs of at most `cap` planes, as even as they come.
 int slab_lx_within(const int size[3], int tile, long long nends, int cap);
+// Whether slabs of lx planes hold more than 180 of nends ends spread evenly.
+bool slabs_overfull(const int size[3], int tile, long long nends, int lx);
 // Multiplier and shift of a division by lx (FastDiv).
 void slab_division(int lx, unsigned by[2]);
 

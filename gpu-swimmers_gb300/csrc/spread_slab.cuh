@@ -65,12 +65,14 @@ struct SpreadLayout {
 // Where the ends of slab `slab` are: its bucket; every pending end when the bucket
 // overflowed, or when there are no buckets (count null: DIRECT_ENDS ends at most,
 // of which a slab picks its own).
+constexpr unsigned SLAB_COUNT = 0x7fffffffu;  // of a count; the other bit: k_ens_step's mark
 struct SlabEnds {
   const EndRecord<float>* ends;
   const unsigned* count;  // [slabs]
   const int* list;        // [slabs][SLAB_BUCKET_CAP]
   int npending;
   const unsigned* max_abs_f;
+  bool dense = false;  // Ends::ANY: more than shared memory holds is to be expected
 };
 
 // Whether the sums of slab `slab` can take the split form: a site takes at
@@ -80,7 +82,7 @@ struct SlabEnds {
 // the same choice.
 __device__ __forceinline__ bool slab_sums_split(const SlabEnds& se, int slab, int nx, int ny,
                                                 int nz) {
-  const unsigned c = se.count ? se.count[slab] : ~0u;
+  const unsigned c = se.count ? se.count[slab] & SLAB_COUNT : ~0u;
   const long long cnt = c > (unsigned)SLAB_BUCKET_CAP ? se.npending : (long long)c;
   return cnt * (nx < 4 || ny < 4 || nz < 4 ? 16 : 1) <= 65535ll;
 }
@@ -113,7 +115,8 @@ __device__ __forceinline__ void add_to_sums(unsigned* fq, int at, int q0, int q1
 // takes the low word's carries (slab_sums_split decides).
 // FEW and MANY are the forms for slabs whose ends fit shared memory and for the others
 // (prologue() of FEW tells, by false), apart so that the usual one has the registers and the
-// instruction cache to itself; ANY decides at run time.
+// instruction cache to itself.  ANY is FEW with a plain form of the other beside it for
+// slabs that say `dense` (batched members with that many ends on every slab).
 enum class Ends { FEW, MANY, ANY };
 template <int TZ, int TY, int H, int BASE, bool SPLIT, Ends ENDS = Ends::FEW>
 struct SlabSpreader {
@@ -125,7 +128,7 @@ struct SlabSpreader {
   const int* list;
   long long s0;
   int cnt;
-  bool in_smem, overflow, direct;
+  bool in_smem, overflow, direct, dense;
   float fx_scale, fx_inv;
   // shared-memory arrays at fixed offsets from smem
   __device__ unsigned* fq() const { return reinterpret_cast<unsigned*>(smem + SL::fq); }
@@ -148,8 +151,9 @@ struct SlabSpreader {
     fx_inv = exp2_int(-e);
     ends = se.ends;
     list = se.list;
+    dense = se.dense;
     direct = se.count == nullptr;
-    const unsigned c = direct ? 0u : se.count[slab];
+    const unsigned c = direct ? 0u : se.count[slab] & SLAB_COUNT;
     overflow = direct || c > (unsigned)SLAB_BUCKET_CAP;
     cnt = overflow ? se.npending : (int)c;
     s0 = (long long)slab * SLAB_BUCKET_CAP;
@@ -179,17 +183,6 @@ struct SlabSpreader {
       if (ly2 + ny <= ey - 1 + 2 * H || lz2 + nz <= ez - 1 + 2 * H) m |= 1ull << 63;
     }
     return m;
-  }
-  __device__ static bool reaches(unsigned long long m, const NodeLocal& nl) {
-    const bool in_y = (nl.y[0] & nl.y[1] & nl.y[2] & nl.y[3]) >= 0;
-    const bool in_z = (nl.z[0] & nl.z[1] & nl.z[2] & nl.z[3]) >= 0;
-    return (m & ~(1ull << 63)) != 0ull && in_y && in_z;
-  }
-  // Whether a node of the end lies in the slab or its surroundings.
-  __device__ bool touches(const EndRecord<float>& g) const {
-    NodeLocal nl;
-    const unsigned long long m = cover(g, nl);
-    return reaches(m, nl);
   }
   __device__ void keep(int q, const EndRecord<float>& g, unsigned long long m,
                        const NodeLocal& nl) const {
@@ -229,7 +222,9 @@ struct SlabSpreader {
         const EndRecord<float>& g = ends[q];
         NodeLocal nl;
         const unsigned long long m = cover(g, nl);
-        if (!reaches(m, nl)) continue;
+        const bool in_y = (nl.y[0] & nl.y[1] & nl.y[2] & nl.y[3]) >= 0;
+        const bool in_z = (nl.z[0] & nl.z[1] & nl.z[2] & nl.z[3]) >= 0;
+        if ((m & ~(1ull << 63)) == 0ull || !in_y || !in_z) continue;
         const int at = atomicAdd(&picked, 1);
         if (at < SPREAD_CAP) keep(at, g, m, nl);
       }
@@ -239,7 +234,7 @@ struct SlabSpreader {
         cnt = picked;
       }
     }
-    if (ENDS == Ends::FEW && !in_smem) return false;
+    if (!in_smem && !(ENDS == Ends::ANY && dense)) return false;
     for (int i = tid; i < 3 * 2 * PLANE; i += nthreads) fq()[i] = 0u;
     __syncthreads();
     if (ENDS == Ends::FEW || in_smem) {
@@ -338,9 +333,9 @@ struct SlabSpreader {
     } else {
       // records from global memory: a lane tests an end, then half a warp adds the nodes
       // of each that covers the plane (with sixteen threads testing every end, 256^3 with
-      // 65,536 swimmers in 100^3 took 45 ms a step)
-      const int lane = t0 & 31, node = lane & 15;
-      const int jy = node >> 2, jz = node & 3;
+      // 65,536 swimmers in 100^3 took 45 ms a step; through shared memory, 256 ends at a
+      // time, 30; like this 10)
+      const int lane = t0 & 31, jy = (lane >> 2) & 3, jz = lane & 3;
       for (int base = t0 - lane; base < cnt; base += stride) {
         const int q = base + lane;
         float w = 0.f;

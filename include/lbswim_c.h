@@ -323,8 +323,8 @@ int lbswim_lattice_set_tau(lbswim_lattice* lat, double tau_s, double tau_b);
  * ensemble advances many independent FP32 solves -- each an FP32 lattice with
  * an optional swimmer array and an optional tracer array, all created and
  * initialised with the calls above -- by the same coupled step as
- * lbswim_system_step, in two batched launches per step replayed from a CUDA
- * graph.  Each member ends exactly where lbswim_system_step would have taken
+ * lbswim_system_step, in two batched launches per step (three with members of more
+ * than 128 swimmers) replayed from a CUDA graph.  Each member ends exactly where lbswim_system_step would have taken
  * it (bit for bit, with the same slab shape).  Membership can change between
  * calls to lbswim_ensemble_step; members stay owned by the caller and must
  * outlive their membership.  A member lattice has fewer than 143M sites and its
