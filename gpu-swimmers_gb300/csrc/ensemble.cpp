@@ -208,9 +208,8 @@ static void build_tables(Ensemble* E) {
     Tracers* T = E->tr[i];
     EnsMember& M = E->hmem[m];
     const int nsw = W ? W->n : 0, ntr = T ? T->n : 0;
-    M.lx = lx[i];
+    M.lx = spread_reserve(L, 2 * nsw, lx[i]);
     M.dense = slabs_overfull(L->size, L->fused_tile, 2ll * nsw, M.lx);
-    spread_reserve(L, 2 * nsw, M.lx);
     for (int a = 0; a < 3; ++a) M.size[a] = L->size[a];
     M.n = L->n;
     M.rho0 = (float)L->rho0;

@@ -344,9 +344,9 @@ void exact_init_from_hydro_f64(Lattice* L);
 // particles.cu: force spreading state
 void spread_materialise(Lattice* L);
 SlabSpread spread_prepare_slabs(Lattice* L);
-// Pending-end storage for `nends` ends and buckets for slabs of lx planes
-// (particles.cu).
-void spread_reserve(Lattice* L, int nends, int lx);
+// Pending-end storage for `nends` ends and buckets for slabs of lx planes, or of as many
+// as it returns (particles.cu).
+int spread_reserve(Lattice* L, int nends, int lx);
 // Dense force (base + spread of the pending ends) of a reduced-precision
 // lattice, bit for bit the force the step kernel spreads (lattice.cu).
 void lattice_force_from_slabs(Lattice* L);

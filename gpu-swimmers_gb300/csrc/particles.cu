@@ -2378,19 +2378,35 @@ static void grow_buckets(Lattice* L, int nslabs, unsigned*& count, int*& list, i
   slabs = nslabs;
 }
 
-void spread_reserve(Lattice* L, int nends, int lx) {
+// Buckets for slabs of lx planes, or, where the device has no room for those of short
+// slabs (4 KB each: a dense lattice in slabs of one plane would take a fifth of its own
+// size), of 32; returns which.
+static int grow_slab_buckets(Lattice* L, int lx, unsigned*& count, int*& list, int& slabs) {
+  const int longer = std::min(32, L->size[0]);
+  try {
+    grow_buckets(L, slabs_of(slab_grid(L, lx)), count, list, slabs);
+  } catch (const LbswimError& e) {
+    if (e.code != LBSWIM_ENOMEM || lx >= longer) throw;
+    (void)cudaGetLastError();
+    lx = longer;
+    grow_buckets(L, slabs_of(slab_grid(L, lx)), count, list, slabs);
+  }
+  return lx;
+}
+
+int spread_reserve(Lattice* L, int nends, int lx) {
   ensure_ends(L, nends);
   SpreadScratch& S = L->spread;
   if (!S.max_abs_force) LB_CUDA(cudaMalloc(&S.max_abs_force, 2 * sizeof(unsigned)));
-  grow_buckets(L, slabs_of(slab_grid(L, lx)), S.bucket_count, S.bucket_list, S.bucket_slabs);
   S.bucket_tile = -1;
+  return grow_slab_buckets(L, lx, S.bucket_count, S.bucket_list, S.bucket_slabs);
 }
 
 // Empty buckets for slabs of S.lx planes.
 static void clear_buckets(Lattice* L) {
   SpreadScratch& S = L->spread;
+  S.lx = grow_slab_buckets(L, S.lx, S.bucket_count, S.bucket_list, S.bucket_slabs);
   const int nslabs = slabs_of(slab_grid(L, S.lx));
-  grow_buckets(L, nslabs, S.bucket_count, S.bucket_list, S.bucket_slabs);
   LB_CUDA(cudaMemsetAsync(S.bucket_count, 0, sizeof(unsigned) * nslabs, L->stream));
   S.bucket_tile = L->fused_tile;
 }
@@ -2638,9 +2654,9 @@ void swimmers_prepare_room(Swimmers* const* w, int nw, Lattice* L) {
   if (!P.max_abs_force) LB_CUDA(cudaMalloc(&P.max_abs_force, 2 * sizeof(unsigned)));
   P.clear_max = true;
   if (nends > DIRECT_ENDS) {
-    P.lx = choose_slab_lx(L, nends);
+    P.lx = grow_slab_buckets(L, choose_slab_lx(L, nends), P.bucket_count, P.bucket_list,
+                             P.bucket_slabs);
     P.clear = slabs_of(slab_grid(L, P.lx));
-    grow_buckets(L, P.clear, P.bucket_count, P.bucket_list, P.bucket_slabs);
   }
 }
 
