@@ -2378,19 +2378,17 @@ static void grow_buckets(Lattice* L, int nslabs, unsigned*& count, int*& list, i
   slabs = nslabs;
 }
 
-// Buckets for slabs of lx planes, or, where the device has no room for those of short
-// slabs (4 KB each: a dense lattice in slabs of one plane would take a fifth of its own
-// size), of 32; returns which.
+// Buckets for slabs of lx planes; those of short slabs (4 KB each, twice: a dense lattice in
+// slabs of one plane takes a fifth of its own size) while they take a quarter of what is
+// free on the device, otherwise of 32 planes.  Returns which.
 static int grow_slab_buckets(Lattice* L, int lx, unsigned*& count, int*& list, int& slabs) {
-  const int longer = std::min(32, L->size[0]);
-  try {
-    grow_buckets(L, slabs_of(slab_grid(L, lx)), count, list, slabs);
-  } catch (const LbswimError& e) {
-    if (e.code != LBSWIM_ENOMEM || lx >= longer) throw;
-    (void)cudaGetLastError();
-    lx = longer;
-    grow_buckets(L, slabs_of(slab_grid(L, lx)), count, list, slabs);
+  const int longer = std::min(32, L->size[0]), nslabs = slabs_of(slab_grid(L, lx));
+  if (lx < longer && (slabs < nslabs || !count)) {
+    size_t free = 0, total = 0;
+    LB_CUDA(cudaMemGetInfo(&free, &total));
+    if (sizeof(int) * (size_t)nslabs * SLAB_BUCKET_CAP > free / 4) lx = longer;
   }
+  grow_buckets(L, slabs_of(slab_grid(L, lx)), count, list, slabs);
   return lx;
 }
 
