@@ -1293,10 +1293,10 @@ static void launch_fused_w(Lattice* L, const FusedArgs& a) {
     launch_fused_i<S, TZ, TY, SPREAD, int, TMA, LOADS>(L, a);
 }
 
-// FP32 steps with ends load late up to three waves of slabs, where the chain of a plane
-// bounds them (us a step late and early: 100x75x130 71.2 and 73.3, 128^3 with 300 swimmers
-// 86.5 and 88.2), early beyond, where DRAM does (160^3, 4 waves, 167.1 and 166.4; 256^3
-// 587 and 578 with 65,536 swimmers, 480 and 469 with 8192); without ends early.
+// FP32 steps with ends load late up to two waves of slabs, where the chain of a plane
+// bounds them (step kernel in us, late and early: 100x75x130 49.2 and 50.2, 144^3 115.6 and
+// 115.9, with few ends 102.4 and 103.9), early beyond, where DRAM does (192^3 232.7 and 230.7,
+// with few ends 199.9 and 197.1; 256^3 529 and 521, 475 and 463); without ends early.
 template <class S, int TZ, int TY, bool SPREAD>
 static void launch_fused(Lattice* L, const FusedArgs& a) {
   if constexpr (TZ == 32) {
@@ -1310,7 +1310,7 @@ static void launch_fused(Lattice* L, const FusedArgs& a) {
   } else if constexpr (SPREAD) {
     const long long slabs = (long long)((a.nz + TZ - 1) / TZ) * ((a.ny + TY - 1) / TY) *
                             ((a.nx + a.lx - 1) / a.lx);
-    if (slabs <= 3ll * fused_ctas<S, false>() * sm_count())
+    if (slabs <= 2ll * fused_ctas<S, false>() * sm_count())
       launch_fused_w<S, TZ, TY, SPREAD, false, Loads::LATE>(L, a);
     else
       launch_fused_w<S, TZ, TY, SPREAD, false, Loads::EARLY>(L, a);

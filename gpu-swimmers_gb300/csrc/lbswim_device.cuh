@@ -30,7 +30,8 @@ __host__ __device__ constexpr double w_of(int p) {
   return p == 0 ? 2.0 / 9.0 : p <= 6 ? 1.0 / 9.0 : 1.0 / 72.0;
 }
 
-// Unsigned division by a divisor fixed at launch: t / d for t < 2^31.
+// Unsigned division by a divisor fixed at launch: t / d for t < 2^31 (Granlund and
+// Montgomery, Division by invariant integers using multiplication, PLDI 1994).
 struct FastDiv {
   unsigned mul, shift;
 };
