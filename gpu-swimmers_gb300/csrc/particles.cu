@@ -518,8 +518,8 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan_apply_total(
 // Force tiles of 4 (x) x 8 (y) x 32 (z) sites.  The end records list every end
 // under the tiles its stencil touches, in buckets of FT_CAP and, past those, chains
 // (TileChains).  Two kernels sum them:
-//  * k_force_fixed (default): the (end, node) contributions are integers of 72 to 84
-//    bits below the tile's largest force, added as three words with shared-memory
+//  * k_force_fixed (default): the (end, node) contributions are integers of 72 (256 ends)
+//    to 84 bits below the tile's largest force, added as three words with shared-memory
 //    atomics that return nothing, and converted once.  All 32 lanes work on the nodes of
 //    an end.  Integer sums do not depend on their order.
 //  * k_force_tile (LBSWIM_COMPAT_EXACT_F64, and suspensions too dense for
@@ -837,9 +837,10 @@ __device__ __forceinline__ double words_to_double(unsigned lo, unsigned mid, int
 // the record loads run under the zeroing: AddForces at 256^3 with 65,536 swimmers 313 us,
 // against 840 in FP64 by site; 65x47x90 with 1074 20 against 76.  Up to two tiles
 // to an SM, the chain of a block's phases bounds the launch: 512 threads shorten
-// each, and the list is read with its count (onto a force 24^3 18.6 -> 15.6 us); with
-// more tiles they cost occupancy (80^3 18.8 -> 23.2; 256^3 224 -> 320), and of a few ends
-// without buckets each tile first picks its own (256^3 with 32 swimmers 199 -> 88 us).
+// each, and the list is read with its count (onto a force 24^3 18.5 -> 14.5 us, 64^3 22.6 ->
+// 19.5); with more tiles they cost occupancy (64x64x80, 384 tiles, 23.0 -> 23.4; 80^3 26.7
+// -> 28.6; 256^3 316 -> 380 alone), and of a few ends without buckets each tile first
+// picks its own (256^3 with 32 swimmers 199 -> 88 us).
 template <int THREADS>
 __global__ void __launch_bounds__(THREADS) k_force_fixed(
     Dims D, TileGrid G, const EndRecord<double>* __restrict__ ends, int nends,
